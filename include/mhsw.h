@@ -54,8 +54,12 @@ extern "C" {
 #define MHSW_ORIENT_REF_IS_A 1
 
 /* ---- forms ----------------------------------------------------------------- */
-#define MHSW_FORM_PLAIN 0    /* one wavefront group per pair, input order */
-#define MHSW_FORM_BATCHED 1  /* length-bucketed, sorted, persistent work-stealing launch */
+/* Both forms give the same results.  They order the pairs by length on the device and run
+ * persistent kernels whose lane groups claim pairs from a queue; the batched form also tunes
+ * their configuration to the batch (mhsw_tuning).  Batches of a few thousand pairs take one
+ * launch for both passes in either form. */
+#define MHSW_FORM_PLAIN 0    /* default configuration */
+#define MHSW_FORM_BATCHED 1  /* configuration picked by timed trials */
 
 typedef struct mhsw_driver mhsw_driver;
 
@@ -99,7 +103,8 @@ typedef struct {
  * call whose length signature (the A-length mix over the kernels' row classes, sampled
  * where the host sees the lengths, and the classes of the longest A and B and of the
  * batch size) moved away from the one the handle last tuned for re-tunes on a strided
- * sample of at most 256k pairs of its batch before aligning it. */
+ * sample of at most 256k pairs of its batch before aligning it.  Batches short enough for
+ * the one-launch path (see MHSW_FORM_PLAIN) are not tuned. */
 typedef struct {
   int32_t threads_per_block;  /* persistent kernels' block size */
   int32_t blocks_per_sm;      /* 0 = the occupancy limit */

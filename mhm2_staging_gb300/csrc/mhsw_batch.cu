@@ -1,18 +1,17 @@
-// mhsw_batch.cu -- batched form of the forward pass.
+// mhsw_batch.cu -- the forward pass over a batch (both forms).
 //
 // The reference launches one block per pair with the block size fixed by the batch's
 // longest sequences (src/adept-sw/driver.cpp:343-368), so uneven batches idle most
-// threads.  Here the pair order is sorted on the device by a key
-//   bucket(len A) << 17 | (131071 - len B)
-// (bucket = rows-per-lane class of the wavefront engine, so a lane group always runs
-// the narrowest engine that fits; longest B first inside a bucket), and one
-// persistent launch of G-lane groups claims pairs from a single atomic counter
+// threads.  Here the pairs are put in order of
+//   (bucket(len A), len B descending)
+// on the device (bucket = rows-per-lane class of the wavefront engine, so a lane group
+// always runs the narrowest engine that fits; longest B first inside a bucket), and
+// persistent launches of G-lane groups claim pairs from an atomic counter
 // (work stealing: a group that finishes early takes the next pair).  Pairs whose
 // score could exceed the int16 range (min(lenA, lenB) * match above the int16
 // capacity) are sent straight to the int32 list.
 #include <algorithm>
 #include <chrono>
-#include <cub/cub.cuh>
 
 #include "mhsw_batch.h"
 #include "mhsw_engine.cuh"
@@ -23,8 +22,6 @@ namespace mhsw {
 
 namespace {
 
-constexpr int kKeyShift = 17;
-constexpr int kSortBits = 20;  // 3 bucket bits above the 17 B-length bits
 // Buckets: 0..3 = A up to 64/96/128/160 rows (8-lane groups, K = 4/6/8/10),
 // 4/5 = up to 192/256 rows (16-lane groups, K = 6/8), 6 = longer A (K = 8 strips),
 // 7 = could exceed the int16 keys: straight to the int32 list.  The tuned row threshold
@@ -51,18 +48,144 @@ __device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int la
   return b;
 }
 
-// Sort keys of items i < m, item i = pair i * stride (stride 1: the whole batch; larger:
-// the tuner's sample); hist (the sample) counts the items per bucket.
-__global__ void k_keys(PairSet ps, Scoring sc, int lane_rows, bool wide_try16, int64_t m, int64_t stride,
-                       uint32_t *keys, uint32_t *idx, int *hist) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i * stride;
-    const int M = ps.a_len[p], N = ps.b_len[p];
-    const int b = (M <= 0 || N <= 0) ? 0 : bucket_of(M, N, sc, lane_rows, wide_try16);
-    const int nb = N < 0 ? 0 : (N > 131071 ? 131071 : N);
-    keys[i] = ((uint32_t)b << kKeyShift) | (uint32_t)(131071 - nb);
-    idx[i] = (uint32_t)p;
-    if (hist) atomicAdd(&hist[b], 1);
+// ---- pair order: a counting sort over (bucket, class of len B, longest first) ---------
+// Length classes are single columns below 1024 and 1/64 of an octave (1.6%) above, so the
+// lane groups of a warp see equal B lengths, which is all the order is for (classes of 4
+// columns cost the forward pass of 800,000 uneven pairs 0.7%).  Order within a bin is
+// whatever the atomics give; no result depends on it.
+constexpr int kLenBins = 1024 + 7 * 64;  // lengths up to 131071
+constexpr int kOrderBins = kBuckets * kLenBins;
+// Batches up to this size are ordered by one block in one launch (serving micro-batches of
+// 4,000 pairs: 9 us against 26 us for the key, radix-sort and split kernels it replaced),
+// larger ones by a histogram and a placement launch.
+constexpr int64_t kOrderOneBlock = 4096;
+
+__device__ __forceinline__ int len_class(int n) {  // 0 = longest
+  n = n < 0 ? 0 : (n > 131071 ? 131071 : n);
+  const int e = 31 - __clz(n | 1);
+  const int c = n < 1024 ? n : 1024 + (e - 10) * 64 + ((n >> (e - 6)) & 63);
+  return kLenBins - 1 - c;
+}
+
+struct OrderArgs {
+  PairSet ps;
+  Scoring sc;
+  int lane_rows;
+  bool wide_try16;
+  int64_t m, stride;  // item i < m is pair i * stride (stride 1: the whole batch; larger: the tuner's sample)
+  int *queue;         // [0], [1]: claim counters of the short and long ranges; [2]: first item of the long range
+  int *first;         // first item of each bucket, then m
+  int *hist, *cursor; // kOrderBins each (zeroed before the two-launch form)
+  uint32_t *order;
+};
+
+__device__ __forceinline__ int order_bin(const OrderArgs &g, int64_t p) {
+  const int M = g.ps.a_len[p], N = g.ps.b_len[p];
+  const int b = (M <= 0 || N <= 0) ? (g.lane_rows > 0 ? 0 : kBucketFirstLong)
+                                   : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16);
+  return b * kLenBins + len_class(N);
+}
+
+// Exclusive prefix sum of the kOrderBins counts in h, in place, by the whole block.
+__device__ void scan_bins(int *h) {
+  __shared__ int warp_sum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int per = (kOrderBins + blockDim.x - 1) / blockDim.x;
+  const int lo = threadIdx.x * per, hi = lo + per < kOrderBins ? lo + per : kOrderBins;
+  int sum = 0;
+  for (int b = lo; b < hi; b++) sum += h[b];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int v = lane < nw ? warp_sum[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    warp_sum[lane] = v;
+  }
+  __syncthreads();
+  int at = incl - sum + (warp > 0 ? warp_sum[warp - 1] : 0);
+  for (int b = lo; b < hi; b++) {
+    const int c = h[b];
+    h[b] = at;
+    at += c;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void write_firsts(const OrderArgs &g, const int *base) {
+  if (threadIdx.x < kBuckets) g.first[threadIdx.x] = base[threadIdx.x * kLenBins];
+  if (threadIdx.x == 0) {
+    g.first[kBuckets] = (int)g.m;
+    g.queue[2] = base[kBucketFirstLong * kLenBins];
+  }
+}
+
+__global__ void __launch_bounds__(1024) k_order_one(OrderArgs g) {
+  __shared__ int h[kOrderBins];
+  for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) h[b] = 0;
+  if (threadIdx.x < 2) g.queue[threadIdx.x] = 0;
+  __syncthreads();
+  int bin[kOrderOneBlock / 1024];
+#pragma unroll
+  for (int k = 0; k < kOrderOneBlock / 1024; k++) {
+    const int64_t i = threadIdx.x + k * 1024;
+    bin[k] = i < g.m ? order_bin(g, i * g.stride) : -1;
+    if (bin[k] >= 0) atomicAdd(&h[bin[k]], 1);
+  }
+  __syncthreads();
+  scan_bins(h);
+  write_firsts(g, h);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kOrderOneBlock / 1024; k++)
+    if (bin[k] >= 0) g.order[atomicAdd(&h[bin[k]], 1)] = (uint32_t)((threadIdx.x + k * 1024) * g.stride);
+}
+
+__global__ void __launch_bounds__(1024) k_order_hist(OrderArgs g) {
+  __shared__ int h[kOrderBins];
+  for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) h[b] = 0;
+  __syncthreads();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.m; i += (int64_t)gridDim.x * blockDim.x)
+    atomicAdd(&h[order_bin(g, i * g.stride)], 1);
+  __syncthreads();
+  for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x)
+    if (h[b]) atomicAdd(&g.hist[b], h[b]);
+}
+
+// Same grid as k_order_hist: each block reserves its run of every bin with one atomic.
+__global__ void __launch_bounds__(1024) k_order_place(OrderArgs g) {
+  extern __shared__ int base[];
+  int *h = base + kOrderBins;
+  for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) {
+    base[b] = g.hist[b];
+    h[b] = 0;
+  }
+  __syncthreads();
+  scan_bins(base);
+  if (blockIdx.x == 0) write_firsts(g, base);
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.m; i += step)
+    atomicAdd(&h[order_bin(g, i * g.stride)], 1);
+  __syncthreads();
+  for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x)
+    if (h[b]) {
+      base[b] += atomicAdd(&g.cursor[b], h[b]);
+      h[b] = 0;
+    }
+  __syncthreads();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.m; i += step) {
+    const int64_t p = i * g.stride;
+    const int b = order_bin(g, p);
+    g.order[base[b] + atomicAdd(&h[b], 1)] = (uint32_t)p;
   }
 }
 
@@ -72,27 +195,14 @@ __device__ __forceinline__ unsigned group_mask_b(int G) {
   return ((1u << G) - 1u) << ((lane32 / G) * G);
 }
 
-// First sorted item of the long-read buckets (the sorted keys are ascending).
-__global__ void k_split(const uint32_t *__restrict__ keys, int64_t n, int *split) {
-  const uint32_t first = (uint32_t)kBucketFirstLong << kKeyShift;
-  int64_t lo = 0, hi = n;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) / 2;
-    if (keys[mid] < first) lo = mid + 1;
-    else hi = mid;
-  }
-  *split = (int)lo;
-}
-
 // Persistent forward kernel over one range of the sorted pair order: 8-lane groups for
 // the short-read buckets (items [0, split)), 16-lane groups for the rest ([split, n)).
 // A group claims its next pair from the range's atomic counter.
-template <int G, bool S2 = false>
+template <int G, bool S2>
 __global__ void __launch_bounds__(256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
-                                                     const uint32_t *__restrict__ keys,
                                                      const uint32_t *__restrict__ order, int64_t n, int *queue,
-                                                     const int *split, int ceiling, WorkLists wl, int pad, int bcap,
-                                                     V16::Pay *scratch, int scratch_stride) {
+                                                     int lane_rows, bool wide_try16, int ceiling, WorkLists wl, int pad,
+                                                     int bcap, V16::Pay *scratch, int scratch_stride) {
   constexpr bool kShort = (G == kGKShort);
   extern __shared__ __align__(16) unsigned char smem[];
   const int gpb = blockDim.x / G;
@@ -110,8 +220,8 @@ __global__ void __launch_bounds__(256) k_fwd_persist(PairSet ps, ResultSet rs, S
   gs.bcap = bcap;
   const int64_t gid = (int64_t)blockIdx.x * gpb + grp;
   V16::Pay *bnd = scratch ? scratch + gid * (int64_t)scratch_stride : nullptr;
-  const int64_t lo = kShort ? 0 : *split;
-  const int64_t hi = kShort ? *split : n;
+  const int64_t lo = kShort ? 0 : queue[2];
+  const int64_t hi = kShort ? queue[2] : n;
   int *counter = queue + (kShort ? 0 : 1);
 
   for (;;) {
@@ -120,10 +230,9 @@ __global__ void __launch_bounds__(256) k_fwd_persist(PairSet ps, ResultSet rs, S
     claim = __shfl_sync(gmask, claim, 0, G);
     const int64_t item = lo + claim;
     if (item >= hi) break;
-    const uint32_t key = keys[item];
     const int64_t p = order[item];
-    const int bucket = (int)(key >> kKeyShift);
     const int M = ps.a_len[p], N = ps.b_len[p];
+    const int bucket = (M <= 0 || N <= 0) ? 0 : bucket_of(M, N, sc, lane_rows, wide_try16);
     if (bucket == kBucketWide) {
       if (lane == 0) {
         rs.flag[p] = kFlagOverflow16;
@@ -194,21 +303,15 @@ cudaError_t grow(T **p, size_t n) {
 }  // namespace
 
 void BatchState::release() {
-  for (uint32_t **q : {&keys_in, &keys_out, &idx_in, &idx_out, &s_keys_in, &s_keys_out, &s_idx_in, &s_idx_out}) {
+  for (uint32_t **q : {&order, &s_order}) {
     if (*q) cudaFree(*q);
     *q = nullptr;
   }
-  for (void **q : {&temp, &s_temp, &scratch}) {
-    if (*q) cudaFree(*q);
-    *q = nullptr;
-  }
-  if (queue) cudaFree(queue);
-  if (s_hist) cudaFree(s_hist);
-  queue = nullptr;
-  s_hist = nullptr;
+  if (scratch) cudaFree(scratch);
+  if (ctl) cudaFree(ctl);
+  scratch = nullptr;
+  ctl = nullptr;
   cap = 0;
-  temp_bytes = 0;
-  s_temp_bytes = 0;
   scratch_bytes = 0;
 }
 
@@ -248,8 +351,13 @@ bool BatchSignature::close_to(const BatchSignature &o) const {
   return true;
 }
 
+bool may_need_int32(const Scoring &sc, int ceiling, int max_a, int max_b) {
+  const long long bound = (long long)std::min(max_a, max_b) * sc.match;
+  return bound > std::min(ceiling, keyed_cap(10));
+}
+
 int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultSet &rs, const WorkLists &wl,
-                    const Scoring &sc, int ceiling, int max_a, int max_b, const BatchSignature &sig,
+                    const Scoring &sc, int ceiling, int max_a, int max_b, const BatchSignature &sig, bool tune,
                     cudaStream_t st, int64_t *launches, const Forks *fk) {
   auto fail = [&](cudaError_t e, const char *what) {
     bs.err = std::string(what) + ": " + cudaGetErrorString(e);
@@ -264,22 +372,17 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   }
   cudaError_t e;
   if ((size_t)n > bs.cap) {
-    size_t c = (size_t)n + (size_t)n / 8 + 1024;
-    if ((e = grow(&bs.keys_in, c)) || (e = grow(&bs.keys_out, c)) || (e = grow(&bs.idx_in, c)) ||
-        (e = grow(&bs.idx_out, c)))
-      return fail(e, "cudaMalloc batch keys");
-    size_t tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, bs.keys_in, bs.keys_out, bs.idx_in, bs.idx_out, (int)c, 0, kSortBits,
-                                    st);
-    if (bs.temp) cudaFree(bs.temp);
-    bs.temp = nullptr;
-    if ((e = cudaMalloc(&bs.temp, tb))) return fail(e, "cudaMalloc sort temp");
-    bs.temp_bytes = tb;
+    const size_t c = (size_t)n + (size_t)n / 8 + 1024;
+    bs.cap = 0;
+    if ((e = grow(&bs.order, c))) return fail(e, "cudaMalloc pair order");
     bs.cap = c;
   }
-  // queue[0], queue[1]: claim counters of the short and long ranges; queue[2]: split item;
-  // queue[4..6]: the same for the tuner's sample
-  if (!bs.queue && (e = cudaMalloc(&bs.queue, sizeof(int) * 8))) return fail(e, "cudaMalloc queue");
+  // [0..7] claim counters and first long item, [8..23] first item of each bucket, then the
+  // bin counts and cursors
+  constexpr size_t kCtlHead = 24;
+  if (!bs.ctl && (e = cudaMalloc(&bs.ctl, sizeof(int) * (kCtlHead + 2 * kOrderBins))))
+    return fail(e, "cudaMalloc order counters");
+  int *queue = bs.ctl;
 
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -296,25 +399,29 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   // strip scratch stride: B, the lane skew and score2 mode's zero-score padding (< 16)
   const int bcap = ((pad + std::max(max_b, 1) + 16 + 2 * kGKLong) + 15) / 16 * 16;
 
-  // keys + device sort of m items (pair i * stride), split point into q[2]
-  auto sort_items = [&](const BatchShape &sh, int64_t m, int64_t stride, uint32_t *kin, uint32_t *kout, uint32_t *iin,
-                        uint32_t *iout, void *temp, size_t temp_bytes, int *q, int *hist) -> int {
-    const int grid = (int)std::min<int64_t>((m + 255) / 256, (int64_t)sms * 32);
-    if (hist && (e = cudaMemsetAsync(hist, 0, sizeof(int) * kBuckets, st))) return fail(e, "memset");
-    k_keys<<<grid, 256, 0, st>>>(ps, sc, sh.lane_rows, sh.wide_try16, m, stride, kin, iin, hist);
-    if ((e = cudaGetLastError())) return fail(e, "keys launch");
-    size_t tb = temp_bytes;
-    e = cub::DeviceRadixSort::SortPairs(temp, tb, kin, kout, iin, iout, (int)m, 0, kSortBits, st);
-    if (e) return fail(e, "radix sort");
-    k_split<<<1, 1, 0, st>>>(kout, m, q + 2);
-    if ((e = cudaGetLastError())) return fail(e, "split launch");
-    if (launches) *launches += 2 + 4;  // keys, split, and the radix sort's passes (approximate)
+  // order of m items (pair i * stride); clears the claim counters
+  auto order_items = [&](const BatchShape &sh, int64_t m, int64_t stride, uint32_t *order) -> int {
+    OrderArgs g{ps, sc, sh.lane_rows, sh.wide_try16, m, stride, queue, bs.ctl + 8, bs.ctl + kCtlHead,
+                bs.ctl + kCtlHead + kOrderBins, order};
+    if (m <= kOrderOneBlock) {
+      k_order_one<<<1, 1024, 0, st>>>(g);
+      if (launches) *launches += 1;
+    } else {
+      if ((e = cudaMemsetAsync(bs.ctl, 0, sizeof(int) * (kCtlHead + 2 * kOrderBins), st))) return fail(e, "memset");
+      // a block an SM at most: each reads and writes all bins, 47 KB
+      const int grid = (int)std::min<int64_t>((m + 4095) / 4096, sms);
+      const size_t smem = 2 * sizeof(int) * kOrderBins;
+      if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_order_place), smem))) return fail(e, "smem attribute");
+      k_order_hist<<<grid, 1024, 0, st>>>(g);
+      k_order_place<<<grid, 1024, smem, st>>>(g);
+      if (launches) *launches += 2;
+    }
+    if ((e = cudaGetLastError())) return fail(e, "order launch");
     return 0;
   };
 
-  // the two persistent launches over m sorted items (keys, order), claim counters in q
-  auto run = [&](const BatchShape &sh, const uint32_t *keys, const uint32_t *order, int64_t m, int *q,
-                 float *ms) -> int {
+  // the two persistent launches over m ordered items
+  auto run = [&](const BatchShape &sh, const uint32_t *order, int64_t m, float *ms) -> int {
     const int threads = sh.groups_per_block * 8;  // block size: 8 groups of 8 lanes or 4 of 16, etc.
     const int gpb_s = threads / kGKShort, gpb_l = threads / kGKLong;
     const size_t smem_s = (size_t)gpb_s * prof_short, smem_l = (size_t)gpb_l * prof_long;
@@ -326,8 +433,15 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_l, klong, threads, smem_l);
     occ_s = std::max(occ_s, 1);
     occ_l = std::max(occ_l, 1);
-    const int grid_s = sms * (sh.blocks_per_sm > 0 ? std::min(sh.blocks_per_sm, occ_s) : occ_s);
-    const int grid_l = sms * (sh.blocks_per_sm > 0 ? std::min(sh.blocks_per_sm, occ_l) : occ_l);
+    // no more blocks than the items fill
+    auto grid_of = [&](int occ, int gpb) {
+      const int64_t full = (int64_t)sms * (sh.blocks_per_sm > 0 ? std::min(sh.blocks_per_sm, occ) : occ);
+      return (int)std::min<int64_t>(full, (m + gpb - 1) / gpb);
+    };
+    const int grid_s = grid_of(occ_s, gpb_s), grid_l = grid_of(occ_l, gpb_l);
+    // every pair is in the short buckets when the longest A is and no score bound sends a
+    // pair to the int32 list
+    const bool any_long = max_a > sh.lane_rows || (long long)std::min(max_a, max_b) * sc.match > keyed_cap(10);
     V16::Pay *scr = nullptr;
     const int stride = bcap;
     if (max_a > 2 * 8 * kGKLong) {
@@ -343,23 +457,26 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
       scr = reinterpret_cast<V16::Pay *>(bs.scratch);
     }
     cudaEvent_t t0 = nullptr, t1 = nullptr;
-    if (ms) {
+    if (ms) {  // a trial: its sample is run again and again in one order
       cudaEventCreate(&t0);
       cudaEventCreate(&t1);
       cudaEventRecord(t0, st);
+      cudaMemsetAsync(queue, 0, 2 * sizeof(int), st);
+      cudaMemsetAsync(wl.ovf_count, 0, sizeof(int), st);
     }
-    cudaMemsetAsync(q, 0, 2 * sizeof(int), st);
-    cudaMemsetAsync(wl.ovf_count, 0, sizeof(int), st);
-    const bool fan = fk && fk->fork;
+    const bool any_short = sh.lane_rows > 0;
+    const bool fan = any_long && any_short && fk && fk->fork;
     if (fan && (e2 = fork_to(*fk, st, 1))) return fail(e2, "fork");
-    klong<<<grid_l, threads, smem_l, fan ? fk->side[0] : st>>>(ps, rs, sc, keys, order, m, q, q + 2, ceiling, wl, pad,
-                                                               bcap, scr, stride);
-    kshort<<<grid_s, threads, smem_s, st>>>(ps, rs, sc, keys, order, m, q, q + 2, ceiling, wl, pad, bcap, nullptr,
-                                             stride);
+    if (any_long)
+      klong<<<grid_l, threads, smem_l, fan ? fk->side[0] : st>>>(ps, rs, sc, order, m, queue, sh.lane_rows, sh.wide_try16,
+                                                                 ceiling, wl, pad, bcap, scr, stride);
+    if (any_short)
+      kshort<<<grid_s, threads, smem_s, st>>>(ps, rs, sc, order, m, queue, sh.lane_rows, sh.wide_try16, ceiling, wl, pad,
+                                               bcap, nullptr, stride);
     e2 = cudaGetLastError();
     if (e2) return fail(e2, "persistent forward launch");
     if (fan && (e2 = join_from(*fk, st, 1))) return fail(e2, "join");
-    if (launches) *launches += 2;
+    if (launches) *launches += (any_long ? 1 : 0) + (any_short ? 1 : 0);
     if (ms) {
       cudaEventRecord(t1, st);
       cudaEventSynchronize(t1);
@@ -373,7 +490,7 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   // a configuration tuned earlier for a signature close to this one is taken back without
   // trials (batches that alternate between workloads, such as full and partial serving
   // micro-batches, tune once each)
-  if (bs.autotune && (!bs.tuned || !sig.close_to(bs.tuned_for))) {
+  if (tune && bs.autotune && (!bs.tuned || !sig.close_to(bs.tuned_for))) {
     for (int k = 0; k < bs.n_cached; k++)
       if (sig.close_to(bs.cached[k].sig)) {
         bs.shape = bs.cached[k].shape;
@@ -382,9 +499,9 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
         break;
       }
   }
-  if (bs.autotune && (!bs.tuned || !sig.close_to(bs.tuned_for))) {
+  if (tune && bs.autotune && (!bs.tuned || !sig.close_to(bs.tuned_for))) {
     // Trials on a strided sample of the batch (every stride-th pair, so its length mix is
-    // the batch's), sorted as the batch is.  Coordinate descent: the launch shape at the
+    // the batch's), ordered as the batch is.  Coordinate descent: the launch shape at the
     // default row threshold; then the 16-lane threshold for A of 129..160 rows; then the
     // int16/int32 split of pairs whose bound exceeds the int16 keys -- each only when the
     // sample has pairs it affects.  Trial results land in the result arrays of the sampled
@@ -392,41 +509,29 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     const auto t_start = std::chrono::steady_clock::now();
     const int64_t stride = (n + kTuneSample - 1) / kTuneSample;
     const int64_t m = (n + stride - 1) / stride;
-    if (!bs.s_keys_in) {
-      const size_t c = (size_t)kTuneSample + 1024;
-      if ((e = grow(&bs.s_keys_in, c)) || (e = grow(&bs.s_keys_out, c)) || (e = grow(&bs.s_idx_in, c)) ||
-          (e = grow(&bs.s_idx_out, c)) || (e = grow(&bs.s_hist, (size_t)kBuckets)))
-        return fail(e, "cudaMalloc tuner sample");
-      size_t tb = 0;
-      cub::DeviceRadixSort::SortPairs(nullptr, tb, bs.s_keys_in, bs.s_keys_out, bs.s_idx_in, bs.s_idx_out, (int)c, 0,
-                                      kSortBits, st);
-      if ((e = cudaMalloc(&bs.s_temp, tb))) return fail(e, "cudaMalloc tuner sort temp");
-      bs.s_temp_bytes = tb;
-    }
-    int *sq = bs.queue + 4;
-    int hist[kBuckets] = {0};
-    auto sample_sort = [&](const BatchShape &sh) -> int {
-      if (sort_items(sh, m, stride, bs.s_keys_in, bs.s_keys_out, bs.s_idx_in, bs.s_idx_out, bs.s_temp,
-                     bs.s_temp_bytes, sq, bs.s_hist))
-        return 1;
-      if ((e = cudaMemcpyAsync(hist, bs.s_hist, sizeof(hist), cudaMemcpyDeviceToHost, st)) ||
+    if (!bs.s_order && (e = grow(&bs.s_order, (size_t)kTuneSample + 1024))) return fail(e, "cudaMalloc tuner sample");
+    int first[kBuckets + 1] = {0};
+    auto in_bucket = [&](int b) { return first[b + 1] - first[b]; };
+    auto sample_order = [&](const BatchShape &sh) -> int {
+      if (order_items(sh, m, stride, bs.s_order)) return 1;
+      if ((e = cudaMemcpyAsync(first, bs.ctl + 8, sizeof(first), cudaMemcpyDeviceToHost, st)) ||
           (e = cudaStreamSynchronize(st)))
-        return fail(e, "tuner histogram");
+        return fail(e, "tuner bucket counts");
       return 0;
     };
     TuneRecord tr;
     tr.tunings = bs.tune.tunings + 1;
     tr.sample_pairs = m;
     auto trial = [&](const BatchShape &sh, float *ms) -> int {
-      if (run(sh, bs.s_keys_out, bs.s_idx_out, m, sq, ms)) return 1;
+      if (run(sh, bs.s_order, m, ms)) return 1;
       if (tr.trials < 16) tr.trial_ms[tr.trials] = *ms;
       tr.trials++;
       return 0;
     };
     BatchShape best;  // defaults: 128-thread blocks, occupancy limit, rows <= 160 in 8-lane groups
-    if (sample_sort(best)) return 1;
+    if (sample_order(best)) return 1;
     float warm = 0.f, best_ms = 1e30f;
-    if (run(best, bs.s_keys_out, bs.s_idx_out, m, sq, &warm)) return 1;  // untimed warm-up
+    if (run(best, bs.s_order, m, &warm)) return 1;  // untimed warm-up
     const BatchShape shapes[] = {{8, 0}, {16, 0}, {32, 0}, {16, 2}, {32, 1}};
     for (const BatchShape &c0 : shapes) {
       BatchShape c = best;
@@ -439,22 +544,22 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
         best = c;
       }
     }
-    if (hist[3] > 0) {  // A of 129..160 rows present: try them in 16-lane groups
+    if (in_bucket(3) > 0) {  // A of 129..160 rows present: try them in 16-lane groups
       BatchShape c = best;
       c.lane_rows = 128;
       float ms = 0.f;
-      if (sample_sort(c) || trial(c, &ms)) return 1;
+      if (sample_order(c) || trial(c, &ms)) return 1;
       if (ms < best_ms) {
         best_ms = ms;
         best = c;
       }
-      if (sample_sort(best)) return 1;  // hist of the kept threshold
+      if (sample_order(best)) return 1;  // bucket counts of the kept threshold
     }
-    if (hist[kBucketWide] > 0 && sc.match <= 63) {  // bound above the int16 keys: try int16 first
+    if (in_bucket(kBucketWide) > 0 && sc.match <= 63) {  // bound above the int16 keys: try int16 first
       BatchShape c = best;
       c.wide_try16 = true;
       float ms = 0.f;
-      if (sample_sort(c) || trial(c, &ms)) return 1;
+      if (sample_order(c) || trial(c, &ms)) return 1;
       if (ms < best_ms) best = c;
     }
     bs.shape = best;
@@ -466,13 +571,16 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     tr.last_call_tuned = true;
     tr.wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
     bs.tune = tr;
+    if ((e = cudaMemsetAsync(wl.ovf_count, 0, sizeof(int), st))) return fail(e, "memset");
   }
 
-  // the batch: keys with the kept configuration, sort, the persistent launches
-  if (sort_items(bs.shape, n, 1, bs.keys_in, bs.keys_out, bs.idx_in, bs.idx_out, bs.temp, bs.temp_bytes, bs.queue,
-                 nullptr))
-    return 1;
-  return run(bs.shape, bs.keys_out, bs.idx_out, n, bs.queue, nullptr);
+  // the batch: ordered with the kept configuration, then the persistent launches.  A plain
+  // batch that does not give every 16-lane group a pair takes those for short reads too:
+  // their shorter chain is what it waits for.
+  BatchShape shape = tune ? bs.shape : BatchShape{};
+  if (!tune && n <= (int64_t)sms * 64) shape.lane_rows = 0;  // any_long holds: max_a > 0
+  if (order_items(shape, n, 1, bs.order)) return 1;
+  return run(shape, bs.order, n, nullptr);
 }
 
 }  // namespace mhsw

@@ -55,17 +55,10 @@ struct TuneRecord {
 
 struct BatchState {
   std::string err;
-  uint32_t *keys_in = nullptr, *keys_out = nullptr;
-  uint32_t *idx_in = nullptr, *idx_out = nullptr;
-  void *temp = nullptr;
-  size_t temp_bytes = 0;
+  uint32_t *order = nullptr;    // the batch's pairs by (bucket, B length descending)
   size_t cap = 0;
-  // the tuner's sample of the batch (sorted like the batch), its sort space
-  uint32_t *s_keys_in = nullptr, *s_keys_out = nullptr, *s_idx_in = nullptr, *s_idx_out = nullptr;
-  void *s_temp = nullptr;
-  size_t s_temp_bytes = 0;
-  int *s_hist = nullptr;  // bucket counts of the sample (device), read by the tuner
-  int *queue = nullptr;
+  uint32_t *s_order = nullptr;  // the tuner's sample of the batch, ordered like it
+  int *ctl = nullptr;           // claim counters, bucket starts and bin counts of one ordered batch
   void *scratch = nullptr;  // strip scratch for A longer than one strip
   size_t scratch_bytes = 0;
   BatchShape shape;
@@ -85,10 +78,11 @@ struct BatchState {
   void release();
 };
 
-// Forward pass of the batched form: computes bucket keys (rows-per-lane class of A,
-// then descending B length), sorts the pair order on the device, and runs the
-// persistent kernel whose lane groups claim pairs from one atomic queue.  Pairs whose
-// score could exceed the int16 ceiling go straight to the int32 list wl.ovf.
+// Forward pass over a batch: puts the pairs in order on the device (rows-per-lane class of
+// A, then descending B length) and runs the persistent kernels whose lane groups claim
+// pairs from an atomic queue.  Pairs whose score could exceed the int16 ceiling go
+// straight to the int32 list wl.ovf.  The plain form (tune = false) runs the default
+// configuration; the batched form (tune = true) the tuned one:
 // A call whose batch signature differs from the one the handle last tuned for takes back
 // the configuration of a close earlier signature (the last eight are kept), or else runs
 // the tuner first: timed trials of the persistent kernels on a strided sample of the batch
@@ -99,7 +93,7 @@ struct BatchState {
 // With side streams (fk), the two persistent launches (8-lane and 16-lane groups) run
 // concurrently, so the tail of one fills with the other.
 int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultSet &rs, const WorkLists &wl,
-                    const Scoring &sc, int ceiling, int max_a, int max_b, const BatchSignature &sig,
+                    const Scoring &sc, int ceiling, int max_a, int max_b, const BatchSignature &sig, bool tune,
                     cudaStream_t st, int64_t *launches, const Forks *fk = nullptr);
 
 }  // namespace mhsw

@@ -235,7 +235,13 @@ struct mhsw_driver {
     double cells = 0;
     uint64_t seq = 0;
     mhsw::PairSet ps;
+    bool brief = false;           // one-launch batch (mhsw_short.cu): events 0 and 4 only
+    const int32_t *from = nullptr;  // a short host batch's results in h_small, copied to copy_to when it completes
+    int32_t *copy_to = nullptr;
   } pend[kSlots];
+  // Short host batches: inputs packed and results written in one pinned buffer per slot,
+  // which the kernel reads and writes in place.
+  HBuf<unsigned char> h_small[kSlots];
   struct InSet {
     DBuf<char> a_seq, b_seq;
     DBuf<int64_t> a_off, b_off;
@@ -287,6 +293,9 @@ struct mhsw_driver {
   int64_t a_bytes = 0, b_bytes = 0;  // arena extents of the staged batch
   bool fwd_issued = false;
   bool rev_issued = false;
+  bool in_place = false;     // the staged batch was not copied to the device
+  bool begins_done = false;  // its begins are in the result arrays already
+  bool brief_batch = false;  // the staged batch took the one-launch path (begins included)
   double fwd_cells = 0;
   int64_t launches = 0;
   // Pair order of the last forward pass when it ran the batched form (its sorted
@@ -382,6 +391,7 @@ struct mhsw_driver {
         if (e) cudaEventDestroy(e);
     if (ev_epoch) cudaEventDestroy(ev_epoch);
     for (auto &h : h_counts_p) h.release();
+    for (auto &h : h_small) h.release();
     h_a.release();
     h_b.release();
     h_aoff.release();
@@ -408,6 +418,14 @@ struct mhsw_driver {
 namespace {
 
 int finish_pending(mhsw_driver *d);
+
+// Forgets the captured graph of a device batch: calls that may resize the handle's buffers
+// outside the batch entry point (whose own calls replace the graph) leave it dangling.
+void drop_graph(mhsw_driver *d) {
+  if (d->gexec) cudaGraphExecDestroy(d->gexec);
+  d->gexec = nullptr;
+  d->gkey_seen = false;
+}
 
 // Device buffers for n pairs and the byte totals; result arrays; lists.
 int ensure_device(mhsw_driver *d, int64_t n, int64_t a_bytes, int64_t b_bytes) {
@@ -643,15 +661,16 @@ int ceiling_for(mhsw_driver *d) {
   return mhsw::keyed_scoring(d->sc) ? std::min(d->ceiling16, mhsw::kCeiling16) : d->ceiling16;
 }
 
-int run_forward(mhsw_driver *d, const mhsw::PairSet &ps, int max_a, int max_b, bool persistent_grid) {
+// The generic engine, one group per pair in input order: scorings the keyed engine cannot
+// hold (a mismatch or ambiguity penalty above the gap-open penalty).
+int run_forward(mhsw_driver *d, const mhsw::PairSet &ps, int max_a, int max_b) {
   mhsw::FwdConfig c16, c32;
-  cudaError_t e = mhsw::plan_forward(d->device, max_a, max_b, false, &c16, mhsw::keyed_scoring(d->sc),
-                                     ps.rowmax16 != nullptr);
+  cudaError_t e = mhsw::plan_forward(d->device, max_a, max_b, false, &c16);
   if (e != cudaSuccess) return d->fail(MHSW_ERR_LIMIT, "B length %d exceeds the kernel limit %d", max_b, mhsw::kMaxB);
   e = mhsw::plan_forward(d->device, max_a, max_b, true, &c32);
   if (e != cudaSuccess) return d->fail(MHSW_ERR_LIMIT, "B length %d exceeds the kernel limit %d", max_b, mhsw::kMaxB);
   const bool strips16 = max_a > 2 * c16.K * c16.G;
-  if (!persistent_grid && !strips16) {
+  if (!strips16) {
     int64_t g = (ps.n + c16.groups_per_block - 1) / c16.groups_per_block;
     c16.grid = (int)std::max<int64_t>(1, std::min<int64_t>(g, 1 << 30));
   }
@@ -684,29 +703,29 @@ int forward_any(mhsw_driver *d, const mhsw::PairSet &ps, int max_a, int max_b, i
 }
 
 int forward_passes(mhsw_driver *d, const mhsw::PairSet &ps, int max_a, int max_b, int form) {
-  // The batched form runs the keyed int16 engine; scorings it cannot hold (a mismatch or
-  // ambiguity penalty above the gap-open penalty) use the plain form.
   d->fwd_order = nullptr;
-  if (form != MHSW_FORM_BATCHED || !mhsw::keyed_scoring(d->sc)) return run_forward(d, ps, max_a, max_b, false);
+  if (!mhsw::keyed_scoring(d->sc)) return run_forward(d, ps, max_a, max_b);
   mhsw::WorkLists wl = work_lists(d, ps.n);
   MHSW_CK(mhsw::reset_lists(wl, d->st), "reset lists");
   d->launches += 1;
   if (mhsw::batched_forward(d->batch, d->device, ps, result_set(d), wl, d->sc, ceiling_for(d), max_a, max_b, d->sig,
-                            d->st, &d->launches, &d->forks))
-    return d->fail(MHSW_ERR_CUDA, "batched forward: %s", d->batch.err.c_str());
-  d->fwd_order = d->batch.idx_out;
+                            form == MHSW_FORM_BATCHED, d->st, &d->launches, &d->forks))
+    return d->fail(MHSW_ERR_CUDA, "forward: %s", d->batch.err.c_str());
+  d->fwd_order = d->batch.order;
   // int32 pass over the pairs the int16 engine could not hold
   mhsw::FwdConfig c16, c32;
-  if (mhsw::plan_forward(d->device, max_a, max_b, false, &c16, false, ps.rowmax16 != nullptr) != cudaSuccess ||
+  if (mhsw::plan_forward(d->device, max_a, max_b, false, &c16) != cudaSuccess ||
       mhsw::plan_forward(d->device, max_a, max_b, true, &c32) != cudaSuccess)
     return d->fail(MHSW_ERR_LIMIT, "B length %d exceeds the kernel limit %d", max_b, mhsw::kMaxB);
   size_t sb = 0;
   int rc = ensure_scratch(d, max_a, max_b, &c16, &c32, &sb);
   if (rc) return rc;
-  MHSW_CK(mhsw::launch_forward(c32, true, ps, result_set(d), d->sc, wl.ovf, wl.ovf_count, 0x7fffffff, d->scratch.p,
-                               wl, d->st),
-          "forward int32 launch");
-  d->launches += 1;
+  if (ps.rowmax16 || mhsw::may_need_int32(d->sc, ceiling_for(d), max_a, max_b)) {
+    MHSW_CK(mhsw::launch_forward(c32, true, ps, result_set(d), d->sc, wl.ovf, wl.ovf_count, 0x7fffffff, d->scratch.p,
+                                 wl, d->st),
+            "forward int32 launch");
+    d->launches += 1;
+  }
   return MHSW_OK;
 }
 
@@ -754,7 +773,62 @@ int check_scoring(mhsw_driver *d, const mhsw::Scoring &s) {
   return MHSW_OK;
 }
 
+// Largest batch whose inputs the one-launch path reads in place from pinned host memory: one
+// buffer, no copies to the device.  Above it the copies' bandwidth is worth their launches.
+constexpr int64_t kInPlaceBytes = 512 << 10;
+
+// Whether one launch takes both passes of a batch (a fixed batch configuration asks for the
+// general path's kernels).
+bool short_passes(mhsw_driver *d, int64_t n, int max_a, int max_b, int form) {
+  return n > 0 && !(form == MHSW_FORM_BATCHED && !d->batch.autotune) &&
+         mhsw::short_batch(d->sc, ceiling_for(d), n, max_a, max_b);
+}
+
+// ... and is all there is to do (CIGAR mode goes on from the code arenas and result arrays).
+bool use_short(mhsw_driver *d, int64_t n, int max_a, int max_b, int form) {
+  return !d->cigar && short_passes(d, n, max_a, max_b, form);
+}
+
+// The score2 arrays alone, as the result set of a one-launch batch.
+int short_results(mhsw_driver *d, int64_t n, mhsw::ResultSet *rs) {
+  d->score2_n = -1;
+  if (!d->score2) return MHSW_OK;
+  MHSW_CK(d->r_score2.reserve((size_t)n + 1), "cudaMalloc results");
+  MHSW_CK(d->r_aend2.reserve((size_t)n + 1), "cudaMalloc results");
+  rs->score2 = d->r_score2.p;
+  rs->a_end2 = d->r_aend2.p;
+  d->score2_n = n;
+  return MHSW_OK;
+}
+
+// Both passes of a short batch whose codes are translated, into the result arrays.
+int run_short_passes(mhsw_driver *d, const mhsw::PairSet &ps, int max_a, int max_b) {
+  d->score2_n = d->score2 ? ps.n : -1;
+  d->fwd_order = nullptr;
+  const mhsw::ResultSet rs = result_set(d);
+  MHSW_CK(mhsw::reset_lists(work_lists(d, ps.n), d->st), "reset lists");
+  MHSW_CK(mhsw::launch_short(ps, d->sc, max_a, max_b, nullptr, nullptr, &rs, false, d->st), "short batch launch");
+  d->launches += 2;
+  return MHSW_OK;
+}
+
+// The staged batch from the pinned buffers to the device.
+int copy_staged(mhsw_driver *d, int64_t n, int64_t ta, int64_t tb) {
+  int rc = ensure_device(d, n, ta, tb);
+  if (rc) return rc;
+  rc = ensure_results(d, n);
+  if (rc) return rc;
+  MHSW_CK(cudaMemcpyAsync(d->a_seq.p, d->h_a.p, (size_t)ta, cudaMemcpyHostToDevice, d->st), "H2D");
+  MHSW_CK(cudaMemcpyAsync(d->b_seq.p, d->h_b.p, (size_t)tb, cudaMemcpyHostToDevice, d->st), "H2D");
+  MHSW_CK(cudaMemcpyAsync(d->a_off.p, d->h_aoff.p, sizeof(int64_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
+  MHSW_CK(cudaMemcpyAsync(d->b_off.p, d->h_boff.p, sizeof(int64_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
+  MHSW_CK(cudaMemcpyAsync(d->a_len.p, d->h_alen.p, sizeof(int32_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
+  MHSW_CK(cudaMemcpyAsync(d->b_len.p, d->h_blen.p, sizeof(int32_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
+  return MHSW_OK;
+}
+
 // Stage a drop-in batch (pointer arrays) into pinned memory and on to the device.
+// A short batch (d->brief_batch, decided here) of few bytes stays in the pinned buffers.
 int stage_strings(mhsw_driver *d, const char *const *reads, const int32_t *read_lens, const char *const *contigs,
                   const int32_t *contig_lens, int32_t n) {
   const bool a_is_read = d->orientation == MHSW_ORIENT_KLIGN;
@@ -797,16 +871,10 @@ int stage_strings(mhsw_driver *d, const char *const *reads, const int32_t *read_
     }
   };
   d->copy_pool.run(parts, copy_part);
-  int rc = ensure_device(d, n, ta, tb);
-  if (rc) return rc;
-  rc = ensure_results(d, n);
-  if (rc) return rc;
-  MHSW_CK(cudaMemcpyAsync(d->a_seq.p, d->h_a.p, (size_t)ta, cudaMemcpyHostToDevice, d->st), "H2D");
-  MHSW_CK(cudaMemcpyAsync(d->b_seq.p, d->h_b.p, (size_t)tb, cudaMemcpyHostToDevice, d->st), "H2D");
-  MHSW_CK(cudaMemcpyAsync(d->a_off.p, d->h_aoff.p, sizeof(int64_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
-  MHSW_CK(cudaMemcpyAsync(d->b_off.p, d->h_boff.p, sizeof(int64_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
-  MHSW_CK(cudaMemcpyAsync(d->a_len.p, d->h_alen.p, sizeof(int32_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
-  MHSW_CK(cudaMemcpyAsync(d->b_len.p, d->h_blen.p, sizeof(int32_t) * n, cudaMemcpyHostToDevice, d->st), "H2D");
+  d->brief_batch = use_short(d, n, ma, mb, d->form);
+  d->in_place = d->brief_batch && ta + tb + 24 * (int64_t)n <= kInPlaceBytes;
+  int rc = MHSW_OK;
+  if (!d->in_place && (rc = copy_staged(d, n, ta, tb))) return rc;
   d->max_a = ma;
   d->max_b = mb;
   d->n_batch = n;
@@ -830,6 +898,52 @@ mhsw::PairSet staged_pairs(mhsw_driver *d) {
   ps.a_code = d->a_code.p;
   ps.b_code = d->b_code.p;
   return ps;
+}
+
+// Score2 mode: the staged batch's second-best scores to the drop-in results.
+int copy_score2(mhsw_driver *d, int64_t n) {
+  if (!d->score2) return MHSW_OK;
+  MHSW_CK(d->h_score2.reserve(2 * (size_t)n), "cudaMallocHost");
+  MHSW_CK(cudaMemcpyAsync(d->h_score2.p, d->r_score2.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, d->st), "D2H");
+  MHSW_CK(cudaMemcpyAsync(d->h_score2.p + n, d->r_aend2.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, d->st), "D2H");
+  return MHSW_OK;
+}
+
+// The staged batch where it lies in pinned host memory.
+mhsw::PairSet pinned_pairs(mhsw_driver *d) {
+  mhsw::PairSet ps{};
+  ps.a_seq = d->h_a.p;
+  ps.a_off = d->h_aoff.p;
+  ps.a_len = d->h_alen.p;
+  ps.b_seq = d->h_b.p;
+  ps.b_off = d->h_boff.p;
+  ps.b_len = d->h_blen.p;
+  ps.n = d->n_batch;
+  return ps;
+}
+
+// A short host batch into the slot's pinned buffer, results behind the inputs.
+int pack_small(mhsw_driver *d, const mhsw_pairs *pairs, int64_t n, int64_t ta, int64_t tb, int slot,
+               mhsw::PairSet *ps, int32_t **out5) {
+  size_t off[7], at = 0;
+  const size_t len[7] = {sizeof(int64_t) * (size_t)n, sizeof(int64_t) * (size_t)n, sizeof(int32_t) * (size_t)n,
+                         sizeof(int32_t) * (size_t)n, (size_t)ta, (size_t)tb, 5 * sizeof(int32_t) * (size_t)n};
+  for (int k = 0; k < 7; k++) {
+    off[k] = at;
+    at += (len[k] + 127) / 128 * 128;
+  }
+  MHSW_CK(d->h_small[slot].reserve(at), "cudaMallocHost");
+  unsigned char *h = d->h_small[slot].p;
+  const void *src[6] = {pairs->a_off, pairs->b_off, pairs->a_len, pairs->b_len, pairs->a_seq, pairs->b_seq};
+  for (int k = 0; k < 6; k++) memcpy(h + off[k], src[k], len[k]);
+  ps->a_off = reinterpret_cast<int64_t *>(h + off[0]);
+  ps->b_off = reinterpret_cast<int64_t *>(h + off[1]);
+  ps->a_len = reinterpret_cast<int32_t *>(h + off[2]);
+  ps->b_len = reinterpret_cast<int32_t *>(h + off[3]);
+  ps->a_seq = reinterpret_cast<char *>(h + off[4]);
+  ps->b_seq = reinterpret_cast<char *>(h + off[5]);
+  *out5 = reinterpret_cast<int32_t *>(h + off[6]);
+  return MHSW_OK;
 }
 
 // A host batch into input set `in`: arenas in 64 MB pieces and the offsets and lengths,
@@ -1090,6 +1204,28 @@ int mhsw_run_kernel_forwards(mhsw_driver *d, const char *const *reads, const int
   if (rc) return rc;
   d->sig = mhsw::batch_signature(d->orientation == MHSW_ORIENT_KLIGN ? read_lens : contig_lens, n, d->max_a,
                                  d->max_b);
+  if (!d->brief_batch) drop_graph(d);
+  if (d->brief_batch) {
+    // one launch for both passes, from the pinned staging buffers into the pinned result views
+    mhsw::OutViews dv, hv;
+    rc = ensure_outviews(d, n, &dv, &hv);
+    if (rc) return rc;
+    d->launches = 1;
+    mhsw::ResultSet rs;
+    if ((rc = short_results(d, n, &rs))) return rc;
+    MHSW_CK(cudaEventRecord(d->ev_t[1], d->st), "event");
+    mhsw::PairSet ps = d->in_place ? pinned_pairs(d) : staged_pairs(d);
+    ps.b_code = nullptr;
+    MHSW_CK(mhsw::launch_short(ps, d->sc, d->max_a, d->max_b, nullptr, &hv, &rs,
+                               d->orientation == MHSW_ORIENT_KLIGN, d->st),
+            "short batch launch");
+    if ((rc = copy_score2(d, n))) return rc;
+    MHSW_CK(cudaEventRecord(d->ev_t[2], d->st), "event");
+    MHSW_CK(cudaEventRecord(d->ev_done, d->st), "event");
+    d->ev_live = true;
+    d->fwd_issued = true;
+    return MHSW_OK;
+  }
   mhsw::PairSet ps = staged_pairs(d);
   if (n > 0) {
     rc = translate_batch(d, &ps, d->a_bytes, d->b_bytes);
@@ -1098,16 +1234,11 @@ int mhsw_run_kernel_forwards(mhsw_driver *d, const char *const *reads, const int
   rc = attach_score2(d, &ps, n, d->a_bytes);
   if (rc) return rc;
   MHSW_CK(cudaEventRecord(d->ev_t[1], d->st), "event");
+  d->begins_done = short_passes(d, n, d->max_a, d->max_b, d->form);
   if (n > 0) {
-    rc = forward_any(d, ps, d->max_a, d->max_b, d->form);
+    rc = d->begins_done ? run_short_passes(d, ps, d->max_a, d->max_b) : forward_any(d, ps, d->max_a, d->max_b, d->form);
     if (rc) return rc;
-    if (ps.rowmax16) {
-      MHSW_CK(d->h_score2.reserve(2 * (size_t)n), "cudaMallocHost");
-      MHSW_CK(cudaMemcpyAsync(d->h_score2.p, d->r_score2.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, d->st),
-              "D2H");
-      MHSW_CK(cudaMemcpyAsync(d->h_score2.p + n, d->r_aend2.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, d->st),
-              "D2H");
-    }
+    if ((rc = copy_score2(d, n))) return rc;
   }
   MHSW_CK(cudaEventRecord(d->ev_t[2], d->st), "event");
   mhsw::OutViews dv, hv;
@@ -1149,11 +1280,37 @@ int mhsw_run_kernel_backwards(mhsw_driver *d, const char *const *reads, const in
   if (!d->fwd_issued) return d->fail(MHSW_ERR_STATE, "run_kernel_backwards without a preceding run_kernel_forwards");
   if ((int64_t)n != d->n_batch)
     return d->fail(MHSW_ERR_ARG, "batch size %d differs from the forward batch (%lld)", n, (long long)d->n_batch);
+  if (d->brief_batch && !d->cigar) {
+    // the begins came with the forward launch
+    MHSW_CK(d->h_counts.reserve(4), "cudaMallocHost");
+    d->h_counts.p[0] = d->h_counts.p[1] = 0;
+    MHSW_CK(cudaEventRecord(d->ev_t[4], d->st), "event");
+    MHSW_CK(cudaEventRecord(d->ev_t[5], d->st), "event");
+    MHSW_CK(cudaEventRecord(d->ev_done, d->st), "event");
+    d->ev_live = true;
+    d->rev_issued = true;
+    return MHSW_OK;
+  }
+  if (d->brief_batch) {
+    // CIGAR mode was switched on between the passes: it needs what the general path leaves
+    // on the device
+    d->brief_batch = false;
+    if (d->in_place) {
+      rc = copy_staged(d, n, d->a_bytes, d->b_bytes);
+      if (rc) return rc;
+    }
+    mhsw::PairSet again = staged_pairs(d);
+    rc = translate_batch(d, &again, d->a_bytes, d->b_bytes);
+    if (rc) return rc;
+    rc = run_short_passes(d, again, d->max_a, d->max_b);
+    if (rc) return rc;
+    d->begins_done = true;
+  }
   mhsw::PairSet ps = staged_pairs(d);
   MHSW_CK(cudaEventRecord(d->ev_t[4], d->st), "event");
   d->cigar_n = -1;
   if (n > 0) {
-    rc = run_reverse(d, ps, d->max_a, d->max_b, d->fwd_order);
+    if (!d->begins_done) rc = run_reverse(d, ps, d->max_a, d->max_b, d->fwd_order);
     if (rc) return rc;
     if (d->cigar) {
       rc = ensure_cigar(d, n);
@@ -1283,9 +1440,12 @@ int finish_slot(mhsw_driver *d, int s) {
     const int rc = finish_cigar(d, pd.ps);
     if (rc) return rc;
   }
-  const int *hc = d->h_counts_p[s].p;
-  d->timing.fwd_ms = elapsed(ev[1], ev[2]);
-  d->timing.rev_ms = elapsed(ev[2], ev[3]);
+  if (pd.copy_to) memcpy(pd.copy_to, pd.from, sizeof(int32_t) * 5 * (size_t)n);
+  // a one-launch batch: both passes are the forward figure
+  const int e1 = pd.brief ? 0 : 1, e2 = pd.brief ? 4 : 2, e3 = pd.brief ? 4 : 3;
+  const int *hc = pd.brief ? nullptr : d->h_counts_p[s].p;
+  d->timing.fwd_ms = elapsed(ev[e1], ev[e2]);
+  d->timing.rev_ms = pd.brief ? 0 : elapsed(ev[2], ev[3]);
   d->timing.total_ms = elapsed(ev[0], ev[4]);
   d->timing.fwd_cells = pd.cells;
   d->timing.n_pairs = n;
@@ -1306,9 +1466,9 @@ int finish_slot(mhsw_driver *d, int s) {
       r.copy_in_end = std::max(r.copy_in_end, (double)elapsed(d->ev_epoch, d->ev_cin[s][1 + k]));
   }
   r.stream_ready = elapsed(d->ev_epoch, ev[0]);
-  r.translated = elapsed(d->ev_epoch, ev[1]);
-  r.forward_done = elapsed(d->ev_epoch, ev[2]);
-  r.begin_done = elapsed(d->ev_epoch, ev[3]);
+  r.translated = elapsed(d->ev_epoch, ev[e1]);
+  r.forward_done = elapsed(d->ev_epoch, ev[e2]);
+  r.begin_done = elapsed(d->ev_epoch, ev[e3]);
   r.done = elapsed(d->ev_epoch, ev[4]);
   d->history[d->history_n % mhsw_driver::kHistory] = r;
   d->history_n++;
@@ -1325,6 +1485,29 @@ int finish_pending(mhsw_driver *d) {
     const int rc = finish_slot(d, oldest);
     if (rc) return rc;
   }
+}
+
+// A batch on the one-launch path: results to res, copied on to the host array out5 when the
+// call completes (out5 null: res is the caller's device array).
+int run_short(mhsw_driver *d, int slot, const mhsw::PairSet &ps, int ma, int mb, double cells, int32_t *res,
+              int32_t *out5) {
+  cudaEvent_t *ev = d->ev_p[slot];
+  d->cigar_n = -1;
+  mhsw::ResultSet rs;
+  if (int rc = short_results(d, ps.n, &rs)) return rc;
+  MHSW_CK(mhsw::launch_short(ps, d->sc, ma, mb, res, nullptr, &rs, false, d->st), "short batch launch");
+  d->launches = 1;
+  MHSW_CK(cudaEventRecord(ev[4], d->st), "event");
+  mhsw_driver::Pending &pd = d->pend[slot];
+  pd.active = true;
+  pd.n = ps.n;
+  pd.cells = cells;
+  pd.seq = ++d->call_seq;
+  pd.ps = ps;
+  pd.brief = true;
+  pd.from = res;
+  pd.copy_to = out5;
+  return MHSW_OK;
 }
 
 // Everything of a batch call up to its completion event, enqueued on the handle's stream;
@@ -1380,6 +1563,13 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
         tb = std::max(tb, pairs->b_off[i] + lb);
         cells += (double)la * (double)lb;
       }
+    }
+    if (mb <= mhsw::kMaxB && use_short(d, n, ma, mb, form) && ta + tb + 24 * n <= kInPlaceBytes) {
+      int32_t *res = nullptr;
+      rc = pack_small(d, pairs, n, ta, tb, slot, &ps, &res);
+      if (rc) return rc;
+      ps.n = n;
+      return run_short(d, slot, ps, ma, mb, cells, res, out5);
     }
     mhsw_driver::InSet &in = d->in_sets[slot];
     MHSW_CK(in.a_seq.reserve((size_t)ta + 16), "cudaMalloc A");
@@ -1441,6 +1631,9 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
   else if (hinted_sizes) d->sig = mhsw::batch_signature(nullptr, n, ma, mb);
   ps.n = n;
   if (mb > mhsw::kMaxB) return d->fail(MHSW_ERR_LIMIT, "sequence of %d bytes exceeds the limit %d", mb, mhsw::kMaxB);
+  // (decided here: a capture switches the tuner off while it runs enqueue)
+  const bool both = short_passes(d, n, ma, mb, form), brief = both && !d->cigar;
+  if (brief && !host_io) return run_short(d, slot, ps, ma, mb, cells, out5, nullptr);
   rc = ensure_results(d, n);
   if (rc) return rc;
   if (n > 0) {
@@ -1465,17 +1658,29 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
     return capturing ? cudaEventRecordWithFlags(ev, d->st, cudaEventRecordExternal) : cudaEventRecord(ev, d->st);
   };
   auto enqueue = [&]() -> int {
+    if (brief) {  // a host batch copied in: one launch for both passes
+      MHSW_CK(mark(ev[1]), "event");
+      mhsw::ResultSet rs;
+      if (int r = short_results(d, n, &rs)) return r;
+      MHSW_CK(mhsw::launch_short(ps, d->sc, ma, mb, d->out5.p, nullptr, &rs, false, d->st), "short batch launch");
+      MHSW_CK(mark(ev[2]), "event");
+      MHSW_CK(mark(ev[3]), "event");
+      MHSW_CK(cudaMemcpyAsync(out5, d->out5.p, sizeof(int32_t) * 5 * n, cudaMemcpyDeviceToHost, d->st), "D2H");
+      d->h_counts_p[slot].p[0] = d->h_counts_p[slot].p[1] = 0;
+      d->launches += 1;
+      return MHSW_OK;
+    }
     if (n > 0) {
       int r = translate_batch(d, &ps, ta, tb);
       if (r) return r;
     }
     MHSW_CK(mark(ev[1]), "event");
     if (n > 0) {
-      int r = forward_any(d, ps, ma, mb, form);
+      int r = both ? run_short_passes(d, ps, ma, mb) : forward_any(d, ps, ma, mb, form);
       if (r) return r;
     }
     MHSW_CK(mark(ev[2]), "event");
-    if (n > 0) {
+    if (n > 0 && !both) {
       int r = run_reverse(d, ps, ma, mb, d->fwd_order);
       if (r) return r;
     }
@@ -1586,6 +1791,8 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
   pd.cells = cells;
   pd.seq = ++d->call_seq;
   pd.ps = ps;
+  pd.brief = false;
+  pd.copy_to = nullptr;
   return MHSW_OK;
 }
 
@@ -1800,6 +2007,20 @@ int align_resident(mhsw_driver *d, const PairSet &in, int64_t a_bytes, int max_a
   if (n <= 0) return MHSW_OK;
   if (!in.b_code || !out5_dev) return d->fail(MHSW_ERR_ARG, "resident batch needs B codes and an output buffer");
   if (max_b > kMaxB) return d->fail(MHSW_ERR_LIMIT, "sequence of %d bytes exceeds the limit %d", max_b, kMaxB);
+  if (use_short(d, n, max_a, max_b, form)) {
+    ResultSet rs;
+    if ((rc = short_results(d, n, &rs))) return rc;
+    MHSW_CK(cudaEventRecord(d->ev_t[0], d->st), "event");
+    MHSW_CK(cudaEventRecord(d->ev_t[1], d->st), "event");
+    MHSW_CK(launch_short(in, d->sc, max_a, max_b, out5_dev, nullptr, &rs, false, d->st), "short batch launch");
+    MHSW_CK(cudaEventRecord(d->ev_t[2], d->st), "event");
+    MHSW_CK(cudaEventRecord(d->ev_t[3], d->st), "event");
+    d->launches = 1;
+    d->timing = mhsw_timing{};
+    d->timing.n_pairs = n;
+    return MHSW_OK;
+  }
+  drop_graph(d);
   rc = ensure_results(d, n);
   if (rc) return rc;
   MHSW_CK(d->a_code.reserve((size_t)a_bytes + 16), "cudaMalloc codes");
@@ -1812,10 +2033,11 @@ int align_resident(mhsw_driver *d, const PairSet &in, int64_t a_bytes, int max_a
   if (rc) return rc;
   MHSW_CK(cudaEventRecord(d->ev_t[1], d->st), "event");
   d->sig = mhsw::batch_signature(nullptr, ps.n, max_a, max_b);
-  rc = forward_any(d, ps, max_a, max_b, form);
+  const bool both = short_passes(d, n, max_a, max_b, form);
+  rc = both ? run_short_passes(d, ps, max_a, max_b) : forward_any(d, ps, max_a, max_b, form);
   if (rc) return rc;
   MHSW_CK(cudaEventRecord(d->ev_t[2], d->st), "event");
-  rc = run_reverse(d, ps, max_a, max_b, d->fwd_order);
+  if (!both) rc = run_reverse(d, ps, max_a, max_b, d->fwd_order);
   if (rc) return rc;
   MHSW_CK(cudaEventRecord(d->ev_t[3], d->st), "event");
   MHSW_CK(launch_pack5(result_set(d), n, out5_dev, d->st), "pack5");

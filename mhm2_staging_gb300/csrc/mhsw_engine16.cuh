@@ -60,11 +60,6 @@ constexpr int kCeiling16 = 4000;  // largest score the keyed int16 engine accept
 // rows-pairs per lane), 16 lanes for longer A (K = 6, 8; strips of 256 rows beyond).
 constexpr int kGKShort = 8;
 constexpr int kGKLong = 16;
-constexpr int kShortRows = 160;
-__host__ __device__ constexpr int keyed_g_for_rows(int rows) { return rows <= kShortRows ? kGKShort : kGKLong; }
-__host__ __device__ constexpr int keyed_k_for_rows(int rows) {
-  return rows <= 64 ? 4 : rows <= 96 ? 6 : rows <= 128 ? 8 : rows <= 160 ? 10 : rows <= 192 ? 6 : 8;
-}
 __host__ __device__ constexpr int keyed_cap(int K) { return K <= 8 ? (1 << 12) - 64 : (1 << 11) - 64; }
 
 constexpr int kCode16Zero = 5;  // score2 mode: SSW's zero-scoring query padding

@@ -20,6 +20,7 @@
 #include <mutex>
 #include <utility>
 
+#include "mhsw_band.cuh"
 #include "mhsw_engine.cuh"
 #include "mhsw_engine16.cuh"
 #include "mhsw_launch.h"
@@ -107,69 +108,6 @@ __global__ void __launch_bounds__(256) k_fwd(PairSet ps, ResultSet rs, Scoring s
   }
 }
 
-// Plain forward pass with the keyed int16 engine (mhsw_engine16.cuh): one G-lane group
-// per pair, grid-stride over [0, n).
-template <int K, int G, bool S2 = false>
-__global__ void __launch_bounds__(256) k_fwd16(PairSet ps, ResultSet rs, Scoring sc, int ceiling, V16::Pay *scratch,
-                                               int scratch_stride, WorkLists wl, int pad, int bcap) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int gpb = blockDim.x / G;
-  const int grp = threadIdx.x / G;
-  const int lane = threadIdx.x % G;
-  const unsigned gmask = group_mask(G);
-  constexpr size_t kProf = group_prof16_bytes<K, G, S2 ? kCode16Zero + 1 : kCodeN + 1>();
-  unsigned char *gbase = smem + (size_t)grp * kProf;  // keyed engine: profile table only
-  GroupSmem gs;
-  gs.prof = reinterpret_cast<uint32_t *>(gbase);
-  gs.prof_lanes = G;
-  gs.bcodes = nullptr;
-  gs.pad = pad;
-  gs.bcap = bcap;
-  constexpr int RS = 2 * K * G;
-  const int64_t gid = (int64_t)blockIdx.x * gpb + grp;
-  const int64_t gstride = (int64_t)gridDim.x * gpb;
-  V16::Pay *bnd = scratch ? scratch + gid * (int64_t)scratch_stride : nullptr;
-  for (int64_t p = gid; p < ps.n; p += gstride) {
-    const int M = ps.a_len[p], N = ps.b_len[p];
-    const int NP = S2 ? ssw_pad16(N) : N;
-    const bool too_long = (N > kMaxB) || (M > RS && (bnd == nullptr || NP > scratch_stride));
-    if (M <= 0 || N <= 0 || too_long) {
-      if (lane == 0) {
-        rs.score[p] = 0;
-        rs.a_end[p] = -1;
-        rs.b_end[p] = 0;
-        rs.flag[p] = too_long ? kFlagTooLong : 0u;
-      }
-      continue;
-    }
-    SeqView A{ps.a_code + ps.a_off[p], 1, M};
-    SeqView B{ps.b_code + ps.b_off[p], 1, N};
-    SweepOut so;
-    RowMaxOut rmo{nullptr, 0};
-    if constexpr (S2) rmo = RowMaxOut{ps.rowmax16 + ps.a_off[p], NP};
-    sweep16<K, G, S2>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo);
-    if (lane == 0) {
-      const int S = key_value(so.key);
-      // score2 mode: SSW's word path pads B to a multiple of 8; where that differs from
-      // the byte-path padding swept here, the int32 pass recomputes the row maxima.
-      const bool word_redo = S2 && S + ssw_bias(sc) >= 255 && ssw_pad8(N) != NP;
-      if (so.overflow || word_redo) {
-        rs.flag[p] = kFlagOverflow16;
-        const int slot = atomicAdd(wl.ovf_count, 1);
-        if (slot < wl.cap) wl.ovf[slot] = p;
-        rs.score[p] = S;
-        rs.a_end[p] = -1;
-        rs.b_end[p] = 0;
-      } else {
-        rs.flag[p] = 0u;
-        rs.score[p] = S;
-        rs.a_end[p] = S > 0 ? key_row(so.key) : -1;
-        rs.b_end[p] = S > 0 ? key_col(so.key) : 0;
-      }
-    }
-  }
-}
-
 // Begin pass, banded.  Each pair's search is first assigned a band class: the
 // narrowest instantiation whose width holds the alignment's largest drift to each side
 // of the end cell's diagonal at the first row cap (band_sides: vertical gaps also cost
@@ -184,48 +122,6 @@ __global__ void __launch_bounds__(256) k_fwd16(PairSet ps, ResultSet rs, Scoring
 // wavefront list.
 __host__ __device__ constexpr int band_half(int c) {  // half-widths 3, 5, 7, 11, 15, 23, 31
   return c == 0 ? 3 : c == 1 ? 5 : c == 2 ? 7 : c == 3 ? 11 : c == 4 ? 15 : c == 5 ? 23 : 31;
-}
-
-__host__ __device__ __forceinline__ int band_first_cap(int S, int mt, int M2) {
-  const long long tt = 2ll * S / (mt > 0 ? mt : 1) + 16;
-  return (int)(tt < M2 ? tt : M2);
-}
-
-// Total gap length g (inserted plus deleted cells) of an alignment that scores S with at
-// most dmax diagonal steps.  Each diagonal step scores at most match, and g gap cells in
-// r >= 1 runs cost r*gO + (g - r)*gE >= g*min(gO, gE) + max(gO - gE, 0), so
-// g*min(gO, gE) + max(gO - gE, 0) <= dmax*match - S (g = 0 when that leaves no room for
-// one gap cell).  (dmax <= 65000 and match <= 127 keep the product inside 32 bits.)
-__host__ __device__ __forceinline__ int gap_cells_bound(int dmax, int S, const Scoring &sc) {
-  const int gmin = sc.gap_open < sc.gap_extend ? sc.gap_open : sc.gap_extend;
-  const int g1 = gmin > 0 ? gmin : 1;
-  const int slack = dmax * sc.match - S - (sc.gap_open > sc.gap_extend ? sc.gap_open - sc.gap_extend : 0);
-  return slack < g1 ? 0 : slack / g1;
-}
-
-// Total gap length any alignment reaching the score within the first t rows can have:
-// its diagonal steps D <= min(t, N2).
-__host__ __device__ __forceinline__ int band_gap_bound(int t, int N2, int S, const Scoring &sc) {
-  return gap_cells_bound(t < N2 ? t : N2, S, sc);
-}
-
-// How far such an alignment can drift from the end cell's diagonal to either side.  I
-// vertical gap cells (a row each, no column) leave at most t - I diagonal steps:
-// S <= (t - I)*match - I*gmin - c, c = max(gO - gE, 0) once, so
-// I <= (t*match - S - c) / (match + gmin); likewise J horizontal gap cells leave at most
-// N2 - J, so J <= (N2*match - S - c) / (match + gmin).  Both are at most the total g.  A
-// band over columns [row - L, row - L + W) holds every such alignment when I <= L and
-// J <= W - 1 - L.
-__host__ __device__ __forceinline__ void band_sides(int t, int N2, int S, const Scoring &sc, int &I, int &J) {
-  const int g = band_gap_bound(t, N2, S, sc);
-  const int gmin = sc.gap_open < sc.gap_extend ? sc.gap_open : sc.gap_extend;
-  const int mg = sc.match + (gmin > 0 ? gmin : 1);
-  const int c = sc.gap_open > sc.gap_extend ? sc.gap_open - sc.gap_extend : 0;
-  const int st = t * sc.match - S - c, sn = N2 * sc.match - S - c;
-  I = st < mg ? 0 : st / mg;
-  J = sn < mg ? 0 : sn / mg;
-  if (I > g) I = g;
-  if (J > g) J = g;
 }
 
 // The narrowest band class whose width holds both sides at the first row cap
@@ -924,23 +820,6 @@ int num_sms(int device) {
   return g_num_sms;
 }
 
-template <int C>
-size_t group_prof16_rt_c(int K, int G) {
-  if (G == kGKShort) {
-    switch (K) {
-      case 4: return group_prof16_bytes<4, kGKShort, C>();
-      case 6: return group_prof16_bytes<6, kGKShort, C>();
-      case 8: return group_prof16_bytes<8, kGKShort, C>();
-      default: return group_prof16_bytes<10, kGKShort, C>();
-    }
-  }
-  return K == 6 ? group_prof16_bytes<6, kGKLong, C>() : group_prof16_bytes<8, kGKLong, C>();
-}
-
-size_t group_prof16_rt(int K, int G, bool s2) {
-  return s2 ? group_prof16_rt_c<kCode16Zero + 1>(K, G) : group_prof16_rt_c<kCodeN + 1>(K, G);
-}
-
 size_t group_prof_rt(bool wide32, int K) {
   if (wide32) return group_prof_bytes<V32, 4, kG>();
   switch (K) {
@@ -969,33 +848,16 @@ cudaError_t launch_fwd_t(const FwdConfig &cfg, const PairSet &ps, const ResultSe
   return cudaGetLastError();
 }
 
-template <int K, int G>
-cudaError_t launch_fwd16_t(const FwdConfig &cfg, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
-                           int ceiling, void *scratch, int scratch_stride, const WorkLists &wl, cudaStream_t st) {
-  auto kern = ps.rowmax16 ? k_fwd16<K, G, true> : k_fwd16<K, G, false>;
-  {
-    cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), cfg.smem);
-    if (e != cudaSuccess) return e;
-  }
-  kern<<<cfg.grid, cfg.groups_per_block * G, cfg.smem, st>>>(ps, rs, sc, ceiling,
-                                                              reinterpret_cast<V16::Pay *>(scratch), scratch_stride,
-                                                              wl, cfg.pad, cfg.bcap);
-  return cudaGetLastError();
-}
-
 }  // namespace
 
 bool keyed_scoring(const Scoring &sc) {
   return sc.mismatch <= sc.gap_open && sc.ambiguity <= sc.gap_open && sc.gap_open >= 1 && sc.gap_extend >= 1;
 }
 
-cudaError_t plan_forward(int device, int max_a, int max_b, bool wide32, FwdConfig *cfg, bool keyed, bool s2) {
+cudaError_t plan_forward(int device, int max_a, int max_b, bool wide32, FwdConfig *cfg) {
   FwdConfig c{};
   c.G = kG;
-  if (keyed && !wide32) {
-    c.G = keyed_g_for_rows(max_a);
-    c.K = keyed_k_for_rows(max_a);
-  } else if (wide32) {
+  if (wide32) {
     c.K = 4;
   } else {
     const int need = (max_a + 2 * kG - 1) / (2 * kG);  // K with 2*K*G >= max_a
@@ -1013,18 +875,14 @@ cudaError_t plan_forward(int device, int max_a, int max_b, bool wide32, FwdConfi
   // room for B, the groups' lane skew and SSW's zero-score padding of score2 mode (< 16)
   c.bcap = ((c.pad + max_b + 16 + 2 * c.G) + 15) / 16 * 16;
   const size_t budget = 100 * 1024;  // keep two blocks per SM possible
-  // the keyed engine reads B from global memory: its group needs the profile table only
-  const size_t per_group =
-      (keyed && !wide32) ? group_prof16_rt(c.K, c.G, s2) : group_prof_rt(wide32, c.K) + (size_t)c.bcap;
+  const size_t per_group = group_prof_rt(wide32, c.K) + (size_t)c.bcap;
   int gpb = 8;
   while (gpb > 1 && (size_t)gpb * per_group > budget) gpb /= 2;
-  if (c.G < kG) gpb *= kG / c.G;  // same block size (128 threads) with smaller groups
   c.groups_per_block = gpb;
   c.smem = (size_t)gpb * per_group;
   if (c.smem > 220 * 1024) return cudaErrorInvalidValue;
   int sms = num_sms(device);
   c.grid = sms * 8;  // grid-stride; callers may lower it
-  c.keyed = keyed && !wide32;
   *cfg = c;
   return cudaSuccess;
 }
@@ -1043,18 +901,6 @@ cudaError_t launch_forward(const FwdConfig &cfg, bool wide32, const PairSet &ps,
   // scratch stride (payloads per group) = B capacity
   const int stride = cfg.bcap;
   if (wide32) return launch_fwd_t<V32, 4>(cfg, ps, rs, sc, list, list_count, ceiling, scratch, stride, wl, st);
-  if (cfg.keyed && !list) {
-    if (cfg.G == kGKShort) {
-      switch (cfg.K) {
-        case 4: return launch_fwd16_t<4, kGKShort>(cfg, ps, rs, sc, ceiling, scratch, stride, wl, st);
-        case 6: return launch_fwd16_t<6, kGKShort>(cfg, ps, rs, sc, ceiling, scratch, stride, wl, st);
-        case 8: return launch_fwd16_t<8, kGKShort>(cfg, ps, rs, sc, ceiling, scratch, stride, wl, st);
-        default: return launch_fwd16_t<10, kGKShort>(cfg, ps, rs, sc, ceiling, scratch, stride, wl, st);
-      }
-    }
-    if (cfg.K == 6) return launch_fwd16_t<6, kGKLong>(cfg, ps, rs, sc, ceiling, scratch, stride, wl, st);
-    return launch_fwd16_t<8, kGKLong>(cfg, ps, rs, sc, ceiling, scratch, stride, wl, st);
-  }
   switch (cfg.K) {
     case 2: return launch_fwd_t<V16, 2>(cfg, ps, rs, sc, list, list_count, ceiling, scratch, stride, wl, st);
     case 3: return launch_fwd_t<V16, 3>(cfg, ps, rs, sc, list, list_count, ceiling, scratch, stride, wl, st);
@@ -1207,7 +1053,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
   // Wide bands: wavefront on the reversed box (count read on the device), in int16 for
   // scores up to kWaveScore16 where a strip plan with scratch exists, int32 otherwise.
   FwdConfig c16, c32;
-  cudaError_t e = plan_forward(device, max_a, max_b, false, &c16, false, false);
+  cudaError_t e = plan_forward(device, max_a, max_b, false, &c16);
   if (e != cudaSuccess) return e;
   e = plan_forward(device, max_a, max_b, true, &c32);
   if (e != cudaSuccess) return e;

@@ -30,7 +30,6 @@ struct FwdConfig {
   int pad;            // leading PAD entries
   int grid;           // blocks (grid-stride over pairs)
   size_t smem;        // dynamic shared memory bytes
-  bool keyed;         // int16 forward uses the keyed engine (mhsw_engine16.cuh)
 };
 
 // Upper bound of B length the forward kernels accept (shared-memory code buffer).
@@ -59,11 +58,9 @@ cudaError_t join_from(const Forks &f, cudaStream_t st, int k);
 // one another's launch.
 cudaError_t raise_smem_limit(const void *func, size_t bytes);
 
-// Chooses K/G/grid/smem for a forward launch over pairs whose A (rows) lengths are at
-// most max_a and B lengths at most max_b.  wide32 selects the int32 engine.
-// s2: score2 mode (the keyed profile table gains the zero-score code).
-cudaError_t plan_forward(int device, int max_a, int max_b, bool wide32, FwdConfig *cfg, bool keyed = false,
-                         bool s2 = false);
+// Chooses K/G/grid/smem for a launch of the generic engine over pairs whose A (rows)
+// lengths are at most max_a and B lengths at most max_b.  wide32 selects the int32 engine.
+cudaError_t plan_forward(int device, int max_a, int max_b, bool wide32, FwdConfig *cfg);
 // Second-best scores (score2 mode) from the row maxima the forward pass wrote.
 cudaError_t launch_score2(const PairSet &ps, const ResultSet &rs, const Scoring &sc, cudaStream_t st);
 
@@ -102,6 +99,22 @@ struct OutViews {
 // part: 1 = ends + score, 2 = begins, 3 = all.
 cudaError_t launch_finalize(const ResultSet &rs, int64_t n, bool a_is_query, int part, const OutViews &ov,
                             cudaStream_t st);
+
+// ---- short batches (mhsw_short.cu) -------------------------------------------------
+// Largest batch (pairs, and pairs times the longest B), A and B the one-launch path takes.
+constexpr int64_t kShortPairs = 8192;
+constexpr int64_t kShortColumns = 14000000;
+constexpr int kShortRowsMax = 512;
+constexpr int kShortColsMax = 8192;
+bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b);
+// Forward and begin pass of a short batch: ps.a_seq raw bytes, B from ps.b_code or, when
+// that is null, ps.b_seq raw bytes; any of them may be pinned host memory.  Results go to out5
+// (n x 5), the drop-in views ov and the general path's arrays rs (each may be null; score2
+// mode when rs holds its arrays, the others of rs being null when only it is wanted).
+cudaError_t launch_short(const PairSet &ps, const Scoring &sc, int max_a, int max_b, int32_t *out5, const OutViews *ov,
+                         const ResultSet *rs, bool a_is_query, cudaStream_t st);
+// True when some pair of a batch with these longest sequences can need the int32 pass.
+bool may_need_int32(const Scoring &sc, int ceiling, int max_a, int max_b);
 
 // Packs results into n x 5 int32 rows (score, a_beg, a_end, b_beg, b_end).
 cudaError_t launch_pack5(const ResultSet &rs, int64_t n, int32_t *out5, cudaStream_t st);

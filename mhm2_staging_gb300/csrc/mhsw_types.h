@@ -39,8 +39,8 @@ struct PairSet {  // device pointers; A = SSW ref (rows), B = SSW query (columns
 };
 
 struct ResultSet {  // device pointers, one entry per pair
-  int32_t *score, *a_end, *b_end, *a_beg, *b_beg;
-  uint32_t *flag;
+  int32_t *score = nullptr, *a_end = nullptr, *b_end = nullptr, *a_beg = nullptr, *b_beg = nullptr;
+  uint32_t *flag = nullptr;
   int32_t *score2 = nullptr, *a_end2 = nullptr;  // score2 mode: SSW's second-best score and its A row
 };
 
