@@ -21,16 +21,25 @@
 //            and X by comparing base codes along the CIGAR's own walk from the box's
 //            start (N against N counts as =), mismatches = X + I + D lengths.
 //
-// GB300 mapping.  One thread per pair; the band is kept diagonal-indexed (k = j - i + w)
-// so the rows slide without moving data: H and E of the previous row live in registers
-// at fixed indices, the A codes of the band in a nibble-packed register window shifted
-// one code per row.  Six instantiations hold half-widths up to 1, 2, 4, 8, 16 and 31
-// (cells per row 3 .. 63); a pair whose band doubles past its kernel's width moves to the
-// next list, and boxes longer than kCigarRowCap rows or bands wider than 31 go to the
-// generic kernel (rows and directions in global memory, host-driven rounds).  Directions
-// take 4 bits per cell (E open/extend, F open/extend, H source) written one row word at
-// a time, coalesced across the warp ([row][word][thread] layout).  The traceback walks
-// the stored directions once, streaming the rows it visits through a ring of prefetched
+// GB300 mapping.  The band is kept diagonal-indexed (k = j - i + w) so the rows slide without
+// moving data.  Two forms:
+//   lanes (k_cigar_lanes)  a group of 8, 16 or 32 lanes takes a pair, lane k band cell k; the
+//     row's F chain is a prefix maximum over the lanes, the four direction bits of the row's
+//     cells are four ballots, kept with the box's codes in shared memory, where the group's
+//     first lane then walks them.  Half-widths up to 15.  A row costs about 45 warp
+//     instructions whatever the group size, but its chain is ~15x shorter than a thread's
+//     chain over the cells, and a class of up to kLanesMost pairs is bound by that chain.
+//   threads (k_cigar_band) one thread per pair, the band in registers: fewer instructions per
+//     pair, for classes large enough to fill the GPU, and for half-widths 16 and 31.  H and E
+//     of the previous row at fixed indices, the A codes of the band in a nibble-packed
+//     register window shifted one code per row.
+// Classes hold half-widths up to 1, 2, 4, 8, 16 and 31; a pair whose band doubles past its
+// kernel's width moves to the next list, and boxes longer than kCigarRowCap rows or bands
+// wider than 31 go to the generic kernel (rows and directions in global memory, host-driven
+// rounds).  Directions
+// take 4 bits per cell (E open/extend, F open/extend, H source).  The thread form writes them
+// one row word at a time, coalesced across the warp ([row][word][thread] layout), walks them
+// once, streaming the rows it visits through a ring of prefetched
 // row words and recording its steps (2 bits each) in thread-local memory; replaying the
 // record counts the ops and mismatches, then writes the ops back to front straight to
 // their place in a shared arena reserved with one atomic per warp.  (The generic kernel,
@@ -747,6 +756,12 @@ __device__ int band_pass(const CigarArgs &g, const Box &bx, int w, uint32_t *dco
   return mx;
 }
 
+// Largest class the lanes form takes (100,000 uneven pairs, classes of about 30,000, 12,000,
+// 10,000 and 4,000 pairs: the four thread kernels took 235, 292, 421 and 624 us one after the
+// other; their time hardly grows up to about 100,000 pairs, the lanes form's does with the
+// pairs).
+constexpr int kLanesMost = 40000;
+
 template <int C>
 __global__ void __launch_bounds__(128) k_cigar_band(CigarArgs g) {
   constexpr int W = cigar_half(C);
@@ -756,8 +771,12 @@ __global__ void __launch_bounds__(128) k_cigar_band(CigarArgs g) {
   int seg0 = 0;
 #pragma unroll
   for (int c = 0; c <= C; c++) seg0 += g.counts[c];
-  const int seg_n = g.counts[1 + C];
-  const int count = seg_n + g.counts[kCigarEsc + C];
+  int seg_n = g.counts[1 + C], list_n = g.counts[kCigarEsc + C];
+  if (cigar_half(C) <= 8) {  // the lanes form takes the smaller segments and the lists
+    if (seg_n <= kLanesMost) seg_n = 0;
+    list_n = 0;
+  }
+  const int count = seg_n + list_n;
   const int2 *list = g.lists + (int64_t)C * g.list_cap;
   uint32_t *dcol = g.dirs + tid;
   // warp-uniform trip count: every lane reaches the arena reservation together
@@ -790,6 +809,213 @@ __global__ void __launch_bounds__(128) k_cigar_band(CigarArgs g) {
     }
     __syncwarp();
     traceback_reg<W>(g, dcol, T, bx, w, p, valid);
+  }
+}
+
+// ---- lanes form ------------------------------------------------------------------------
+
+constexpr int kLaneRowsA = kCigarRowCap + 32;  // A codes of a box: at most rows + 15 columns
+constexpr int kLaneWarps = 4;
+
+template <int LG>
+__host__ __device__ constexpr size_t lanes_warp_bytes() {  // one warp: direction words of a row, then the groups' codes
+  return (size_t)kCigarRowCap * 16 + (32 / LG) * (size_t)(kLaneRowsA + kCigarRowCap);
+}
+
+// One banded DP pass at half-width w for the groups with `go`; the same cells, ties and
+// quirks as band_pass.  F along the row as a prefix maximum: with H' = max(E, 0, diagonal),
+// F(k) + k*gE = max(F(kstart) + kstart*gE, max over kstart <= m < k of H'(m) - gO + (m+1)*gE),
+// and F(k) opened where the last term of that maximum exceeds the others.
+template <int LG>
+__device__ int lanes_pass(const CigarArgs &g, const uint8_t *A, const uint8_t *B, int rows, int ref_len, int w, bool go,
+                          int k, int all_rows, uint4 *dirs) {
+  constexpr unsigned full = 0xffffffffu;
+  const int gO = g.gO, gE = g.gE;
+  const int up_add = (k + 1) * gE - gO;
+  const unsigned mine = __ballot_sync(full, go);  // lanes whose directions this pass writes
+  int H = 0, E = 0, mx = 0;
+  for (int i = 0; i < all_rows; i++) {
+    const int kstart = max(0, w - i), kend = min(2 * w, ref_len - 1 - i + w);
+    const bool v = go && i < rows && k >= kstart && k <= kend;
+    int hu = __shfl_down_sync(full, H, 1, LG), eu = __shfl_down_sync(full, E, 1, LG);
+    if (k == kend && i >= 1 && i <= w + 1 && ref_len <= i + w) hu = eu = 0;
+    const int a = hu - gO, b = eu - gE;
+    const int e = max(a, b);
+    const int ca = v ? (int)A[i - w + k] : 0, cb = v ? (int)B[i] : 0;
+    const int dg = H + sub_score(g, ca, cb);
+    const int hp = __vimax_s32_relu(e, dg);
+    const int u = v ? hp + up_add : -(1 << 28);
+    int in = u;
+#pragma unroll
+    for (int o = 1; o < LG; o <<= 1) {
+      const int t = __shfl_up_sync(full, in, o, LG);
+      if (k >= o) in = max(in, t);
+    }
+    const int base = (kstart - 1) * gE;  // F of the row's first cell is -gE (gap open >= gap extend)
+    in = max(in, base);
+    int ex = __shfl_up_sync(full, in, 1, LG);
+    if (k == 0) ex = base;
+    const int f = ex - k * gE;
+    const int m1 = __vimax_s32_relu(e, f);
+    const bool gap = m1 > dg, from_e = e > max(f, 0), same = ca == cb;
+    uint4 d;
+    d.x = __ballot_sync(full, v && a > b);
+    d.y = __ballot_sync(full, v && u > ex) << 1;  // the next cell's F opened
+    d.z = __ballot_sync(full, v && (gap ? from_e : same));
+    d.w = __ballot_sync(full, v && (gap ? !from_e : same));
+    if ((threadIdx.x & 31) == 0) {
+      if (mine != full) {  // keep the other groups' bits
+        const uint4 o = dirs[i];
+        d.x = (d.x & mine) | (o.x & ~mine);
+        d.y = (d.y & mine) | (o.y & ~mine);
+        d.z = (d.z & mine) | (o.z & ~mine);
+        d.w = (d.w & mine) | (o.w & ~mine);
+      }
+      dirs[i] = d;
+    }
+    if (v) {
+      H = max(hp, f);
+      E = e;
+      mx = max(mx, H);
+    }
+  }
+#pragma unroll
+  for (int o = LG / 2; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(full, mx, o, LG));
+  __syncwarp();
+  return mx;
+}
+
+// The walk over a group's directions (bit sh + k of a row's words).  Counts ops and
+// mismatches or (EMIT) writes the ops to out[0 .. nops) back to front; j_end is the column
+// where it stops.  shift: that column of an earlier walk; where it is not 0, M steps compare
+// the bases shifted by it (see replay_path).
+template <bool EMIT>
+__device__ bool lanes_walk(const uint4 *dirs, int sh, const uint8_t *A, const uint8_t *B, const Box &bx, int w, int shift,
+                           int *j_end, int *nops, int *mism, uint32_t *out) {
+  int t = 0, mis = 0, rl = 0;
+  uint32_t rk = 0;
+  auto emit = [&](uint32_t kind, int len) {
+    if (EMIT) out[*nops - 1 - t] = ((uint32_t)len << 4) | kind;
+    ++t;
+  };
+  auto cell = [&](uint32_t kind) {
+    mis += kind != kOpEq;
+    if (kind == rk) {
+      ++rl;
+    } else {
+      if (rl > 0) emit(rk, rl);
+      rk = kind;
+      rl = 1;
+    }
+  };
+  if (bx.tail > 0) emit(kOpS, bx.tail);
+  int i = bx.rows - 1, j = bx.ref_len - 1, st = 2;
+  while (i > 0) {
+    const int k = j - i + w;
+    if (j < 0 || k < 0 || k > 2 * w) return false;
+    const uint4 d = dirs[i];
+    const int b = sh + k;
+    const uint32_t hs = ((d.z >> b) & 1u) | (((d.w >> b) & 1u) << 1);
+    const int eff = st != 2 ? st : (hs == 1u ? 0 : hs == 2u ? 1 : 2);
+    if (eff == 2) cell((shift ? A[j - shift] != B[i] : hs != 3u) ? kOpX : kOpEq);
+    else cell(eff == 0 ? kOpI : kOpD);
+    st = eff == 0 ? (((d.x >> b) & 1u) ? 2 : 0) : eff == 1 ? (((d.y >> b) & 1u) ? 2 : 1) : 2;
+    i -= eff != 1;
+    j -= eff != 0;
+  }
+  cell(A[0] != B[0] ? kOpX : kOpEq);  // the cell where the walk stopped: one more M
+  emit(rk, rl);
+  if (bx.bb > 0) emit(kOpS, bx.bb);
+  if (!EMIT) {
+    *j_end = j;
+    *nops = t;
+    *mism = mis;
+  }
+  return true;
+}
+
+// Pairs of the segments of classes c_lo .. c_hi (none when together they exceed kLanesMost
+// and the thread form takes them), or of class c_lo's escalation list.
+template <int LG>
+__global__ void __launch_bounds__(kLaneWarps * 32) k_cigar_lanes(CigarArgs g, int c_lo, int c_hi, bool from_list) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr int PPW = 32 / LG;
+  constexpr unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, grp = lane / LG, k = lane % LG;
+  unsigned char *mine = smem + (size_t)(threadIdx.x >> 5) * lanes_warp_bytes<LG>();
+  uint4 *dirs = reinterpret_cast<uint4 *>(mine);
+  uint8_t *A = mine + (size_t)kCigarRowCap * 16 + grp * (kLaneRowsA + kCigarRowCap);
+  uint8_t *B = A + kLaneRowsA;
+  int first = 0, count = 0;
+  if (from_list) {
+    count = g.counts[kCigarEsc + c_lo];
+  } else {
+    for (int c = 0; c <= c_lo; c++) first += g.counts[c];
+    for (int c = c_lo; c <= c_hi; c++) {
+      const int m = g.counts[1 + c];
+      if (m <= kLanesMost) count += m;
+      else if (count == 0) first += m;  // its thread kernel takes it (a following class starts after it)
+    }
+  }
+  const int64_t warps = (int64_t)gridDim.x * kLaneWarps;
+  for (int64_t base = ((int64_t)blockIdx.x * kLaneWarps + (threadIdx.x >> 5)) * PPW; base < count; base += warps * PPW) {
+    const int64_t e = base + grp;
+    bool valid = e < count;
+    int p = 0, w = 0, S = 0;
+    Box bx{};
+    if (valid) {
+      if (from_list) {
+        const int2 ent = g.lists[(int64_t)c_lo * g.list_cap + e];
+        p = ent.x;
+        w = ent.y;
+      } else {
+        p = (int)g.sorted[first + e];
+      }
+      bx = make_box(g, p);
+      if (!from_list) w = abs(bx.ref_len - bx.rows) + 1;
+      S = g.score[p];
+      for (int t = k; t < bx.ref_len; t += LG) A[t] = bx.A[t];
+      for (int t = k; t < bx.rows; t += LG) B[t] = bx.B[t];
+    }
+    __syncwarp();
+    const int all_rows = __reduce_max_sync(full, bx.rows);
+    bool go = valid;
+    for (;;) {  // SSW's doubling: until the band's maximum reaches the score
+      if (go && 2 * w + 1 > LG) {
+        if (k == 0) list_push(g, list_for(w, bx.rows), p, w, bx.rows, bx.ref_len);
+        go = valid = false;
+      }
+      if (!__any_sync(full, go)) break;
+      const int mx = lanes_pass<LG>(g, A, B, bx.rows, bx.ref_len, w, go, k, all_rows, dirs);
+      if (go) {
+        if (mx >= S) go = false;
+        else w *= 2;
+      }
+    }
+    int nops = 0, mism = 0, j_end = 0;
+    bool ok = valid && k == 0;
+    if (ok) {
+      ok = lanes_walk<false>(dirs, grp * LG, A, B, bx, w, 0, &j_end, &nops, &mism, nullptr);
+      int again = 0;
+      if (ok && j_end != 0) ok = lanes_walk<false>(dirs, grp * LG, A, B, bx, w, j_end, &again, &nops, &mism, nullptr);
+      if (!ok) {
+        g.nops[p] = -1;
+        atomicAdd(&g.counts[kCigarWalkErrors], 1);
+      }
+    }
+    const int64_t at = reserve_arena(g, ok ? nops : 0, true);
+    if (ok) {
+      if (at + nops > g.arena_cap) {  // arena full: the host grows it and runs the pass again
+        g.nops[p] = -1;
+        atomicAdd(&g.counts[kCigarArenaFull], 1);
+      } else {
+        lanes_walk<true>(dirs, grp * LG, A, B, bx, w, j_end, nullptr, &nops, nullptr, g.arena + at);
+        g.op_off[p] = at;
+        g.nops[p] = nops;
+        g.mism[p] = mism;
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -949,10 +1175,21 @@ cudaError_t launch_band(const CigarArgs &g, int sms, size_t dirs_bytes, cudaStre
   return cudaGetLastError();
 }
 
+template <int LG>
+cudaError_t launch_lanes(const CigarArgs &g, int sms, int64_t most, int c_lo, int c_hi, bool from_list, cudaStream_t st) {
+  constexpr size_t smem = kLaneWarps * lanes_warp_bytes<LG>();
+  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_cigar_lanes<LG>), smem);
+  if (e) return e;
+  const int64_t need = (most + kLaneWarps * (32 / LG) - 1) / (kLaneWarps * (32 / LG));
+  k_cigar_lanes<LG><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * 4)), kLaneWarps * 32, smem, st>>>(
+      g, c_lo, c_hi, from_list);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_cigar(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const CigarBufs &cb, int sms,
-                         const uint32_t *order, cudaStream_t st, int64_t *launches) {
+                         const uint32_t *order, cudaStream_t st, int64_t *launches, const Forks *fk) {
   const CigarArgs g = make_args(ps, rs, sc, cb);
   k_cigar_reset<<<1, 32, 0, st>>>(cb.counts, cb.cursor);
   const int64_t n = ps.n;
@@ -965,15 +1202,33 @@ cudaError_t launch_cigar(const PairSet &ps, const ResultSet &rs, const Scoring &
                                         13, st);
     if (e) return e;
   }
-  k_cigar_diag<<<sms * 8, 128, 0, st>>>(g);
+  // The classes are independent up to their escalations: diagonal boxes, the lanes kernels
+  // and (where a class can be large enough for it) the thread kernels, which share the
+  // direction scratch and so follow one another, run side by side.
+  const bool fan = fk && fk->fork;
+  if (fan && (e = fork_to(*fk, st, 4))) return e;
+  cudaStream_t cs[4] = {st, st, st, st};
+  if (fan) std::copy(fk->side, fk->side + 4, cs);
+  if ((e = launch_lanes<32>(g, sms, n, 3, 3, false, cs[0]))) return e;
+  if ((e = launch_lanes<16>(g, sms, n, 2, 2, false, cs[1]))) return e;
+  if ((e = launch_lanes<8>(g, sms, n, 0, 1, false, cs[2]))) return e;
+  k_cigar_diag<<<sms * 8, 128, 0, cs[3]>>>(g);
   if ((e = cudaGetLastError())) return e;
-  if ((e = launch_band<0>(g, sms, cb.dirs_bytes, st))) return e;
-  if ((e = launch_band<1>(g, sms, cb.dirs_bytes, st))) return e;
-  if ((e = launch_band<2>(g, sms, cb.dirs_bytes, st))) return e;
-  if ((e = launch_band<3>(g, sms, cb.dirs_bytes, st))) return e;
+  const bool large = n > kLanesMost;
+  if (large) {
+    if ((e = launch_band<0>(g, sms, cb.dirs_bytes, st))) return e;
+    if ((e = launch_band<1>(g, sms, cb.dirs_bytes, st))) return e;
+    if ((e = launch_band<2>(g, sms, cb.dirs_bytes, st))) return e;
+    if ((e = launch_band<3>(g, sms, cb.dirs_bytes, st))) return e;
+  }
+  if (fan && (e = join_from(*fk, st, 4))) return e;
+  // escalated pairs (a list feeds the next class's), then the wide classes
+  if (large && (e = launch_lanes<8>(g, sms, n, 1, 1, true, st))) return e;
+  if ((e = launch_lanes<16>(g, sms, n, 2, 2, true, st))) return e;
+  if ((e = launch_lanes<32>(g, sms, n, 3, 3, true, st))) return e;
   if ((e = launch_band<4>(g, sms, cb.dirs_bytes, st))) return e;
   if ((e = launch_band<5>(g, sms, cb.dirs_bytes, st))) return e;
-  if (launches) *launches += 3 + kCigarClasses + 4;  // + the radix sort's passes (approximate)
+  if (launches) *launches += 2 + 4 + 4 + (large ? 5 : 0) + 4;  // + the radix sort's passes (approximate)
   return cudaSuccess;
 }
 

@@ -541,7 +541,7 @@ mhsw::CigarBufs cigar_bufs(mhsw_driver *d, int64_t n) {
 // (all stream-ordered; part of a captured graph when the batch is captured).
 int enqueue_cigar(mhsw_driver *d, const mhsw::PairSet &ps) {
   MHSW_CK(mhsw::launch_cigar(ps, result_set(d), d->sc, cigar_bufs(d, ps.n), d->sms, d->fwd_order, d->st,
-                              &d->launches),
+                              &d->launches, &d->forks),
           "CIGAR launch");
   MHSW_CK(cudaMemcpyAsync(d->h_ccounts.p, d->c_counts.p, sizeof(int) * mhsw::kCigarCounters, cudaMemcpyDeviceToHost,
                           d->st),
