@@ -24,10 +24,10 @@
 // GB300 mapping.  The band is kept diagonal-indexed (k = j - i + w) so the rows slide without
 // moving data.  Two forms:
 //   lanes (k_cigar_lanes)  a group of 8, 16 or 32 lanes takes a pair, lane k band cell k; the
-//     row's F chain is a prefix maximum over the lanes, the four direction bits of the row's
-//     cells are four ballots, kept with the box's codes in shared memory, where the group's
-//     first lane then walks them.  Half-widths up to 15.  A row costs about 45 warp
-//     instructions whatever the group size, but its chain is ~15x shorter than a thread's
+//     row's F chain is a prefix maximum over the lanes; each lane collects its cells' direction
+//     bits over 32 rows a word, kept with the box's codes in shared memory, where the group's
+//     first lane then walks them, up to 32 diagonal steps at a time.  Half-widths up to 15.  A row costs about 50 warp
+//     instructions whatever the group size, but its chain is far shorter than a thread's
 //     chain over the cells, and a class of up to kLanesMost pairs is bound by that chain.
 //   threads (k_cigar_band) one thread per pair, the band in registers: fewer instructions per
 //     pair, for classes large enough to fill the GPU, and for half-widths 16 and 31.  H and E
@@ -814,69 +814,78 @@ __global__ void __launch_bounds__(128) k_cigar_band(CigarArgs g) {
 
 // ---- lanes form ------------------------------------------------------------------------
 
-constexpr int kLaneRowsA = kCigarRowCap + 32;  // A codes of a box: at most rows + 15 columns
 constexpr int kLaneWarps = 4;
+constexpr int kLanePad = 16;  // the lanes' A reads run past both ends of the box by the band
 
+// One warp's shared memory for boxes of up to `rows` rows (a multiple of 32): four direction
+// words per lane and 32 rows (bit = row), then each group's A and B codes.
 template <int LG>
-__host__ __device__ constexpr size_t lanes_warp_bytes() {  // one warp: direction words of a row, then the groups' codes
-  return (size_t)kCigarRowCap * 16 + (32 / LG) * (size_t)(kLaneRowsA + kCigarRowCap);
+__host__ __device__ constexpr size_t lanes_warp_bytes(int rows) {
+  return (size_t)rows * 16 + (32 / LG) * (size_t)(2 * rows + 4 * kLanePad);
 }
 
 // One banded DP pass at half-width w for the groups with `go`; the same cells, ties and
 // quirks as band_pass.  F along the row as a prefix maximum: with H' = max(E, 0, diagonal),
 // F(k) + k*gE = max(F(kstart) + kstart*gE, max over kstart <= m < k of H'(m) - gO + (m+1)*gE),
-// and F(k) opened where the last term of that maximum exceeds the others.
+// and F(k) opened where the last term of that maximum exceeds the others (that bit is kept
+// by lane k - 1).  Lane k's cells are rows lo .. hi - 1; lanes outside the row's band pass on
+// F's start value, which only reaches lanes right of the band or its first cell.
 template <int LG>
 __device__ int lanes_pass(const CigarArgs &g, const uint8_t *A, const uint8_t *B, int rows, int ref_len, int w, bool go,
-                          int k, int all_rows, uint4 *dirs) {
+                          int k, int all_rows, uint32_t *dirs) {
   constexpr unsigned full = 0xffffffffu;
-  const int gO = g.gO, gE = g.gE;
-  const int up_add = (k + 1) * gE - gO;
-  const unsigned mine = __ballot_sync(full, go);  // lanes whose directions this pass writes
-  int H = 0, E = 0, mx = 0;
-  for (int i = 0; i < all_rows; i++) {
-    const int kstart = max(0, w - i), kend = min(2 * w, ref_len - 1 - i + w);
-    const bool v = go && i < rows && k >= kstart && k <= kend;
-    int hu = __shfl_down_sync(full, H, 1, LG), eu = __shfl_down_sync(full, E, 1, LG);
-    if (k == kend && i >= 1 && i <= w + 1 && ref_len <= i + w) hu = eu = 0;
-    const int a = hu - gO, b = eu - gE;
-    const int e = max(a, b);
-    const int ca = v ? (int)A[i - w + k] : 0, cb = v ? (int)B[i] : 0;
-    const int dg = H + sub_score(g, ca, cb);
-    const int hp = __vimax_s32_relu(e, dg);
-    const int u = v ? hp + up_add : -(1 << 28);
-    int in = u;
+  const int gO = g.gO, gE = g.gE, mt = g.match, xs = -g.mismatch, ns = -g.amb;
+  const int lo = max(0, w - k);
+  const int hi = go && k <= 2 * w ? min(rows, ref_len + w - k) : 0;
+  const unsigned span = hi > lo ? (unsigned)(hi - lo) : 0u;
+  // the row where this lane's cell is the row's last and its upper neighbour reads 0 (the
+  // cleared edge cell), or -1
+  const int edge = ref_len - 1 + w - k;
+  const int clob = edge >= 1 && edge <= w + 1 && k < 2 * w ? edge : -1;
+  const int up_add = (k + 1) * gE - gO, kge = k * gE;
+  const uint8_t *Ak = A + (k - w);
+  int H = 0, E = 0, mx = 0, base = (w - 1) * gE;
+  for (int i0 = 0; i0 < all_rows; i0 += 32) {
+    uint32_t d0 = 0, d1 = 0, d2 = 0, d3 = 0, bit = 1;
+    const int top = min(32, all_rows - i0);
+    for (int r = 0; r < top; r++, bit <<= 1, base -= gE) {
+      const int i = i0 + r;
+      const bool v = (unsigned)(i - lo) < span;
+      int hu = __shfl_down_sync(full, H, 1, LG), eu = __shfl_down_sync(full, E, 1, LG);
+      if (i == clob) hu = eu = 0;
+      const int ca = Ak[i], cb = B[i];
+      const bool same = ca == cb;
+      int sv = same ? mt : xs;
+      if ((ca | cb) & kCodeN) sv = ns;
+      const int a = hu - gO, b = eu - gE;
+      const int e = max(a, b);
+      const int dg = H + sv;
+      const int hp = __vimax_s32_relu(e, dg);
+      const int u = v ? hp + up_add : base;
+      int in = u;
 #pragma unroll
-    for (int o = 1; o < LG; o <<= 1) {
-      const int t = __shfl_up_sync(full, in, o, LG);
-      if (k >= o) in = max(in, t);
-    }
-    const int base = (kstart - 1) * gE;  // F of the row's first cell is -gE (gap open >= gap extend)
-    in = max(in, base);
-    int ex = __shfl_up_sync(full, in, 1, LG);
-    if (k == 0) ex = base;
-    const int f = ex - k * gE;
-    const int m1 = __vimax_s32_relu(e, f);
-    const bool gap = m1 > dg, from_e = e > max(f, 0), same = ca == cb;
-    uint4 d;
-    d.x = __ballot_sync(full, v && a > b);
-    d.y = __ballot_sync(full, v && u > ex) << 1;  // the next cell's F opened
-    d.z = __ballot_sync(full, v && (gap ? from_e : same));
-    d.w = __ballot_sync(full, v && (gap ? !from_e : same));
-    if ((threadIdx.x & 31) == 0) {
-      if (mine != full) {  // keep the other groups' bits
-        const uint4 o = dirs[i];
-        d.x = (d.x & mine) | (o.x & ~mine);
-        d.y = (d.y & mine) | (o.y & ~mine);
-        d.z = (d.z & mine) | (o.z & ~mine);
-        d.w = (d.w & mine) | (o.w & ~mine);
+      for (int o = 1; o < LG; o <<= 1) in = max(in, __shfl_up_sync(full, in, o, LG));
+      int ex = __shfl_up_sync(full, in, 1, LG);
+      if (k == 0) ex = -gE;  // F of the row's first cell (gap open >= gap extend)
+      const int f = ex - kge;
+      const int fr = max(f, 0);
+      const bool gap = max(e, fr) > dg, from_e = e > fr;
+      if (v) {
+        if (a > b) d0 |= bit;
+        if (u > ex) d1 |= bit;
+        if (gap ? from_e : same) d2 |= bit;
+        if (gap ? !from_e : same) d3 |= bit;
+        H = max(hp, f);
+        E = e;
+        mx = max(mx, H);
       }
-      dirs[i] = d;
     }
-    if (v) {
-      H = max(hp, f);
-      E = e;
-      mx = max(mx, H);
+    if (go) {
+      uint32_t *d = dirs + (i0 >> 5) * 128 + (threadIdx.x & 31);
+      d[0] = d0;
+      d[32] = d1;
+      d[64] = d2;
+      d[96] = d3;
     }
   }
 #pragma unroll
@@ -885,27 +894,28 @@ __device__ int lanes_pass(const CigarArgs &g, const uint8_t *A, const uint8_t *B
   return mx;
 }
 
-// The walk over a group's directions (bit sh + k of a row's words).  Counts ops and
-// mismatches or (EMIT) writes the ops to out[0 .. nops) back to front; j_end is the column
-// where it stops.  shift: that column of an earlier walk; where it is not 0, M steps compare
-// the bases shifted by it (see replay_path).
+// The walk over a group's directions (column grp0 + k of the words).  Along a diagonal the
+// rows of one lane lie in one word, so runs of = and of X are counted up to 32 at a time.
+// Counts ops and mismatches or (EMIT) writes the ops to out[0 .. nops) back to front; j_end is
+// the column where it stops.  shift: that column of an earlier walk; where it is not 0, M
+// steps compare the bases shifted by it (see replay_path).
 template <bool EMIT>
-__device__ bool lanes_walk(const uint4 *dirs, int sh, const uint8_t *A, const uint8_t *B, const Box &bx, int w, int shift,
-                           int *j_end, int *nops, int *mism, uint32_t *out) {
+__device__ bool lanes_walk(const uint32_t *dirs, int grp0, const uint8_t *A, const uint8_t *B, const Box &bx, int w,
+                           int shift, int *j_end, int *nops, int *mism, uint32_t *out) {
   int t = 0, mis = 0, rl = 0;
   uint32_t rk = 0;
   auto emit = [&](uint32_t kind, int len) {
     if (EMIT) out[*nops - 1 - t] = ((uint32_t)len << 4) | kind;
     ++t;
   };
-  auto cell = [&](uint32_t kind) {
-    mis += kind != kOpEq;
+  auto cells = [&](uint32_t kind, int n) {
+    if (kind != kOpEq) mis += n;
     if (kind == rk) {
-      ++rl;
+      rl += n;
     } else {
       if (rl > 0) emit(rk, rl);
       rk = kind;
-      rl = 1;
+      rl = n;
     }
   };
   if (bx.tail > 0) emit(kOpS, bx.tail);
@@ -913,17 +923,36 @@ __device__ bool lanes_walk(const uint4 *dirs, int sh, const uint8_t *A, const ui
   while (i > 0) {
     const int k = j - i + w;
     if (j < 0 || k < 0 || k > 2 * w) return false;
-    const uint4 d = dirs[i];
-    const int b = sh + k;
-    const uint32_t hs = ((d.z >> b) & 1u) | (((d.w >> b) & 1u) << 1);
-    const int eff = st != 2 ? st : (hs == 1u ? 0 : hs == 2u ? 1 : 2);
-    if (eff == 2) cell((shift ? A[j - shift] != B[i] : hs != 3u) ? kOpX : kOpEq);
-    else cell(eff == 0 ? kOpI : kOpD);
-    st = eff == 0 ? (((d.x >> b) & 1u) ? 2 : 0) : eff == 1 ? (((d.y >> b) & 1u) ? 2 : 1) : 2;
-    i -= eff != 1;
-    j -= eff != 0;
+    const uint32_t *d = dirs + (i >> 5) * 128 + grp0 + k;
+    const int b = i & 31;
+    if (st == 2) {
+      const uint32_t z = d[64], y = d[96];
+      const bool zb = (z >> b) & 1u, yb = (y >> b) & 1u;
+      if (zb == yb) {  // the diagonal: = (both set) or X (neither)
+        const uint32_t m = zb ? z & y : ~(z | y);
+        const int run = min(min(__clz(~(m << (31 - b))), b + 1), min(i, j + 1));
+        if (shift == 0) {
+          cells(zb ? kOpEq : kOpX, run);
+        } else {
+          for (int r = 0; r < run; r++) cells(A[j - r - shift] != B[i - r] ? kOpX : kOpEq, 1);
+        }
+        i -= run;
+        j -= run;
+        continue;
+      }
+      st = zb ? 0 : 1;  // from E or from F
+    }
+    if (st == 0) {
+      cells(kOpI, 1);
+      if ((d[0] >> b) & 1u) st = 2;
+      --i;
+    } else {
+      cells(kOpD, 1);
+      if (k > 0 && k > w - i && ((d[31] >> b) & 1u)) st = 2;  // lane k - 1's bit; the row's first cell extends
+      --j;
+    }
   }
-  cell(A[0] != B[0] ? kOpX : kOpEq);  // the cell where the walk stopped: one more M
+  cells(A[0] != B[0] ? kOpX : kOpEq, 1);  // the cell where the walk stopped: one more M
   emit(rk, rl);
   if (bx.bb > 0) emit(kOpS, bx.bb);
   if (!EMIT) {
@@ -937,15 +966,16 @@ __device__ bool lanes_walk(const uint4 *dirs, int sh, const uint8_t *A, const ui
 // Pairs of the segments of classes c_lo .. c_hi (none when together they exceed kLanesMost
 // and the thread form takes them), or of class c_lo's escalation list.
 template <int LG>
-__global__ void __launch_bounds__(kLaneWarps * 32) k_cigar_lanes(CigarArgs g, int c_lo, int c_hi, bool from_list) {
+__global__ void __launch_bounds__(kLaneWarps * 32) k_cigar_lanes(CigarArgs g, int c_lo, int c_hi, bool from_list,
+                                                                 int row_cap) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int PPW = 32 / LG;
   constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, grp = lane / LG, k = lane % LG;
-  unsigned char *mine = smem + (size_t)(threadIdx.x >> 5) * lanes_warp_bytes<LG>();
-  uint4 *dirs = reinterpret_cast<uint4 *>(mine);
-  uint8_t *A = mine + (size_t)kCigarRowCap * 16 + grp * (kLaneRowsA + kCigarRowCap);
-  uint8_t *B = A + kLaneRowsA;
+  unsigned char *mine = smem + (size_t)(threadIdx.x >> 5) * lanes_warp_bytes<LG>(row_cap);
+  uint32_t *dirs = reinterpret_cast<uint32_t *>(mine);
+  uint8_t *A = mine + (size_t)row_cap * 16 + grp * (2 * row_cap + 4 * kLanePad) + kLanePad;
+  uint8_t *B = A + row_cap + 3 * kLanePad;
   int first = 0, count = 0;
   if (from_list) {
     count = g.counts[kCigarEsc + c_lo];
@@ -974,6 +1004,11 @@ __global__ void __launch_bounds__(kLaneWarps * 32) k_cigar_lanes(CigarArgs g, in
       bx = make_box(g, p);
       if (!from_list) w = abs(bx.ref_len - bx.rows) + 1;
       S = g.score[p];
+      if (bx.rows > row_cap || bx.ref_len > row_cap) {  // longer than the stated longest A
+        if (k == 0) list_push(g, kCigarClasses, p, w, bx.rows, bx.ref_len);
+        valid = false;
+        bx.rows = bx.ref_len = 0;
+      }
       for (int t = k; t < bx.ref_len; t += LG) A[t] = bx.A[t];
       for (int t = k; t < bx.rows; t += LG) B[t] = bx.B[t];
     }
@@ -1176,20 +1211,23 @@ cudaError_t launch_band(const CigarArgs &g, int sms, size_t dirs_bytes, cudaStre
 }
 
 template <int LG>
-cudaError_t launch_lanes(const CigarArgs &g, int sms, int64_t most, int c_lo, int c_hi, bool from_list, cudaStream_t st) {
-  constexpr size_t smem = kLaneWarps * lanes_warp_bytes<LG>();
+cudaError_t launch_lanes(const CigarArgs &g, int sms, int64_t most, int max_a, int c_lo, int c_hi, bool from_list,
+                         cudaStream_t st) {
+  // a box in these classes has at most 14 rows more than its A columns (8 columns more than rows)
+  const int row_cap = std::min((max_a + 15 + 31) / 32 * 32, kCigarRowCap + 32);
+  const size_t smem = kLaneWarps * lanes_warp_bytes<LG>(row_cap);
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_cigar_lanes<LG>), smem);
   if (e) return e;
   const int64_t need = (most + kLaneWarps * (32 / LG) - 1) / (kLaneWarps * (32 / LG));
-  k_cigar_lanes<LG><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * 4)), kLaneWarps * 32, smem, st>>>(
-      g, c_lo, c_hi, from_list);
+  k_cigar_lanes<LG><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * 8)), kLaneWarps * 32, smem, st>>>(
+      g, c_lo, c_hi, from_list, row_cap);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_cigar(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const CigarBufs &cb, int sms,
-                         const uint32_t *order, cudaStream_t st, int64_t *launches, const Forks *fk) {
+                         const uint32_t *order, int max_a, cudaStream_t st, int64_t *launches, const Forks *fk) {
   const CigarArgs g = make_args(ps, rs, sc, cb);
   k_cigar_reset<<<1, 32, 0, st>>>(cb.counts, cb.cursor);
   const int64_t n = ps.n;
@@ -1209,9 +1247,9 @@ cudaError_t launch_cigar(const PairSet &ps, const ResultSet &rs, const Scoring &
   if (fan && (e = fork_to(*fk, st, 4))) return e;
   cudaStream_t cs[4] = {st, st, st, st};
   if (fan) std::copy(fk->side, fk->side + 4, cs);
-  if ((e = launch_lanes<32>(g, sms, n, 3, 3, false, cs[0]))) return e;
-  if ((e = launch_lanes<16>(g, sms, n, 2, 2, false, cs[1]))) return e;
-  if ((e = launch_lanes<8>(g, sms, n, 0, 1, false, cs[2]))) return e;
+  if ((e = launch_lanes<32>(g, sms, n, max_a, 3, 3, false, cs[0]))) return e;
+  if ((e = launch_lanes<16>(g, sms, n, max_a, 2, 2, false, cs[1]))) return e;
+  if ((e = launch_lanes<8>(g, sms, n, max_a, 0, 1, false, cs[2]))) return e;
   k_cigar_diag<<<sms * 8, 128, 0, cs[3]>>>(g);
   if ((e = cudaGetLastError())) return e;
   const bool large = n > kLanesMost;
@@ -1223,9 +1261,9 @@ cudaError_t launch_cigar(const PairSet &ps, const ResultSet &rs, const Scoring &
   }
   if (fan && (e = join_from(*fk, st, 4))) return e;
   // escalated pairs (a list feeds the next class's), then the wide classes
-  if (large && (e = launch_lanes<8>(g, sms, n, 1, 1, true, st))) return e;
-  if ((e = launch_lanes<16>(g, sms, n, 2, 2, true, st))) return e;
-  if ((e = launch_lanes<32>(g, sms, n, 3, 3, true, st))) return e;
+  if (large && (e = launch_lanes<8>(g, sms, n, max_a, 1, 1, true, st))) return e;
+  if ((e = launch_lanes<16>(g, sms, n, max_a, 2, 2, true, st))) return e;
+  if ((e = launch_lanes<32>(g, sms, n, max_a, 3, 3, true, st))) return e;
   if ((e = launch_band<4>(g, sms, cb.dirs_bytes, st))) return e;
   if ((e = launch_band<5>(g, sms, cb.dirs_bytes, st))) return e;
   if (launches) *launches += 2 + 4 + 4 + (large ? 5 : 0) + 4;  // + the radix sort's passes (approximate)

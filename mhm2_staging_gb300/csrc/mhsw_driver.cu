@@ -207,6 +207,7 @@ struct mhsw_driver {
   bool cigar = false;
   int64_t cigar_n = -1;        // pairs of the last batch whose CIGARs are in the arena
   int64_t cigar_total = -1;    // ops in pair order (after the ordered copy), -1 before it
+  int cigar_max_a = 0;         // longest A of the batch the CIGAR pass runs on
   double cigar_ms = 0;
   int64_t cigar_generic = 0;   // pairs of the last batch that took the generic kernel
   int sms = 152;
@@ -540,8 +541,8 @@ mhsw::CigarBufs cigar_bufs(mhsw_driver *d, int64_t n) {
 // Classification and the register-band kernels, then the counters' copy to the host
 // (all stream-ordered; part of a captured graph when the batch is captured).
 int enqueue_cigar(mhsw_driver *d, const mhsw::PairSet &ps) {
-  MHSW_CK(mhsw::launch_cigar(ps, result_set(d), d->sc, cigar_bufs(d, ps.n), d->sms, d->fwd_order, d->st,
-                              &d->launches, &d->forks),
+  MHSW_CK(mhsw::launch_cigar(ps, result_set(d), d->sc, cigar_bufs(d, ps.n), d->sms, d->fwd_order,
+                              d->cigar_max_a, d->st, &d->launches, &d->forks),
           "CIGAR launch");
   MHSW_CK(cudaMemcpyAsync(d->h_ccounts.p, d->c_counts.p, sizeof(int) * mhsw::kCigarCounters, cudaMemcpyDeviceToHost,
                           d->st),
@@ -1315,6 +1316,7 @@ int mhsw_run_kernel_backwards(mhsw_driver *d, const char *const *reads, const in
     if (d->cigar) {
       rc = ensure_cigar(d, n);
       if (rc) return rc;
+      d->cigar_max_a = d->max_a;
       MHSW_CK(cudaEventRecord(d->ev_c[0], d->st), "event");
       rc = enqueue_cigar(d, ps);
       if (rc) return rc;
@@ -1649,6 +1651,7 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
   if (d->cigar && n > 0) {
     rc = ensure_cigar(d, n);
     if (rc) return rc;
+    d->cigar_max_a = ma;
   }
   // Everything from translation to the result copy, on the handle's stream.
   // Phase events recorded inside a capture become external event nodes, so a replayed
@@ -2032,6 +2035,7 @@ int align_resident(mhsw_driver *d, const PairSet &in, int64_t a_bytes, int max_a
   rc = attach_score2(d, &ps, n, a_bytes);
   if (rc) return rc;
   MHSW_CK(cudaEventRecord(d->ev_t[1], d->st), "event");
+  d->cigar_max_a = max_a;
   d->sig = mhsw::batch_signature(nullptr, ps.n, max_a, max_b);
   const bool both = short_passes(d, n, max_a, max_b, form);
   rc = both ? run_short_passes(d, ps, max_a, max_b) : forward_any(d, ps, max_a, max_b, form);

@@ -159,9 +159,10 @@ struct CigarBufs {           // device buffers of the CIGAR pass
 
 // Classification and the register-band kernels (no host synchronisation).  Pairs left
 // for the generic kernel are in cb.generic (count in cb.counts[kCigarGeneric]).  order
-// (may be null): a pair order to classify in (the batched forward pass's sorted order).
+// (may be null): a pair order to classify in (the forward pass's); max_a: the longest A.
 cudaError_t launch_cigar(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const CigarBufs &cb, int sms,
-                         const uint32_t *order, cudaStream_t st, int64_t *launches, const Forks *fk = nullptr);
+                         const uint32_t *order, int max_a, cudaStream_t st, int64_t *launches,
+                         const Forks *fk = nullptr);
 // Temporary bytes of the (class, rows) sort of n pairs.
 cudaError_t cigar_sort_temp_bytes(int64_t n, size_t *bytes);
 // Generic kernel over `count` entries (device copy), `threads` threads with a slice of
