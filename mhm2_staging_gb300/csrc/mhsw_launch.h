@@ -113,6 +113,10 @@ bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b
 // mode when rs holds its arrays, the others of rs being null when only it is wanted).
 cudaError_t launch_short(const PairSet &ps, const Scoring &sc, int max_a, int max_b, int32_t *out5, const OutViews *ov,
                          const ResultSet *rs, bool a_is_query, cudaStream_t st);
+// The forward pass alone: out3 (n x 3) = score, a_end, b_end; -1 three times for a pair outside
+// max_a or max_b.
+cudaError_t launch_short_forward(const PairSet &ps, const Scoring &sc, int max_a, int max_b, int32_t *out3,
+                                 cudaStream_t st);
 // True when some pair of a batch with these longest sequences can need the int32 pass.
 bool may_need_int32(const Scoring &sc, int ceiling, int max_a, int max_b);
 

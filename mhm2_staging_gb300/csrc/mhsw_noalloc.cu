@@ -8,11 +8,15 @@
 //     and cudaFree may imply, because other streams of the same process must keep
 //     running meanwhile.
 // This entry point serves them.  It computes what the forward pass of the driver
-// computes -- score, A end and B end per pair, bit-exact with SSW -- with one kernel
-// whose every piece of scratch memory (per lane group: the translated A and B codes, the
-// staged B codes and the strip boundary of long A) lives in one file-scope device array
-// of fixed size.  The kernel is a variant of k_fwd<V32, 4, 16> (mhsw_kernels.cu), the
-// int32 wavefront forward kernel, grid-stride over the batch, exact at every score.
+// computes -- score, A end and B end per pair, bit-exact with SSW -- with all its scratch
+// memory in one file-scope device array of fixed size:
+//   short batches   one launch, scratch in shared memory only (mhsw_short.cu);
+//   other batches   the pair order (mhsw_order.cuh, in the array), then the keyed int16 engine
+//                   in persistent kernels whose lane groups claim pairs in that order
+//                   (k_fwd_noalloc16) and translate each pair's codes into their share of the
+//                   array; pairs whose score bound exceeds the int16 keys, and every pair of a
+//                   scoring the keyed engine cannot hold, go to the int32 engine
+//                   (k_fwd_noalloc, a variant of k_fwd<V32, 4, 16>).
 //
 // Nothing here calls cudaMalloc, cudaFree or any library routine that allocates.
 // The first call on a device does a one-time set-up with that device current: it looks
@@ -29,7 +33,9 @@
 
 #include "../../include/mhsw.h"
 #include "mhsw_engine.cuh"
+#include "mhsw_engine16.cuh"
 #include "mhsw_launch.h"
+#include "mhsw_order.cuh"
 
 namespace mhsw {
 namespace {
@@ -69,7 +75,8 @@ __device__ __forceinline__ unsigned na_group_mask() {
   return ((1u << kNaG) - 1u) << ((lane32 / kNaG) * kNaG);
 }
 
-// One kNaG-lane group per pair, grid-stride over [0, n).  Group gid owns bytes
+// One kNaG-lane group per pair, grid-stride over [0, n), or over the items of the pair order
+// from its wide bucket on (order != null).  Group gid owns bytes
 // [gid * stride, (gid + 1) * stride) of the scratch array; the host sizes the grid so
 // that every group's share lies inside it.  Each pair's scratch is written (codes
 // translated, B codes staged, boundary written by strip s before strip s + 1 reads it)
@@ -78,7 +85,8 @@ __global__ void __launch_bounds__(kNaG * kNaGroupsPerBlock)
     k_fwd_noalloc(const char *__restrict__ a_seq, const int64_t *__restrict__ a_off,
                   const int32_t *__restrict__ a_len, const char *__restrict__ b_seq,
                   const int64_t *__restrict__ b_off, const int32_t *__restrict__ b_len, int64_t n, Scoring sc,
-                  int max_a, int max_b, unsigned char *scratch, NaLayout lay, int32_t *__restrict__ out3) {
+                  int max_a, int max_b, unsigned char *scratch, NaLayout lay, const uint32_t *order, const int *wide_first,
+                  int32_t *__restrict__ out3) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr size_t kProf = group_prof_bytes<V32, kNaK, kNaG>();
   const int gpb = blockDim.x / kNaG;
@@ -99,7 +107,8 @@ __global__ void __launch_bounds__(kNaG * kNaGroupsPerBlock)
   gs.pad = lay.pad;
   gs.bcap = lay.bcap;
 
-  for (int64_t i = gid; i < n; i += gstride) {
+  for (int64_t it = (order ? *wide_first : 0) + gid; it < n; it += gstride) {
+    const int64_t i = order ? (int64_t)order[it] : it;
     const int M = a_len[i], N = b_len[i];
     if (M < 0 || N < 0 || M > max_a || N > max_b) {  // outside the stated maxima
       if (lane == 0) {
@@ -136,7 +145,89 @@ __global__ void __launch_bounds__(kNaG * kNaGroupsPerBlock)
   }
 }
 
+// Keyed engine over one range of the pair order: G-lane groups claim items of the short-read
+// buckets (G = 8) or of the longer ones up to the wide bucket (G = 16) and translate a pair's
+// A and B into their share of the scratch array.  50,000 mixed reads (5.1e9 cells): 7.14 -> 1.34 ms
+// a call against the int32 engine in input order, whose shares and registers let 372 blocks run.
+template <int G, bool HALF>
+__global__ void __launch_bounds__(128)
+    k_fwd_noalloc16(PairSet ps, Scoring sc, int max_a, int max_b, int lane_rows, const uint32_t *__restrict__ order,
+                    int *queue, const int *first, unsigned char *scratch, size_t share, size_t a_cap, size_t b_cap,
+                    int32_t *__restrict__ out3) {
+  constexpr bool kShort = G == kGKShort;
+  constexpr int kPer = kShort ? 10 : 8;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int grp = threadIdx.x / G, lane = threadIdx.x % G;
+  const unsigned gmask = ((1u << G) - 1u) << (((threadIdx.x & 31) / G) * G);
+  GroupSmem gs;
+  gs.prof = reinterpret_cast<uint32_t *>(smem + (size_t)grp * group_prof16_bytes<kPer, G>());
+  gs.prof_lanes = G;
+  gs.bcodes = nullptr;
+  gs.pad = 0;
+  gs.bcap = 0;
+  unsigned char *mine = scratch + ((size_t)blockIdx.x * (128 / G) + grp) * share;
+  uint8_t *ac = mine, *bc = mine + a_cap;
+  V16::Pay *bnd = reinterpret_cast<V16::Pay *>(mine + a_cap + b_cap);
+  const int lo = kShort ? 0 : queue[2], hi = kShort ? queue[2] : first[kBucketWide];
+  auto translate = [&](uint8_t *dst, const char *src, int len) {
+    int x = lane;
+    for (; x + 3 * G < len; x += 4 * G) {  // four loads in flight
+      const uint8_t v0 = (uint8_t)src[x], v1 = (uint8_t)src[x + G], v2 = (uint8_t)src[x + 2 * G], v3 = (uint8_t)src[x + 3 * G];
+      dst[x] = c_code[v0];
+      dst[x + G] = c_code[v1];
+      dst[x + 2 * G] = c_code[v2];
+      dst[x + 3 * G] = c_code[v3];
+    }
+    for (; x < len; x += G) dst[x] = c_code[(uint8_t)src[x]];
+  };
+  for (;;) {
+    int claim = 0;
+    if (lane == 0) claim = atomicAdd(queue + (kShort ? 0 : 1), 1);
+    claim = __shfl_sync(gmask, claim, 0, G);
+    if (lo + claim >= hi) break;
+    const int64_t p = order[lo + claim];
+    const int M = ps.a_len[p], N = ps.b_len[p];
+    int r[3] = {0, -1, 0};
+    if (M < 0 || N < 0 || M > max_a || N > max_b) {  // outside the stated maxima
+      r[0] = r[2] = -1;
+    } else if (M > 0 && N > 0) {
+      translate(ac, ps.a_seq + ps.a_off[p], M);
+      translate(bc, ps.b_seq + ps.b_off[p], N);
+      __syncwarp(gmask);
+      SeqView A{ac, 1, M}, B{bc, 1, N};
+      SweepOut so;
+      const int bucket = bucket_of(M, N, sc, lane_rows, false);
+      if constexpr (kShort) {
+        switch (bucket) {
+          case 0: sweep16<4, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+          case 1: sweep16<6, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+          case 2: sweep16<8, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+          default: sweep16<10, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+        }
+      } else {
+        if (bucket == 4) sweep16<6, G, false, HALF>(A, B, sc, gs, lane, gmask, bnd, INT_MAX, so);
+        else sweep16<8, G, false, HALF>(A, B, sc, gs, lane, gmask, bnd, INT_MAX, so);
+      }
+      r[0] = key_value(so.key);
+      if (r[0] > 0) {
+        r[1] = key_row(so.key);
+        r[2] = key_col(so.key);
+      }
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) out3[3 * p + k] = r[k];
+    }
+    __syncwarp(gmask);  // the next pair overwrites this pair's codes
+  }
+}
+
+constexpr size_t na16_smem_short() { return 16 * group_prof16_bytes<10, kGKShort>(); }
+constexpr size_t na16_smem_long() { return 8 * group_prof16_bytes<8, kGKLong>(); }
+constexpr int64_t kNaChunk = 2 << 20;  // pairs ordered at once (their order takes 8 MiB of the array)
+
 struct NaDevice {
+  int occ_short = 1, occ_long = 1;
   bool ready = false;
   unsigned char *scratch = nullptr;
   int sms = 0;
@@ -180,6 +271,17 @@ int na_setup(int dev, NaDevice **out, char *errbuf, size_t errlen) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fwd_noalloc, kNaG * kNaGroupsPerBlock, smem);
     if (e != cudaSuccess)
       return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
+    // limits and occupancy of the keyed kernels and the order's, so later calls only launch
+    for (auto k : {k_fwd_noalloc16<kGKLong, false>, k_fwd_noalloc16<kGKLong, true>}) {
+      if ((e = raise_smem_limit(reinterpret_cast<const void *>(k), na16_smem_long())) ||
+          (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_long, k, 128, na16_smem_long())))
+        return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "keyed kernel set-up: %s", cudaGetErrorString(e));
+    }
+    if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_fwd_noalloc16<kGKShort, false>), na16_smem_short())) ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_short, k_fwd_noalloc16<kGKShort, false>, 128,
+                                                           na16_smem_short())) ||
+        (e = raise_smem_limit(reinterpret_cast<const void *>(k_order_place), 2 * sizeof(int) * kOrderBins)))
+      return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "keyed kernel set-up: %s", cudaGetErrorString(e));
     d.scratch = static_cast<unsigned char *>(p);
     d.sms = sms;
     d.blocks_per_sm = occ > 0 ? occ : 1;
@@ -232,17 +334,78 @@ extern "C" int mhsw_forward_noalloc(const mhsw_pairs *pairs, short match_score, 
   int rc = na_setup(dev, &d, errbuf, errlen);
   if (rc) return rc;
 
-  // Block size: kNaGroupsPerBlock groups, or fewer when the scratch holds fewer groups.
-  const int gpb = (int)std::min<int64_t>(kNaGroupsPerBlock, fit);
-  int64_t blocks = std::min<int64_t>(fit / gpb, (int64_t)d->sms * d->blocks_per_sm);
-  blocks = std::min<int64_t>(blocks, (n + gpb - 1) / gpb);
-  if (blocks < 1) blocks = 1;
-  // blocks * gpb <= fit: the last group's share ends inside the scratch array.
-  const size_t smem = (size_t)gpb * group_prof_bytes<V32, kNaK, kNaG>();
-  k_fwd_noalloc<<<(unsigned)blocks, gpb * kNaG, smem, static_cast<cudaStream_t>(stream)>>>(
-      pairs->a_seq, pairs->a_off, pairs->a_len, pairs->b_seq, pairs->b_off, pairs->b_len, n, sc, max_a, max_b,
-      d->scratch, lay, out3);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  PairSet ps{};
+  ps.a_seq = pairs->a_seq;
+  ps.a_off = pairs->a_off;
+  ps.a_len = pairs->a_len;
+  ps.b_seq = pairs->b_seq;
+  ps.b_off = pairs->b_off;
+  ps.b_len = pairs->b_len;
+  ps.n = n;
+  auto launch_fail = [&](cudaError_t err) {
+    return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "launch: %s", cudaGetErrorString(err));
+  };
+  const int ceiling = kCeiling16;
+  if (short_batch(sc, ceiling, n, max_a, max_b)) {
+    if ((e = launch_short_forward(ps, sc, max_a, max_b, out3, st))) return launch_fail(e);
+    return MHSW_OK;
+  }
+  // int32 engine over n pairs in input order (order null) or the order's wide bucket, with the
+  // scratch array from `at` on
+  auto run32 = [&](const PairSet &q, int64_t m, size_t at, const uint32_t *order, const int *wide_first, int32_t *out) {
+    const int64_t room = (int64_t)((kNoAllocScratchBytes - at) / lay.stride);  // lane groups whose scratch fits
+    // Block size: kNaGroupsPerBlock groups, or fewer when the scratch holds fewer groups.
+    const int gpb = (int)std::min<int64_t>(kNaGroupsPerBlock, room);
+    int64_t blocks = std::min<int64_t>(room / gpb, (int64_t)d->sms * d->blocks_per_sm);
+    blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, (m + gpb - 1) / gpb));
+    // blocks * gpb <= room: the last group's share ends inside the scratch array.
+    const size_t smem = (size_t)gpb * group_prof_bytes<V32, kNaK, kNaG>();
+    k_fwd_noalloc<<<(unsigned)blocks, gpb * kNaG, smem, st>>>(q.a_seq, q.a_off, q.a_len, q.b_seq, q.b_off, q.b_len, m, sc,
+                                                              max_a, max_b, d->scratch + at, lay, order, wide_first, out);
+    return cudaGetLastError();
+  };
+  // Keyed engine: the array holds the order's control block and the order of a chunk, then the
+  // shares (codes, and the strip boundary of A above 256 rows).
+  const int64_t chunk = std::min<int64_t>(n, kNaChunk);
+  const size_t head = round_up(kOrderCtl * sizeof(int) + (size_t)chunk * sizeof(uint32_t), 256);
+  const size_t a_cap = round_up((size_t)max_a, 16), b_cap = round_up((size_t)max_b, 16);
+  const size_t share = a_cap + b_cap + (max_a > 256 ? round_up((size_t)max_b * sizeof(V16::Pay), 16) : 0);
+  const int64_t room = (int64_t)((kNoAllocScratchBytes - head) / share);
+  const bool wide = may_need_int32(sc, ceiling, max_a, max_b);
+  if (!keyed_scoring(sc) || room < 16 || (wide && kNoAllocScratchBytes - head < lay.stride)) {
+    if ((e = run32(ps, n, 0, nullptr, nullptr, out3))) return launch_fail(e);
+    return MHSW_OK;
+  }
+  int *ctl = reinterpret_cast<int *>(d->scratch);
+  uint32_t *order = reinterpret_cast<uint32_t *>(ctl + kOrderCtl);
+  unsigned char *shares = d->scratch + head;
+  const bool half = (long long)std::min(max_a, max_b) * sc.match <= kHalfCap;
+  auto klong = half ? k_fwd_noalloc16<kGKLong, true> : k_fwd_noalloc16<kGKLong, false>;
+  for (int64_t at = 0; at < n; at += chunk) {
+    PairSet q = ps;
+    q.n = std::min(chunk, n - at);
+    q.a_off += at;
+    q.a_len += at;
+    q.b_off += at;
+    q.b_len += at;
+    // as in the plain form: 16-lane groups for all while a batch does not fill them
+    const int lane_rows = q.n <= (int64_t)d->sms * 64 ? 0 : 160;
+    if ((e = order_pairs(q, sc, lane_rows, false, q.n, 1, ctl, order, d->sms, st, nullptr, max_a,
+                         max_b)))
+      return launch_fail(e);
+    auto grid_of = [&](int occ, int gpb) {
+      const int64_t b = std::min<int64_t>((int64_t)d->sms * occ, (q.n + gpb - 1) / gpb);
+      return (unsigned)std::min<int64_t>(b, room / gpb);
+    };
+    if (max_a > lane_rows)
+      klong<<<grid_of(d->occ_long, 8), 128, na16_smem_long(), st>>>(q, sc, max_a, max_b, lane_rows, order, ctl, ctl + 8,
+                                                                   shares, share, a_cap, b_cap, out3 + 3 * at);
+    if (lane_rows > 0)
+      k_fwd_noalloc16<kGKShort, false><<<grid_of(d->occ_short, 16), 128, na16_smem_short(), st>>>(
+          q, sc, max_a, max_b, lane_rows, order, ctl, ctl + 8, shares, share, a_cap, b_cap, out3 + 3 * at);
+    if ((e = cudaGetLastError())) return launch_fail(e);
+    if (wide && (e = run32(q, q.n, head, order, ctl + 8 + kBucketWide, out3 + 3 * at))) return launch_fail(e);
+  }
   return MHSW_OK;
 }

@@ -45,6 +45,7 @@ struct ShortArgs {
   int max_a, max_b;
   int prof_bytes;
   int32_t *out5;  // n x 5, or null
+  int32_t *out3;  // n x 3 (score, a_end, b_end), or null: forward pass only
   OutViews ov;    // drop-in views (null pointers: not written)
   ResultSet rs;   // the general path's result arrays (null pointers: not written)
   bool a_is_query;
@@ -232,6 +233,12 @@ __device__ __forceinline__ int16_t short_of(int v) {
 }
 
 __device__ __forceinline__ void write_result(const ShortArgs &g, int64_t p, const int (&r)[5]) {
+  if (g.out3) {
+    g.out3[3 * p] = r[0];
+    g.out3[3 * p + 1] = r[2];
+    g.out3[3 * p + 2] = r[4];
+    return;
+  }
   if (g.out5) {
 #pragma unroll
     for (int k = 0; k < 5; k++) g.out5[5 * p + k] = r[k];
@@ -305,10 +312,12 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
         warp_score2(rowmax, M, S > 0 ? key_row(k) : -1, word, lane, s2, s2_at);
       }
       if (S > 0) {
-        const int ie = key_row(k), je = key_col(k);
         r[0] = S;
-        r[2] = ie;
-        r[4] = je;
+        r[2] = key_row(k);
+        r[4] = key_col(k);
+      }
+      if (S > 0 && !g.out3) {
+        const int ie = r[2], je = r[4];
         const int M2 = ie + 1, N2 = je + 1;
         // the reversed box's first t rows and the columns reachable within them, N codes
         // around them
@@ -335,6 +344,7 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
         r[3] = je - key_col(q);
       }
     }
+    if (g.out3 && (M < 0 || N < 0 || M > g.max_a || N > g.max_b)) r[0] = r[2] = r[4] = -1;  // outside the stated maxima
     if (lane == 0) {
       write_result(g, p, r);
       if constexpr (S2) {
@@ -353,9 +363,22 @@ bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b
          !may_need_int32(sc, ceiling, max_a, max_b);
 }
 
+static cudaError_t launch(ShortArgs g, cudaStream_t st) {
+  if (g.ps.n <= 0) return cudaSuccess;
+  const bool small = g.max_a <= 256, s2 = g.rs.score2 != nullptr;
+  g.prof_bytes = (int)(s2 ? (small ? Prof16<4, kCode16Zero + 1>::bytes(32) : Prof16<8, kCode16Zero + 1>::bytes(32))
+                          : (small ? Prof16<4>::bytes(32) : Prof16<8>::bytes(32)));
+  const size_t smem =
+      ((size_t)g.prof_bytes + (s2 ? (small ? 512 : 1024) + 16 : 0) + 2 * kShortPad + (size_t)g.max_b + 15) / 16 * 16;
+  auto kern = s2 ? (small ? k_short<4, true> : k_short<8, true>) : (small ? k_short<4, false> : k_short<8, false>);
+  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+  if (e != cudaSuccess) return e;
+  kern<<<(unsigned)g.ps.n, 32, smem, st>>>(g);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_short(const PairSet &ps, const Scoring &sc, int max_a, int max_b, int32_t *out5, const OutViews *ov,
                          const ResultSet *rs, bool a_is_query, cudaStream_t st) {
-  if (ps.n <= 0) return cudaSuccess;
   ShortArgs g{};
   g.ps = ps;
   g.sc = sc;
@@ -363,17 +386,20 @@ cudaError_t launch_short(const PairSet &ps, const Scoring &sc, int max_a, int ma
   g.max_b = max_b;
   g.out5 = out5;
   if (ov) g.ov = *ov;
-  g.rs = rs ? *rs : ResultSet{};
+  if (rs) g.rs = *rs;
   g.a_is_query = a_is_query;
-  const bool small = max_a <= 256, s2 = g.rs.score2 != nullptr;
-  g.prof_bytes = (int)(s2 ? (small ? Prof16<4, kCode16Zero + 1>::bytes(32) : Prof16<8, kCode16Zero + 1>::bytes(32))
-                          : (small ? Prof16<4>::bytes(32) : Prof16<8>::bytes(32)));
-  const size_t smem = ((size_t)g.prof_bytes + (s2 ? (small ? 512 : 1024) + 16 : 0) + 2 * kShortPad + (size_t)max_b + 15) / 16 * 16;
-  auto kern = s2 ? (small ? k_short<4, true> : k_short<8, true>) : (small ? k_short<4, false> : k_short<8, false>);
-  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)ps.n, 32, smem, st>>>(g);
-  return cudaGetLastError();
+  return launch(g, st);
+}
+
+cudaError_t launch_short_forward(const PairSet &ps, const Scoring &sc, int max_a, int max_b, int32_t *out3,
+                                 cudaStream_t st) {
+  ShortArgs g{};
+  g.ps = ps;
+  g.sc = sc;
+  g.max_a = max_a;
+  g.max_b = max_b;
+  g.out3 = out3;
+  return launch(g, st);
 }
 
 }  // namespace mhsw
