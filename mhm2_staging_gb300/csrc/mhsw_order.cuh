@@ -37,6 +37,12 @@ __device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int la
   return b;
 }
 
+// Buckets of the protein kernels: A up to 128/192/256 rows (16-lane groups, K = 4/6/8), up to
+// 384/512 (32-lane groups, K = 6/8), longer (strips of 512).
+__host__ __device__ constexpr int protein_bucket(int M) {
+  return M <= 128 ? 0 : M <= 192 ? 1 : M <= 256 ? 2 : M <= 384 ? 4 : M <= 512 ? 5 : kBucketStrip;
+}
+
 // ---- pair order: a counting sort over (bucket, class of len B, longest first) ---------
 // Length classes are single columns below 1024 and 1/64 of an octave (1.6%) above, so the
 // lane groups of a warp see equal B lengths, which is all the order is for (classes of 4
@@ -67,12 +73,13 @@ struct OrderArgs {
   int *hist, *cursor; // kOrderBins each (zeroed before the two-launch form)
   uint32_t *order;
   int max_a, max_b;   // pairs longer than these go with the empty ones
+  bool protein;       // buckets by protein_bucket (sc unused)
 };
 
 __device__ __forceinline__ int order_bin(const OrderArgs &g, int64_t p) {
   const int M = g.ps.a_len[p], N = g.ps.b_len[p];
   const int b = (M <= 0 || N <= 0 || M > g.max_a || N > g.max_b) ? (g.lane_rows > 0 ? 0 : kBucketFirstLong)
-                                   : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16);
+                : g.protein ? protein_bucket(M) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16);
   return b * kLenBins + len_class(N);
 }
 
@@ -187,9 +194,9 @@ constexpr size_t kOrderCtl = kOrderHead + 2 * kOrderBins;
 // Orders m items (pair i * stride) into `order`; clears the claim counters.
 inline cudaError_t order_pairs(const PairSet &ps, const Scoring &sc, int lane_rows, bool wide_try16, int64_t m,
                                int64_t stride, int *ctl, uint32_t *order, int sms, cudaStream_t st, int64_t *launches,
-                               int max_a = INT_MAX, int max_b = INT_MAX) {
+                               int max_a = INT_MAX, int max_b = INT_MAX, bool protein = false) {
   OrderArgs g{ps, sc, lane_rows, wide_try16, m, stride, ctl, ctl + 8, ctl + kOrderHead, ctl + kOrderHead + kOrderBins,
-              order, max_a, max_b};
+              order, max_a, max_b, protein};
   if (m <= kOrderOneBlock) {
     k_order_one<<<1, 1024, 0, st>>>(g);
     if (launches) *launches += 1;

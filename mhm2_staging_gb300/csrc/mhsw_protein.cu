@@ -8,12 +8,19 @@
 // extended at gap_extend), end = the lexicographically smallest (A row, B column) holding
 // it, begin = the same rule on the reversed prefixes A[0..a_end], B[0..b_end].
 //
-// GB300 mapping: one warp per pair, lanes along A (K rows a lane, 32K rows a strip), B's
+// GB300 mapping: the keyed int16 wavefront of mhsw_engine16.cuh (k_protein16) -- a group of 16
+// lanes (A up to 256 rows) or 32 takes a pair, forward and begin sweep, claiming pairs in
+// length order.  The substitution scores of a lane's rows are bytes: one 128-bit shared load per
+// step gives the column's scores for all of them, and one byte permute per cell pair spreads two
+// of them into the halves of a word (a 24-code table of words, as the DNA engine's, would leave
+// room for 4 warps an SM).  Pairs whose score leaves the keys (4032), and matrices whose
+// scores do not fit the bytes (below -gap open, or above 127 - gap open), take the int32
+// kernels: one warp per pair, lanes along A (K rows a lane, 32K rows a strip), B's
 // columns swept as a skewed wavefront -- lane l works on column t - l at step t and hands
 // its bottom row's H and E to lane l + 1 by shuffle; strips hand their last row to the next
 // through a per-warp global row.  int32 cells with DPX add-max / 3-way relu-max; the
 // scoring matrix sits in shared memory, indexed by the row's code * 24 + the column's code.
-// The begin pass is the same kernel on reversed views of the prefixes ending at the ends.
+// The begin pass is the same sweep on reversed views of the prefixes ending at the ends.
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
@@ -21,9 +28,12 @@
 
 #include "../../include/mhsw.h"
 #include "mhsw_internal.h"
+#include "mhsw_engine16.cuh"
 #include "mhsw_launch.h"
+#include "mhsw_order.cuh"
 #include "mhsw_types.h"
 
+namespace mhsw {
 namespace {
 
 constexpr int kAA = 24;              // matrix dimension
@@ -32,21 +42,38 @@ constexpr int kPK = 8;               // rows per lane
 constexpr int kPRows = 32 * kPK;     // rows per strip
 constexpr int kNegBig = -(1 << 28);  // "minus infinity" for E and F at the borders
 
-// bytes -> codes (0..23); any byte >= 91 or encoded outside [0, 24) sets *bad and gets 0
-__global__ void k_protein_encode(const char *__restrict__ src, uint8_t *__restrict__ dst, int64_t nbytes,
+// bytes -> codes (0..23) of both arenas; any byte >= 91 or encoded outside [0, 24) sets *bad
+// and gets 0.  Four bytes a step where source and destination are aligned.
+__global__ void k_protein_encode(const char *__restrict__ a, uint8_t *__restrict__ ac, int64_t na,
+                                 const char *__restrict__ b, uint8_t *__restrict__ bc, int64_t nb,
                                  const int16_t *__restrict__ enc, int *bad) {
-  __shared__ int16_t senc[kEnc];
-  for (int k = threadIdx.x; k < kEnc; k += blockDim.x) senc[k] = enc[k];
-  __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nbytes; i += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned char c = (unsigned char)src[i];
-    int v = c < kEnc ? senc[c] : -1;
-    if (v < 0 || v >= kAA) {
-      atomicOr(bad, 1);
-      v = 0;
-    }
-    dst[i] = (uint8_t)v;
+  __shared__ uint8_t tab[256];
+  for (int k = threadIdx.x; k < 256; k += blockDim.x) {
+    const int v = k < kEnc ? enc[k] : -1;
+    tab[k] = (uint8_t)(v < 0 || v >= kAA ? 0xff : v);
   }
+  __syncthreads();
+  bool wrong = false;
+  auto one = [&](unsigned c) -> unsigned {
+    const unsigned v = tab[c];
+    wrong |= v == 0xff;
+    return v == 0xff ? 0u : v;
+  };
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int side = 0; side < 2; side++) {
+    const char *src = side ? b : a;
+    uint8_t *dst = side ? bc : ac;
+    const int64_t n = side ? nb : na;
+    const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 3) == 0;
+    const int64_t words = vec ? n / 4 : 0;
+    for (int64_t i = tid; i < words; i += step) {
+      const uint32_t w = reinterpret_cast<const uint32_t *>(src)[i];
+      reinterpret_cast<uint32_t *>(dst)[i] =
+          one(w & 0xff) | (one((w >> 8) & 0xff) << 8) | (one((w >> 16) & 0xff) << 16) | (one(w >> 24) << 24);
+    }
+    for (int64_t i = words * 4 + tid; i < n; i += step) dst[i] = (uint8_t)one((unsigned char)src[i]);
+  }
+  if (wrong) atomicOr(bad, 1);
 }
 
 struct PArgs {
@@ -60,7 +87,259 @@ struct PArgs {
   int32_t *a_beg, *b_beg;          // begins written
   int2 *rows;                      // per warp slot: H, E of a strip's last row (max_n each)
   int64_t max_n;
+  const uint32_t *list;            // int32 kernels: the pairs to take (null: all n)
+  const int *list_n;
 };
+
+// ---- keyed int16 kernels ------------------------------------------------------------------
+
+constexpr int kPadCol = kAA;                 // code of columns outside B: scores -gap open
+constexpr int kPCodes = kAA + 1;
+constexpr int kPWords = (kPCodes + 3) / 4;   // words of one row code's biased scores
+
+struct P16Args {
+  PArgs p;
+  const uint32_t *order;
+  int *ctl;                        // the order's control block
+  uint32_t *bound;                 // per group: strip boundary (max_n words; lo H, hi E^)
+  uint32_t *over;                  // pairs whose score left the keys
+  int *over_n;
+  int wide_from;                   // min(M, N) from which a pair goes straight to int32
+};
+
+// One step (Step16 of mhsw_engine16.cuh) with byte scores: lo words of this step's column, hi
+// words of the previous one.  Bytes are below 128, so the permute's sign bytes are zeros.
+template <int K>
+struct StepP {
+  static constexpr uint32_t kKeyMask = KeyBits<K>::kMask;
+  __device__ static __forceinline__ void run(int t, uint32_t zH, uint32_t zE, uint32_t sel, uint32_t l0, uint32_t l1,
+                                             uint32_t p0, uint32_t p1, uint32_t (&H)[K], uint32_t (&F)[K],
+                                             uint32_t &Hlast, uint32_t &Ecout, uint32_t &HtopPrev, uint32_t &Kl,
+                                             uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t one, uint32_t eight) {
+    uint32_t Ev = prmt_sel(zE, Ecout, sel);
+    const uint32_t Htop = prmt_sel(zH, Hlast, sel);
+    uint32_t Hd = HtopPrev;
+    HtopPrev = Htop;
+    uint32_t key[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t i = k & 3;
+      const uint32_t W = prmt_sel(k < 4 ? l0 : l1, k < 4 ? p0 : p1, i | ((8 | i) << 4) | ((4 + i) << 8) | ((12 + i) << 12));
+      const uint32_t Q = mad_u32(Hd, one, W);
+      const uint32_t m = __vimax3_s16x2(Q, Ev, F[k]);
+      const uint32_t Hn = __viaddmax_s16x2_relu(m, NGO, 0u);
+      Ev = __viaddmax_s16x2(Ev, NGE, Hn);
+      F[k] = __viaddmax_s16x2(F[k], NGE, Hn);
+      Hd = H[k];
+      H[k] = Hn;
+      key[k] = mad_u32(Hn, eight, (uint32_t)(kKeyMask - k) * 0x00010001u);
+    }
+    uint32_t Kn = Kl;
+#pragma unroll
+    for (int k = 0; k < K; k += 2) Kn = __vimax3_s16x2(Kn, key[k], key[k + 1]);
+    Hlast = H[K - 1];
+    Ecout = Ev;
+    const uint32_t msk = sign_mask16(Kn - Kl + 0x7fff7fffu);
+    const uint32_t tt = (uint32_t)t * 0x00010001u;
+    Jp = (msk & tt) | (~msk & Jp);
+    Kl = Kn;
+  }
+};
+
+// Sweep of A (a[adir * i], i < M) over B (b[bdir * j], j < N): the best key, and whether the
+// score left the keys.  MULTI: A in strips of 2*K*G rows, the boundary row in bnd.
+template <int K, int G, bool MULTI>
+__device__ unsigned long long protein_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, int bdir, int N,
+                                            const uint32_t *rowtab, uint4 *tab, int lane, unsigned gmask, uint32_t *bnd,
+                                            uint32_t NGE, uint32_t NGO, uint32_t one, int &overflow) {
+  constexpr int KB = KeyBits<K>::kBits;
+  constexpr uint32_t KMASK = KeyBits<K>::kMask;
+  using ST = StepP<K>;
+  const uint32_t scale = one << KB;
+  const int nstrips = MULTI ? (M + 2 * K * G - 1) / (2 * K * G) : 1;
+  const int T_end = N + 2 * G - 1;
+  unsigned long long best = 0ull;
+  overflow = 0;
+  for (int s = 0; s < nstrips; s++) {
+    const int row0 = s * 2 * K * G + lane * 2 * K;
+    __syncwarp(gmask);
+    // the strip's table: for four rows at a time, their scores against four codes are
+    // transposed to one word per code
+    {
+      uint32_t *tw = reinterpret_cast<uint32_t *>(tab);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {  // words: lo rows 0-3, 4-7, hi rows 0-3, 4-7
+        if ((q & 1) * 4 >= K) continue;
+        const int r0 = row0 + (q >= 2 ? K : 0) + (q & 1) * 4;
+        const uint32_t *rw[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) rw[x] = rowtab + (r0 + x < M ? (int)a[adir * (r0 + x)] : kAA) * kPWords;
+        for (int c = 0; c < kPWords; c++) {
+          const uint32_t w0 = rw[0][c], w1 = rw[1][c], w2 = rw[2][c], w3 = rw[3][c];
+          const uint32_t x0 = __byte_perm(w0, w1, 0x5140), x1 = __byte_perm(w2, w3, 0x5140);  // codes 0, 1
+          const uint32_t y0 = __byte_perm(w0, w1, 0x7362), y1 = __byte_perm(w2, w3, 0x7362);  // codes 2, 3
+          uint32_t *o = tw + ((4 * c) * G + lane) * 4 + q;
+          o[0] = __byte_perm(x0, x1, 0x5410);
+          if (4 * c + 1 < kPCodes) o[4 * G] = __byte_perm(x0, x1, 0x7632);
+          if (4 * c + 2 < kPCodes) o[8 * G] = __byte_perm(y0, y1, 0x5410);
+          if (4 * c + 3 < kPCodes) o[12 * G] = __byte_perm(y0, y1, 0x7632);
+        }
+      }
+    }
+    __syncwarp(gmask);
+    const bool first = s == 0, last = s == nstrips - 1;
+    uint32_t H[K], F[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) H[k] = F[k] = 0u;
+    uint32_t p0 = 0u, p1 = 0u;  // the previous column's hi scores (before column 0: -gap open)
+    uint32_t Hlast = 0u, Ecout = 0u, HtopPrev = 0u, Kl = 0u, Jp = 0u;
+    const uint32_t sel = lane == 0 && first ? 0x54BBu : 0x5432u;
+    const int j0 = -2 * lane;
+    auto code_at = [&](int j) -> int { return (unsigned)j < (unsigned)N ? (int)b[bdir * j] : kPadCol; };
+    const uint8_t *bl = b + bdir * j0;
+    int ceven = code_at(j0), codd = code_at(j0 + 1);
+    int t = 0;
+    auto step = [&](int tt, int c) {
+      const uint4 v = tab[c * G + lane];
+      uint32_t zH = __shfl_up_sync(gmask, Hlast, 1, G), zE = __shfl_up_sync(gmask, Ecout, 1, G);
+      if (MULTI && lane == 0 && !first) {
+        const uint32_t w = tt < N ? bnd[tt] : 0u;
+        zH = __byte_perm(w, 0u, 0x1000);
+        zE = w;
+      }
+      ST::run(tt, zH, zE, sel, v.x, v.y, p0, p1, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale);
+      p0 = v.z;
+      p1 = v.w;
+      if (MULTI && !last && lane == G - 1) {
+        const int jh = tt - 2 * lane - 1;
+        if (jh >= 0 && jh < N) bnd[jh] = __byte_perm(Hlast, Ecout, 0x7632);
+      }
+    };
+    auto two = [&](auto guarded) {
+      constexpr bool kGuard = decltype(guarded)::value;
+      int c = ceven;
+      ceven = kGuard ? code_at(t + 2 + j0) : (int)bl[bdir * (t + 2)];
+      step(t, c);
+      c = codd;
+      codd = kGuard ? code_at(t + 3 + j0) : (int)bl[bdir * (t + 3)];
+      step(t + 1, c);
+    };
+    // (the phases of sweep16_impl; an odd step count runs one step more over pad columns)
+    for (; t < T_end && t < 2 * G - 4; t += 2) two(std::true_type{});
+    for (; t + 6 < N - 3;) {
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        two(std::false_type{});
+        t += 2;
+      }
+    }
+    for (; t < T_end; t += 2) two(std::true_type{});
+
+    unsigned long long kbest = 0ull;
+    int vmax = 0;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+      const uint32_t key = half ? (Kl >> 16) : (Kl & 0xffffu);
+      const int v = (int)(key >> KB), r = row0 + (half ? K : 0) + (int)KMASK - (int)(key & KMASK);
+      const int col = (int)(half ? (Jp >> 16) : (Jp & 0xffffu)) - 2 * lane - half;
+      vmax = v > vmax ? v : vmax;
+      if (v > 0 && r < M) {
+        const unsigned long long kk = best_key(v, r, col);
+        kbest = kk > kbest ? kk : kbest;
+      }
+    }
+    if (vmax > KeyBits<K>::kCap) overflow = 1;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const unsigned long long other = __shfl_xor_sync(gmask, kbest, o, G);
+      kbest = other > kbest ? other : kbest;
+      overflow |= __shfl_xor_sync(gmask, overflow, o, G);
+    }
+    if (kbest > best) best = kbest;
+    __syncwarp(gmask);
+  }
+  return best;
+}
+
+// The narrowest instantiation of the group that holds M rows.
+template <int G>
+__device__ __forceinline__ unsigned long long protein_rows(const uint8_t *a, int adir, int M, const uint8_t *b, int bdir,
+                                                           int N, const uint32_t *rowtab, uint4 *tab, int lane,
+                                                           unsigned gmask, uint32_t *bnd, uint32_t NGE, uint32_t NGO,
+                                                           uint32_t one, int &over) {
+  if (M <= 8 * G) return protein_sweep<4, G, false>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
+  if (M <= 12 * G) return protein_sweep<6, G, false>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
+  if (G == 16 || M <= 16 * G)
+    return protein_sweep<8, G, false>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
+  return protein_sweep<8, G, true>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
+}
+
+// Persistent: G-lane groups claim pairs of their range of the order (16 lanes: A up to 256
+// rows) and run both passes.  The begin sweep first covers score + 32 reversed rows (an
+// alignment scores at least about one a row), then the whole prefix if the score is not there.
+template <int G>
+__global__ void __launch_bounds__(128) k_protein16(P16Args g) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint32_t rowtab[kPCodes * kPWords];
+  const PArgs &p = g.p;
+  for (int k = threadIdx.x; k < kPCodes * kPWords; k += blockDim.x) {
+    const int a = k / kPWords, c0 = (k % kPWords) * 4;
+    uint32_t w = 0;
+    for (int x = 0; x < 4; x++)
+      if (a < kAA && c0 + x < kAA) w |= (uint32_t)(p.mat[a * kAA + c0 + x] + p.gO) << (8 * x);
+    rowtab[k] = w;
+  }
+  __syncthreads();
+  const int grp = threadIdx.x / G, lane = threadIdx.x % G;
+  const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (((threadIdx.x & 31) / G) * G);
+  uint4 *tab = reinterpret_cast<uint4 *>(smem) + (size_t)grp * kPCodes * G;
+  uint32_t *bnd = g.bound ? g.bound + ((int64_t)blockIdx.x * (128 / G) + grp) * p.max_n : nullptr;
+  const uint32_t NGE = V16::splat(-p.gE), NGO = V16::splat(-p.gO);
+  const uint32_t one = (uint32_t)(p.gO >> 30) + 1u;  // a 1 the compiler cannot fold
+  const int lo = G == 16 ? 0 : g.ctl[2], hi = G == 16 ? g.ctl[2] : (int)p.n;
+  for (;;) {
+    int claim = 0;
+    if (lane == 0) claim = atomicAdd(g.ctl + (G == 16 ? 0 : 1), 1);
+    claim = __shfl_sync(gmask, claim, 0, G);
+    if (lo + claim >= hi) break;
+    const uint32_t i = g.order[lo + claim];
+    const int M = p.a_len[i], N = p.b_len[i];
+    const uint8_t *a = p.a_code + p.a_off[i], *b = p.b_code + p.b_off[i];
+    int S = 0, ie = -1, je = 0, ib = -1, jb = 0, over = 0;
+    if (M > 0 && N > 0) {
+      if (min(M, N) >= g.wide_from || N > 65000) {
+        over = 1;
+      } else {
+        const unsigned long long k = protein_rows<G>(a, 1, M, b, 1, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
+        S = key_value(k);
+        if (S > 0 && !over) {
+          ie = key_row(k);
+          je = key_col(k);
+          int t = min(ie + 1, S + 32), dummy;
+          unsigned long long q =
+              protein_rows<G>(a + ie, -1, t, b + je, -1, je + 1, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, dummy);
+          if (key_value(q) != S && t < ie + 1)
+            q = protein_rows<G>(a + ie, -1, ie + 1, b + je, -1, je + 1, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, dummy);
+          ib = ie - key_row(q);
+          jb = je - key_col(q);
+        }
+      }
+    }
+    if (lane == 0) {
+      if (over) {
+        g.over[atomicAdd(g.over_n, 1)] = i;
+      } else {
+        p.score[i] = S;
+        p.a_end[i] = ie;
+        p.b_end[i] = je;
+        p.a_beg[i] = ib;
+        p.b_beg[i] = jb;
+      }
+    }
+  }
+}
+
+// ---- int32 kernels ------------------------------------------------------------------------
 
 // One pass: forward (REV = false) over the whole pairs, or the begin pass (REV = true)
 // over the reversed prefixes that end at each pair's end.
@@ -74,7 +353,9 @@ __global__ void __launch_bounds__(128) k_protein(PArgs g) {
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   int2 *bound = g.rows + warp * g.max_n;
   const int gO = g.gO, gE = g.gE;
-  for (int64_t p = warp; p < g.n; p += nwarps) {
+  const int64_t total = g.list ? (int64_t)*g.list_n : g.n;
+  for (int64_t it = warp; it < total; it += nwarps) {
+    const int64_t p = g.list ? (int64_t)g.list[it] : it;
     int M, N;
     const uint8_t *A = g.a_code + g.a_off[p], *B = g.b_code + g.b_off[p];
     int ie = 0, je = 0;
@@ -220,8 +501,11 @@ __global__ void k_protein_pack(const int32_t *score, const int32_t *a_beg, const
 }
 
 }  // namespace
+}  // namespace mhsw
 
 extern "C" {
+
+using namespace mhsw;
 
 int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *scoring_matrix,
                        const int16_t *encoding, int32_t *out5, int host_io) {
@@ -237,30 +521,42 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
   cudaStream_t st = static_cast<cudaStream_t>(mhsw::driver_stream(d));
   int gO = 0, gE = 0;
   mhsw::driver_gaps(d, &gO, &gE);
-  // extents: host batches are scanned here; device batches read their lengths back
-  std::vector<int32_t> la((size_t)n), lb((size_t)n);
-  std::vector<int64_t> oa((size_t)n), ob((size_t)n);
+  // extents: host batches are scanned in place; device batches read their lengths back
+  std::vector<int32_t> dl(host_io ? 0 : 2 * (size_t)n);
+  std::vector<int64_t> dof(host_io ? 0 : 2 * (size_t)n);
+  const int32_t *la = pairs->a_len, *lb = pairs->b_len;
+  const int64_t *oa = pairs->a_off, *ob = pairs->b_off;
   cudaError_t e = cudaSuccess;
-  if (host_io) {
-    std::memcpy(la.data(), pairs->a_len, sizeof(int32_t) * n);
-    std::memcpy(lb.data(), pairs->b_len, sizeof(int32_t) * n);
-    std::memcpy(oa.data(), pairs->a_off, sizeof(int64_t) * n);
-    std::memcpy(ob.data(), pairs->b_off, sizeof(int64_t) * n);
-  } else {
-    e = cudaMemcpyAsync(la.data(), pairs->a_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
-    if (!e) e = cudaMemcpyAsync(lb.data(), pairs->b_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
-    if (!e) e = cudaMemcpyAsync(oa.data(), pairs->a_off, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st);
-    if (!e) e = cudaMemcpyAsync(ob.data(), pairs->b_off, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st);
+  if (!host_io) {
+    e = cudaMemcpyAsync(dl.data(), pairs->a_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
+    if (!e) e = cudaMemcpyAsync(dl.data() + n, pairs->b_len, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
+    if (!e) e = cudaMemcpyAsync(dof.data(), pairs->a_off, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st);
+    if (!e) e = cudaMemcpyAsync(dof.data() + n, pairs->b_off, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st);
     if (!e) e = cudaStreamSynchronize(st);
     if (e) return MHSW_ERR_CUDA;
+    la = dl.data();
+    lb = la + n;
+    oa = dof.data();
+    ob = oa + n;
   }
-  int64_t ta = 0, tb = 0, max_n = 1;
+  int64_t ta = 0, tb = 0, max_n = 1, max_m = 1;
   for (int64_t i = 0; i < n; i++) {
-    if (la[(size_t)i] < 0 || lb[(size_t)i] < 0 || oa[(size_t)i] < 0 || ob[(size_t)i] < 0) return MHSW_ERR_ARG;
-    ta = std::max(ta, oa[(size_t)i] + la[(size_t)i]);
-    tb = std::max(tb, ob[(size_t)i] + lb[(size_t)i]);
-    max_n = std::max<int64_t>(max_n, lb[(size_t)i]);
+    if (la[i] < 0 || lb[i] < 0 || oa[i] < 0 || ob[i] < 0) return MHSW_ERR_ARG;
+    ta = std::max(ta, oa[i] + la[i]);
+    tb = std::max(tb, ob[i] + lb[i]);
+    max_n = std::max<int64_t>(max_n, lb[i]);
+    max_m = std::max<int64_t>(max_m, la[i]);
   }
+  // the keyed int16 kernels take matrices whose biased scores fit seven bits; a pair's score
+  // is at most min(M, N) * top
+  int top = 0, low = 0;
+  for (int k = 0; k < kAA * kAA; k++) {
+    top = std::max(top, (int)scoring_matrix[k]);
+    low = std::min(low, (int)scoring_matrix[k]);
+  }
+  const bool keyed = low >= -gO && top <= 63 && top + gO <= 127 && n <= 0x7fffffff;
+  const int wide_from = top > 0 ? 30000 / top : INT_MAX;  // H itself leaves int16 from there on
+  const bool over_possible = !keyed || std::min(max_m, max_n) * top > KeyBits<8>::kCap || max_n > 65000;
   char *as = nullptr, *bs = nullptr;
   int64_t *ao = nullptr, *bo = nullptr;
   int32_t *al = nullptr, *bl = nullptr;
@@ -269,11 +565,24 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
   int32_t *mat = nullptr, *sc = nullptr, *ae = nullptr, *be = nullptr, *ab = nullptr, *bb = nullptr, *o5 = nullptr;
   int *bad = nullptr;
   int2 *rows = nullptr;
+  int *ctl = nullptr;
+  uint32_t *order = nullptr, *over = nullptr, *bound = nullptr;
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // one warp per pair at a time; 24 resident warps per SM (76 registers x 128 threads
   // fits 6 blocks of 4 warps) to cover the row chain's latency
   const int64_t warps = std::min<int64_t>(n, (int64_t)sms * 24);
+  const size_t smem16 = 8 * (size_t)kPCodes * 16 * sizeof(uint4), smem32 = 4 * (size_t)kPCodes * 32 * sizeof(uint4);
+  int occ16 = 1, occ32 = 1;
+  if (keyed) {
+    e = raise_smem_limit(reinterpret_cast<const void *>(k_protein16<16>), smem16);
+    if (!e) e = raise_smem_limit(reinterpret_cast<const void *>(k_protein16<32>), smem32);
+    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ16, k_protein16<16>, 128, smem16);
+    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ32, k_protein16<32>, 128, smem32);
+    if (e) return MHSW_ERR_CUDA;
+  }
+  const int64_t blocks16 = std::min<int64_t>((n + 7) / 8, (int64_t)sms * occ16);
+  const int64_t blocks32 = std::min<int64_t>((n + 3) / 4, (int64_t)sms * occ32);
   // the call's arrays, laid out in the handle's call arena (sized by a first pass)
   auto lay = [&](mhsw::Carve &c) {
     if (host_io) {
@@ -295,7 +604,13 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
     c.take(&ab, (size_t)n);
     c.take(&bb, (size_t)n);
     c.take(&bad, 1);
-    c.take(&rows, (size_t)(warps * max_n));
+    if (keyed) {
+      c.take(&ctl, kOrderCtl + 1);
+      c.take(&order, (size_t)n);
+      c.take(&over, (size_t)n);
+      if (max_m > 512) c.take(&bound, (size_t)(blocks32 * 4 * max_n));
+    }
+    if (over_possible) c.take(&rows, (size_t)(warps * max_n));
   };
   mhsw::Carve sizing;
   lay(sizing);
@@ -327,17 +642,35 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
   if (!e) e = cudaMemcpyAsync(enc, encoding, sizeof(int16_t) * kEnc, cudaMemcpyHostToDevice, st);
   if (!e) e = cudaMemsetAsync(bad, 0, sizeof(int), st);
   if (!e) {
-    k_protein_encode<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((ta + 255) / 256, 4096)), 256, 0, st>>>(
-        as, ac, ta, enc, bad);
-    k_protein_encode<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((tb + 255) / 256, 4096)), 256, 0, st>>>(
-        bs, bc, tb, enc, bad);
+    const int64_t steps = (std::max(ta, tb) / 4 + 255) / 256;
+    k_protein_encode<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(steps, (int64_t)sms * 16)), 256, 0, st>>>(
+        as, ac, ta, bs, bc, tb, enc, bad);
     e = cudaGetLastError();
   }
+  PArgs g{ac, bc, ao, bo, al, bl, n, mat, gO, gE, sc, ae, be, ab, bb, rows, max_n, nullptr, nullptr};
+  if (!e && keyed) {
+    PairSet ps{};
+    ps.a_len = al;
+    ps.b_len = bl;
+    ps.n = n;
+    int *over_n = ctl + kOrderCtl;
+    e = cudaMemsetAsync(over_n, 0, sizeof(int), st);
+    if (!e) e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, true);
+    if (!e) {
+      const P16Args q{g, order, ctl, bound, over, over_n, wide_from};
+      if (max_m > 256) k_protein16<32><<<(unsigned)blocks32, 128, smem32, st>>>(q);
+      k_protein16<16><<<(unsigned)blocks16, 128, smem16, st>>>(q);
+      e = cudaGetLastError();
+    }
+    g.list = over;
+    g.list_n = over_n;
+  }
   if (!e) {
-    PArgs g{ac, bc, ao, bo, al, bl, n, mat, gO, gE, sc, ae, be, ab, bb, rows, max_n};
-    const unsigned blocks = (unsigned)((warps * 32 + 127) / 128);
-    k_protein<false><<<blocks, 128, 0, st>>>(g);
-    k_protein<true><<<blocks, 128, 0, st>>>(g);
+    if (over_possible) {
+      const unsigned blocks = (unsigned)((warps * 32 + 127) / 128);
+      k_protein<false><<<blocks, 128, 0, st>>>(g);
+      k_protein<true><<<blocks, 128, 0, st>>>(g);
+    }
     k_protein_pack<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(sc, ab, ae, bb, be, n, o5);
     e = cudaGetLastError();
   }
