@@ -37,9 +37,9 @@ __device__ __forceinline__ unsigned group_mask_b(int G) {
 // HALF: no pair's score can exceed kHalfCap.
 template <int G, bool S2, bool HALF>
 __global__ void __launch_bounds__(256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
-                                                     const uint32_t *__restrict__ order, int64_t n, int *queue,
-                                                     int lane_rows, bool wide_try16, int ceiling, WorkLists wl, int pad,
-                                                     int bcap, V16::Pay *scratch, int scratch_stride) {
+                                                     const uint32_t *__restrict__ order, int *queue, int lane_rows,
+                                                     bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap,
+                                                     V16::Pay *scratch, int scratch_stride) {
   constexpr bool kShort = (G == kGKShort);
   extern __shared__ __align__(16) unsigned char smem[];
   const int gpb = blockDim.x / G;
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256) k_fwd_persist(PairSet ps, ResultSet rs, S
   const int64_t gid = (int64_t)blockIdx.x * gpb + grp;
   V16::Pay *bnd = scratch ? scratch + gid * (int64_t)scratch_stride : nullptr;
   const int64_t lo = kShort ? 0 : queue[2];
-  const int64_t hi = kShort ? queue[2] : n;
+  const int64_t hi = kShort ? queue[2] : queue[8 + kBucketLong];
   int *counter = queue + (kShort ? 0 : 1);
 
   for (;;) {
@@ -233,13 +233,18 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
                   : (half ? k_fwd_persist<kGKLong, false, true> : k_fwd_persist<kGKLong, false, false>);
   const size_t prof_short = s2 ? group_prof16_bytes<10, kGKShort, kCode16Zero + 1>() : group_prof16_bytes<10, kGKShort>();
   const size_t prof_long = s2 ? group_prof16_bytes<8, kGKLong, kCode16Zero + 1>() : group_prof16_bytes<8, kGKLong>();
+  // long pairs take blocks of their own (not in score2 mode, which needs their row maxima, nor
+  // under a lowered int16 ceiling, which asks for the int32 pass)
+  const bool longs = max_a > kLongRows && !s2 && wl.long_bnd && ceiling >= kCeiling16;
+  const int long_rows = longs ? kLongRows : INT_MAX;
   const int pad = 2 * kGKLong;
   // strip scratch stride: B, the lane skew and score2 mode's zero-score padding (< 16)
   const int bcap = ((pad + std::max(max_b, 1) + 16 + 2 * kGKLong) + 15) / 16 * 16;
 
   // order of m items (pair i * stride); clears the claim counters
   auto order_items = [&](const BatchShape &sh, int64_t m, int64_t stride, uint32_t *order) -> int {
-    if ((e = order_pairs(ps, sc, sh.lane_rows, sh.wide_try16, m, stride, bs.ctl, order, sms, st, launches)))
+    if ((e = order_pairs(ps, sc, sh.lane_rows, sh.wide_try16, m, stride, bs.ctl, order, sms, st, launches, INT_MAX,
+                         INT_MAX, long_rows)))
       return fail(e, "order launch");
     return 0;
   };
@@ -292,10 +297,10 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     const bool fan = any_long && any_short && fk && fk->fork;
     if (fan && (e2 = fork_to(*fk, st, 1))) return fail(e2, "fork");
     if (any_long)
-      klong<<<grid_l, threads, smem_l, fan ? fk->side[0] : st>>>(ps, rs, sc, order, m, queue, sh.lane_rows, sh.wide_try16,
+      klong<<<grid_l, threads, smem_l, fan ? fk->side[0] : st>>>(ps, rs, sc, order, queue, sh.lane_rows, sh.wide_try16,
                                                                  ceiling, wl, pad, bcap, scr, stride);
     if (any_short)
-      kshort<<<grid_s, threads, smem_s, st>>>(ps, rs, sc, order, m, queue, sh.lane_rows, sh.wide_try16, ceiling, wl, pad,
+      kshort<<<grid_s, threads, smem_s, st>>>(ps, rs, sc, order, queue, sh.lane_rows, sh.wide_try16, ceiling, wl, pad,
                                                bcap, nullptr, stride);
     e2 = cudaGetLastError();
     if (e2) return fail(e2, "persistent forward launch");
@@ -404,6 +409,11 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   BatchShape shape = tune ? bs.shape : BatchShape{};
   if (!tune && n <= (int64_t)sms * 64) shape.lane_rows = 0;  // any_long holds: max_a > 0
   if (order_items(shape, n, 1, bs.order)) return 1;
+  if (longs) {
+    if ((e = launch_long_forward(plan_long(n, max_b, sms), ps, rs, sc, bs.order, queue + 8 + kBucketLong, wl, st)))
+      return fail(e, "long pair launch");
+    if (launches) *launches += 1;
+  }
   return run(shape, bs.order, n, nullptr);
 }
 

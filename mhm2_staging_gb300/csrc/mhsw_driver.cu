@@ -191,6 +191,7 @@ struct mhsw_driver {
   DBuf<int> l_counts;
   DBuf<uint8_t> a_code, b_code;  // base codes of the current batch
   DBuf<unsigned char> scratch;
+  DBuf<uint32_t> long_bnd;  // strip boundaries of the long-pair kernels
   DBuf<unsigned char> call_arena;  // one call's own arrays (caller side, protein), kept between calls
   DBuf<unsigned char> outv;  // 5 x int16 + 5 x int32 arrays
   DBuf<int32_t> out5;
@@ -339,6 +340,7 @@ struct mhsw_driver {
     b_code.release();
     l_counts.release();
     scratch.release();
+    long_bnd.release();
     call_arena.release();
     outv.release();
     out5.release();
@@ -449,7 +451,7 @@ int ensure_results(mhsw_driver *d, int64_t n) {
   MHSW_CK(d->l_ovf.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_wide.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_bands.reserve((size_t)n + 1), "cudaMalloc lists");
-  MHSW_CK(d->l_counts.reserve(2 + 2 * mhsw::kBandClasses), "cudaMalloc lists");
+  MHSW_CK(d->l_counts.reserve(4 + 2 * mhsw::kBandClasses), "cudaMalloc lists");
   return MHSW_OK;
 }
 
@@ -626,6 +628,8 @@ mhsw::WorkLists work_lists(mhsw_driver *d, int64_t n) {
   wl.wide_count = d->l_counts.p + 1;
   wl.bands = d->l_bands.p;
   wl.band_counts = d->l_counts.p + 2;
+  wl.long_next = d->l_counts.p + 2 + 2 * mhsw::kBandClasses;
+  wl.long_bnd = d->long_bnd.p;
   wl.cap = n;
   return wl;
 }
@@ -706,6 +710,8 @@ int forward_any(mhsw_driver *d, const mhsw::PairSet &ps, int max_a, int max_b, i
 int forward_passes(mhsw_driver *d, const mhsw::PairSet &ps, int max_a, int max_b, int form) {
   d->fwd_order = nullptr;
   if (!mhsw::keyed_scoring(d->sc)) return run_forward(d, ps, max_a, max_b);
+  if (max_a > mhsw::kLongRows)
+    MHSW_CK(d->long_bnd.reserve(mhsw::plan_long(ps.n, max_b, d->sms).bytes / sizeof(uint32_t)), "cudaMalloc strips");
   mhsw::WorkLists wl = work_lists(d, ps.n);
   MHSW_CK(mhsw::reset_lists(wl, d->st), "reset lists");
   d->launches += 1;

@@ -156,14 +156,15 @@ __device__ __forceinline__ bool band_outgrown(int t, int N2, int S, const Scorin
 // their begin written here.
 // s_cap: the largest score the band kernels take (the packed int16 kernels hold scores up
 // to kBand16Score); pairs above it go to the wavefront list too.
-__device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc, int64_t p, int s_cap) {
+// longs: searches over many rows go to the wide list, where the long-pair kernel takes them.
+__device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc, int64_t p, int s_cap, bool longs) {
   const int S = rs.score[p];
   if ((rs.flag[p] & kFlagTooLong) || S <= 0) {
     rs.a_beg[p] = -1;
     rs.b_beg[p] = 0;
     return -1;
   }
-  if (S > s_cap) return kBandClasses;
+  if (S > s_cap || (longs && long_begin(band_first_cap(S, sc.match, rs.a_end[p] + 1), S))) return kBandClasses;
   return band_fit(S, rs.a_end[p] + 1, rs.b_end[p] + 1, sc);
 }
 
@@ -185,13 +186,13 @@ __device__ __forceinline__ void append_agg(int64_t *list, int *count, int64_t ca
 
 // Pass 1: count the pairs of each band class.
 __global__ void __launch_bounds__(256) k_rev_count(ResultSet rs, Scoring sc, const uint32_t *__restrict__ order,
-                                                   int64_t n, int *band_counts, int s_cap) {
+                                                   int64_t n, int *band_counts, int s_cap, bool longs) {
   __shared__ int cnt[kBandClasses];
   if (threadIdx.x < kBandClasses) cnt[threadIdx.x] = 0;
   __syncthreads();
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = order ? (int64_t)order[idx] : idx;
-    const int c = band_class(rs, sc, p, s_cap);
+    const int c = band_class(rs, sc, p, s_cap, longs);
     if (c >= 0 && c < kBandClasses) atomicAdd(&cnt[c], 1);
   }
   __syncthreads();
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(256) k_rev_count(ResultSet rs, Scoring sc, con
 // Pass 2: place each pair in its class segment (segments in class order, each filled in
 // the batch's order); wider pairs go to the wavefront list.
 __global__ void __launch_bounds__(256) k_rev_scatter(ResultSet rs, Scoring sc, const uint32_t *__restrict__ order,
-                                                     int64_t n, WorkLists wl, int s_cap) {
+                                                     int64_t n, WorkLists wl, int s_cap, bool longs) {
   int off[kBandClasses];
   int acc = 0;
 #pragma unroll
@@ -215,7 +216,9 @@ __global__ void __launch_bounds__(256) k_rev_scatter(ResultSet rs, Scoring sc, c
     const int S = rs.score[p];
     int c = -1;
     if (!((rs.flag[p] & kFlagTooLong) || S <= 0)) {
-      c = S <= s_cap ? band_fit(S, rs.a_end[p] + 1, rs.b_end[p] + 1, sc) : kBandClasses;
+      const int M2 = rs.a_end[p] + 1;
+      c = S > s_cap || (longs && long_begin(band_first_cap(S, sc.match, M2), S)) ? kBandClasses
+                                                                                 : band_fit(S, M2, rs.b_end[p] + 1, sc);
     }
     // one append per class present in the warp: lanes of a class share one atomic
     const unsigned act = __activemask();
@@ -708,7 +711,7 @@ constexpr int kWaveScore16 = 16000;
 template <class VT, int K, int G>
 __global__ void __launch_bounds__(256) k_rev_wave(PairSet ps, ResultSet rs, Scoring sc, WorkLists wl,
                                                   typename VT::Pay *scratch, int scratch_stride, int pad, int bcap,
-                                                  int s_lo, int s_hi) {
+                                                  int s_lo, int s_hi, bool longs) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lanes = blockDim.x;
   const int gpb = lanes / G;
@@ -734,6 +737,7 @@ __global__ void __launch_bounds__(256) k_rev_wave(PairSet ps, ResultSet rs, Scor
     if (S < s_lo || S > s_hi) continue;
     const int ie = rs.a_end[p], je = rs.b_end[p];
     const int M2 = ie + 1;
+    if (longs && long_begin(band_first_cap(S, sc.match, M2), S)) continue;
     const int dmax = M2 < je + 1 ? M2 : je + 1;
     const long long gbl = gap_cells_bound(dmax, S, sc);
     long long n2 = (long long)M2 + gbl + 1;
@@ -807,6 +811,7 @@ __global__ void k_reset_lists(WorkLists wl) {
   *wl.ovf_count = 0;
   *wl.wide_count = 0;
   for (int i = 0; i < 2 * kBandClasses; i++) wl.band_counts[i] = 0;
+  wl.long_next[0] = wl.long_next[1] = 0;
 }
 
 int g_num_sms = 0;
@@ -976,28 +981,28 @@ static bool wave_launch_ok(FwdConfig c, int max_a, void *scratch, size_t scratch
 template <class VT, int K>
 static cudaError_t launch_rev_wave_t(FwdConfig c, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
                                      const WorkLists &wl, void *scratch, size_t scratch_bytes, int max_a, int sms,
-                                     int s_lo, int s_hi, cudaStream_t st) {
+                                     int s_lo, int s_hi, bool longs, cudaStream_t st) {
   typename VT::Pay *scr = nullptr;
   // without scratch, pairs longer than a strip are reported (kFlagTooLong), as before
   wave_plan<VT>(c, max_a, scratch, scratch_bytes, sms, &scr);
   auto kern = k_rev_wave<VT, K, kG>;
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), c.smem);
   if (e != cudaSuccess) return e;
-  kern<<<c.grid, c.groups_per_block * kG, c.smem, st>>>(ps, rs, sc, wl, scr, c.bcap, c.pad, c.bcap, s_lo, s_hi);
+  kern<<<c.grid, c.groups_per_block * kG, c.smem, st>>>(ps, rs, sc, wl, scr, c.bcap, c.pad, c.bcap, s_lo, s_hi, longs);
   return cudaGetLastError();
 }
 
 static cudaError_t launch_rev_wave16(const FwdConfig &c, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
                                      const WorkLists &wl, void *scratch, size_t scratch_bytes, int max_a, int sms,
-                                     cudaStream_t st) {
+                                     bool longs, cudaStream_t st) {
   switch (c.K) {
-    case 2: return launch_rev_wave_t<V16, 2>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, st);
-    case 3: return launch_rev_wave_t<V16, 3>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, st);
-    case 4: return launch_rev_wave_t<V16, 4>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, st);
-    case 5: return launch_rev_wave_t<V16, 5>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, st);
-    case 6: return launch_rev_wave_t<V16, 6>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, st);
-    case 7: return launch_rev_wave_t<V16, 7>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, st);
-    default: return launch_rev_wave_t<V16, 8>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, st);
+    case 2: return launch_rev_wave_t<V16, 2>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
+    case 3: return launch_rev_wave_t<V16, 3>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
+    case 4: return launch_rev_wave_t<V16, 4>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
+    case 5: return launch_rev_wave_t<V16, 5>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
+    case 6: return launch_rev_wave_t<V16, 6>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
+    case 7: return launch_rev_wave_t<V16, 7>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
+    default: return launch_rev_wave_t<V16, 8>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
   }
 }
 
@@ -1005,6 +1010,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
                            int max_b, void *scratch, size_t scratch_bytes, const WorkLists &wl, cudaStream_t st,
                            const uint32_t *order, const Forks *fk) {
   const int sms = num_sms(device);
+  const bool longs = max_a > kLongRows && wl.long_bnd && keyed_scoring(sc);
   if (ps.n > 0) {
     const int grid = (int)std::min<int64_t>((ps.n + 255) / 256, (int64_t)sms * 8);
     const int gridb = sms * 8;
@@ -1015,8 +1021,9 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
     const bool bi = sc.gap_open > 0 && sc.mismatch <= sc.gap_open && sc.ambiguity <= sc.gap_open &&
                     sc.match + sc.gap_open <= 255;
     const int s_cap = bi ? kBand16Score : 0x7fffffff;
-    k_rev_count<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl.band_counts, s_cap);
-    k_rev_scatter<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap);
+    const bool force = longs && ps.n <= kLongBeginPairs;
+    k_rev_count<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl.band_counts, s_cap, force);
+    k_rev_scatter<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap, force);
     // The classes are independent: with side streams they run concurrently, so the
     // latency-bound narrow classes share the SMs with the wide ones.
     cudaStream_t cs[kBandClasses];
@@ -1050,6 +1057,10 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
       if (e != cudaSuccess) return e;
     }
   }
+  if (longs) {
+    const cudaError_t e = launch_long_reverse(plan_long(ps.n, max_b, sms), ps, rs, sc, wl, st);
+    if (e != cudaSuccess) return e;
+  }
   // Wide bands: wavefront on the reversed box (count read on the device), in int16 for
   // scores up to kWaveScore16 where a strip plan with scratch exists, int32 otherwise.
   FwdConfig c16, c32;
@@ -1059,11 +1070,11 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
   if (e != cudaSuccess) return e;
   int split = 0;  // largest score the int16 launch takes
   if (wave_launch_ok<V16>(c16, max_a, scratch, scratch_bytes, sms)) {
-    e = launch_rev_wave16(c16, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, st);
+    e = launch_rev_wave16(c16, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, longs, st);
     if (e != cudaSuccess) return e;
     split = kWaveScore16;
   }
-  return launch_rev_wave_t<V32, 4>(c32, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, split + 1, 0x7fffffff, st);
+  return launch_rev_wave_t<V32, 4>(c32, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, split + 1, 0x7fffffff, longs, st);
 }
 
 cudaError_t raise_smem_limit(const void *func, size_t bytes) {

@@ -20,6 +20,8 @@ struct WorkLists {
   int64_t *bands;     // begin-pass pairs grouped by band class (one segment per class)
   int *band_counts;   // kBandClasses pair counts, then kBandClasses scatter cursors
   int64_t cap;        // capacity of each list
+  int *long_next;     // claim counters of the long-pair kernels (forward, begin)
+  uint32_t *long_bnd; // their strip boundaries (LongPlan::bytes), or null
 };
 
 struct FwdConfig {
@@ -122,6 +124,28 @@ bool may_need_int32(const Scoring &sc, int ceiling, int max_a, int max_b);
 
 // Packs results into n x 5 int32 rows (score, a_beg, a_end, b_beg, b_end).
 cudaError_t launch_pack5(const ResultSet &rs, int64_t n, int32_t *out5, cudaStream_t st);
+
+// ---- long pairs (mhsw_long.cu) -------------------------------------------------------
+// A pair with more rows than this (and, in the begin pass, a search whose first row cap is
+// above it) takes a block of its own when its score bound is at most kLongScore (keyed
+// scorings; not in score2 mode).
+constexpr int kLongRows = 1024;
+constexpr int kLongScore = 32000;
+constexpr size_t kLongScratch = size_t(512) << 20;  // strip boundaries, at most
+// Batches up to this size send every such begin search there; in larger ones the banded
+// kernels (a thread per pair, far fewer cells) have pairs enough to fill the GPU.
+constexpr int64_t kLongBeginPairs = 4096;
+__host__ __device__ inline bool long_begin(int rows, int score) { return rows > kLongRows && score <= kLongScore; }
+struct LongPlan {
+  int warps = 0, grid = 0;
+  int64_t cols = 0;
+  size_t bytes = 0;
+};
+LongPlan plan_long(int64_t n, int max_b, int sms);
+cudaError_t launch_long_forward(const LongPlan &pl, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
+                                const uint32_t *order, const int *first, const WorkLists &wl, cudaStream_t st);
+cudaError_t launch_long_reverse(const LongPlan &pl, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
+                                const WorkLists &wl, cudaStream_t st);
 
 // ---- CIGAR pass (mhsw_cigar.cu) ----------------------------------------------------
 constexpr int kCigarClasses = 6;     // register-band traceback kernels, half-widths 1, 2, 4, 8, 16, 31

@@ -280,7 +280,7 @@ int na_setup(int dev, NaDevice **out, char *errbuf, size_t errlen) {
     if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_fwd_noalloc16<kGKShort, false>), na16_smem_short())) ||
         (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_short, k_fwd_noalloc16<kGKShort, false>, 128,
                                                            na16_smem_short())) ||
-        (e = raise_smem_limit(reinterpret_cast<const void *>(k_order_place), 2 * sizeof(int) * kOrderBins)))
+        (e = order_smem_limits()))
       return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "keyed kernel set-up: %s", cudaGetErrorString(e));
     d.scratch = static_cast<unsigned char *>(p);
     d.sms = sms;

@@ -15,17 +15,20 @@ namespace {
 
 // Buckets: 0..3 = A up to 64/96/128/160 rows (8-lane groups, K = 4/6/8/10),
 // 4/5 = up to 192/256 rows (16-lane groups, K = 6/8), 6 = longer A (K = 8 strips),
-// 7 = could exceed the int16 keys: straight to the int32 list.  The tuned row threshold
+// 7 = could exceed the int16 keys: straight to the int32 list; 8 = A above long_rows rows: a
+// block of its own (mhsw_long.cu).  The tuned row threshold
 // (lane_rows, 160 or 128) moves A of 129..160 rows between bucket 3 and bucket 4.
 constexpr int kBucketFirstLong = 4;
 constexpr int kBucketStrip = 6;
 constexpr int kBucketWide = 7;
-constexpr int kBuckets = 8;
+constexpr int kBucketLong = 8;
+constexpr int kBuckets = 9;
 __host__ __device__ constexpr int bucket_k(int b) {
   return b == 0 ? 4 : b == 1 ? 6 : b == 2 ? 8 : b == 3 ? 10 : b == 4 ? 6 : 8;
 }
 
-__device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int lane_rows, bool wide_try16) {
+__device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int lane_rows, bool wide_try16,
+                                         int long_rows = INT_MAX) {
   const int b = M <= lane_rows ? (M <= 64 ? 0 : M <= 96 ? 1 : M <= 128 ? 2 : 3)
                                : (M <= 192 ? 4 : M <= 256 ? 5 : kBucketStrip);
   // wide_try16: the int16 engine's ceiling test sends the pairs that do overflow to int32.
@@ -33,6 +36,7 @@ __device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int la
   // fits a 16-bit key: the capacity leaves 64 values of margin and H grows by at most match
   // per step, so it holds for match <= 63; larger matches keep the bound routing.
   const long long bound = (long long)(M < N ? M : N) * sc.match;
+  if (M > long_rows && bound <= kLongScore) return kBucketLong;
   if ((!wide_try16 || sc.match > 63) && bound > keyed_cap(bucket_k(b))) return kBucketWide;
   return b;
 }
@@ -73,13 +77,14 @@ struct OrderArgs {
   int *hist, *cursor; // kOrderBins each (zeroed before the two-launch form)
   uint32_t *order;
   int max_a, max_b;   // pairs longer than these go with the empty ones
+  int long_rows;      // longest A of the persistent kernels
   bool protein;       // buckets by protein_bucket (sc unused)
 };
 
 __device__ __forceinline__ int order_bin(const OrderArgs &g, int64_t p) {
   const int M = g.ps.a_len[p], N = g.ps.b_len[p];
   const int b = (M <= 0 || N <= 0 || M > g.max_a || N > g.max_b) ? (g.lane_rows > 0 ? 0 : kBucketFirstLong)
-                : g.protein ? protein_bucket(M) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16);
+                : g.protein ? protein_bucket(M) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.long_rows);
   return b * kLenBins + len_class(N);
 }
 
@@ -127,7 +132,7 @@ __device__ __forceinline__ void write_firsts(const OrderArgs &g, const int *base
 }
 
 __global__ void __launch_bounds__(1024) k_order_one(OrderArgs g) {
-  __shared__ int h[kOrderBins];
+  extern __shared__ int h[];
   for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) h[b] = 0;
   if (threadIdx.x < 2) g.queue[threadIdx.x] = 0;
   __syncthreads();
@@ -148,7 +153,7 @@ __global__ void __launch_bounds__(1024) k_order_one(OrderArgs g) {
 }
 
 __global__ void __launch_bounds__(1024) k_order_hist(OrderArgs g) {
-  __shared__ int h[kOrderBins];
+  extern __shared__ int h[];
   for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) h[b] = 0;
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.m; i += (int64_t)gridDim.x * blockDim.x)
@@ -160,8 +165,8 @@ __global__ void __launch_bounds__(1024) k_order_hist(OrderArgs g) {
 
 // Same grid as k_order_hist: each block reserves its run of every bin with one atomic.
 __global__ void __launch_bounds__(1024) k_order_place(OrderArgs g) {
-  extern __shared__ int base[];
-  int *h = base + kOrderBins;
+  extern __shared__ int h[];
+  int *base = h + kOrderBins;
   for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) {
     base[b] = g.hist[b];
     h[b] = 0;
@@ -191,25 +196,31 @@ __global__ void __launch_bounds__(1024) k_order_place(OrderArgs g) {
 constexpr size_t kOrderHead = 24;
 constexpr size_t kOrderCtl = kOrderHead + 2 * kOrderBins;
 
+constexpr size_t kOrderSmem = sizeof(int) * kOrderBins;  // of the one-block and histogram kernels; twice of the placement
+inline cudaError_t order_smem_limits() {
+  cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_order_one), kOrderSmem);
+  if (!e) e = raise_smem_limit(reinterpret_cast<const void *>(k_order_hist), kOrderSmem);
+  return e ? e : raise_smem_limit(reinterpret_cast<const void *>(k_order_place), 2 * kOrderSmem);
+}
+
 // Orders m items (pair i * stride) into `order`; clears the claim counters.
 inline cudaError_t order_pairs(const PairSet &ps, const Scoring &sc, int lane_rows, bool wide_try16, int64_t m,
                                int64_t stride, int *ctl, uint32_t *order, int sms, cudaStream_t st, int64_t *launches,
-                               int max_a = INT_MAX, int max_b = INT_MAX, bool protein = false) {
+                               int max_a = INT_MAX, int max_b = INT_MAX, int long_rows = INT_MAX, bool protein = false) {
   OrderArgs g{ps, sc, lane_rows, wide_try16, m, stride, ctl, ctl + 8, ctl + kOrderHead, ctl + kOrderHead + kOrderBins,
-              order, max_a, max_b, protein};
+              order, max_a, max_b, long_rows, protein};
+  cudaError_t e = order_smem_limits();
+  if (e) return e;
   if (m <= kOrderOneBlock) {
-    k_order_one<<<1, 1024, 0, st>>>(g);
+    k_order_one<<<1, 1024, kOrderSmem, st>>>(g);
     if (launches) *launches += 1;
     return cudaGetLastError();
   }
-  cudaError_t e = cudaMemsetAsync(ctl, 0, sizeof(int) * kOrderCtl, st);
-  if (e) return e;
-  // a block an SM at most: each reads and writes all bins, 47 KB
+  if ((e = cudaMemsetAsync(ctl, 0, sizeof(int) * kOrderCtl, st))) return e;
+  // a block an SM at most: each reads and writes all bins, 53 KB
   const int grid = (int)std::min<int64_t>((m + 4095) / 4096, sms);
-  const size_t smem = 2 * sizeof(int) * kOrderBins;
-  if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_order_place), smem))) return e;
-  k_order_hist<<<grid, 1024, 0, st>>>(g);
-  k_order_place<<<grid, 1024, smem, st>>>(g);
+  k_order_hist<<<grid, 1024, kOrderSmem, st>>>(g);
+  k_order_place<<<grid, 1024, 2 * kOrderSmem, st>>>(g);
   if (launches) *launches += 2;
   return cudaGetLastError();
 }

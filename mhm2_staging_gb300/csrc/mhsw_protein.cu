@@ -655,7 +655,7 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
     ps.n = n;
     int *over_n = ctl + kOrderCtl;
     e = cudaMemsetAsync(over_n, 0, sizeof(int), st);
-    if (!e) e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, true);
+    if (!e) e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, INT_MAX, true);
     if (!e) {
       const P16Args q{g, order, ctl, bound, over, over_n, wide_from};
       if (max_m > 256) k_protein16<32><<<(unsigned)blocks32, 128, smem32, st>>>(q);
