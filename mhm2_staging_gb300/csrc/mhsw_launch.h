@@ -137,7 +137,7 @@ constexpr size_t kLongScratch = size_t(512) << 20;  // strip boundaries, at most
 constexpr int64_t kLongBeginPairs = 4096;
 __host__ __device__ inline bool long_begin(int rows, int score) { return rows > kLongRows && score <= kLongScore; }
 struct LongPlan {
-  int warps = 0, grid = 0;
+  int warps = 0, cluster = 0, clusters = 0;  // warps a block, blocks a cluster, clusters
   int64_t cols = 0;
   size_t bytes = 0;
 };

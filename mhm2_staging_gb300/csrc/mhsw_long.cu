@@ -1,11 +1,12 @@
-// mhsw_long.cu -- long pairs: one block per pair, a warp per strip of A's rows.
+// mhsw_long.cu -- long pairs: a cluster of blocks per pair, a warp per strip of A's rows.
 //
 // A lane group that takes a pair of several thousand rows alone walks its strips one after
 // another: 60 pairs of 1-12 kb kept 60 groups of 16 lanes busy for 0.3 s on 152 SMs.  Here the
 // strips of a pair run at the same time.  Warp w takes strips w, w + W, ... (512 rows each, 16 a
 // lane); strip s follows strip s - 1 by about 130 columns, reading its last row's H and E^ from a
 // row in global memory that the producer publishes 32 columns at a time through a progress
-// word in shared memory.  A strip only ever waits for an earlier one and a warp takes its
+// word.  While the pairs are few, a pair's strips go round the blocks of a cluster (4 SMs, 32
+// warps), so a scheduler has one strip rather than four.  A strip only ever waits for an earlier one and a warp takes its
 // strips in order, so the waits end; each is bounded all the same and reports the pair as
 // inconsistent if it gives up.
 //
@@ -34,7 +35,31 @@ namespace {
 constexpr int kLK = 8;                  // row pairs per lane
 constexpr int kLRows = 2 * kLK * 32;    // rows per strip
 constexpr int kLChunk = 32;             // columns between progress updates
-constexpr int kLongWaits = 1 << 22;     // polls before a wait gives up (seconds)
+constexpr int kLongWaits = 1 << 22;     // polls (of L2) before a wait gives up (seconds)
+
+constexpr int kLongWarps = 32;          // warps on one pair, at most
+
+// Shared by the blocks of a cluster, in global memory.
+struct LongShared {
+  unsigned long long prog[kLongWarps];  // per warp: strip << 32 | columns published (absolute)
+  unsigned long long best;
+  int claim, failed;
+};
+
+__device__ __forceinline__ void cluster_barrier() {  // all threads of the cluster; orders their memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_fence() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
+__device__ __forceinline__ int cluster_rank() {
+  int r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ int cluster_size() {
+  int r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
 
 struct LongArgs {
   PairSet ps;
@@ -46,17 +71,14 @@ struct LongArgs {
   const int *list_n;
   int64_t list_cap;
   int *next;               // claim counter
-  uint32_t *bnd;           // per block: one row of `cols` words per warp
+  LongShared *shared;      // per cluster
+  uint32_t *bnd;           // per cluster: one row of `cols` words per warp
   int64_t cols;
 };
 
-struct LongShared {
-  unsigned long long prog[16];  // per warp: strip << 32 | columns published (absolute)
-  unsigned long long best;
-  int claim, failed;
-};
-
-// The keyed step with keys above a base (nbase: its negative, per half).
+// The keyed step with keys above a base (nbase: its negative, per half).  LAZY (gap open >= gap
+// extend): the chain down the rows is one add-max per row (ShortStep in mhsw_short.cu).
+template <bool LAZY>
 __device__ __forceinline__ void long_step(int t, uint32_t zH, uint32_t zE, const uint32_t (&Wlo)[kLK],
                                           const uint32_t (&Phi)[kLK], uint32_t (&H)[kLK], uint32_t (&F)[kLK],
                                           uint32_t &Hlast, uint32_t &Ecout, uint32_t &HtopPrev, uint32_t &Kl,
@@ -70,9 +92,16 @@ __device__ __forceinline__ void long_step(int t, uint32_t zH, uint32_t zE, const
 #pragma unroll
   for (int k = 0; k < kLK; k++) {
     const uint32_t Q = mad_u32(mad_u32(Hd, one, Wlo[k]), one, Phi[k]);
-    const uint32_t m = __vimax3_s16x2(Q, Ev, F[k]);
-    const uint32_t Hn = __viaddmax_s16x2_relu(m, NGO, 0u);
-    Ev = __viaddmax_s16x2(Ev, NGE, Hn);
+    uint32_t Hn;
+    if constexpr (LAZY) {
+      const uint32_t Hp = __viaddmax_s16x2_relu(__vmaxs2(Q, F[k]), NGO, 0u);
+      Hn = __viaddmax_s16x2(Ev, NGO, Hp);
+      Ev = __viaddmax_s16x2(Ev, NGE, Hp);
+    } else {
+      const uint32_t m = __vimax3_s16x2(Q, Ev, F[k]);
+      Hn = __viaddmax_s16x2_relu(m, NGO, 0u);
+      Ev = __viaddmax_s16x2(Ev, NGE, Hn);
+    }
     F[k] = __viaddmax_s16x2(F[k], NGE, Hn);
     Hd = H[k];
     H[k] = Hn;
@@ -90,14 +119,15 @@ __device__ __forceinline__ void long_step(int t, uint32_t zH, uint32_t zE, const
 }
 
 // Sweep of rows [0, M) (a[adir * i]) over columns [0, N) (b[bdir * j]), row i limited to
-// [i - I, i + J], by all warps of the block; best cell in sh.best.  goal > 0: strips after one
+// [i - I, i + J], by all W warps of the cluster (this one is number `warp`); best cell in sh.best.  goal > 0: strips after one
 // that reached it stop.
+template <bool LAZY>
 __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, int bdir, int N, int I, int J, int goal,
-                           const Scoring &sc, uint32_t *prof, uint32_t *bnd, int64_t cols, LongShared &sh) {
+                           const Scoring &sc, uint32_t *prof, uint32_t *bnd, int64_t cols, LongShared &sh, int warp, int W) {
   using ST = Step16<kLK, 32>;
   using L = Prof16<kLK>;
   constexpr unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const uint32_t NGE = V16::splat(-sc.gap_extend), NGO = V16::splat(-sc.gap_open);
   const uint32_t one = (uint32_t)(sc.gap_open >> 30) + 1u, eight = one << 3;  // not folded by the compiler
   const int nstrips = (M + kLRows - 1) / kLRows;
@@ -130,17 +160,21 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
         }
     }
     __syncwarp();
-    // waits until the strip above has published its columns below `col` (or ended)
+    // waits until the strip above has published its columns below `col` (or ended).  `seen` is
+    // its progress word as loaded a chunk ago, so a strip that is not held up does not stand
+    // still for the word's latency.
+    const int pw = (s + W - 1) % W;
+    unsigned long long seen = 0ull;
     auto await = [&](int col) -> bool {
       if (s == 0) return true;
       const unsigned long long want = ((unsigned long long)(s - 1) << 32) | (unsigned)col;
-      const int pw = (s - 1) % W;
       int polls = 0;
-      while (prog[pw] < want) {
+      while (seen < want) {
         if (++polls > kLongWaits || *(volatile int *)&sh.failed) return false;
-        __nanosleep(64);
+        seen = prog[pw];
       }
-      __threadfence_block();
+      cluster_fence();
+      seen = prog[pw];
       return true;
     };
     auto load_top = [&](int t) -> uint32_t {  // boundary words of columns c0 + t + lane
@@ -157,13 +191,15 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
     const int first_top = (int)__reduce_max_sync(full, max(cur & 0xffffu, HtopPrev));
     int base_lo = max(first_top - 1024, 0), base_hi = base_lo;
     uint32_t nbase = V16::pack(-base_lo, -base_hi);
-    uint32_t H[kLK], F[kLK], Wlo[kLK], HA[kLK], HB[kLK];
+    uint32_t H[kLK], F[kLK], lo[kLK], hi[kLK], hp[kLK];  // this column's words, the last column's hi words
 #pragma unroll
-    for (int k = 0; k < kLK; k++) H[k] = F[k] = HB[k] = 0u;
+    for (int k = 0; k < kLK; k++) H[k] = F[k] = hp[k] = 0u;
     uint32_t Hlast = 0u, Ecout = 0u, Kl = 0u, Jp = 0u;
     const int j0 = c0 - 2 * lane;
     auto code_at = [&](int j) -> int { return j >= c0 && j < c1 ? (int)b[(int64_t)bdir * j] : kCodeN; };
-    int ceven = code_at(j0), codd = code_at(j0 + 1);
+    // a step's words are loaded a step ahead of their use, its code three ahead
+    ST::load(tab, code_at(j0), lane, lo, hi);
+    int c1s = code_at(j0 + 1), c2s = code_at(j0 + 2);
     const int steps = ncols > 0 ? ncols + 63 : 0;
     for (int t0 = 0; t0 < steps && ok; t0 += kLChunk) {
       ok = await(min(c0 + t0 + 2 * kLChunk, pc1));
@@ -178,37 +214,30 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
         constexpr bool kGuard = decltype(guarded)::value;
         const uint8_t *bl = b + (int64_t)bdir * j0;
 #pragma unroll
-        for (int u = 0; u < 8; u += 2) {
+        for (int u = 0; u < 8; u++) {
           const int t = tb + u;
-          auto top = [&](int tt, uint32_t &zH, uint32_t &zE) {
-            const uint32_t w = __shfl_sync(full, cur, tt & 31);
-            zH = __shfl_up_sync(full, Hlast, 1);
-            zE = __shfl_up_sync(full, Ecout, 1);
-            if (lane == 0) {
-              zH = w << 16;
-              zE = w;
-            }
-          };
-          auto put = [&](int tt) {
-            const int jh = c0 + tt - 63;  // the last lane's high-half column
-            if (!last && lane == 31 && jh >= c0 && jh < c1) out_row[jh] = __byte_perm(Hlast, Ecout, 0x7632);
-          };
-          uint32_t zH, zE;
-          int c = ceven;
-          ceven = kGuard ? code_at(j0 + t + 2) : (int)bl[(int64_t)bdir * (t + 2)];
-          ST::load(tab, c, lane, Wlo, HA);
-          top(t, zH, zE);
-          long_step(t, zH, zE, Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, eight, nbase);
-          put(t);
-          c = codd;
-          codd = kGuard ? code_at(j0 + t + 3) : (int)bl[(int64_t)bdir * (t + 3)];
-          ST::load(tab, c, lane, Wlo, HB);
-          top(t + 1, zH, zE);
-          long_step(t + 1, zH, zE, Wlo, HA, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, eight, nbase);
-          put(t + 1);
+          const uint32_t w = __shfl_sync(full, cur, t & 31);
+          uint32_t zH = __shfl_up_sync(full, Hlast, 1), zE = __shfl_up_sync(full, Ecout, 1);
+          if (lane == 0) {
+            zH = w << 16;
+            zE = w;
+          }
+          uint32_t nlo[kLK], nhi[kLK];
+          ST::load(tab, c1s, lane, nlo, nhi);
+          c1s = c2s;
+          c2s = kGuard ? code_at(j0 + t + 3) : (int)bl[(int64_t)bdir * (t + 3)];
+          long_step<LAZY>(t, zH, zE, lo, hp, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, eight, nbase);
+#pragma unroll
+          for (int k = 0; k < kLK; k++) {
+            hp[k] = hi[k];
+            lo[k] = nlo[k];
+            hi[k] = nhi[k];
+          }
+          const int jh = c0 + t - 63;  // the last lane's high-half column
+          if (!last && lane == 31 && jh >= c0 && jh < c1) out_row[jh] = __byte_perm(Hlast, Ecout, 0x7632);
         }
       };
-      // every lane's look-ahead columns j0 + t + 2 .. + 3 lie in [c0, c1)
+      // every lane's look-ahead column j0 + t + 3 lies in [c0, c1)
       const bool inside = t0 >= 64 && t0 + kLChunk + 4 <= ncols;
       for (int tb = t0; tb < t0 + kLChunk; tb += 8) {
         if (inside) eight_steps(tb, std::false_type{});
@@ -226,14 +255,14 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
       if (!last && lane == 31) {
         const int done = min(t0 + kLChunk - 63, ncols);
         if (done > 0) {
-          __threadfence_block();
+          cluster_fence();
           prog[warp] = ((unsigned long long)s << 32) | (unsigned)(c0 + done);
         }
       }
     }
     if (!ok && lane == 0) sh.failed = 1;
     if (lane == 31) {
-      __threadfence_block();
+      cluster_fence();
       prog[warp] = ((unsigned long long)s << 32) | 0xffffffffu;
     }
     unsigned long long best = 0ull;
@@ -259,21 +288,33 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
   }
 }
 
-template <bool REV>
-__global__ void __launch_bounds__(512) k_long(LongArgs g) {
+template <bool REV, bool LAZY>
+__global__ void __launch_bounds__(256, 2) k_long(LongArgs g) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ LongShared sh;
-  const int warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  uint32_t *prof = reinterpret_cast<uint32_t *>(smem + (size_t)warp * Prof16<kLK>::bytes(32));
-  uint32_t *bnd = g.bnd + (int64_t)blockIdx.x * W * g.cols;
+  const int C = cluster_size(), rank = cluster_rank();
+  const int W = (int)(blockDim.x >> 5) * C, warp = (int)(threadIdx.x >> 5) * C + rank;  // strips go round the blocks
+  const int cluster = blockIdx.x / C;
+  uint32_t *prof = reinterpret_cast<uint32_t *>(smem + (size_t)(threadIdx.x >> 5) * Prof16<kLK>::bytes(32));
+  uint32_t *bnd = g.bnd + (int64_t)cluster * W * g.cols;
+  LongShared &sh = g.shared[cluster];
+  volatile LongShared &vs = sh;
+  const bool lead = rank == 0 && threadIdx.x == 0;
   const Scoring sc = g.sc;
   const int64_t lo = REV ? 0 : *g.first;
   const int64_t hi = REV ? (*g.list_n < g.list_cap ? *g.list_n : g.list_cap) : g.ps.n;
+  auto reset = [&]() {
+    if (rank == 0 && threadIdx.x < kLongWarps) vs.prog[threadIdx.x] = 0ull;
+    if (lead) {
+      vs.best = 0ull;
+      vs.failed = 0;
+    }
+    cluster_barrier();
+  };
   for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) sh.claim = atomicAdd(g.next, 1);
-    __syncthreads();
-    const int64_t item = lo + sh.claim;
+    cluster_barrier();
+    if (lead) vs.claim = atomicAdd(g.next, 1);
+    cluster_barrier();
+    const int64_t item = lo + vs.claim;
     if (item >= hi) break;
     const int64_t p = REV ? g.list[item] : (int64_t)g.order[item];
     if (REV) {
@@ -282,47 +323,44 @@ __global__ void __launch_bounds__(512) k_long(LongArgs g) {
       if (!long_begin(band_first_cap(S, sc.match, M2), S)) continue;  // the wavefront kernels take it
       const uint8_t *a = g.ps.a_code + g.ps.a_off[p] + ie, *b = g.ps.b_code + g.ps.b_off[p] + je;
       int t = band_first_cap(S, sc.match, M2);
+      unsigned long long best;
+      bool failed;
       for (;;) {
         int I, J;
         band_sides(t, N2, S, sc, I, J);
-        __syncthreads();
-        if (threadIdx.x < 16) sh.prog[threadIdx.x] = 0ull;
-        if (threadIdx.x == 0) {
-          sh.best = 0ull;
-          sh.failed = 0;
-        }
-        __syncthreads();
-        long_sweep(a, -1, t, b, -1, (int)min((long long)N2, (long long)t + J), I, J, S, sc, prof, bnd, g.cols, sh);
-        __syncthreads();
-        if (key_value(sh.best) >= S || t >= M2 || sh.failed) break;
+        reset();
+        long_sweep<LAZY>(a, -1, t, b, -1, (int)min((long long)N2, (long long)t + J), I, J, S, sc, prof, bnd, g.cols, sh, warp, W);
+        cluster_barrier();
+        best = vs.best;
+        failed = vs.failed;
+        if (key_value(best) >= S || t >= M2 || failed) break;
         t = t < M2 / 2 ? 2 * t : M2;
+        cluster_barrier();  // all have read the outcome before it is reset
       }
-      if (threadIdx.x == 0) {
-        if (key_value(sh.best) != S || sh.failed) {
+      if (lead) {
+        if (key_value(best) != S || failed) {
           g.rs.flag[p] |= kFlagTooLong;  // inconsistent
           g.rs.a_beg[p] = -1;
           g.rs.b_beg[p] = 0;
         } else {
-          g.rs.a_beg[p] = ie - key_row(sh.best);
-          g.rs.b_beg[p] = je - key_col(sh.best);
+          g.rs.a_beg[p] = ie - key_row(best);
+          g.rs.b_beg[p] = je - key_col(best);
         }
       }
     } else {
       const int M = g.ps.a_len[p], N = g.ps.b_len[p];
-      if (threadIdx.x < 16) sh.prog[threadIdx.x] = 0ull;
-      if (threadIdx.x == 0) {
-        sh.best = 0ull;
-        sh.failed = 0;
-      }
-      __syncthreads();
-      long_sweep(g.ps.a_code + g.ps.a_off[p], 1, M, g.ps.b_code + g.ps.b_off[p], 1, N, M, N, 0, sc, prof, bnd, g.cols, sh);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        const int S = key_value(sh.best);
-        g.rs.flag[p] = sh.failed ? kFlagTooLong : 0u;
-        g.rs.score[p] = sh.failed ? 0 : S;
-        g.rs.a_end[p] = S > 0 && !sh.failed ? key_row(sh.best) : -1;
-        g.rs.b_end[p] = S > 0 && !sh.failed ? key_col(sh.best) : 0;
+      reset();
+      long_sweep<LAZY>(g.ps.a_code + g.ps.a_off[p], 1, M, g.ps.b_code + g.ps.b_off[p], 1, N, M, N, 0, sc, prof, bnd, g.cols, sh,
+                 warp, W);
+      cluster_barrier();
+      if (lead) {
+        const bool failed = vs.failed;
+        const unsigned long long best = vs.best;
+        const int S = failed ? 0 : key_value(best);
+        g.rs.flag[p] = failed ? kFlagTooLong : 0u;
+        g.rs.score[p] = S;
+        g.rs.a_end[p] = S > 0 ? key_row(best) : -1;
+        g.rs.b_end[p] = S > 0 ? key_col(best) : 0;
       }
     }
   }
@@ -332,26 +370,47 @@ constexpr size_t long_smem(int warps) { return (size_t)warps * Prof16<kLK>::byte
 
 template <bool REV>
 cudaError_t launch(LongArgs g, const LongPlan &pl, cudaStream_t st) {
-  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_long<REV>), long_smem(pl.warps));
+  auto kern = g.sc.gap_open >= g.sc.gap_extend ? k_long<REV, true> : k_long<REV, false>;
+  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), long_smem(pl.warps));
   if (e != cudaSuccess) return e;
-  k_long<REV><<<pl.grid, pl.warps * 32, long_smem(pl.warps), st>>>(g);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(pl.clusters * pl.cluster));
+  cfg.blockDim = dim3((unsigned)(pl.warps * 32));
+  cfg.dynamicSmemBytes = long_smem(pl.warps);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)pl.cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, g);
 }
 
 }  // namespace
 
-// Few pairs: 16 warps a block, so a pair's strips all run at once; many: 4, so the SMs stay
-// full with pairs of three strips and more.
+// Blocks of 4 warps, four an SM.  Few pairs: clusters of 8 blocks, so nearly every strip of every
+// pair runs at once and on a scheduler of its own; with more pairs smaller clusters, so the SMs
+// stay full with pairs of three strips and more.
 LongPlan plan_long(int64_t n, int max_b, int sms) {
   LongPlan pl;
-  pl.warps = n <= 2 * (int64_t)sms ? 16 : 4;
+  pl.warps = 4;
+  pl.cluster = n <= sms / 2 ? 8 : n <= sms ? 4 : n <= 2 * (int64_t)sms ? 2 : 1;
   pl.cols = (std::max(max_b, 1) + 63) / 64 * 64;
   const int per_sm = 16 / pl.warps;
-  pl.grid = (int)std::min<int64_t>(n, (int64_t)sms * per_sm);
-  const int64_t fit = (int64_t)(kLongScratch / sizeof(uint32_t)) / (pl.warps * pl.cols);
-  pl.grid = (int)std::max<int64_t>(1, std::min<int64_t>(pl.grid, fit));
-  pl.bytes = (size_t)pl.grid * pl.warps * (size_t)pl.cols * sizeof(uint32_t);
+  const size_t per = (size_t)pl.cluster * pl.warps * (size_t)pl.cols * sizeof(uint32_t) + sizeof(LongShared);
+  pl.clusters = (int)std::min<int64_t>(n, (int64_t)sms * per_sm / pl.cluster);
+  pl.clusters = (int)std::max<int64_t>(1, std::min<int64_t>(pl.clusters, (int64_t)(kLongScratch / per)));
+  pl.bytes = (size_t)pl.clusters * per + 256;
   return pl;
+}
+
+// The clusters' shared words lie in front of their boundary rows.
+static void carve(LongArgs &g, const LongPlan &pl, const WorkLists &wl) {
+  g.shared = reinterpret_cast<LongShared *>(wl.long_bnd);
+  const size_t head = ((size_t)pl.clusters * sizeof(LongShared) + 255) / 256 * 256;
+  g.bnd = wl.long_bnd + head / sizeof(uint32_t);
+  g.cols = pl.cols;
 }
 
 cudaError_t launch_long_forward(const LongPlan &pl, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
@@ -363,8 +422,7 @@ cudaError_t launch_long_forward(const LongPlan &pl, const PairSet &ps, const Res
   g.order = order;
   g.first = first;
   g.next = wl.long_next;
-  g.bnd = wl.long_bnd;
-  g.cols = pl.cols;
+  carve(g, pl, wl);
   return launch<false>(g, pl, st);
 }
 
@@ -378,8 +436,7 @@ cudaError_t launch_long_reverse(const LongPlan &pl, const PairSet &ps, const Res
   g.list_n = wl.wide_count;
   g.list_cap = wl.cap;
   g.next = wl.long_next + 1;
-  g.bnd = wl.long_bnd;
-  g.cols = pl.cols;
+  carve(g, pl, wl);
   return launch<true>(g, pl, st);
 }
 
