@@ -138,6 +138,7 @@ constexpr int64_t kLongBeginPairs = 4096;
 __host__ __device__ inline bool long_begin(int rows, int score) { return rows > kLongRows && score <= kLongScore; }
 struct LongPlan {
   int warps = 0, cluster = 0, clusters = 0;  // warps a block, blocks a cluster, clusters
+  bool spread = false;  // a block an SM
   int64_t cols = 0;
   size_t bytes = 0;
 };

@@ -366,17 +366,20 @@ __global__ void __launch_bounds__(256, 2) k_long(LongArgs g) {
   }
 }
 
-constexpr size_t long_smem(int warps) { return (size_t)warps * Prof16<kLK>::bytes(32); }
+size_t long_smem(const LongPlan &pl) {
+  const size_t need = (size_t)pl.warps * Prof16<kLK>::bytes(32);
+  return pl.spread ? std::max(need, size_t(120) << 10) : need;  // above half an SM's
+}
 
 template <bool REV>
 cudaError_t launch(LongArgs g, const LongPlan &pl, cudaStream_t st) {
   auto kern = g.sc.gap_open >= g.sc.gap_extend ? k_long<REV, true> : k_long<REV, false>;
-  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), long_smem(pl.warps));
+  const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), long_smem(pl));
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(pl.clusters * pl.cluster));
   cfg.blockDim = dim3((unsigned)(pl.warps * 32));
-  cfg.dynamicSmemBytes = long_smem(pl.warps);
+  cfg.dynamicSmemBytes = long_smem(pl);
   cfg.stream = st;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;
@@ -389,15 +392,19 @@ cudaError_t launch(LongArgs g, const LongPlan &pl, cudaStream_t st) {
 
 }  // namespace
 
-// Blocks of 4 warps, four an SM.  Few pairs: clusters of 8 blocks, so nearly every strip of every
-// pair runs at once and on a scheduler of its own; with more pairs smaller clusters, so the SMs
-// stay full with pairs of three strips and more.
+// While there are SMs for it, a block an SM (by its shared memory: the hardware would put a
+// cluster's blocks together otherwise) in clusters of 8 blocks of 4 warps or 4 of 8, so nearly
+// every strip of a pair runs at once and on a scheduler of its own; with many pairs blocks of 4
+// warps, four an SM, which stay full with pairs of three strips and more.  Forward pass of 60
+// pairs of 1-12 kb: clusters of 4 x 8 warps 2.55 ms, 8 x 4 3.15 (and 2.8-3.0 without the spreading),
+// 2 x 8 3.97; of 20 pairs 2.51, 2.08 and 3.95.
 LongPlan plan_long(int64_t n, int max_b, int sms) {
   LongPlan pl;
-  pl.warps = 4;
-  pl.cluster = n <= sms / 2 ? 8 : n <= sms ? 4 : n <= 2 * (int64_t)sms ? 2 : 1;
+  pl.spread = n <= sms;
+  pl.cluster = n <= sms / 8 ? 8 : n <= sms ? 4 : n <= 2 * (int64_t)sms ? 2 : 1;
+  pl.warps = pl.cluster == 4 || pl.cluster == 2 ? 8 : 4;
   pl.cols = (std::max(max_b, 1) + 63) / 64 * 64;
-  const int per_sm = 16 / pl.warps;
+  const int per_sm = pl.spread ? 1 : 16 / pl.warps;
   const size_t per = (size_t)pl.cluster * pl.warps * (size_t)pl.cols * sizeof(uint32_t) + sizeof(LongShared);
   pl.clusters = (int)std::min<int64_t>(n, (int64_t)sms * per_sm / pl.cluster);
   pl.clusters = (int)std::max<int64_t>(1, std::min<int64_t>(pl.clusters, (int64_t)(kLongScratch / per)));
