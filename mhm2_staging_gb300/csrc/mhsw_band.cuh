@@ -48,4 +48,14 @@ __host__ __device__ __forceinline__ void band_sides(int t, int N2, int S, const 
   if (J > g) J = g;
 }
 
+// Whether the warp-per-pair begin kernel (mhsw_short.cu) takes a search: its rows, columns and
+// score fit that kernel's tile and keys.
+constexpr int kWarpBeginRows = 512, kWarpBeginCols = 2048, kWarpBeginScore = 4000;
+__host__ __device__ __forceinline__ bool warp_begin(int M2, int N2, int S, const Scoring &sc) {
+  if (M2 > kWarpBeginRows || S > kWarpBeginScore) return false;
+  int I, J;
+  band_sides(M2, N2, S, sc, I, J);
+  return (M2 + J < N2 ? M2 + J : N2) <= kWarpBeginCols;
+}
+
 }  // namespace mhsw

@@ -451,7 +451,7 @@ int ensure_results(mhsw_driver *d, int64_t n) {
   MHSW_CK(d->l_ovf.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_wide.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_bands.reserve((size_t)n + 1), "cudaMalloc lists");
-  MHSW_CK(d->l_counts.reserve(4 + 2 * mhsw::kBandClasses), "cudaMalloc lists");
+  MHSW_CK(d->l_counts.reserve(5 + 2 * mhsw::kBandClasses), "cudaMalloc lists");
   return MHSW_OK;
 }
 
@@ -630,6 +630,7 @@ mhsw::WorkLists work_lists(mhsw_driver *d, int64_t n) {
   wl.band_counts = d->l_counts.p + 2;
   wl.long_next = d->l_counts.p + 2 + 2 * mhsw::kBandClasses;
   wl.long_bnd = d->long_bnd.p;
+  wl.esc_count = d->l_counts.p + 4 + 2 * mhsw::kBandClasses;
   wl.cap = n;
   return wl;
 }

@@ -151,13 +151,20 @@ __device__ __forceinline__ bool band_outgrown(int t, int N2, int S, const Scorin
   return I > L || J > 2 * G - L;
 }
 
+// The class a search goes to: band_fit's, or the wide list when that is at least top_class and
+// the warp kernel takes it.
+__device__ __forceinline__ int band_route(int S, int M2, int N2, const Scoring &sc, int top_class) {
+  const int c = band_fit(S, M2, N2, sc);
+  return c >= top_class && c < kBandClasses && warp_begin(M2, N2, S, sc) ? kBandClasses : c;
+}
+
 // Band class of pair p (0 .. kBandClasses-1), kBandClasses for the wavefront, or -1 when
 // there is nothing to search (score 0, or a pair the forward pass rejected); those get
 // their begin written here.
 // s_cap: the largest score the band kernels take (the packed int16 kernels hold scores up
 // to kBand16Score); pairs above it go to the wavefront list too.
 // longs: searches over many rows go to the wide list, where the long-pair kernel takes them.
-__device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc, int64_t p, int s_cap, bool longs) {
+__device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc, int64_t p, int s_cap, bool longs, int top_class) {
   const int S = rs.score[p];
   if ((rs.flag[p] & kFlagTooLong) || S <= 0) {
     rs.a_beg[p] = -1;
@@ -165,10 +172,10 @@ __device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc
     return -1;
   }
   if (S > s_cap || (longs && long_begin(band_first_cap(S, sc.match, rs.a_end[p] + 1), S))) return kBandClasses;
-  return band_fit(S, rs.a_end[p] + 1, rs.b_end[p] + 1, sc);
+  return band_route(S, rs.a_end[p] + 1, rs.b_end[p] + 1, sc, top_class);
 }
 
-// Warp-aggregated append of p to list[*count] (one atomic per distinct counter).
+// Warp-aggregated append of p to the end of the list, downwards (one atomic per warp).
 __device__ __forceinline__ void append_agg(int64_t *list, int *count, int64_t cap, int64_t p, bool want) {
   const unsigned act = __activemask();
   const unsigned sel = __ballot_sync(act, want);
@@ -180,19 +187,20 @@ __device__ __forceinline__ void append_agg(int64_t *list, int *count, int64_t ca
   base = __shfl_sync(act, base, leader);
   if (want) {
     const int slot = base + __popc(sel & ((1u << lane32) - 1u));
-    if (slot < cap) list[slot] = p;
+    if (slot < cap) list[cap - 1 - slot] = p;
   }
 }
 
 // Pass 1: count the pairs of each band class.
 __global__ void __launch_bounds__(256) k_rev_count(ResultSet rs, Scoring sc, const uint32_t *__restrict__ order,
-                                                   int64_t n, int *band_counts, int s_cap, bool longs) {
+                                                   int64_t n, int *band_counts, int s_cap, bool longs,
+                                                   int top_class) {
   __shared__ int cnt[kBandClasses];
   if (threadIdx.x < kBandClasses) cnt[threadIdx.x] = 0;
   __syncthreads();
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = order ? (int64_t)order[idx] : idx;
-    const int c = band_class(rs, sc, p, s_cap, longs);
+    const int c = band_class(rs, sc, p, s_cap, longs, top_class);
     if (c >= 0 && c < kBandClasses) atomicAdd(&cnt[c], 1);
   }
   __syncthreads();
@@ -202,7 +210,8 @@ __global__ void __launch_bounds__(256) k_rev_count(ResultSet rs, Scoring sc, con
 // Pass 2: place each pair in its class segment (segments in class order, each filled in
 // the batch's order); wider pairs go to the wavefront list.
 __global__ void __launch_bounds__(256) k_rev_scatter(ResultSet rs, Scoring sc, const uint32_t *__restrict__ order,
-                                                     int64_t n, WorkLists wl, int s_cap, bool longs) {
+                                                     int64_t n, WorkLists wl, int s_cap, bool longs,
+                                                     int top_class) {
   int off[kBandClasses];
   int acc = 0;
 #pragma unroll
@@ -218,7 +227,7 @@ __global__ void __launch_bounds__(256) k_rev_scatter(ResultSet rs, Scoring sc, c
     if (!((rs.flag[p] & kFlagTooLong) || S <= 0)) {
       const int M2 = rs.a_end[p] + 1;
       c = S > s_cap || (longs && long_begin(band_first_cap(S, sc.match, M2), S)) ? kBandClasses
-                                                                                 : band_fit(S, M2, rs.b_end[p] + 1, sc);
+                                                                                 : band_route(S, M2, rs.b_end[p] + 1, sc, top_class);
     }
     // one append per class present in the warp: lanes of a class share one atomic
     const unsigned act = __activemask();
@@ -443,7 +452,7 @@ __global__ void __launch_bounds__(128) k_rev_band(PairSet ps, ResultSet rs, Scor
       if (found || t >= M2) break;
       t = cap_rows(2 * t);
     }
-    append_agg(wl.wide, wl.wide_count, wl.cap, p, escalate);
+    append_agg(wl.wide, wl.esc_count, wl.cap, p, escalate);
     if (escalate) continue;
     if (!found || fi >= M2 || fj < 0 || fj >= N2) {
       rs.flag[p] |= kFlagTooLong;  // inconsistent; reported as an error by the driver
@@ -627,7 +636,7 @@ __global__ void __launch_bounds__(128) k_rev_band16(PairSet ps, ResultSet rs, Sc
       if (found || t >= M2) break;
       t = cap_rows(2 * t);
     }
-    append_agg(wl.wide, wl.wide_count, wl.cap, p, escalate);
+    append_agg(wl.wide, wl.esc_count, wl.cap, p, escalate);
     if (escalate) continue;
     if (!found || fi < 0 || fi >= M2 || fj < 0 || fj >= N2) {
       rs.flag[p] |= kFlagTooLong;  // inconsistent; reported as an error by the driver
@@ -711,7 +720,7 @@ constexpr int kWaveScore16 = 16000;
 template <class VT, int K, int G>
 __global__ void __launch_bounds__(256) k_rev_wave(PairSet ps, ResultSet rs, Scoring sc, WorkLists wl,
                                                   typename VT::Pay *scratch, int scratch_stride, int pad, int bcap,
-                                                  int s_lo, int s_hi, bool longs) {
+                                                  int s_lo, int s_hi, bool longs, bool warps) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lanes = blockDim.x;
   const int gpb = lanes / G;
@@ -727,17 +736,20 @@ __global__ void __launch_bounds__(256) k_rev_wave(PairSet ps, ResultSet rs, Scor
   gs.pad = pad;
   gs.bcap = bcap;
   constexpr int RS = 2 * K * G;
-  const int64_t total = *wl.wide_count < wl.cap ? *wl.wide_count : wl.cap;
+  const int64_t listed = *wl.wide_count < wl.cap ? *wl.wide_count : wl.cap;
+  const int64_t total = listed + *wl.esc_count;
   const int64_t gid = (int64_t)blockIdx.x * gpb + grp;
   const int64_t gstride = (int64_t)gridDim.x * gpb;
   typename VT::Pay *bnd = scratch ? scratch + gid * (int64_t)scratch_stride : nullptr;
   for (int64_t i = gid; i < total; i += gstride) {
-    const int64_t p = wl.wide[i];
+    const int64_t p = wl.wide[i < listed ? i : wl.cap - 1 - (i - listed)];
     const int S = rs.score[p];
     if (S < s_lo || S > s_hi) continue;
     const int ie = rs.a_end[p], je = rs.b_end[p];
     const int M2 = ie + 1;
-    if (longs && long_begin(band_first_cap(S, sc.match, M2), S)) continue;
+    if (i < listed && ((longs && long_begin(band_first_cap(S, sc.match, M2), S)) ||
+                       (warps && warp_begin(M2, je + 1, S, sc))))
+      continue;  // taken by the long-pair or the warp kernel
     const int dmax = M2 < je + 1 ? M2 : je + 1;
     const long long gbl = gap_cells_bound(dmax, S, sc);
     long long n2 = (long long)M2 + gbl + 1;
@@ -810,6 +822,7 @@ __global__ void k_pack5(ResultSet rs, int64_t n, int32_t *out5) {
 __global__ void k_reset_lists(WorkLists wl) {
   *wl.ovf_count = 0;
   *wl.wide_count = 0;
+  *wl.esc_count = 0;
   for (int i = 0; i < 2 * kBandClasses; i++) wl.band_counts[i] = 0;
   wl.long_next[0] = wl.long_next[1] = 0;
 }
@@ -981,28 +994,28 @@ static bool wave_launch_ok(FwdConfig c, int max_a, void *scratch, size_t scratch
 template <class VT, int K>
 static cudaError_t launch_rev_wave_t(FwdConfig c, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
                                      const WorkLists &wl, void *scratch, size_t scratch_bytes, int max_a, int sms,
-                                     int s_lo, int s_hi, bool longs, cudaStream_t st) {
+                                     int s_lo, int s_hi, bool longs, bool warps, cudaStream_t st) {
   typename VT::Pay *scr = nullptr;
   // without scratch, pairs longer than a strip are reported (kFlagTooLong), as before
   wave_plan<VT>(c, max_a, scratch, scratch_bytes, sms, &scr);
   auto kern = k_rev_wave<VT, K, kG>;
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), c.smem);
   if (e != cudaSuccess) return e;
-  kern<<<c.grid, c.groups_per_block * kG, c.smem, st>>>(ps, rs, sc, wl, scr, c.bcap, c.pad, c.bcap, s_lo, s_hi, longs);
+  kern<<<c.grid, c.groups_per_block * kG, c.smem, st>>>(ps, rs, sc, wl, scr, c.bcap, c.pad, c.bcap, s_lo, s_hi, longs, warps);
   return cudaGetLastError();
 }
 
 static cudaError_t launch_rev_wave16(const FwdConfig &c, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
                                      const WorkLists &wl, void *scratch, size_t scratch_bytes, int max_a, int sms,
-                                     bool longs, cudaStream_t st) {
+                                     bool longs, bool warps, cudaStream_t st) {
   switch (c.K) {
-    case 2: return launch_rev_wave_t<V16, 2>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
-    case 3: return launch_rev_wave_t<V16, 3>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
-    case 4: return launch_rev_wave_t<V16, 4>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
-    case 5: return launch_rev_wave_t<V16, 5>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
-    case 6: return launch_rev_wave_t<V16, 6>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
-    case 7: return launch_rev_wave_t<V16, 7>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
-    default: return launch_rev_wave_t<V16, 8>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, st);
+    case 2: return launch_rev_wave_t<V16, 2>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
+    case 3: return launch_rev_wave_t<V16, 3>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
+    case 4: return launch_rev_wave_t<V16, 4>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
+    case 5: return launch_rev_wave_t<V16, 5>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
+    case 6: return launch_rev_wave_t<V16, 6>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
+    case 7: return launch_rev_wave_t<V16, 7>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
+    default: return launch_rev_wave_t<V16, 8>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
   }
 }
 
@@ -1011,6 +1024,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
                            const uint32_t *order, const Forks *fk) {
   const int sms = num_sms(device);
   const bool longs = max_a > kLongRows && wl.long_bnd && keyed_scoring(sc);
+  const bool warps = keyed_scoring(sc) && sc.gap_open >= sc.gap_extend;  // (the warp kernel's step)
   if (ps.n > 0) {
     const int grid = (int)std::min<int64_t>((ps.n + 255) / 256, (int64_t)sms * 8);
     const int gridb = sms * 8;
@@ -1022,14 +1036,19 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
                     sc.match + sc.gap_open <= 255;
     const int s_cap = bi ? kBand16Score : 0x7fffffff;
     const bool force = longs && ps.n <= kLongBeginPairs;
-    k_rev_count<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl.band_counts, s_cap, force);
-    k_rev_scatter<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap, force);
+    const int top_class = warps && ps.n <= kWarpBeginPairs ? kBandClasses - 2 : kBandClasses;
+    k_rev_count<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl.band_counts, s_cap, force, top_class);
+    k_rev_scatter<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap, force, top_class);
     // The classes are independent: with side streams they run concurrently, so the
     // latency-bound narrow classes share the SMs with the wide ones.
     cudaStream_t cs[kBandClasses];
     const bool fan = fk && fk->fork;
     if (fan) {
-      cudaError_t e = fork_to(*fk, st, kBandClasses);
+      cudaError_t e = fork_to(*fk, st, kBandClasses + 1);
+      if (e != cudaSuccess) return e;
+    }
+    if (warps) {
+      const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, longs, fan ? fk->side[kBandClasses] : st);
       if (e != cudaSuccess) return e;
     }
     for (int c = 0; c < kBandClasses; c++) cs[c] = fan ? fk->side[c] : st;
@@ -1053,7 +1072,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (fan) {
-      e = join_from(*fk, st, kBandClasses);
+      e = join_from(*fk, st, kBandClasses + 1);
       if (e != cudaSuccess) return e;
     }
   }
@@ -1061,7 +1080,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
     const cudaError_t e = launch_long_reverse(plan_long(ps.n, max_b, sms), ps, rs, sc, wl, st);
     if (e != cudaSuccess) return e;
   }
-  // Wide bands: wavefront on the reversed box (count read on the device), in int16 for
+  // Searches no kernel took so far: wavefront on the reversed box (counts read on the device), in int16 for
   // scores up to kWaveScore16 where a strip plan with scratch exists, int32 otherwise.
   FwdConfig c16, c32;
   cudaError_t e = plan_forward(device, max_a, max_b, false, &c16);
@@ -1070,11 +1089,11 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
   if (e != cudaSuccess) return e;
   int split = 0;  // largest score the int16 launch takes
   if (wave_launch_ok<V16>(c16, max_a, scratch, scratch_bytes, sms)) {
-    e = launch_rev_wave16(c16, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, longs, st);
+    e = launch_rev_wave16(c16, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, longs, warps, st);
     if (e != cudaSuccess) return e;
     split = kWaveScore16;
   }
-  return launch_rev_wave_t<V32, 4>(c32, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, split + 1, 0x7fffffff, longs, st);
+  return launch_rev_wave_t<V32, 4>(c32, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, split + 1, 0x7fffffff, longs, warps, st);
 }
 
 cudaError_t raise_smem_limit(const void *func, size_t bytes) {

@@ -15,8 +15,10 @@ constexpr int kBandClasses = 7;  // banded begin-pass instantiations (half-width
 struct WorkLists {
   int64_t *ovf;       // pairs whose int16 forward pass crossed the ceiling
   int *ovf_count;
-  int64_t *wide;      // pairs whose reverse band is wider than the banded kernels handle
+  int64_t *wide;      // pairs whose reverse band is wider than the banded kernels handle, and from
+                      // the end (wide[cap - 1] down) those that outgrew theirs on the way
   int *wide_count;
+  int *esc_count;
   int64_t *bands;     // begin-pass pairs grouped by band class (one segment per class)
   int *band_counts;   // kBandClasses pair counts, then kBandClasses scatter cursors
   int64_t cap;        // capacity of each list
@@ -124,6 +126,12 @@ bool may_need_int32(const Scoring &sc, int ceiling, int max_a, int max_b);
 
 // Packs results into n x 5 int32 rows (score, a_beg, a_end, b_beg, b_end).
 cudaError_t launch_pack5(const ResultSet &rs, int64_t n, int32_t *out5, cudaStream_t st);
+
+// Begin searches of the wide list by a warp each (mhsw_short.cu), where warp_begin holds.
+// Batches up to this size send the two widest band classes there too.
+constexpr int64_t kWarpBeginPairs = 40000;
+cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const WorkLists &wl, int sms,
+                            bool longs, cudaStream_t st);
 
 // ---- long pairs (mhsw_long.cu) -------------------------------------------------------
 // A pair with more rows than this (and, in the begin pass, a search whose first row cap is

@@ -356,7 +356,56 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
   }
 }
 
+// Begin searches of the wide list, a warp each: bands wider than the banded kernels hold, and (in
+// batches up to kWarpBeginPairs) the widest of their classes, whose threads walk a row pair in
+// 0.5 us -- 250 rows took 130-160 us however few the pairs.  Same search as k_short's.
+__global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scoring sc, WorkLists wl, bool longs) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint32_t *prof = reinterpret_cast<uint32_t *>(smem);
+  uint8_t *bc = smem + Prof16<8>::bytes(32) + kShortPad;  // reversed: bc[j] = column j of the box
+  const int lane = threadIdx.x;
+  const uint32_t one = (uint32_t)(sc.gap_open >> 30) + 1u;  // a 1 the compiler cannot fold
+  const int64_t total = *wl.wide_count < wl.cap ? *wl.wide_count : wl.cap;
+  for (int64_t it = blockIdx.x; it < total; it += gridDim.x) {
+    const int64_t p = wl.wide[it];
+    const int S = rs.score[p], ie = rs.a_end[p], je = rs.b_end[p];
+    const int M2 = ie + 1, N2 = je + 1;
+    if ((longs && long_begin(band_first_cap(S, sc.match, M2), S)) || !warp_begin(M2, N2, S, sc)) continue;
+    const uint8_t *a = ps.a_code + ps.a_off[p] + ie, *b = ps.b_code + ps.b_off[p] + je;
+    unsigned long long q = 0ull;
+    for (int t = band_first_cap(S, sc.match, M2);; t = M2) {
+      int I, J;
+      band_sides(t, N2, S, sc, I, J);
+      const int n2 = t + J < N2 ? t + J : N2;
+      __syncwarp();
+      for (int j = lane - kShortPad; j < n2 + kShortPad; j += 32)
+        bc[j] = (uint8_t)((unsigned)j < (unsigned)n2 ? (int)b[-j] : kCodeN);
+      __syncwarp();
+      q = sweep_rows<8, false>(t, n2, [&](int i) { return (int)a[-i]; }, bc, 1, sc, prof, lane, one, nullptr);
+      if (key_value(q) == S || t == M2) break;
+    }
+    if (lane == 0) {
+      if (key_value(q) != S) {
+        rs.flag[p] |= kFlagTooLong;  // inconsistent
+        rs.a_beg[p] = -1;
+        rs.b_beg[p] = 0;
+      } else {
+        rs.a_beg[p] = ie - key_row(q);
+        rs.b_beg[p] = je - key_col(q);
+      }
+    }
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const WorkLists &wl, int sms,
+                            bool longs, cudaStream_t st) {
+  constexpr size_t smem = Prof16<8>::bytes(32) + 2 * kShortPad + kWarpBeginCols;
+  const int64_t grid = std::min<int64_t>(ps.n, (int64_t)sms * 12);
+  k_rev_warp<<<(unsigned)grid, 32, smem, st>>>(ps, rs, sc, wl, longs);
+  return cudaGetLastError();
+}
 
 bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b) {
   return n <= kShortPairs && n * (int64_t)max_b <= kShortColumns && sc.gap_open >= sc.gap_extend && max_a <= kShortRowsMax && max_b <= kShortColsMax && keyed_scoring(sc) &&
