@@ -747,8 +747,8 @@ __global__ void __launch_bounds__(256) k_rev_wave(PairSet ps, ResultSet rs, Scor
     if (S < s_lo || S > s_hi) continue;
     const int ie = rs.a_end[p], je = rs.b_end[p];
     const int M2 = ie + 1;
-    if (i < listed && ((longs && long_begin(band_first_cap(S, sc.match, M2), S)) ||
-                       (warps && warp_begin(M2, je + 1, S, sc))))
+    if ((i < listed && longs && long_begin(band_first_cap(S, sc.match, M2), S)) ||
+        (warps && warp_begin(M2, je + 1, S, sc)))
       continue;  // taken by the long-pair or the warp kernel
     const int dmax = M2 < je + 1 ? M2 : je + 1;
     const long long gbl = gap_cells_bound(dmax, S, sc);
@@ -1036,7 +1036,11 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
                     sc.match + sc.gap_open <= 255;
     const int s_cap = bi ? kBand16Score : 0x7fffffff;
     const bool force = longs && ps.n <= kLongBeginPairs;
-    const int top_class = warps && ps.n <= kWarpBeginPairs ? kBandClasses - 2 : kBandClasses;
+    // The narrowest class that goes to the warp kernel: it costs about ten times a banded
+    // search's instructions but not a thread's latency.  Begin pass, classes 7 / 5 / 4 / 3 from:
+    // 9000 mixed pairs 184 / 135 / 127 / 123 us, 20,000 220 / 180 / 214 / 239, 100,000 uneven
+    // 362 / 324 / 463 / 733, 800,000 1390 / 1707 / 2680 / 4952.
+    const int top_class = !warps || ps.n > 250000 ? kBandClasses : ps.n > 12000 ? 5 : 4;
     k_rev_count<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl.band_counts, s_cap, force, top_class);
     k_rev_scatter<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap, force, top_class);
     // The classes are independent: with side streams they run concurrently, so the
@@ -1048,7 +1052,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
       if (e != cudaSuccess) return e;
     }
     if (warps) {
-      const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, longs, fan ? fk->side[kBandClasses] : st);
+      const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, longs, false, fan ? fk->side[kBandClasses] : st);
       if (e != cudaSuccess) return e;
     }
     for (int c = 0; c < kBandClasses; c++) cs[c] = fan ? fk->side[c] : st;
@@ -1080,6 +1084,14 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
     const cudaError_t e = launch_long_reverse(plan_long(ps.n, max_b, sms), ps, rs, sc, wl, st);
     if (e != cudaSuccess) return e;
   }
+  if (warps && ps.n > 0) {
+    const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, longs, true, st);
+    if (e != cudaSuccess) return e;
+  }
+  // every search fits the warp kernel's tile and keys: nothing is left
+  if (warps && max_a <= kWarpBeginRows && max_b <= kWarpBeginCols &&
+      (long long)std::min(max_a, max_b) * sc.match <= kWarpBeginScore)
+    return cudaSuccess;
   // Searches no kernel took so far: wavefront on the reversed box (counts read on the device), in int16 for
   // scores up to kWaveScore16 where a strip plan with scratch exists, int32 otherwise.
   FwdConfig c16, c32;

@@ -127,11 +127,10 @@ bool may_need_int32(const Scoring &sc, int ceiling, int max_a, int max_b);
 // Packs results into n x 5 int32 rows (score, a_beg, a_end, b_beg, b_end).
 cudaError_t launch_pack5(const ResultSet &rs, int64_t n, int32_t *out5, cudaStream_t st);
 
-// Begin searches of the wide list by a warp each (mhsw_short.cu), where warp_begin holds.
-// Batches up to this size send the two widest band classes there too.
-constexpr int64_t kWarpBeginPairs = 40000;
+// Begin searches of the wide list (escaped: those that outgrew their band) by a warp each
+// (mhsw_short.cu), where warp_begin holds.
 cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const WorkLists &wl, int sms,
-                            bool longs, cudaStream_t st);
+                            bool longs, bool escaped, cudaStream_t st);
 
 // ---- long pairs (mhsw_long.cu) -------------------------------------------------------
 // A pair with more rows than this (and, in the begin pass, a search whose first row cap is

@@ -356,21 +356,23 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
   }
 }
 
-// Begin searches of the wide list, a warp each: bands wider than the banded kernels hold, and (in
-// batches up to kWarpBeginPairs) the widest of their classes, whose threads walk a row pair in
+// Begin searches of the wide list, a warp each: bands wider than the banded kernels hold, those
+// that outgrew theirs, and in all but the largest batches the widest of their classes, whose threads walk a row pair in
 // 0.5 us -- 250 rows took 130-160 us however few the pairs.  Same search as k_short's.
-__global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scoring sc, WorkLists wl, bool longs) {
+__global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scoring sc, WorkLists wl, bool longs,
+                                                 bool escaped) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t *prof = reinterpret_cast<uint32_t *>(smem);
   uint8_t *bc = smem + Prof16<8>::bytes(32) + kShortPad;  // reversed: bc[j] = column j of the box
   const int lane = threadIdx.x;
   const uint32_t one = (uint32_t)(sc.gap_open >> 30) + 1u;  // a 1 the compiler cannot fold
-  const int64_t total = *wl.wide_count < wl.cap ? *wl.wide_count : wl.cap;
+  // escaped: the searches that outgrew their band, from the end of the list
+  const int64_t total = escaped ? *wl.esc_count : *wl.wide_count < wl.cap ? *wl.wide_count : wl.cap;
   for (int64_t it = blockIdx.x; it < total; it += gridDim.x) {
-    const int64_t p = wl.wide[it];
+    const int64_t p = wl.wide[escaped ? wl.cap - 1 - it : it];
     const int S = rs.score[p], ie = rs.a_end[p], je = rs.b_end[p];
     const int M2 = ie + 1, N2 = je + 1;
-    if ((longs && long_begin(band_first_cap(S, sc.match, M2), S)) || !warp_begin(M2, N2, S, sc)) continue;
+    if ((longs && !escaped && long_begin(band_first_cap(S, sc.match, M2), S)) || !warp_begin(M2, N2, S, sc)) continue;
     const uint8_t *a = ps.a_code + ps.a_off[p] + ie, *b = ps.b_code + ps.b_off[p] + je;
     unsigned long long q = 0ull;
     for (int t = band_first_cap(S, sc.match, M2);; t = M2) {
@@ -400,10 +402,10 @@ __global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scori
 }  // namespace
 
 cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const WorkLists &wl, int sms,
-                            bool longs, cudaStream_t st) {
+                            bool longs, bool escaped, cudaStream_t st) {
   constexpr size_t smem = Prof16<8>::bytes(32) + 2 * kShortPad + kWarpBeginCols;
   const int64_t grid = std::min<int64_t>(ps.n, (int64_t)sms * 12);
-  k_rev_warp<<<(unsigned)grid, 32, smem, st>>>(ps, rs, sc, wl, longs);
+  k_rev_warp<<<(unsigned)grid, 32, smem, st>>>(ps, rs, sc, wl, longs, escaped);
   return cudaGetLastError();
 }
 
