@@ -34,9 +34,11 @@ __device__ __forceinline__ unsigned group_mask_b(int G) {
 // Persistent forward kernel over one range of the sorted pair order: 8-lane groups for
 // the short-read buckets (items [0, split)), 16-lane groups for the rest ([split, n)).
 // A group claims its next pair from the range's atomic counter.
-// HALF: no pair's score can exceed kHalfCap.
+// HALF: no pair's score can exceed kHalfCap.  The 16-lane kernel in half mode is held to 102
+// registers (640 threads an SM: five blocks of 128 instead of four; 30,011 pairs against
+// 2-8 kb 6.98 -> 6.85 ms, 150,001 mixed reads 3.40 -> 3.34); the others lose or spill there.
 template <int G, bool S2, bool HALF>
-__global__ void __launch_bounds__(256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
+__global__ void __launch_bounds__(G == kGKLong && HALF && !S2 ? 640 : 256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
                                                      const uint32_t *__restrict__ order, int *queue, int lane_rows,
                                                      bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap,
                                                      V16::Pay *scratch, int scratch_stride) {
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(256) k_fwd_persist(PairSet ps, ResultSet rs, S
   const int lane = threadIdx.x % G;
   const unsigned gmask = group_mask_b(G);
   constexpr int kC = S2 ? kCode16Zero + 1 : kCodeN + 1;
-  constexpr size_t kProf = kShort ? group_prof16_bytes<10, G, kC>() : group_prof16_bytes<8, G, kC>();
+  constexpr size_t kProf = kShort ? group_prof16_bytes<10, G, kC, HALF>() : group_prof16_bytes<8, G, kC, HALF>();
   unsigned char *gbase = smem + (size_t)grp * kProf;  // keyed engine: profile table only
   GroupSmem gs;
   gs.prof = reinterpret_cast<uint32_t *>(gbase);
@@ -224,15 +226,21 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     return 1;
   }
   const bool s2 = ps.rowmax16 != nullptr;
-  // Half mode where the scores allow it, except in the 8-lane kernel outside score2 mode
-  // (800,000 uneven pairs: forward pass 13.33 ms with it, 13.22 without).
+  // half mode where the scores allow it
   const bool half = (long long)std::min(max_a, max_b) * sc.match <= kHalfCap;
   auto kshort = s2 ? (half ? k_fwd_persist<kGKShort, true, true> : k_fwd_persist<kGKShort, true, false>)
-                   : k_fwd_persist<kGKShort, false, false>;
+                   : (half ? k_fwd_persist<kGKShort, false, true> : k_fwd_persist<kGKShort, false, false>);
   auto klong = s2 ? (half ? k_fwd_persist<kGKLong, true, true> : k_fwd_persist<kGKLong, true, false>)
                   : (half ? k_fwd_persist<kGKLong, false, true> : k_fwd_persist<kGKLong, false, false>);
-  const size_t prof_short = s2 ? group_prof16_bytes<10, kGKShort, kCode16Zero + 1>() : group_prof16_bytes<10, kGKShort>();
-  const size_t prof_long = s2 ? group_prof16_bytes<8, kGKLong, kCode16Zero + 1>() : group_prof16_bytes<8, kGKLong>();
+  // profile table of a group, one of (codes, form)
+  auto prof_of = [&](auto full, auto full_s2, auto half_w, auto half_s2) -> size_t {
+    return half ? (s2 ? half_s2 : half_w) : (s2 ? full_s2 : full);
+  };
+  constexpr int kZ = kCode16Zero + 1, kN = kCodeN + 1;
+  const size_t prof_short = prof_of(group_prof16_bytes<10, kGKShort, kN>(), group_prof16_bytes<10, kGKShort, kZ>(),
+                                    group_prof16_bytes<10, kGKShort, kN, true>(), group_prof16_bytes<10, kGKShort, kZ, true>());
+  const size_t prof_long = prof_of(group_prof16_bytes<8, kGKLong, kN>(), group_prof16_bytes<8, kGKLong, kZ>(),
+                                   group_prof16_bytes<8, kGKLong, kN, true>(), group_prof16_bytes<8, kGKLong, kZ, true>());
   // long pairs take blocks of their own (not in score2 mode, which needs their row maxima, nor
   // under a lowered int16 ceiling, which asks for the int32 pass)
   const bool longs = max_a > kLongRows && !s2 && wl.long_bnd && ceiling >= kCeiling16;

@@ -46,9 +46,10 @@
 // first normal binade above, with one spacing -- so adding patterns with fp16 adds is exact
 // integer arithmetic while sums stay below 2048, and the integer maxima order them as
 // before.  The two adds forming Hdiag + s + gO and the relu(m - gO) then run on the FMA
-// pipe at twice the rate of the integer multiply-adds and off the DPX pipe.  Measured
-// (forward pass, integer form -> half): 30,011 pairs of 250 bp against 2-8 kb 7.34 -> 7.06 ms,
-// 150,001 mixed reads 3.53 -> 3.44 ms; the relu alone or the adds alone gain less or lose.
+// pipe at twice the rate of the integer multiply-adds and off the DPX pipe.  As fused
+// multiply-adds by (1, 0) and (0, 1) the two adds also pick their half of a word, so the
+// table holds one word per row pair instead of two (Prof16H): the integer form's loads kept
+// the shared-memory pipe 70% busy next to 71% of the issue slots.
 //
 // Score2 mode (S2) also produces what SSW's second-best score is computed from
 // (ssw_core.cpp:489, :513-536): each A row's maximum of H, over B extended to P columns
@@ -88,9 +89,24 @@ struct Prof16 {
   __host__ __device__ static constexpr int hi_elem(int w) { return w < 4 * kQ ? w % 4 : 2 + w - 4 * kQ; }
 };
 
-template <int KMAX, int G, int CODES = kCodeN + 1>
+// Half mode's table: one word per row pair (low row's score in the low half, high row's in the
+// high half); a step's adds take one half each of this column's and the last column's words.
+template <int K, int CODES = kCodeN + 1>
+struct Prof16H {
+  static_assert(K % 2 == 0, "row pairs per lane must be even");
+  static constexpr int kCodes = CODES;
+  static constexpr int kQ = K / 4;            // 128-bit vectors per (code, lane), then
+  static constexpr bool kRem = (K % 4) != 0;  // one 64-bit vector
+  __host__ __device__ static constexpr size_t bytes(int lanes) { return (size_t)kCodes * K * lanes * 4; }
+  // word w of (code c, lane): the 128-bit vectors of a code lie [q][lane], the 64-bit ones after them
+  __host__ __device__ static constexpr int word(int c, int w, int lane, int lanes) {
+    return c * K * lanes + (w < 4 * kQ ? ((w / 4) * lanes + lane) * 4 + w % 4 : 4 * kQ * lanes + lane * 2 + (w - 4 * kQ));
+  }
+};
+
+template <int KMAX, int G, int CODES = kCodeN + 1, bool HALF = false>
 __host__ __device__ constexpr size_t group_prof16_bytes() {
-  return Prof16<KMAX, CODES>::bytes(G);
+  return HALF ? Prof16H<KMAX, CODES>::bytes(G) : Prof16<KMAX, CODES>::bytes(G);
 }
 
 // Where score2 mode writes the row maxima (rowmax[row] for the pair's A rows) and the
@@ -103,9 +119,15 @@ struct RowMaxOut {
 // Largest score bound of half mode: H + s + gO < 2048 with match and gO at most 127.
 constexpr int kHalfCap = 1792;
 
-__device__ __forceinline__ uint32_t add_f16x2(uint32_t a, uint32_t b) {
+// a + the low (high) half of w
+__device__ __forceinline__ uint32_t add_lo_f16x2(uint32_t a, uint32_t w) {
   uint32_t r;
-  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0x00003C00u), "r"(a));
+  return r;
+}
+__device__ __forceinline__ uint32_t add_hi_f16x2(uint32_t a, uint32_t w) {
+  uint32_t r;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0x3C000000u), "r"(a));
   return r;
 }
 // relu(a + c) of fp16 pairs (a * 1 + c)
@@ -169,7 +191,7 @@ struct Step16 {
       // halves never carry: all terms >= 0, sum < 2^15.  Written as multiply-adds by a
       // runtime 1 so they issue on the FMA pipe, not the integer ALU pipe the DP saturates.
       uint32_t Q, Hn;
-      if constexpr (HALF) Q = add_f16x2(add_f16x2(Hd, Wlo[k]), Phi[k]);
+      if constexpr (HALF) Q = add_hi_f16x2(add_lo_f16x2(Hd, Wlo[k]), Phi[k]);
       else Q = mad_u32(mad_u32(Hd, one, Wlo[k]), one, Phi[k]);
       const uint32_t m = __vimax3_s16x2(Q, Ev, F[k]);
       if constexpr (HALF) Hn = add_relu_f16x2(m, NGO);
@@ -192,6 +214,24 @@ struct Step16 {
     const uint32_t tt = (uint32_t)t * 0x00010001u;
     Jp = (msk & tt) | (~msk & Jp);
     Kl = Kn;
+  }
+  // Half mode: the words of code c (Wlo of this step, Phi of the next).
+  __device__ static __forceinline__ void load_half(const uint32_t *tab, int c, int lane, uint32_t (&W)[K]) {
+    using LH = Prof16H<K, L::kCodes>;
+    const uint32_t *b = tab + c * (K * G);
+#pragma unroll
+    for (int q = 0; q < LH::kQ; q++) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(b + (q * G + lane) * 4);
+      W[4 * q + 0] = v.x;
+      W[4 * q + 1] = v.y;
+      W[4 * q + 2] = v.z;
+      W[4 * q + 3] = v.w;
+    }
+    if constexpr (LH::kRem) {
+      const uint2 v = *reinterpret_cast<const uint2 *>(b + 4 * LH::kQ * G + lane * 2);
+      W[K - 2] = v.x;
+      W[K - 1] = v.y;
+    }
   }
   // Words of code c: low words into Wlo (used at this step), high words into Whi (used
   // at the next step by the high half).
@@ -263,6 +303,10 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
           const int shi = (S2 && c == kCode16Zero) ? (ahi == kCodePad ? -sc.gap_open : 0) : sub_score(ahi, c, sc, sc.gap_open);
           const uint32_t vlo = (uint32_t)(slo + sc.gap_open) & 0xffffu;
           const uint32_t vhi = ((uint32_t)(shi + sc.gap_open) & 0xffffu) << 16;
+          if constexpr (HALF) {
+            tw[Prof16H<K, L::kCodes>::word(c, w, lane, G)] = vlo | vhi;
+            continue;
+          }
           tw[((c * L::kNV + L::lo_vec(w)) * G + lane) * 4 + L::lo_elem(w)] = vlo;
           tw[((c * L::kNV + L::hi_vec(w)) * G + lane) * 4 + L::hi_elem(w)] = vhi;
         }
@@ -331,17 +375,19 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
       // even step: hi words into HA; the high half uses HB (previous column)
       int c = ceven;
       ceven = kGuard ? code_at(t + 2 + j0) : (int)bl[t + 2];
-      ST::load(tab, c, lane, Wlo, HA);
+      if constexpr (HALF) ST::load_half(gs.prof, c, lane, HA);
+      else ST::load(tab, c, lane, Wlo, HA);
       uint32_t zH, zE;
       top(t, zH, zE);
-      ST::run(t, zH, zE, sel, Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm, vmask_at(t));
+      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm, vmask_at(t));
       out_bnd(t);
       // odd step: hi words into HB; the high half uses HA
       c = codd;
       codd = kGuard ? code_at(t + 3 + j0) : (int)bl[t + 3];
-      ST::load(tab, c, lane, Wlo, HB);
+      if constexpr (HALF) ST::load_half(gs.prof, c, lane, HB);
+      else ST::load(tab, c, lane, Wlo, HB);
       top(t + 1, zH, zE);
-      ST::run(t + 1, zH, zE, sel, Wlo, HA, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm,
+      ST::run(t + 1, zH, zE, sel, HALF ? HB : Wlo, HA, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm,
               vmask_at(t + 1));
       out_bnd(t + 1);
     };
@@ -361,10 +407,11 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
     }
     for (; t + 1 < T_end; t += 2) two_steps(std::true_type{});
     if (t < T_end) {
-      ST::load(tab, ceven, lane, Wlo, HA);
+      if constexpr (HALF) ST::load_half(gs.prof, ceven, lane, HA);
+      else ST::load(tab, ceven, lane, Wlo, HA);
       uint32_t zH, zE;
       top(t, zH, zE);
-      ST::run(t, zH, zE, sel, Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm, vmask_at(t));
+      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm, vmask_at(t));
       out_bnd(t);
     }
 

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(128)
   const int grp = threadIdx.x / G, lane = threadIdx.x % G;
   const unsigned gmask = ((1u << G) - 1u) << (((threadIdx.x & 31) / G) * G);
   GroupSmem gs;
-  gs.prof = reinterpret_cast<uint32_t *>(smem + (size_t)grp * group_prof16_bytes<kPer, G>());
+  gs.prof = reinterpret_cast<uint32_t *>(smem + (size_t)grp * group_prof16_bytes<kPer, G, kCodeN + 1, HALF>());
   gs.prof_lanes = G;
   gs.bcodes = nullptr;
   gs.pad = 0;
