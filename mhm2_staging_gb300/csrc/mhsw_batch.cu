@@ -34,11 +34,11 @@ __device__ __forceinline__ unsigned group_mask_b(int G) {
 // Persistent forward kernel over one range of the sorted pair order: 8-lane groups for
 // the short-read buckets (items [0, split)), 16-lane groups for the rest ([split, n)).
 // A group claims its next pair from the range's atomic counter.
-// HALF: no pair's score can exceed kHalfCap.  The 16-lane kernel in half mode is held to 102
+// MODE: the engine's (mhsw_engine16.cuh).  The 16-lane kernel in the half modes is held to 102
 // registers (640 threads an SM: five blocks of 128 instead of four; 30,011 pairs against
 // 2-8 kb 6.98 -> 6.85 ms, 150,001 mixed reads 3.40 -> 3.34); the others lose or spill there.
-template <int G, bool S2, bool HALF>
-__global__ void __launch_bounds__(G == kGKLong && HALF && !S2 ? 640 : 256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
+template <int G, bool S2, int MODE>
+__global__ void __launch_bounds__(G == kGKLong && MODE != kModeInt && !S2 ? 640 : 256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
                                                      const uint32_t *__restrict__ order, int *queue, int lane_rows,
                                                      bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap,
                                                      V16::Pay *scratch, int scratch_stride) {
@@ -49,7 +49,8 @@ __global__ void __launch_bounds__(G == kGKLong && HALF && !S2 ? 640 : 256) k_fwd
   const int lane = threadIdx.x % G;
   const unsigned gmask = group_mask_b(G);
   constexpr int kC = S2 ? kCode16Zero + 1 : kCodeN + 1;
-  constexpr size_t kProf = kShort ? group_prof16_bytes<10, G, kC, HALF>() : group_prof16_bytes<8, G, kC, HALF>();
+  constexpr size_t kProf = kShort ? group_prof16_bytes<10, G, kC, MODE != kModeInt>()
+                                  : group_prof16_bytes<8, G, kC, MODE != kModeInt>();
   unsigned char *gbase = smem + (size_t)grp * kProf;  // keyed engine: profile table only
   GroupSmem gs;
   gs.prof = reinterpret_cast<uint32_t *>(gbase);
@@ -101,14 +102,14 @@ __global__ void __launch_bounds__(G == kGKLong && HALF && !S2 ? 640 : 256) k_fwd
     if constexpr (S2) rmo = RowMaxOut{ps.rowmax16 + ps.a_off[p], NP};
     if constexpr (kShort) {
       switch (bucket) {
-        case 0: sweep16<4, G, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
-        case 1: sweep16<6, G, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
-        case 2: sweep16<8, G, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
-        default: sweep16<10, G, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
+        case 0: sweep16<4, G, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
+        case 1: sweep16<6, G, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
+        case 2: sweep16<8, G, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
+        default: sweep16<10, G, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo); break;
       }
     } else {
-      if (bucket == 4) sweep16<6, G, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo);
-      else sweep16<8, G, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo);
+      if (bucket == 4) sweep16<6, G, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo);
+      else sweep16<8, G, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, so, rmo);
     }
     if (lane == 0) {
       const int S = key_value(so.key);
@@ -226,20 +227,28 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     return 1;
   }
   const bool s2 = ps.rowmax16 != nullptr;
-  // half mode where the scores allow it
-  const bool half = (long long)std::min(max_a, max_b) * sc.match <= kHalfCap;
-  auto kshort = s2 ? (half ? k_fwd_persist<kGKShort, true, true> : k_fwd_persist<kGKShort, true, false>)
-                   : (half ? k_fwd_persist<kGKShort, false, true> : k_fwd_persist<kGKShort, false, false>);
-  auto klong = s2 ? (half ? k_fwd_persist<kGKLong, true, true> : k_fwd_persist<kGKLong, true, false>)
-                  : (half ? k_fwd_persist<kGKLong, false, true> : k_fwd_persist<kGKLong, false, false>);
+  // The engine's mode by the largest score of each kernel's pairs (8-lane groups take at most
+  // 160 rows).
+  const int mode_s = mode_for((long long)std::min({max_a, max_b, 160}) * sc.match, 10);
+  const int mode_l = mode_for((long long)std::min(max_a, max_b) * sc.match, 8);
+  using Kern = decltype(&k_fwd_persist<kGKShort, false, kModeInt>);
+  auto pick = [&](int mode, Kern i, Kern h, Kern t, Kern i2, Kern h2, Kern t2) -> Kern {
+    return mode == kModeStep ? (s2 ? t2 : t) : mode == kModeHalf ? (s2 ? h2 : h) : (s2 ? i2 : i);
+  };
+  const Kern kshort = pick(mode_s, k_fwd_persist<kGKShort, false, 0>, k_fwd_persist<kGKShort, false, 1>,
+                           k_fwd_persist<kGKShort, false, 2>, k_fwd_persist<kGKShort, true, 0>,
+                           k_fwd_persist<kGKShort, true, 1>, k_fwd_persist<kGKShort, true, 2>);
+  const Kern klong = pick(mode_l, k_fwd_persist<kGKLong, false, 0>, k_fwd_persist<kGKLong, false, 1>,
+                          k_fwd_persist<kGKLong, false, 2>, k_fwd_persist<kGKLong, true, 0>,
+                          k_fwd_persist<kGKLong, true, 1>, k_fwd_persist<kGKLong, true, 2>);
   // profile table of a group, one of (codes, form)
-  auto prof_of = [&](auto full, auto full_s2, auto half_w, auto half_s2) -> size_t {
-    return half ? (s2 ? half_s2 : half_w) : (s2 ? full_s2 : full);
+  auto prof_of = [&](bool h, size_t full, size_t full_s2, size_t half_w, size_t half_s2) -> size_t {
+    return h ? (s2 ? half_s2 : half_w) : (s2 ? full_s2 : full);
   };
   constexpr int kZ = kCode16Zero + 1, kN = kCodeN + 1;
-  const size_t prof_short = prof_of(group_prof16_bytes<10, kGKShort, kN>(), group_prof16_bytes<10, kGKShort, kZ>(),
+  const size_t prof_short = prof_of(mode_s != kModeInt, group_prof16_bytes<10, kGKShort, kN>(), group_prof16_bytes<10, kGKShort, kZ>(),
                                     group_prof16_bytes<10, kGKShort, kN, true>(), group_prof16_bytes<10, kGKShort, kZ, true>());
-  const size_t prof_long = prof_of(group_prof16_bytes<8, kGKLong, kN>(), group_prof16_bytes<8, kGKLong, kZ>(),
+  const size_t prof_long = prof_of(mode_l != kModeInt, group_prof16_bytes<8, kGKLong, kN>(), group_prof16_bytes<8, kGKLong, kZ>(),
                                    group_prof16_bytes<8, kGKLong, kN, true>(), group_prof16_bytes<8, kGKLong, kZ, true>());
   // long pairs take blocks of their own (not in score2 mode, which needs their row maxima, nor
   // under a lowered int16 ceiling, which asks for the int32 pass)

@@ -41,15 +41,24 @@
 //     holds a sign-replicate selector instead (H and E^ are never negative, so the
 //     replicated sign bytes are zero).
 //
-// Half mode (HALF, every score of the batch at most kHalfCap): small integers as fp16 bit
-// patterns.  A pattern n in [0, 2047] is the fp16 value n * 2^-24 -- subnormal below 1024, the
-// first normal binade above, with one spacing -- so adding patterns with fp16 adds is exact
-// integer arithmetic while sums stay below 2048, and the integer maxima order them as
-// before.  The two adds forming Hdiag + s + gO and the relu(m - gO) then run on the FMA
-// pipe at twice the rate of the integer multiply-adds and off the DPX pipe.  As fused
-// multiply-adds by (1, 0) and (0, 1) the two adds also pick their half of a word, so the
-// table holds one word per row pair instead of two (Prof16H): the integer form's loads kept
-// the shared-memory pipe 70% busy next to 71% of the issue slots.
+// Modes of the engine, by the largest score the kernel's pairs can reach (mode_cap):
+//   kModeInt   the integer step above.
+//   kModeHalf  small integers as fp16 bit patterns.  A pattern n in [0, 2047] is the fp16 value
+//              n * 2^-24 -- subnormal below 1024, the first normal binade above, with one
+//              spacing -- so adding patterns with fp16 adds is exact integer arithmetic while
+//              sums stay below 2048, and the integer maxima order them as before.  The two adds
+//              forming Hdiag + s + gO and the relu(m - gO) then run on the FMA pipe at twice
+//              the rate of the integer multiply-adds and off the DPX pipe.  As fused
+//              multiply-adds by (1, 0) and (0, 1) the two adds also pick their half of a word,
+//              so the table holds one word per row pair instead of two (Prof16H): the integer
+//              form's loads kept the shared-memory pipe 70% busy next to 71% of the issue slots.
+//   kModeStep  half mode with keys that also hold the step within a block of eight, below the
+//              row: the largest key of a block is its largest score at the smallest row, then
+//              the first step, so the running key and its step are brought up to date once a
+//              block instead of once a step (four instructions of about 80).
+// Forward pass, int / half / step: 800,000 uneven pairs 13.19 / 12.91 / 12.63 ms, 30,011 pairs of
+// 250 bp against 2-8 kb 7.34 / 6.74 / 6.67.  Unsigned keys (twice the cap), or a key that ages
+// in place of step constants, give half of the last gain back.
 //
 // Score2 mode (S2) also produces what SSW's second-best score is computed from
 // (ssw_core.cpp:489, :513-536): each A row's maximum of H, over B extended to P columns
@@ -116,8 +125,15 @@ struct RowMaxOut {
   int P;
 };
 
-// Largest score bound of half mode: H + s + gO < 2048 with match and gO at most 127.
-constexpr int kHalfCap = 1792;
+enum : int { kModeInt = 0, kModeHalf = 1, kModeStep = 2 };
+// Largest score bound of a mode: half sums stay below 2048 with match and gO at most 127; step
+// keys hold the score above the row and three step bits.
+__host__ __device__ constexpr int mode_cap(int mode, int K) {
+  return mode == kModeStep ? (1 << (K <= 8 ? 9 : 8)) - 64 : mode == kModeHalf ? 1792 : 0x7fffffff;
+}
+__host__ __device__ constexpr int mode_for(long long bound, int K) {
+  return bound <= mode_cap(kModeStep, K) ? kModeStep : bound <= mode_cap(kModeHalf, K) ? kModeHalf : kModeInt;
+}
 
 // a + the low (high) half of w
 __device__ __forceinline__ uint32_t add_lo_f16x2(uint32_t a, uint32_t w) {
@@ -169,18 +185,20 @@ struct KeyBits {
   static constexpr int kCap = (1 << (15 - kBits)) - 64;  // largest score a key holds, with margin
 };
 
-template <int K, int G, bool S2 = false, bool HALF = false>
+template <int K, int G, bool S2 = false, int MODE = kModeInt>
 struct Step16 {
+  static constexpr bool HALF = MODE != kModeInt, STEP = MODE == kModeStep;
   using L = Prof16<K, S2 ? kCode16Zero + 1 : kCodeN + 1>;
   static constexpr uint32_t kKeyMask = KeyBits<K>::kMask;
   // NGO: -gO in both halves as integers, or (HALF) as negative fp16 patterns.
+  // STEP: u is the step within its block, Kl the block's largest key (fold_block).
   // S2: Rm[k] keeps each row's running maximum over valid columns; vmask is 0 in a half
   // whose column is valid at this step and -16384 otherwise (an add-max then ignores it).
   __device__ static __forceinline__ void run(int t, uint32_t zH, uint32_t zE, uint32_t sel, const uint32_t (&Wlo)[K],
                                              const uint32_t (&Phi)[K], uint32_t (&H)[K], uint32_t (&F)[K],
                                              uint32_t &Hlast, uint32_t &Ecout, uint32_t &HtopPrev,
                                              uint32_t &Kl, uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t one,
-                                             uint32_t eight, uint32_t (&Rm)[K], uint32_t vmask) {
+                                             uint32_t eight, uint32_t (&Rm)[K], uint32_t vmask, int u) {
     uint32_t Ev = prmt_sel(zE, Ecout, sel);  // lo: from the left lane, hi: own lo half
     const uint32_t Htop = prmt_sel(zH, Hlast, sel);
     uint32_t Hd = HtopPrev;
@@ -200,8 +218,16 @@ struct Step16 {
       F[k] = __viaddmax_s16x2(F[k], NGE, Hn);
       Hd = H[k];
       H[k] = Hn;
-      key[k] = mad_u32(Hn, eight, (uint32_t)(kKeyMask - k) * 0x00010001u);
+      if constexpr (STEP) key[k] = mad_u32(Hn, eight, ((uint32_t)(kKeyMask - k) * 8u + 7u - (uint32_t)u) * 0x00010001u);
+      else key[k] = mad_u32(Hn, eight, (uint32_t)(kKeyMask - k) * 0x00010001u);
       if constexpr (S2) Rm[k] = __viaddmax_s16x2(Hn, vmask, Rm[k]);
+    }
+    if constexpr (STEP) {
+#pragma unroll
+      for (int k = 0; k < K; k += 2) Kl = __vimax3_s16x2(Kl, key[k], key[k + 1]);
+      Hlast = H[K - 1];
+      Ecout = Ev;
+      return;
     }
     // running key per half (keys are non-negative int16): K/2 three-way maxima
     uint32_t Kn = Kl;
@@ -214,6 +240,15 @@ struct Step16 {
     const uint32_t tt = (uint32_t)t * 0x00010001u;
     Jp = (msk & tt) | (~msk & Jp);
     Kl = Kn;
+  }
+  // Step mode: the running key (score, row; step bits 0) and its step after a block of steps from
+  // t on whose largest key is Kb.
+  __device__ static __forceinline__ void fold_block(int t, uint32_t Kb, uint32_t &Kl, uint32_t &Jp) {
+    const uint32_t n = __vmaxs2(Kb & 0xFFF8FFF8u, Kl);
+    const uint32_t grown = sign_mask16(n - Kl + 0x7fff7fffu);
+    const uint32_t at = (uint32_t)t * 0x00010001u + 0x00070007u - (Kb & 0x00070007u);
+    Jp = (grown & at) | (~grown & Jp);
+    Kl = n;
   }
   // Half mode: the words of code c (Wlo of this step, Phi of the next).
   __device__ static __forceinline__ void load_half(const uint32_t *tab, int c, int lane, uint32_t (&W)[K]) {
@@ -264,19 +299,22 @@ struct Step16 {
 // Forward sweep of one pair with the keyed engine.  B is read directly from its code
 // array in global memory (one byte per lane per step, loaded two steps ahead); the
 // shared memory of the group holds only the profile table.  A must be a forward view.
-template <int K, int G, bool MULTI, bool S2 = false, bool HALF = false>
+template <int K, int G, bool MULTI, bool S2 = false, int MODE = kModeInt>
 __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &sc, const GroupSmem &gs, int lane,
                              unsigned gmask, V16::Pay *bnd, int ceiling, SweepOut &out, const RowMaxOut &rmo) {
-  using ST = Step16<K, G, S2, HALF>;
+  using ST = Step16<K, G, S2, MODE>;
+  constexpr bool HALF = ST::HALF, STEP = ST::STEP;
   using L = typename ST::L;
   constexpr int RS = 2 * K * G;
-  constexpr int KB = KeyBits<K>::kBits;
   constexpr uint32_t KMASK = KeyBits<K>::kMask;
+  constexpr int KS = STEP ? 3 : 0;  // step bits below the row bits
+  constexpr int KB = KeyBits<K>::kBits + KS;
   const int M = A.len, N = B.len;
   const uint32_t NGE = V16::splat(-sc.gap_extend);
   const uint32_t NGO = HALF ? (uint32_t)(0x8000 | sc.gap_open) * 0x00010001u : V16::splat(-sc.gap_open);
   const uint8_t *bg = B.base;
-  if (ceiling > KeyBits<K>::kCap) ceiling = KeyBits<K>::kCap;
+  constexpr int kCap = STEP ? mode_cap(MODE, K) : KeyBits<K>::kCap;
+  if (ceiling > kCap) ceiling = kCap;
 
   unsigned long long best = 0ull;
   int overflow = 0;
@@ -370,7 +408,10 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
     const uint8_t *bl = bg + j0;
     // Two steps; `guarded` (std::true_type / std::false_type) says whether the look-ahead
     // codes need the bounds test.
-    auto two_steps = [&](auto guarded) {
+    // (STEP: u is the first one's place in its block, Kb the block's largest key).
+    uint32_t Kb = 0u;
+    uint32_t &Kr = STEP ? Kb : Kl;
+    auto two_steps = [&](auto guarded, int u) {
       constexpr bool kGuard = decltype(guarded)::value;
       // even step: hi words into HA; the high half uses HB (previous column)
       int c = ceven;
@@ -379,7 +420,8 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
       else ST::load(tab, c, lane, Wlo, HA);
       uint32_t zH, zE;
       top(t, zH, zE);
-      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm, vmask_at(t));
+      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
+              vmask_at(t), u);
       out_bnd(t);
       // odd step: hi words into HB; the high half uses HA
       c = codd;
@@ -387,32 +429,47 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
       if constexpr (HALF) ST::load_half(gs.prof, c, lane, HB);
       else ST::load(tab, c, lane, Wlo, HB);
       top(t + 1, zH, zE);
-      ST::run(t + 1, zH, zE, sel, HALF ? HB : Wlo, HA, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm,
-              vmask_at(t + 1));
+      ST::run(t + 1, zH, zE, sel, HALF ? HB : Wlo, HA, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
+              vmask_at(t + 1), u + 1);
       out_bnd(t + 1);
     };
     // The look-ahead columns t+2+j0 and t+3+j0 lie in [0, N) for every lane of the group
     // (j0 = -2 lane, lane < G) when 2G-4 <= t <= N-4.
     const int tm0 = 2 * G - 4, tm1 = N - 3;
-    for (; t + 1 < T_end && t < tm0; t += 2) two_steps(std::true_type{});
+    auto fold = [&](int t0) {
+      if constexpr (STEP) {
+        ST::fold_block(t0, Kb, Kl, Jp);
+        Kb = 0u;
+      }
+    };
+    for (; t + 1 < T_end && t < tm0; t += 2) {
+      two_steps(std::true_type{}, 0);
+      fold(t);
+    }
     // eight steps per iteration in the middle phase (the loop's own instructions and the
     // register moves at its back edge are paid once per eight steps); its last few steps
     // go to the guarded drain loop, which keeps one copy of the step code fewer
     for (; t + 6 < tm1;) {
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        two_steps(std::false_type{});
+        two_steps(std::false_type{}, 2 * u);
         t += 2;
       }
+      fold(t - 8);
     }
-    for (; t + 1 < T_end; t += 2) two_steps(std::true_type{});
+    for (; t + 1 < T_end; t += 2) {
+      two_steps(std::true_type{}, 0);
+      fold(t);
+    }
     if (t < T_end) {
       if constexpr (HALF) ST::load_half(gs.prof, ceven, lane, HA);
       else ST::load(tab, ceven, lane, Wlo, HA);
       uint32_t zH, zE;
       top(t, zH, zE);
-      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm, vmask_at(t));
+      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
+              vmask_at(t), 0);
       out_bnd(t);
+      fold(t);
     }
 
     if constexpr (S2) {
@@ -430,7 +487,7 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
     for (int half = 0; half < 2; half++) {
       const uint32_t key = half ? (Kl >> 16) : (Kl & 0xffffu);
       const int v = (int)(key >> KB);
-      const int k = (int)KMASK - (int)(key & KMASK);
+      const int k = (int)KMASK - (int)((key >> KS) & KMASK);
       const int r = row0 + (half ? K : 0) + k;
       const int jstep = (int)(half ? (Jp >> 16) : (Jp & 0xffffu));
       const int col = jstep - 2 * lane - half;
@@ -454,14 +511,14 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
   out.overflow = overflow;
 }
 
-template <int K, int G, bool S2 = false, bool HALF = false>
+template <int K, int G, bool S2 = false, int MODE = kModeInt>
 __device__ __forceinline__ void sweep16(const SeqView &A, const SeqView &B, const Scoring &sc, const GroupSmem &gs,
                                         int lane, unsigned gmask, V16::Pay *bnd, int ceiling, SweepOut &out,
                                         const RowMaxOut &rmo = RowMaxOut{nullptr, 0}) {
   if (A.len > 2 * K * G)
-    sweep16_impl<K, G, true, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, out, rmo);
+    sweep16_impl<K, G, true, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, out, rmo);
   else
-    sweep16_impl<K, G, false, S2, HALF>(A, B, sc, gs, lane, gmask, bnd, ceiling, out, rmo);
+    sweep16_impl<K, G, false, S2, MODE>(A, B, sc, gs, lane, gmask, bnd, ceiling, out, rmo);
 }
 
 }  // namespace mhsw

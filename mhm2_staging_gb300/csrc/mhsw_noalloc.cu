@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(kNaG * kNaGroupsPerBlock)
 // buckets (G = 8) or of the longer ones up to the wide bucket (G = 16) and translate a pair's
 // A and B into their share of the scratch array.  50,000 mixed reads (5.1e9 cells): 7.14 -> 1.34 ms
 // a call against the int32 engine in input order, whose shares and registers let 372 blocks run.
-template <int G, bool HALF>
-__global__ void __launch_bounds__(128)
+template <int G, int MODE>
+__global__ void __launch_bounds__(128, G == kGKLong && MODE != kModeInt ? 5 : 4)
     k_fwd_noalloc16(PairSet ps, Scoring sc, int max_a, int max_b, int lane_rows, const uint32_t *__restrict__ order,
                     int *queue, const int *first, unsigned char *scratch, size_t share, size_t a_cap, size_t b_cap,
                     int32_t *__restrict__ out3) {
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(128)
   const int grp = threadIdx.x / G, lane = threadIdx.x % G;
   const unsigned gmask = ((1u << G) - 1u) << (((threadIdx.x & 31) / G) * G);
   GroupSmem gs;
-  gs.prof = reinterpret_cast<uint32_t *>(smem + (size_t)grp * group_prof16_bytes<kPer, G, kCodeN + 1, HALF>());
+  gs.prof = reinterpret_cast<uint32_t *>(smem + (size_t)grp * group_prof16_bytes<kPer, G, kCodeN + 1, MODE != kModeInt>());
   gs.prof_lanes = G;
   gs.bcodes = nullptr;
   gs.pad = 0;
@@ -199,14 +199,14 @@ __global__ void __launch_bounds__(128)
       const int bucket = bucket_of(M, N, sc, lane_rows, false);
       if constexpr (kShort) {
         switch (bucket) {
-          case 0: sweep16<4, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
-          case 1: sweep16<6, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
-          case 2: sweep16<8, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
-          default: sweep16<10, G, false, HALF>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+          case 0: sweep16<4, G, false, MODE>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+          case 1: sweep16<6, G, false, MODE>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+          case 2: sweep16<8, G, false, MODE>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
+          default: sweep16<10, G, false, MODE>(A, B, sc, gs, lane, gmask, nullptr, INT_MAX, so); break;
         }
       } else {
-        if (bucket == 4) sweep16<6, G, false, HALF>(A, B, sc, gs, lane, gmask, bnd, INT_MAX, so);
-        else sweep16<8, G, false, HALF>(A, B, sc, gs, lane, gmask, bnd, INT_MAX, so);
+        if (bucket == 4) sweep16<6, G, false, MODE>(A, B, sc, gs, lane, gmask, bnd, INT_MAX, so);
+        else sweep16<8, G, false, MODE>(A, B, sc, gs, lane, gmask, bnd, INT_MAX, so);
       }
       r[0] = key_value(so.key);
       if (r[0] > 0) {
@@ -222,12 +222,26 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-constexpr size_t na16_smem_short() { return 16 * group_prof16_bytes<10, kGKShort>(); }
-constexpr size_t na16_smem_long() { return 8 * group_prof16_bytes<8, kGKLong>(); }
+using Na16Kern = decltype(&k_fwd_noalloc16<kGKShort, kModeInt>);
+// The two kernels by mode, and the shared memory of a block.
+Na16Kern na16_short(int mode) {
+  return mode == kModeStep ? k_fwd_noalloc16<kGKShort, 2> : mode == kModeHalf ? k_fwd_noalloc16<kGKShort, 1>
+                                                                              : k_fwd_noalloc16<kGKShort, 0>;
+}
+Na16Kern na16_long(int mode) {
+  return mode == kModeStep ? k_fwd_noalloc16<kGKLong, 2> : mode == kModeHalf ? k_fwd_noalloc16<kGKLong, 1>
+                                                                             : k_fwd_noalloc16<kGKLong, 0>;
+}
+size_t na16_smem_short(int mode) {
+  return 16 * (mode ? group_prof16_bytes<10, kGKShort, kCodeN + 1, true>() : group_prof16_bytes<10, kGKShort>());
+}
+size_t na16_smem_long(int mode) {
+  return 8 * (mode ? group_prof16_bytes<8, kGKLong, kCodeN + 1, true>() : group_prof16_bytes<8, kGKLong>());
+}
 constexpr int64_t kNaChunk = 2 << 20;  // pairs ordered at once (their order takes 8 MiB of the array)
 
 struct NaDevice {
-  int occ_short = 1, occ_long = 1;
+  int occ_short[3] = {1, 1, 1}, occ_long[3] = {1, 1, 1};  // by mode
   bool ready = false;
   unsigned char *scratch = nullptr;
   int sms = 0;
@@ -272,15 +286,13 @@ int na_setup(int dev, NaDevice **out, char *errbuf, size_t errlen) {
     if (e != cudaSuccess)
       return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
     // limits and occupancy of the keyed kernels and the order's, so later calls only launch
-    for (auto k : {k_fwd_noalloc16<kGKLong, false>, k_fwd_noalloc16<kGKLong, true>}) {
-      if ((e = raise_smem_limit(reinterpret_cast<const void *>(k), na16_smem_long())) ||
-          (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_long, k, 128, na16_smem_long())))
+    for (int m = 0; m < 3; m++)
+      if ((e = raise_smem_limit(reinterpret_cast<const void *>(na16_long(m)), na16_smem_long(m))) ||
+          (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_long[m], na16_long(m), 128, na16_smem_long(m))) ||
+          (e = raise_smem_limit(reinterpret_cast<const void *>(na16_short(m)), na16_smem_short(m))) ||
+          (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_short[m], na16_short(m), 128, na16_smem_short(m))))
         return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "keyed kernel set-up: %s", cudaGetErrorString(e));
-    }
-    if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_fwd_noalloc16<kGKShort, false>), na16_smem_short())) ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_short, k_fwd_noalloc16<kGKShort, false>, 128,
-                                                           na16_smem_short())) ||
-        (e = order_smem_limits()))
+    if ((e = order_smem_limits()))
       return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "keyed kernel set-up: %s", cudaGetErrorString(e));
     d.scratch = static_cast<unsigned char *>(p);
     d.sms = sms;
@@ -380,8 +392,8 @@ extern "C" int mhsw_forward_noalloc(const mhsw_pairs *pairs, short match_score, 
   int *ctl = reinterpret_cast<int *>(d->scratch);
   uint32_t *order = reinterpret_cast<uint32_t *>(ctl + kOrderCtl);
   unsigned char *shares = d->scratch + head;
-  const bool half = (long long)std::min(max_a, max_b) * sc.match <= kHalfCap;
-  auto klong = half ? k_fwd_noalloc16<kGKLong, true> : k_fwd_noalloc16<kGKLong, false>;
+  const int mode_s = mode_for((long long)std::min({max_a, max_b, 160}) * sc.match, 10);
+  const int mode_l = mode_for((long long)std::min(max_a, max_b) * sc.match, 8);
   for (int64_t at = 0; at < n; at += chunk) {
     PairSet q = ps;
     q.n = std::min(chunk, n - at);
@@ -399,10 +411,10 @@ extern "C" int mhsw_forward_noalloc(const mhsw_pairs *pairs, short match_score, 
       return (unsigned)std::min<int64_t>(b, room / gpb);
     };
     if (max_a > lane_rows)
-      klong<<<grid_of(d->occ_long, 8), 128, na16_smem_long(), st>>>(q, sc, max_a, max_b, lane_rows, order, ctl, ctl + 8,
-                                                                   shares, share, a_cap, b_cap, out3 + 3 * at);
+      na16_long(mode_l)<<<grid_of(d->occ_long[mode_l], 8), 128, na16_smem_long(mode_l), st>>>(
+          q, sc, max_a, max_b, lane_rows, order, ctl, ctl + 8, shares, share, a_cap, b_cap, out3 + 3 * at);
     if (lane_rows > 0)
-      k_fwd_noalloc16<kGKShort, false><<<grid_of(d->occ_short, 16), 128, na16_smem_short(), st>>>(
+      na16_short(mode_s)<<<grid_of(d->occ_short[mode_s], 16), 128, na16_smem_short(mode_s), st>>>(
           q, sc, max_a, max_b, lane_rows, order, ctl, ctl + 8, shares, share, a_cap, b_cap, out3 + 3 * at);
     if ((e = cudaGetLastError())) return launch_fail(e);
     if (wide && (e = run32(q, q.n, head, order, ctl + 8 + kBucketWide, out3 + 3 * at))) return launch_fail(e);
