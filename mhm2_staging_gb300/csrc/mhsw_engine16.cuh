@@ -192,13 +192,15 @@ struct Step16 {
   static constexpr uint32_t kKeyMask = KeyBits<K>::kMask;
   // NGO: -gO in both halves as integers, or (HALF) as negative fp16 patterns.
   // STEP: u is the step within its block, Kl the block's largest key (fold_block).
+  // inside: both halves' columns are valid in every lane (vmask unused).
   // S2: Rm[k] keeps each row's running maximum over valid columns; vmask is 0 in a half
   // whose column is valid at this step and -16384 otherwise (an add-max then ignores it).
   __device__ static __forceinline__ void run(int t, uint32_t zH, uint32_t zE, uint32_t sel, const uint32_t (&Wlo)[K],
                                              const uint32_t (&Phi)[K], uint32_t (&H)[K], uint32_t (&F)[K],
                                              uint32_t &Hlast, uint32_t &Ecout, uint32_t &HtopPrev,
                                              uint32_t &Kl, uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t one,
-                                             uint32_t eight, uint32_t (&Rm)[K], uint32_t vmask, int u) {
+                                             uint32_t eight, uint32_t (&Rm)[K], uint32_t vmask, int u,
+                                             bool inside) {
     uint32_t Ev = prmt_sel(zE, Ecout, sel);  // lo: from the left lane, hi: own lo half
     const uint32_t Htop = prmt_sel(zH, Hlast, sel);
     uint32_t Hd = HtopPrev;
@@ -220,7 +222,7 @@ struct Step16 {
       H[k] = Hn;
       if constexpr (STEP) key[k] = mad_u32(Hn, eight, ((uint32_t)(kKeyMask - k) * 8u + 7u - (uint32_t)u) * 0x00010001u);
       else key[k] = mad_u32(Hn, eight, (uint32_t)(kKeyMask - k) * 0x00010001u);
-      if constexpr (S2) Rm[k] = __viaddmax_s16x2(Hn, vmask, Rm[k]);
+      if constexpr (S2) Rm[k] = inside ? __vmaxs2(Hn, Rm[k]) : __viaddmax_s16x2(Hn, vmask, Rm[k]);
     }
     if constexpr (STEP) {
 #pragma unroll
@@ -421,7 +423,7 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
       uint32_t zH, zE;
       top(t, zH, zE);
       ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
-              vmask_at(t), u);
+              kGuard ? vmask_at(t) : 0u, u, !kGuard);
       out_bnd(t);
       // odd step: hi words into HB; the high half uses HA
       c = codd;
@@ -430,12 +432,13 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
       else ST::load(tab, c, lane, Wlo, HB);
       top(t + 1, zH, zE);
       ST::run(t + 1, zH, zE, sel, HALF ? HB : Wlo, HA, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
-              vmask_at(t + 1), u + 1);
+              kGuard ? vmask_at(t + 1) : 0u, u + 1, !kGuard);
       out_bnd(t + 1);
     };
     // The look-ahead columns t+2+j0 and t+3+j0 lie in [0, N) for every lane of the group
     // (j0 = -2 lane, lane < G) when 2G-4 <= t <= N-4.
-    const int tm0 = 2 * G - 4, tm1 = N - 3;
+    // From t = 2G on the current columns do as well (the row maxima's plain form needs it).
+    const int tm0 = S2 ? 2 * G : 2 * G - 4, tm1 = N - 3;
     auto fold = [&](int t0) {
       if constexpr (STEP) {
         ST::fold_block(t0, Kb, Kl, Jp);
@@ -467,7 +470,7 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
       uint32_t zH, zE;
       top(t, zH, zE);
       ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
-              vmask_at(t), 0);
+              vmask_at(t), 0, false);
       out_bnd(t);
       fold(t);
     }
