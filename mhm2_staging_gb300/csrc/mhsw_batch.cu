@@ -34,11 +34,12 @@ __device__ __forceinline__ unsigned group_mask_b(int G) {
 // Persistent forward kernel over one range of the sorted pair order: 8-lane groups for
 // the short-read buckets (items [0, split)), 16-lane groups for the rest ([split, n)).
 // A group claims its next pair from the range's atomic counter.
-// MODE: the engine's (mhsw_engine16.cuh).  The 16-lane kernel in the half modes is held to 102
-// registers (640 threads an SM: five blocks of 128 instead of four; 30,011 pairs against
-// 2-8 kb 6.98 -> 6.85 ms, 150,001 mixed reads 3.40 -> 3.34); the others lose or spill there.
+// MODE: the engine's (mhsw_engine16.cuh).  In the half modes the 16-lane kernel is held to 80
+// registers (six blocks of 128 an SM) and the 8-lane one to 96 (five): 800,000 uneven pairs
+// 12.51 -> 12.23 ms and 30,011 pairs against 2-8 kb 6.55 -> 6.47 against 96 and 128; the score2
+// kernels, which keep a row maximum per row pair, lose or spill there.
 template <int G, bool S2, int MODE>
-__global__ void __launch_bounds__(G == kGKLong && MODE != kModeInt && !S2 ? 640 : 256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
+__global__ void __launch_bounds__(MODE != kModeInt && !S2 ? (G == kGKLong ? 768 : 640): 256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
                                                      const uint32_t *__restrict__ order, int *queue, int lane_rows,
                                                      bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap,
                                                      V16::Pay *scratch, int scratch_stride) {

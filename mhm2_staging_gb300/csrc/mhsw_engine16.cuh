@@ -174,9 +174,7 @@ __device__ __forceinline__ uint32_t sign_mask16(uint32_t x) {
   return r;
 }
 
-// One wavefront step of the keyed engine for one lane.  W holds this step's profile
-// words (lo words used now), Phi the high words of the previous step; both are
-// register arrays of the caller, alternated between steps so no copies are needed.
+// One wavefront step of the keyed engine for one lane (Step16::run).
 // Arg-max key of a cell: H << kKeyBits | (kKeyMask - k), k = row within the lane half.
 template <int K>
 struct KeyBits {
@@ -195,48 +193,55 @@ struct Step16 {
   // inside: both halves' columns are valid in every lane (vmask unused).
   // S2: Rm[k] keeps each row's running maximum over valid columns; vmask is 0 in a half
   // whose column is valid at this step and -16384 otherwise (an add-max then ignores it).
+  // P[k] is the diagonal input of row k with the high half's score already added: a step adds the
+  // low half's score to it (the column's word), and once a row's H is known the high half's score
+  // of the same word to that, for the next step.  So a word is used in the step that loads it, and
+  // P[k] is replaced right after its only use (no word kept for the next step, no H beside it):
+  // 2K registers fewer, and fewer moves at the end of the unrolled steps.  The relu of H on the
+  // integer pipe for every fourth row, to even the pipes out, costs 3%; sixteen steps an
+  // iteration cost 2-4%.
   __device__ static __forceinline__ void run(int t, uint32_t zH, uint32_t zE, uint32_t sel, const uint32_t (&Wlo)[K],
-                                             const uint32_t (&Phi)[K], uint32_t (&H)[K], uint32_t (&F)[K],
-                                             uint32_t &Hlast, uint32_t &Ecout, uint32_t &HtopPrev,
-                                             uint32_t &Kl, uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t one,
-                                             uint32_t eight, uint32_t (&Rm)[K], uint32_t vmask, int u,
-                                             bool inside) {
+                                             const uint32_t (&Whi)[K], uint32_t (&P)[K], uint32_t (&F)[K],
+                                             uint32_t &Hlast, uint32_t &Ecout, uint32_t &Kl, uint32_t &Jp, uint32_t NGE,
+                                             uint32_t NGO, uint32_t one, uint32_t eight, uint32_t (&Rm)[K],
+                                             uint32_t vmask, int u, bool inside) {
     uint32_t Ev = prmt_sel(zE, Ecout, sel);  // lo: from the left lane, hi: own lo half
     const uint32_t Htop = prmt_sel(zH, Hlast, sel);
-    uint32_t Hd = HtopPrev;
-    HtopPrev = Htop;
+    // halves never carry: all terms >= 0, sum < 2^15.  Written as multiply-adds by a
+    // runtime 1 so they issue on the FMA pipe, not the integer ALU pipe the DP saturates.
+    auto add_lo = [&](uint32_t h, uint32_t w) { return HALF ? add_lo_f16x2(h, w) : mad_u32(h, one, w); };
+    auto add_hi = [&](uint32_t h, uint32_t w) { return HALF ? add_hi_f16x2(h, w) : mad_u32(h, one, w); };
+    uint32_t Q = add_lo(P[0], Wlo[0]);
+    P[0] = add_hi(Htop, Whi[0]);
     uint32_t key[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      // halves never carry: all terms >= 0, sum < 2^15.  Written as multiply-adds by a
-      // runtime 1 so they issue on the FMA pipe, not the integer ALU pipe the DP saturates.
-      uint32_t Q, Hn;
-      if constexpr (HALF) Q = add_hi_f16x2(add_lo_f16x2(Hd, Wlo[k]), Phi[k]);
-      else Q = mad_u32(mad_u32(Hd, one, Wlo[k]), one, Phi[k]);
+      uint32_t Hn;
       const uint32_t m = __vimax3_s16x2(Q, Ev, F[k]);
       if constexpr (HALF) Hn = add_relu_f16x2(m, NGO);
       else Hn = __viaddmax_s16x2_relu(m, NGO, 0u);
+      if (k + 1 < K) {
+        Q = add_lo(P[k + 1], Wlo[k + 1]);
+        P[k + 1] = add_hi(Hn, Whi[k + 1]);
+      } else {
+        Hlast = Hn;
+      }
       Ev = __viaddmax_s16x2(Ev, NGE, Hn);
       F[k] = __viaddmax_s16x2(F[k], NGE, Hn);
-      Hd = H[k];
-      H[k] = Hn;
       if constexpr (STEP) key[k] = mad_u32(Hn, eight, ((uint32_t)(kKeyMask - k) * 8u + 7u - (uint32_t)u) * 0x00010001u);
       else key[k] = mad_u32(Hn, eight, (uint32_t)(kKeyMask - k) * 0x00010001u);
       if constexpr (S2) Rm[k] = inside ? __vmaxs2(Hn, Rm[k]) : __viaddmax_s16x2(Hn, vmask, Rm[k]);
     }
+    Ecout = Ev;
     if constexpr (STEP) {
 #pragma unroll
       for (int k = 0; k < K; k += 2) Kl = __vimax3_s16x2(Kl, key[k], key[k + 1]);
-      Hlast = H[K - 1];
-      Ecout = Ev;
       return;
     }
     // running key per half (keys are non-negative int16): K/2 three-way maxima
     uint32_t Kn = Kl;
 #pragma unroll
     for (int k = 0; k < K; k += 2) Kn = __vimax3_s16x2(Kn, key[k], key[k + 1]);
-    Hlast = H[K - 1];
-    Ecout = Ev;
     // record the step where the running key strictly grows
     const uint32_t msk = sign_mask16(Kn - Kl + 0x7fff7fffu);
     const uint32_t tt = (uint32_t)t * 0x00010001u;
@@ -252,7 +257,7 @@ struct Step16 {
     Jp = (grown & at) | (~grown & Jp);
     Kl = n;
   }
-  // Half mode: the words of code c (Wlo of this step, Phi of the next).
+  // Half mode: the words of code c.
   __device__ static __forceinline__ void load_half(const uint32_t *tab, int c, int lane, uint32_t (&W)[K]) {
     using LH = Prof16H<K, L::kCodes>;
     const uint32_t *b = tab + c * (K * G);
@@ -270,8 +275,7 @@ struct Step16 {
       W[K - 1] = v.y;
     }
   }
-  // Words of code c: low words into Wlo (used at this step), high words into Whi (used
-  // at the next step by the high half).
+  // Words of code c: low words into Wlo, high words into Whi.
   __device__ static __forceinline__ void load(const uint4 *tab, int c, int lane, uint32_t (&Wlo)[K],
                                               uint32_t (&Whi)[K]) {
     const uint4 *b = tab + c * L::kNV * G + lane;
@@ -332,39 +336,54 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
     const int row0 = s * RS + lane * 2 * K;
     __syncwarp(gmask);
     // Profile words: lo word k = s(A[row0+k], c) + gO; hi word k = (s(A[row0+K+k], c) + gO) << 16.
+    // Rows past A score -gO (0 biased).  A's codes are read once, a word is its row pair's
+    // mismatch word plus the match's surplus in the halves that match.
     {
       uint32_t *tw = gs.prof;
-      for (int c = 0; c < L::kCodes; c++) {
-#pragma unroll
-        for (int w = 0; w < K; w++) {
-          const int alo = A.code(row0 + w), ahi = A.code(row0 + K + w);
-          // the zero code scores 0 against real rows (biased gO); rows past A stay at -gO
-          const int slo = (S2 && c == kCode16Zero) ? (alo == kCodePad ? -sc.gap_open : 0) : sub_score(alo, c, sc, sc.gap_open);
-          const int shi = (S2 && c == kCode16Zero) ? (ahi == kCodePad ? -sc.gap_open : 0) : sub_score(ahi, c, sc, sc.gap_open);
-          const uint32_t vlo = (uint32_t)(slo + sc.gap_open) & 0xffffu;
-          const uint32_t vhi = ((uint32_t)(shi + sc.gap_open) & 0xffffu) << 16;
-          if constexpr (HALF) {
-            tw[Prof16H<K, L::kCodes>::word(c, w, lane, G)] = vlo | vhi;
-            continue;
-          }
-          tw[((c * L::kNV + L::lo_vec(w)) * G + lane) * 4 + L::lo_elem(w)] = vlo;
-          tw[((c * L::kNV + L::hi_vec(w)) * G + lane) * 4 + L::hi_elem(w)] = vhi;
+      auto put = [&](int c, int w, uint32_t v) {
+        if constexpr (HALF) {
+          tw[Prof16H<K, L::kCodes>::word(c, w, lane, G)] = v;
+        } else {
+          tw[((c * L::kNV + L::lo_vec(w)) * G + lane) * 4 + L::lo_elem(w)] = v & 0xffffu;
+          tw[((c * L::kNV + L::hi_vec(w)) * G + lane) * 4 + L::hi_elem(w)] = v & 0xffff0000u;
         }
+      };
+      const uint32_t miss = (uint32_t)(sc.gap_open - sc.mismatch), vn = (uint32_t)(sc.gap_open - sc.ambiguity);
+      const uint32_t plus = (uint32_t)(sc.match + sc.mismatch);
+      int alo[K], ahi[K];
+      uint32_t base[K];
+#pragma unroll
+      for (int w = 0; w < K; w++) {
+        alo[w] = A.code(row0 + w);
+        ahi[w] = A.code(row0 + K + w);
+      }
+      auto both = [&](int w, uint32_t v) {  // v in the halves whose row is in A
+        return (alo[w] == kCodePad ? 0u : v) | (ahi[w] == kCodePad ? 0u : v << 16);
+      };
+#pragma unroll
+      for (int w = 0; w < K; w++) {
+        base[w] = (alo[w] == kCodePad ? 0u : alo[w] == kCodeN ? vn : miss) |
+                  (ahi[w] == kCodePad ? 0u : ahi[w] == kCodeN ? vn : miss) << 16;
+        put(kCodeN, w, both(w, vn));
+        if constexpr (S2) put(kCode16Zero, w, both(w, (uint32_t)sc.gap_open));  // scores 0 against real rows
+      }
+#pragma unroll 1
+      for (int c = 0; c < kCodeN; c++) {
+#pragma unroll
+        for (int w = 0; w < K; w++) put(c, w, base[w] + (alo[w] == c ? plus : 0u) + (ahi[w] == c ? plus << 16 : 0u));
       }
     }
     __syncwarp(gmask);
 
     const bool first_strip = (s == 0);
     const bool last_strip = (s == nstrips - 1);
-    uint32_t H[K], F[K], Wlo[K], HA[K], HB[K];
+    uint32_t P[K], F[K], Wlo[K], Whi[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      H[k] = 0u;
+      P[k] = 0u;  // high words before column 0 are 0 (biased)
       F[k] = 0u;  // F^ = F + gO with F = -gO before column 0
     }
-#pragma unroll
-    for (int w = 0; w < K; w++) HB[w] = 0u;  // hi words before column 0 (biased 0)
-    uint32_t Hlast = 0u, Ecout = 0u, HtopPrev = 0u;
+    uint32_t Hlast = 0u, Ecout = 0u;
     // lane 0 of the first strip reads zeros above: the selector replicates the sign of a
     // top byte of its own (non-negative) H and E^ words; other lanes take the left lane's hi halves
     const uint32_t sel = (lane == 0 && first_strip) ? 0x54BBu : 0x5432u;
@@ -374,9 +393,9 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
 #pragma unroll
     for (int k = 0; k < K; k++) Rm[k] = 0u;
     const int j0 = -2 * lane;  // lo column at step 0
-    auto code_at = [&](int j) -> int {
-      if ((unsigned)j < (unsigned)N) return (int)bg[j];
-      return (S2 && (unsigned)j < (unsigned)NP) ? kCode16Zero : kCodeN;
+    auto code_at = [&](int j) -> int {  // (a load in bounds for every j: no branch around it)
+      const int c = (int)bg[max(0, min(j, N - 1))];
+      return (unsigned)j < (unsigned)N ? c : S2 && (unsigned)j < (unsigned)NP ? kCode16Zero : kCodeN;
     };
     // score2 mode: 0 in a half whose column is inside [0, NP) at step t, else -16384
     auto vmask_at = [&](int t) -> uint32_t {
@@ -413,27 +432,21 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
     // (STEP: u is the first one's place in its block, Kb the block's largest key).
     uint32_t Kb = 0u;
     uint32_t &Kr = STEP ? Kb : Kl;
-    auto two_steps = [&](auto guarded, int u) {
+    auto step = [&](int t, int &code, auto guarded, int u) {
       constexpr bool kGuard = decltype(guarded)::value;
-      // even step: hi words into HA; the high half uses HB (previous column)
-      int c = ceven;
-      ceven = kGuard ? code_at(t + 2 + j0) : (int)bl[t + 2];
-      if constexpr (HALF) ST::load_half(gs.prof, c, lane, HA);
-      else ST::load(tab, c, lane, Wlo, HA);
+      const int c = code;
+      code = kGuard ? code_at(t + 2 + j0) : (int)bl[t + 2];
+      if constexpr (HALF) ST::load_half(gs.prof, c, lane, Wlo);
+      else ST::load(tab, c, lane, Wlo, Whi);
       uint32_t zH, zE;
       top(t, zH, zE);
-      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
+      ST::run(t, zH, zE, sel, Wlo, HALF ? Wlo : Whi, P, F, Hlast, Ecout, Kr, Jp, NGE, NGO, one, scale, Rm,
               kGuard ? vmask_at(t) : 0u, u, !kGuard);
       out_bnd(t);
-      // odd step: hi words into HB; the high half uses HA
-      c = codd;
-      codd = kGuard ? code_at(t + 3 + j0) : (int)bl[t + 3];
-      if constexpr (HALF) ST::load_half(gs.prof, c, lane, HB);
-      else ST::load(tab, c, lane, Wlo, HB);
-      top(t + 1, zH, zE);
-      ST::run(t + 1, zH, zE, sel, HALF ? HB : Wlo, HA, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
-              kGuard ? vmask_at(t + 1) : 0u, u + 1, !kGuard);
-      out_bnd(t + 1);
+    };
+    auto two_steps = [&](auto guarded, int u) {
+      step(t, ceven, guarded, u);
+      step(t + 1, codd, guarded, u + 1);
     };
     // The look-ahead columns t+2+j0 and t+3+j0 lie in [0, N) for every lane of the group
     // (j0 = -2 lane, lane < G) when 2G-4 <= t <= N-4.
@@ -465,13 +478,7 @@ __device__ void sweep16_impl(const SeqView &A, const SeqView &B, const Scoring &
       fold(t);
     }
     if (t < T_end) {
-      if constexpr (HALF) ST::load_half(gs.prof, ceven, lane, HA);
-      else ST::load(tab, ceven, lane, Wlo, HA);
-      uint32_t zH, zE;
-      top(t, zH, zE);
-      ST::run(t, zH, zE, sel, HALF ? HA : Wlo, HB, H, F, Hlast, Ecout, HtopPrev, Kr, Jp, NGE, NGO, one, scale, Rm,
-              vmask_at(t), 0, false);
-      out_bnd(t);
+      step(t, ceven, std::true_type{}, 0);
       fold(t);
     }
 
