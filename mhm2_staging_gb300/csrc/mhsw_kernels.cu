@@ -1052,7 +1052,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
       if (e != cudaSuccess) return e;
     }
     if (warps) {
-      const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, longs, false, fan ? fk->side[kBandClasses] : st);
+      const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, max_a, max_b, longs, false, fan ? fk->side[kBandClasses] : st);
       if (e != cudaSuccess) return e;
     }
     for (int c = 0; c < kBandClasses; c++) cs[c] = fan ? fk->side[c] : st;
@@ -1085,7 +1085,7 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
     if (e != cudaSuccess) return e;
   }
   if (warps && ps.n > 0) {
-    const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, longs, true, st);
+    const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, max_a, max_b, longs, true, st);
     if (e != cudaSuccess) return e;
   }
   // every search fits the warp kernel's tile and keys: nothing is left

@@ -130,7 +130,7 @@ cudaError_t launch_pack5(const ResultSet &rs, int64_t n, int32_t *out5, cudaStre
 // Begin searches of the wide list (escaped: those that outgrew their band) by a warp each
 // (mhsw_short.cu), where warp_begin holds.
 cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const WorkLists &wl, int sms,
-                            bool longs, bool escaped, cudaStream_t st);
+                            int max_a, int max_b, bool longs, bool escaped, cudaStream_t st);
 
 // ---- long pairs (mhsw_long.cu) -------------------------------------------------------
 // A pair with more rows than this (and, in the begin pass, a search whose first row cap is

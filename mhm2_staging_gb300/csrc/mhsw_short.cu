@@ -39,6 +39,13 @@ __device__ __forceinline__ int base_code(unsigned char x) {  // SSW's table (c_c
   return u == 'A' || u == 'U' ? 0 : u == 'C' ? 1 : u == 'G' ? 2 : u == 'T' ? 3 : kCodeN;
 }
 
+// Bytes of a warp's profile table.
+template <int K, bool S2>
+__host__ __device__ constexpr int warp_prof(bool step) {
+  constexpr int kCodes = S2 ? kCode16Zero + 1 : kCodeN + 1;
+  return (int)(step ? Prof16H<K, kCodes>::bytes(32) : Prof16<K, kCodes>::bytes(32));
+}
+
 struct ShortArgs {
   PairSet ps;  // a_seq raw; b_code when the codes are resident, else b_seq raw
   Scoring sc;
@@ -57,46 +64,68 @@ struct ShortArgs {
 // open >= gap extend, which short_batch checks), so E^' = max(E^ - gE, H') all the same.  That
 // is one add-max per row on the chain instead of three operations, for one more
 // instruction per cell pair: worth it where a warp has its scheduler nearly to itself.
-// S2 (score2 mode) keeps each row's maximum over the valid columns in Rm, as Step16 does.
-template <int R, bool S2>
+// S2 (score2 mode) keeps each row's maximum over the valid columns in Rm, as Step16 does; STEP
+// (scores up to 448: kModeStep) takes its half arithmetic, step keys and one table word a row pair.
+template <int R, bool S2, bool STEP>
 struct ShortStep {
   static_assert(R == 2 || R == 3 || R == 4 || R == 6 || R == 8, "row pairs per lane");
   static constexpr int kLay = R == 3 ? 4 : R;  // table layout (R = 3: that of 4, the last words unused)
-  using L = Prof16<kLay, S2 ? kCode16Zero + 1 : kCodeN + 1>;
+  static constexpr int kCodes = S2 ? kCode16Zero + 1 : kCodeN + 1;
+  using L = Prof16<kLay, kCodes>;
+  using LH = Prof16H<kLay, kCodes>;
+  using Eng = Step16<kLay, 32, S2, STEP ? kModeStep : kModeInt>;
   static constexpr uint32_t kKeyMask = KeyBits<R>::kMask;
-  __device__ static __forceinline__ void load(const uint4 *tab, int c, int lane, uint32_t (&lo)[kLay], uint32_t (&hi)[kLay]) {
-    Step16<kLay, 32, S2>::load(tab, c, lane, lo, hi);
+  static constexpr int kStepBits = STEP ? 3 : 0;
+  __device__ static __forceinline__ void load(const uint32_t *tab, int c, int lane, uint32_t (&lo)[kLay], uint32_t (&hi)[kLay]) {
+    if constexpr (STEP) Eng::load_half(tab, c, lane, lo);
+    else Eng::load(reinterpret_cast<const uint4 *>(tab), c, lane, lo, hi);
   }
-  __device__ static __forceinline__ void run(int t, uint32_t zH, uint32_t zE, uint32_t sel, const uint32_t (&Wlo)[kLay],
-                                             const uint32_t (&Phi)[kLay], uint32_t (&H)[R], uint32_t (&F)[R],
-                                             uint32_t &Hlast, uint32_t &Ecout, uint32_t &HtopPrev, uint32_t &Kl,
-                                             uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t one, uint32_t scale,
-                                             uint32_t (&Rm)[R], uint32_t vmask) {
+  __device__ static __forceinline__ void put(uint32_t *tab, int c, int w, int lane, uint32_t v) {
+    if constexpr (STEP) {
+      tab[LH::word(c, w, lane, 32)] = v;
+    } else {
+      tab[((c * L::kNV + L::lo_vec(w)) * 32 + lane) * 4 + L::lo_elem(w)] = v & 0xffffu;
+      tab[((c * L::kNV + L::hi_vec(w)) * 32 + lane) * 4 + L::hi_elem(w)] = v & 0xffff0000u;
+    }
+  }
+  // P: the diagonal inputs with the high half's score added, as in Step16::run.
+  __device__ static __forceinline__ void run(int t, int u, uint32_t zH, uint32_t zE, uint32_t sel,
+                                             const uint32_t (&Wlo)[kLay], const uint32_t (&Whi)[kLay], uint32_t (&P)[R],
+                                             uint32_t (&F)[R], uint32_t &Hlast, uint32_t &Ecout, uint32_t &Kl,
+                                             uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t NGOh, uint32_t one,
+                                             uint32_t scale, uint32_t (&Rm)[R], uint32_t vmask) {
     uint32_t Ev = prmt_sel(zE, Ecout, sel);
     const uint32_t Htop = prmt_sel(zH, Hlast, sel);
-    uint32_t Hd = HtopPrev, Kn = Kl;
-    HtopPrev = Htop;
+    auto add_lo = [&](uint32_t h, uint32_t w) { return STEP ? add_lo_f16x2(h, w) : mad_u32(h, one, w); };
+    auto add_hi = [&](uint32_t h, uint32_t w) { return STEP ? add_hi_f16x2(h, w) : mad_u32(h, one, w); };
+    uint32_t Q = add_lo(P[0], Wlo[0]), Kn = Kl;
+    P[0] = add_hi(Htop, Whi[0]);
     uint32_t key[R];
 #pragma unroll
     for (int k = 0; k < R; k++) {
-      const uint32_t Q = mad_u32(mad_u32(Hd, one, Wlo[k]), one, Phi[k]);
-      const uint32_t Hp = __viaddmax_s16x2_relu(__vmaxs2(Q, F[k]), NGO, 0u);
+      const uint32_t m = __vmaxs2(Q, F[k]);
+      const uint32_t Hp = STEP ? add_relu_f16x2(m, NGOh) : __viaddmax_s16x2_relu(m, NGO, 0u);
       const uint32_t Hn = __viaddmax_s16x2(Ev, NGO, Hp);
       Ev = __viaddmax_s16x2(Ev, NGE, Hp);
       F[k] = __viaddmax_s16x2(F[k], NGE, Hn);
-      Hd = H[k];
-      H[k] = Hn;
-      key[k] = mad_u32(Hn, scale, (uint32_t)(kKeyMask - k) * 0x00010001u);
+      if (k + 1 < R) {
+        Q = add_lo(P[k + 1], Wlo[k + 1]);
+        P[k + 1] = add_hi(Hn, Whi[k + 1]);
+      } else {
+        Hlast = Hn;
+      }
+      key[k] = mad_u32(Hn, scale, ((uint32_t)(kKeyMask - k) * (STEP ? 8u : 1u) + (STEP ? 7u - (uint32_t)u : 0u)) * 0x00010001u);
       if constexpr (S2) Rm[k] = __viaddmax_s16x2(Hn, vmask, Rm[k]);
     }
 #pragma unroll
     for (int k = 0; k + 1 < R; k += 2) Kn = __vimax3_s16x2(Kn, key[k], key[k + 1]);
     if constexpr (R % 2 != 0) Kn = __vmaxs2(Kn, key[R - 1]);
-    Hlast = H[R - 1];
     Ecout = Ev;
-    const uint32_t msk = sign_mask16(Kn - Kl + 0x7fff7fffu);
-    const uint32_t tt = (uint32_t)t * 0x00010001u;
-    Jp = (msk & tt) | (~msk & Jp);
+    if constexpr (!STEP) {
+      const uint32_t msk = sign_mask16(Kn - Kl + 0x7fff7fffu);
+      const uint32_t tt = (uint32_t)t * 0x00010001u;
+      Jp = (msk & tt) | (~msk & Jp);
+    }
     Kl = Kn;
   }
 };
@@ -105,56 +134,62 @@ struct ShortStep {
 // them, with kShortPad N codes on either side.  Returns the best key (same in every lane).
 // A step's profile words are loaded a step ahead of their use, its code three ahead.  S2: N
 // includes SSW's zero-score padding; rowmax[row] receives each row's maximum.
-template <int R, bool S2, class RowCode>
+template <int R, bool S2, bool STEP, class RowCode>
 __device__ __forceinline__ unsigned long long sweep_warp(int M, int N, RowCode row, const uint8_t *b, int dir,
                                                          const Scoring &sc, uint32_t *prof, int lane, uint32_t one,
                                                          uint16_t *rowmax) {
-  using ST = ShortStep<R, S2>;
-  using L = typename ST::L;
+  using ST = ShortStep<R, S2, STEP>;
   constexpr int K = ST::kLay;
-  constexpr int KB = KeyBits<R>::kBits;
+  constexpr int KS = ST::kStepBits, KB = KeyBits<R>::kBits + KS;
   constexpr uint32_t KMASK = KeyBits<R>::kMask;
   const uint32_t NGE = V16::splat(-sc.gap_extend), NGO = V16::splat(-sc.gap_open);
+  const uint32_t NGOh = (uint32_t)(0x8000 | sc.gap_open) * 0x00010001u;
   const int row0 = lane * 2 * R;
   int alo[R], ahi[R];
+  uint32_t base[R];
 #pragma unroll
   for (int w = 0; w < R; w++) {
     alo[w] = row0 + w < M ? row(row0 + w) : kCodePad;
     ahi[w] = row0 + R + w < M ? row(row0 + R + w) : kCodePad;
   }
   __syncwarp();
-  for (int c = 0; c < L::kCodes; c++) {
+  {  // profile words, as sweep16_impl builds them
+    const uint32_t miss = (uint32_t)(sc.gap_open - sc.mismatch), vn = (uint32_t)(sc.gap_open - sc.ambiguity);
+    const uint32_t plus = (uint32_t)(sc.match + sc.mismatch);
+    auto both = [&](int w, uint32_t v) {  // v in the halves whose row is in A
+      return (alo[w] == kCodePad ? 0u : v) | (ahi[w] == kCodePad ? 0u : v << 16);
+    };
 #pragma unroll
     for (int w = 0; w < R; w++) {
-      int slo = sub_score(alo[w], c, sc, sc.gap_open), shi = sub_score(ahi[w], c, sc, sc.gap_open);
-      if (S2 && c == kCode16Zero) {  // scores 0 against real rows; rows past A stay at -gO
-        slo = alo[w] == kCodePad ? -sc.gap_open : 0;
-        shi = ahi[w] == kCodePad ? -sc.gap_open : 0;
-      }
-      prof[((c * L::kNV + L::lo_vec(w)) * 32 + lane) * 4 + L::lo_elem(w)] = (uint32_t)(slo + sc.gap_open);
-      prof[((c * L::kNV + L::hi_vec(w)) * 32 + lane) * 4 + L::hi_elem(w)] = (uint32_t)(shi + sc.gap_open) << 16;
+      base[w] = (alo[w] == kCodePad ? 0u : alo[w] == kCodeN ? vn : miss) |
+                (ahi[w] == kCodePad ? 0u : ahi[w] == kCodeN ? vn : miss) << 16;
+      ST::put(prof, kCodeN, w, lane, both(w, vn));
+      if constexpr (S2) ST::put(prof, kCode16Zero, w, lane, both(w, (uint32_t)sc.gap_open));  // scores 0 against real rows
     }
+#pragma unroll
+    for (int c = 0; c < kCodeN; c++)
+#pragma unroll
+      for (int w = 0; w < R; w++)
+        ST::put(prof, c, w, lane, base[w] + (alo[w] == c ? plus : 0u) + (ahi[w] == c ? plus << 16 : 0u));
   }
   __syncwarp();
-  const uint4 *tab = reinterpret_cast<const uint4 *>(prof);
-  uint32_t H[R], F[R], Rm[R], lo[K], hi[K], hp[K];
+  uint32_t P[R], F[R], Rm[R], lo[K], hi[K];
 #pragma unroll
-  for (int k = 0; k < R; k++) H[k] = F[k] = Rm[k] = 0u;
-#pragma unroll
-  for (int k = 0; k < K; k++) hp[k] = 0u;
-  uint32_t Hlast = 0u, Ecout = 0u, HtopPrev = 0u, Kl = 0u, Jp = 0u;
+  for (int k = 0; k < R; k++) P[k] = F[k] = Rm[k] = 0u;
+  uint32_t Hlast = 0u, Ecout = 0u, Kl = 0u, Jp = 0u;
   const uint32_t sel = lane == 0 ? 0x54BBu : 0x5432u;
   const uint32_t scale = one << KB;
   const int steps = N + 63;  // the last lane's high half ends at step N + 62
   const uint8_t *bl = b - 2 * lane * dir;
-  ST::load(tab, bl[0], lane, lo, hi);
+  ST::load(prof, bl[0], lane, lo, hi);
   int c1 = bl[dir], c2 = bl[2 * dir];
   for (int t = 0; t < steps; t += 4) {
+    uint32_t Kb = 0u;
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       const uint32_t zH = __shfl_up_sync(0xffffffffu, Hlast, 1), zE = __shfl_up_sync(0xffffffffu, Ecout, 1);
       uint32_t nlo[K], nhi[K];
-      ST::load(tab, c1, lane, nlo, nhi);
+      ST::load(prof, c1, lane, nlo, nhi);
       c1 = c2;
       c2 = bl[(t + u + 3) * dir];
       uint32_t vmask = 0u;  // S2: -16384 in a half whose column lies outside [0, N)
@@ -162,14 +197,15 @@ __device__ __forceinline__ unsigned long long sweep_warp(int M, int N, RowCode r
         const int jl = t + u - 2 * lane;
         vmask = ((unsigned)jl < (unsigned)N ? 0u : 0x0000C000u) | ((unsigned)(jl - 1) < (unsigned)N ? 0u : 0xC0000000u);
       }
-      ST::run(t + u, zH, zE, sel, lo, hp, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, scale, Rm, vmask);
+      ST::run(t + u, u, zH, zE, sel, lo, STEP ? lo : hi, P, F, Hlast, Ecout, STEP ? Kb : Kl, Jp, NGE, NGO, NGOh, one, scale,
+              Rm, vmask);
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        hp[k] = hi[k];
         lo[k] = nlo[k];
-        hi[k] = nhi[k];
+        if constexpr (!STEP) hi[k] = nhi[k];
       }
     }
+    if constexpr (STEP) ST::Eng::fold_block(t, Kb, Kl, Jp);
   }
   if constexpr (S2) {
 #pragma unroll
@@ -183,7 +219,7 @@ __device__ __forceinline__ unsigned long long sweep_warp(int M, int N, RowCode r
 #pragma unroll
   for (int half = 0; half < 2; half++) {
     const uint32_t key = half ? (Kl >> 16) : (Kl & 0xffffu);
-    const int v = (int)(key >> KB), r = row0 + (half ? R : 0) + (int)KMASK - (int)(key & KMASK);
+    const int v = (int)(key >> KB), r = row0 + (half ? R : 0) + (int)KMASK - (int)((key >> KS) & KMASK);
     const int col = (int)(half ? (Jp >> 16) : (Jp & 0xffffu)) - 2 * lane - half;
     if (v > 0 && r < M) {
       const unsigned long long kk = best_key(v, r, col);
@@ -199,17 +235,17 @@ __device__ __forceinline__ unsigned long long sweep_warp(int M, int N, RowCode r
 }
 
 // The narrowest instantiation that holds M rows (M <= 64 * KMAX).
-template <int KMAX, bool S2, class RowCode>
+template <int KMAX, bool S2, bool STEP, class RowCode>
 __device__ __forceinline__ unsigned long long sweep_rows(int M, int N, RowCode row, const uint8_t *b, int dir,
                                                          const Scoring &sc, uint32_t *prof, int lane, uint32_t one,
                                                          uint16_t *rowmax) {
-  if (M <= 128) return sweep_warp<2, S2>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
-  if (M <= 192) return sweep_warp<3, S2>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
+  if (M <= 128) return sweep_warp<2, S2, STEP>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
+  if (M <= 192) return sweep_warp<3, S2, STEP>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
   if constexpr (KMAX >= 6) {
-    if (M > 384) return sweep_warp<8, S2>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
-    if (M > 256) return sweep_warp<6, S2>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
+    if (M > 384) return sweep_warp<8, S2, STEP>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
+    if (M > 256) return sweep_warp<6, S2, STEP>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
   }
-  return sweep_warp<4, S2>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
+  return sweep_warp<4, S2, STEP>(M, N, row, b, dir, sc, prof, lane, one, rowmax);
 }
 
 // SSW's second-best score from the row maxima: see k_score2 in mhsw_kernels.cu.
@@ -270,7 +306,7 @@ __device__ __forceinline__ void write_result(const ShortArgs &g, int64_t p, cons
 // One warp per pair, one warp per block (so the pairs of a short batch spread over the SMs).
 // Shared memory: the profile table, in score2 mode the row maxima, then B's codes between
 // two pads.
-template <int KMAX, bool S2>
+template <int KMAX, bool S2, bool STEP>
 __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t *prof = reinterpret_cast<uint32_t *>(smem);
@@ -300,14 +336,14 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
       auto row = [&](int i) { return base_code(a[i]); };
       int np = S2 ? ssw_pad16(N) : N;
       stage(np);
-      const unsigned long long k = sweep_rows<KMAX, S2>(M, np, row, bc, 1, sc, prof, lane, one, rowmax);
+      const unsigned long long k = sweep_rows<KMAX, S2, STEP>(M, np, row, bc, 1, sc, prof, lane, one, rowmax);
       const int S = key_value(k);
       if constexpr (S2) {
         const bool word = S + ssw_bias(sc) >= 255;
         if (word && ssw_pad8(N) != np) {  // SSW's word path pads B less
           np = ssw_pad8(N);
           stage(np);
-          sweep_rows<KMAX, S2>(M, np, row, bc, 1, sc, prof, lane, one, rowmax);
+          sweep_rows<KMAX, S2, STEP>(M, np, row, bc, 1, sc, prof, lane, one, rowmax);
         }
         warp_score2(rowmax, M, S > 0 ? key_row(k) : -1, word, lane, s2, s2_at);
       }
@@ -331,7 +367,7 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
             if (je - n2 - x >= 0) bc[je - n2 - x] = kCodeN;
           }
           __syncwarp();
-          return sweep_rows<KMAX, false>(t, n2, [&](int i) { return base_code(a[ie - i]); }, bc + je, -1, sc, prof,
+          return sweep_rows<KMAX, false, STEP>(t, n2, [&](int i) { return base_code(a[ie - i]); }, bc + je, -1, sc, prof,
                                          lane, one, nullptr);
         };
         const int t0 = band_first_cap(S, sc.match, M2);
@@ -359,11 +395,12 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
 // Begin searches of the wide list, a warp each: bands wider than the banded kernels hold, those
 // that outgrew theirs, and in all but the largest batches the widest of their classes, whose threads walk a row pair in
 // 0.5 us -- 250 rows took 130-160 us however few the pairs.  Same search as k_short's.
+template <bool STEP>
 __global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scoring sc, WorkLists wl, bool longs,
                                                  bool escaped) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t *prof = reinterpret_cast<uint32_t *>(smem);
-  uint8_t *bc = smem + Prof16<8>::bytes(32) + kShortPad;  // reversed: bc[j] = column j of the box
+  uint8_t *bc = smem + warp_prof<8, false>(STEP) + kShortPad;  // reversed: bc[j] = column j of the box
   const int lane = threadIdx.x;
   const uint32_t one = (uint32_t)(sc.gap_open >> 30) + 1u;  // a 1 the compiler cannot fold
   // escaped: the searches that outgrew their band, from the end of the list
@@ -383,7 +420,7 @@ __global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scori
       for (int j = lane - kShortPad; j < n2 + kShortPad; j += 32)
         bc[j] = (uint8_t)((unsigned)j < (unsigned)n2 ? (int)b[-j] : kCodeN);
       __syncwarp();
-      q = sweep_rows<8, false>(t, n2, [&](int i) { return (int)a[-i]; }, bc, 1, sc, prof, lane, one, nullptr);
+      q = sweep_rows<8, false, STEP>(t, n2, [&](int i) { return (int)a[-i]; }, bc, 1, sc, prof, lane, one, nullptr);
       if (key_value(q) == S || t == M2) break;
     }
     if (lane == 0) {
@@ -402,10 +439,11 @@ __global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scori
 }  // namespace
 
 cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scoring &sc, const WorkLists &wl, int sms,
-                            bool longs, bool escaped, cudaStream_t st) {
-  constexpr size_t smem = Prof16<8>::bytes(32) + 2 * kShortPad + kWarpBeginCols;
+                            int max_a, int max_b, bool longs, bool escaped, cudaStream_t st) {
+  const bool step = mode_for((long long)std::min(max_a, max_b) * sc.match, 8) == kModeStep;
+  const size_t smem = warp_prof<8, false>(step) + 2 * kShortPad + kWarpBeginCols;
   const int64_t grid = std::min<int64_t>(ps.n, (int64_t)sms * 12);
-  k_rev_warp<<<(unsigned)grid, 32, smem, st>>>(ps, rs, sc, wl, longs, escaped);
+  (step ? k_rev_warp<true> : k_rev_warp<false>)<<<(unsigned)grid, 32, smem, st>>>(ps, rs, sc, wl, longs, escaped);
   return cudaGetLastError();
 }
 
@@ -417,11 +455,13 @@ bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b
 static cudaError_t launch(ShortArgs g, cudaStream_t st) {
   if (g.ps.n <= 0) return cudaSuccess;
   const bool small = g.max_a <= 256, s2 = g.rs.score2 != nullptr;
-  g.prof_bytes = (int)(s2 ? (small ? Prof16<4, kCode16Zero + 1>::bytes(32) : Prof16<8, kCode16Zero + 1>::bytes(32))
-                          : (small ? Prof16<4>::bytes(32) : Prof16<8>::bytes(32)));
+  const bool step = mode_for((long long)std::min(g.max_a, g.max_b) * g.sc.match, 8) == kModeStep;
+  g.prof_bytes = s2 ? (small ? warp_prof<4, true>(step) : warp_prof<8, true>(step))
+                    : (small ? warp_prof<4, false>(step) : warp_prof<8, false>(step));
   const size_t smem =
       ((size_t)g.prof_bytes + (s2 ? (small ? 512 : 1024) + 16 : 0) + 2 * kShortPad + (size_t)g.max_b + 15) / 16 * 16;
-  auto kern = s2 ? (small ? k_short<4, true> : k_short<8, true>) : (small ? k_short<4, false> : k_short<8, false>);
+  auto kern = s2 ? (small ? k_short<4, true, false> : k_short<8, true, false>) : (small ? k_short<4, false, false> : k_short<8, false, false>);
+  if (step) kern = s2 ? (small ? k_short<4, true, true> : k_short<8, true, true>) : (small ? k_short<4, false, true> : k_short<8, false, true>);
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
   if (e != cudaSuccess) return e;
   kern<<<(unsigned)g.ps.n, 32, smem, st>>>(g);
