@@ -77,24 +77,24 @@ struct LongArgs {
 };
 
 // The keyed step with keys above a base (nbase: its negative, per half).  LAZY (gap open >= gap
-// extend): the chain down the rows is one add-max per row (ShortStep in mhsw_short.cu).
+// extend): the chain down the rows is one add-max per row (ShortStep in mhsw_short.cu), and the
+// relu is a maximum with gO before the subtraction, which then runs on the multiply-add pipe (a
+// warp has a scheduler to itself here, and the integer pipe is what it waits for).
 template <bool LAZY>
 __device__ __forceinline__ void long_step(int t, uint32_t zH, uint32_t zE, const uint32_t (&Wlo)[kLK],
-                                          const uint32_t (&Phi)[kLK], uint32_t (&H)[kLK], uint32_t (&F)[kLK],
-                                          uint32_t &Hlast, uint32_t &Ecout, uint32_t &HtopPrev, uint32_t &Kl,
-                                          uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t one, uint32_t eight,
-                                          uint32_t nbase) {
+                                          const uint32_t (&Whi)[kLK], uint32_t (&P)[kLK], uint32_t (&F)[kLK],
+                                          uint32_t &Hlast, uint32_t &Ecout, uint32_t &Kl, uint32_t &Jp, uint32_t NGE,
+                                          uint32_t NGO, uint32_t GO, uint32_t one, uint32_t eight, uint32_t nbase) {
   uint32_t Ev = __byte_perm(zE, Ecout, 0x5432);
   const uint32_t Htop = __byte_perm(zH, Hlast, 0x5432);
-  uint32_t Hd = HtopPrev;
-  HtopPrev = Htop;
+  uint32_t Q = mad_u32(P[0], one, Wlo[0]);
+  P[0] = mad_u32(Htop, one, Whi[0]);
   uint32_t key[kLK];
 #pragma unroll
   for (int k = 0; k < kLK; k++) {
-    const uint32_t Q = mad_u32(mad_u32(Hd, one, Wlo[k]), one, Phi[k]);
     uint32_t Hn;
     if constexpr (LAZY) {
-      const uint32_t Hp = __viaddmax_s16x2_relu(__vmaxs2(Q, F[k]), NGO, 0u);
+      const uint32_t Hp = mad_u32(__vimax3_s16x2(Q, F[k], GO), one, 0u - GO);  // (no borrow: halves >= gO)
       Hn = __viaddmax_s16x2(Ev, NGO, Hp);
       Ev = __viaddmax_s16x2(Ev, NGE, Hp);
     } else {
@@ -103,14 +103,17 @@ __device__ __forceinline__ void long_step(int t, uint32_t zH, uint32_t zE, const
       Ev = __viaddmax_s16x2(Ev, NGE, Hn);
     }
     F[k] = __viaddmax_s16x2(F[k], NGE, Hn);
-    Hd = H[k];
-    H[k] = Hn;
+    if (k + 1 < kLK) {
+      Q = mad_u32(P[k + 1], one, Wlo[k + 1]);
+      P[k + 1] = mad_u32(Hn, one, Whi[k + 1]);
+    } else {
+      Hlast = Hn;
+    }
     key[k] = mad_u32(__viaddmax_s16x2_relu(Hn, nbase, 0u), eight, (uint32_t)(7 - k) * 0x00010001u);
   }
   uint32_t Kn = Kl;
 #pragma unroll
   for (int k = 0; k < kLK; k += 2) Kn = __vimax3_s16x2(Kn, key[k], key[k + 1]);
-  Hlast = H[kLK - 1];
   Ecout = Ev;
   const uint32_t msk = sign_mask16(Kn - Kl + 0x7fff7fffu);
   const uint32_t tt = (uint32_t)t * 0x00010001u;
@@ -129,6 +132,7 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
   constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const uint32_t NGE = V16::splat(-sc.gap_extend), NGO = V16::splat(-sc.gap_open);
+  const uint32_t GO = V16::splat(sc.gap_open);
   const uint32_t one = (uint32_t)(sc.gap_open >> 30) + 1u, eight = one << 3;  // not folded by the compiler
   const int nstrips = (M + kLRows - 1) / kLRows;
   auto c0_of = [&](int s) { return max(0, s * kLRows - I); };
@@ -191,9 +195,10 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
     const int first_top = (int)__reduce_max_sync(full, max(cur & 0xffffu, HtopPrev));
     int base_lo = max(first_top - 1024, 0), base_hi = base_lo;
     uint32_t nbase = V16::pack(-base_lo, -base_hi);
-    uint32_t H[kLK], F[kLK], lo[kLK], hi[kLK], hp[kLK];  // this column's words, the last column's hi words
+    uint32_t P[kLK], F[kLK], lo[kLK], hi[kLK];  // (P: Step16::run of mhsw_engine16.cuh)
 #pragma unroll
-    for (int k = 0; k < kLK; k++) H[k] = F[k] = hp[k] = 0u;
+    for (int k = 0; k < kLK; k++) P[k] = F[k] = 0u;
+    P[0] = HtopPrev;  // (the high halves start a column later, at 0)
     uint32_t Hlast = 0u, Ecout = 0u, Kl = 0u, Jp = 0u;
     const int j0 = c0 - 2 * lane;
     auto code_at = [&](int j) -> int { return j >= c0 && j < c1 ? (int)b[(int64_t)bdir * j] : kCodeN; };
@@ -226,10 +231,9 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
           ST::load(tab, c1s, lane, nlo, nhi);
           c1s = c2s;
           c2s = kGuard ? code_at(j0 + t + 3) : (int)bl[(int64_t)bdir * (t + 3)];
-          long_step<LAZY>(t, zH, zE, lo, hp, H, F, Hlast, Ecout, HtopPrev, Kl, Jp, NGE, NGO, one, eight, nbase);
+          long_step<LAZY>(t, zH, zE, lo, hi, P, F, Hlast, Ecout, Kl, Jp, NGE, NGO, GO, one, eight, nbase);
 #pragma unroll
           for (int k = 0; k < kLK; k++) {
-            hp[k] = hi[k];
             lo[k] = nlo[k];
             hi[k] = nhi[k];
           }
