@@ -86,7 +86,7 @@ typedef struct {
   double fwd_cells;   /* sum over pairs of len(A) * len(B) */
   int64_t n_pairs;
   int64_t n_overflow16;  /* pairs re-run in int32 */
-  int64_t n_rev_wide;    /* begin searches that used the wavefront path */
+  int64_t n_rev_wide;    /* begin searches wider than the banded kernels */
   int64_t launches;      /* kernels launched by the call (a graph replay counts its kernels) */
   int64_t graph_replays; /* CUDA graph launches by this handle so far: a device-resident batch
                           * aligned again with the same pointers, sizes and settings is

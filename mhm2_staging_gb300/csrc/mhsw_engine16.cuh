@@ -9,8 +9,8 @@
 //     Then X^' = max(X^ - gE, H) uses H directly, and
 //       H = max(max(Hdiag + s + gO, E^, F^) - gO, 0)
 //     is one 3-way max and one add-max-relu.  Hdiag + s + gO is formed with integer
-//     multiply-adds (FMA pipe) from two table words, one per half, each already
-//     biased by +gO; this needs s + gO >= 0 for every score (mismatch and ambiguity
+//     multiply-adds (FMA pipe) of two score words, one per half, each already
+//     biased by +gO (the high half's as soon as Hdiag is known, a step earlier); this needs s + gO >= 0 for every score (mismatch and ambiguity
 //     not above the gap-open penalty), which the driver checks before choosing this
 //     engine.  Rows past the end of A score -gO (biased 0); columns outside B read as
 //     N (score -ambiguity <= 0).  Cells left of column 0 then stay exactly 0, and every
@@ -24,12 +24,12 @@
 //     first column at which that row reached that score -- the lexicographic rule of
 //     SSW (ssw_core.cpp:474-506).  Keys need H < 2^(15-b), so this engine flags pairs
 //     whose score reaches the ceiling (at most KeyBits::kCap) for the int32 engine.
-//  3. The profile table holds separate low-half and high-half words for the five B
-//     codes, loaded as 128-bit vectors: K/4 vectors of low words, K/4 of high words and,
+//  3. In integer mode the profile table holds separate low-half and high-half words for the
+//     five B codes, loaded as 128-bit vectors: K/4 vectors of low words, K/4 of high words and,
 //     when K is 2 mod 4, one vector holding the last two low and the last two high
 //     words (every load is a full 128-bit vector, conflict-free across the groups of a
-//     warp).  The high words loaded at step t serve the high half at step t+1 (the step
-//     loop is unrolled by two so the two word sets alternate registers).
+//     warp).  A step uses the words it loads: the low ones for its own low half, the high ones
+//     for the next step's high half (Step16::run).
 //  4. B codes are read from global memory (each loaded two steps before its use) instead
 //     of being staged in shared memory, so a group's shared memory is its profile table only.
 //     The sweep runs in three phases: the middle one, where every lane's look-ahead column
@@ -57,7 +57,7 @@
 //              the first step, so the running key and its step are brought up to date once a
 //              block instead of once a step (four instructions of about 80).
 // Forward pass, int / half / step: 800,000 uneven pairs 13.19 / 12.91 / 12.63 ms, 30,011 pairs of
-// 250 bp against 2-8 kb 7.34 / 6.74 / 6.67.  Unsigned keys (twice the cap), or a key that ages
+// 250 bp against 2-8 kb 7.34 / 6.74 / 6.67 (12.02 and 6.47 with the diagonal of Step16::run).  Unsigned keys (twice the cap), or a key that ages
 // in place of step constants, give half of the last gain back.
 //
 // Score2 mode (S2) also produces what SSW's second-best score is computed from

@@ -3,7 +3,7 @@
 // Forward  : k_fwd<V16|V32, K, G>  -- the wavefront engine of mhsw_engine.cuh, one
 //            G-lane group per pair (the reference's one-block-per-pair
 //            sequence_dna_kernel, src/adept-sw/kernel.cpp:160-333, replaced).
-// Begin    : k_rev_banded          -- one thread per pair, banded DP on the reversed
+// Begin    : k_rev_band16, k_rev_band -- one thread per pair, banded DP on the reversed
 //            prefixes A[0..a_end], B[0..b_end] (the reference's reverse pass,
 //            src/ssw/ssw_core.cpp:1166-1178 and src/adept-sw/kernel.cpp:335-509).
 //            Exact: every cell holding the score lies on an alignment from the end
@@ -11,8 +11,9 @@
 //            g*min(gO,gE) + max(gO-gE, 0) <= D*match - score with
 //            D <= min(a_end+1, b_end+1) diagonal steps,
 //            so the band |j - i| <= g contains it and banding only lowers other cells.
-//            k_rev_wave runs the wavefront engine on the reversed box for the rare
-//            pairs whose band is wider than the widest banded instantiation.
+//            Bands wider than the widest banded instantiation go to the warp-per-search
+//            kernel (mhsw_short.cu), long pairs' to theirs (mhsw_long.cu), and what neither
+//            holds to k_rev_wave, the wavefront engine on the reversed box.
 // Output   : k_finalize / k_pack5  -- orientation mapping into the caller's arrays.
 #include <algorithm>
 #include <cstdio>

@@ -81,9 +81,10 @@ cudaError_t launch_forward(const FwdConfig &cfg, bool wide32, const PairSet &ps,
 // substitution score plus the gap-open penalty is non-negative.
 bool keyed_scoring(const Scoring &sc);
 
-// Begin pass: banded thread-per-pair kernels (bands of up to 16, 32, 64 cells, each
-// escalating to the next), then the wavefront kernel on reversed prefixes for the pairs
-// left in wl.wide.  order (may be null) is the pair order of the first kernel.
+// Begin pass: banded thread-per-pair kernels (seven band classes of up to 63 cells) beside the
+// warp-per-search kernel for the wider ones, then the long pairs' kernel and the wavefront
+// kernel on reversed prefixes for what is left in wl.wide.  order (may be null) is the pair
+// order the classes are laid out in.
 cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, const Scoring &sc, int max_a,
                            int max_b, void *scratch, size_t scratch_bytes, const WorkLists &wl, cudaStream_t st,
                            const uint32_t *order, const Forks *fk = nullptr);
