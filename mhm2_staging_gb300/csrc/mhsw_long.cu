@@ -166,9 +166,11 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
     __syncwarp();
     // waits until the strip above has published its columns below `col` (or ended).  `seen` is
     // its progress word as loaded a chunk ago, so a strip that is not held up does not stand
-    // still for the word's latency.
+    // still for the word's latency; and `fenced` says that the fence of this strip's own publishing
+    // came after that load, which then orders this strip's reads as well (one fence a chunk).
     const int pw = (s + W - 1) % W;
     unsigned long long seen = 0ull;
+    bool fenced = false;
     auto await = [&](int col) -> bool {
       if (s == 0) return true;
       const unsigned long long want = ((unsigned long long)(s - 1) << 32) | (unsigned)col;
@@ -176,9 +178,11 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
       while (seen < want) {
         if (++polls > kLongWaits || *(volatile int *)&sh.failed) return false;
         seen = prog[pw];
+        fenced = false;
       }
-      cluster_fence();
+      if (!fenced) cluster_fence();
       seen = prog[pw];
+      fenced = false;
       return true;
     };
     auto load_top = [&](int t) -> uint32_t {  // boundary words of columns c0 + t + lane
@@ -256,12 +260,11 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
         }
       }
       cur = nxt;
-      if (!last && lane == 31) {
-        const int done = min(t0 + kLChunk - 63, ncols);
-        if (done > 0) {
-          cluster_fence();
-          prog[warp] = ((unsigned long long)s << 32) | (unsigned)(c0 + done);
-        }
+      const int done = min(t0 + kLChunk - 63, ncols);
+      if (!last && done > 0) {
+        cluster_fence();  // by every lane: lane 31 publishes, all read the row above
+        fenced = true;
+        if (lane == 31) prog[warp] = ((unsigned long long)s << 32) | (unsigned)(c0 + done);
       }
     }
     if (!ok && lane == 0) sh.failed = 1;
