@@ -189,7 +189,7 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
       const int j = c0 + t + lane;
       return s > 0 && j < pc1 && j < c1 ? *(volatile const uint32_t *)(top_row + j) : 0u;
     };
-    bool ok = await(min(c0 + kLChunk, pc1));
+    bool ok = __all_sync(full, await(min(c0 + kLChunk, pc1)));  // (the warp's lanes go on or give up together)
     uint32_t cur = ok ? load_top(0) : 0u;
     // H above-left of the strip's first cell, and the base of both halves: the first columns may
     // take large values from the row above at once
@@ -211,12 +211,12 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
     int c1s = code_at(j0 + 1), c2s = code_at(j0 + 2);
     const int steps = ncols > 0 ? ncols + 63 : 0;
     for (int t0 = 0; t0 < steps && ok; t0 += kLChunk) {
-      ok = await(min(c0 + t0 + 2 * kLChunk, pc1));
+      ok = __all_sync(full, await(min(c0 + t0 + 2 * kLChunk, pc1)));
       if (goal > 0 && s > 0) {
         // An earlier strip reached the score: nothing here can win.  Tested after the wait: a
         // strip that stopped this way ends its successor's wait without its columns.
         const unsigned long long bk = *(volatile unsigned long long *)&sh.best;
-        if (key_value(bk) == goal && key_row(bk) < s * kLRows) break;
+        if (__any_sync(full, key_value(bk) == goal && key_row(bk) < s * kLRows)) break;
       }
       const uint32_t nxt = ok ? load_top(t0 + kLChunk) : 0u;
       auto eight_steps = [&](int tb, auto guarded) {
