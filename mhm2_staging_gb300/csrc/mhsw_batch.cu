@@ -215,6 +215,7 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   if ((size_t)n > bs.cap) {
     const size_t c = (size_t)n + (size_t)n / 8 + 1024;
     bs.cap = 0;
+    bs.moves++;
     if ((e = grow(&bs.order, c))) return fail(e, "cudaMalloc pair order");
     bs.cap = c;
   }
@@ -294,6 +295,7 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     if (max_a > 2 * 8 * kGKLong) {
       const size_t need = (size_t)grid_l * gpb_l * (size_t)stride * sizeof(V16::Pay);
       if (need > bs.scratch_bytes) {
+        bs.moves++;
         if (bs.scratch) cudaFree(bs.scratch);
         bs.scratch = nullptr;
         bs.scratch_bytes = 0;

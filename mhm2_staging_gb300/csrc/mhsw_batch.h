@@ -61,6 +61,7 @@ struct BatchState {
   int *ctl = nullptr;           // claim counters, bucket starts and bin counts of one ordered batch
   void *scratch = nullptr;  // strip scratch for A longer than one strip
   size_t scratch_bytes = 0;
+  uint64_t moves = 0;       // reallocations of order and scratch
   BatchShape shape;
   BatchSignature tuned_for;
   bool tuned = false;

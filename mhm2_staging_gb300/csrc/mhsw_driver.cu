@@ -29,12 +29,17 @@
 
 namespace {
 
+// A device buffer that grows, counting its reallocations in a counter of its owner's: a captured
+// graph holds buffers by address and is replayed only while their counter stands where it did.
 template <class T>
 struct DBuf {
   T *p = nullptr;
   size_t cap = 0;
+  uint64_t &moves;
+  explicit DBuf(uint64_t &owner_moves) : moves(owner_moves) {}
   cudaError_t reserve(size_t n) {
     if (n <= cap) return cudaSuccess;
+    moves++;
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
@@ -179,29 +184,31 @@ struct mhsw_driver {
   cudaStream_t st = nullptr;
   cudaEvent_t ev_done = nullptr;
   bool ev_live = false;
+  uint64_t moves = 0;    // reallocations of the device buffers a graph may hold ...
+  uint64_t unheld = 0;   // ... and of those it never does
   cudaEvent_t ev_t[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
 
   // device batch
-  DBuf<char> a_seq, b_seq;
-  DBuf<int64_t> a_off, b_off;
-  DBuf<int32_t> a_len, b_len;
-  DBuf<int32_t> r_score, r_aend, r_bend, r_abeg, r_bbeg;
-  DBuf<uint32_t> r_flag;
-  DBuf<int64_t> l_ovf, l_wide, l_bands;
-  DBuf<int> l_counts;
-  DBuf<uint8_t> a_code, b_code;  // base codes of the current batch
-  DBuf<unsigned char> scratch;
-  DBuf<uint32_t> long_bnd;  // strip boundaries of the long-pair kernels
-  DBuf<unsigned char> call_arena;  // one call's own arrays (caller side, protein), kept between calls
-  DBuf<unsigned char> outv;  // 5 x int16 + 5 x int32 arrays
-  DBuf<int32_t> out5;
+  DBuf<char> a_seq{unheld}, b_seq{unheld};
+  DBuf<int64_t> a_off{unheld}, b_off{unheld};
+  DBuf<int32_t> a_len{unheld}, b_len{unheld};
+  DBuf<int32_t> r_score{moves}, r_aend{moves}, r_bend{moves}, r_abeg{moves}, r_bbeg{moves};
+  DBuf<uint32_t> r_flag{moves};
+  DBuf<int64_t> l_ovf{moves}, l_wide{moves}, l_bands{moves};
+  DBuf<int> l_counts{moves};
+  DBuf<uint8_t> a_code{moves}, b_code{moves};  // base codes of the current batch
+  DBuf<unsigned char> scratch{moves};
+  DBuf<uint32_t> long_bnd{moves};  // strip boundaries of the long-pair kernels
+  DBuf<unsigned char> call_arena{unheld};  // one call's own arrays (caller side, protein), kept between calls
+  DBuf<unsigned char> outv{unheld};  // 5 x int16 + 5 x int32 arrays
+  DBuf<int32_t> out5{unheld};
   mhsw::BatchState batch;     // batched-form work buffers
   CopyPool copy_pool;         // host threads for staging a block's strings
   mhsw::BatchSignature sig;   // length signature of the batch being aligned (the tuner's key)
   // score2 mode: SSW's second-best score per pair (row maxima arenas, results)
   bool score2 = false;
   int64_t score2_n = -1;  // pairs of the last batch whose second-best scores are in r_score2
-  DBuf<int32_t> rowmax16, rowmax8, r_score2, r_aend2;
+  DBuf<int32_t> rowmax16{moves}, rowmax8{moves}, r_score2{moves}, r_aend2{moves};
   HBuf<int32_t> h_score2;  // drop-in protocol: score2 then a_end2, n each
   mhsw::Forks forks;          // side streams for launches that overlap on the device
   // CIGAR mode: SSW's report_cigar output per pair (ops arena, lists, scratch)
@@ -212,16 +219,16 @@ struct mhsw_driver {
   double cigar_ms = 0;
   int64_t cigar_generic = 0;   // pairs of the last batch that took the generic kernel
   int sms = 152;
-  DBuf<int32_t> c_nops, c_mism;
-  DBuf<int64_t> c_off, c_ordoff, c_c64;
-  DBuf<uint32_t> c_arena, c_ordops, c_dirs;
-  DBuf<unsigned long long> c_cursor;
-  DBuf<int> c_counts;
-  DBuf<int2> c_lists;
-  DBuf<int4> c_generic, c_gsorted;
-  DBuf<uint32_t> c_keys_in, c_keys_out, c_idx_in, c_idx_out;
-  DBuf<unsigned char> c_sort_temp;
-  DBuf<unsigned char> c_pool, c_temp;
+  DBuf<int32_t> c_nops{moves}, c_mism{moves};
+  DBuf<int64_t> c_off{moves}, c_ordoff{unheld}, c_c64{unheld};
+  DBuf<uint32_t> c_arena{moves}, c_ordops{unheld}, c_dirs{moves};
+  DBuf<unsigned long long> c_cursor{moves};
+  DBuf<int> c_counts{moves};
+  DBuf<int2> c_lists{moves};
+  DBuf<int4> c_generic{moves}, c_gsorted{unheld};
+  DBuf<uint32_t> c_keys_in{moves}, c_keys_out{moves}, c_idx_in{moves}, c_idx_out{moves};
+  DBuf<unsigned char> c_sort_temp{moves};
+  DBuf<unsigned char> c_pool{unheld}, c_temp{unheld};
   HBuf<int> h_ccounts;
   cudaEvent_t ev_c[2] = {nullptr, nullptr};
   // Batch calls enqueued (mhsw_align_pairs_async) and not yet completed: up to kSlots,
@@ -245,9 +252,10 @@ struct mhsw_driver {
   // which the kernel reads and writes in place.
   HBuf<unsigned char> h_small[kSlots];
   struct InSet {
-    DBuf<char> a_seq, b_seq;
-    DBuf<int64_t> a_off, b_off;
-    DBuf<int32_t> a_len, b_len;
+    uint64_t unheld = 0;  // (a graph is of a resident batch: it reads no input set)
+    DBuf<char> a_seq{unheld}, b_seq{unheld};
+    DBuf<int64_t> a_off{unheld}, b_off{unheld};
+    DBuf<int32_t> a_len{unheld}, b_len{unheld};
     cudaEvent_t free_ev = nullptr;  // recorded after the kernels of the set's last call
     bool used = false;
   } in_sets[kSlots];
@@ -278,7 +286,11 @@ struct mhsw_driver {
   };
   GraphKey gkey{};
   bool gkey_seen = false;
+  uint64_t gmoves = 0;  // buffer_moves() when the batch of gkey had been enqueued
   cudaGraphExec_t gexec = nullptr;
+  int64_t glaunches = 0;             // kernels of the graph
+  const uint32_t *gorder = nullptr;  // fwd_order of the captured batch
+  uint64_t buffer_moves() const { return moves + batch.moves; }
   bool use_graphs = true;
   int64_t graph_launches = 0;  // replays so far (diagnostics)
 
@@ -421,14 +433,6 @@ struct mhsw_driver {
 namespace {
 
 int finish_pending(mhsw_driver *d);
-
-// Forgets the captured graph of a device batch: calls that may resize the handle's buffers
-// outside the batch entry point (whose own calls replace the graph) leave it dangling.
-void drop_graph(mhsw_driver *d) {
-  if (d->gexec) cudaGraphExecDestroy(d->gexec);
-  d->gexec = nullptr;
-  d->gkey_seen = false;
-}
 
 // Device buffers for n pairs and the byte totals; result arrays; lists.
 int ensure_device(mhsw_driver *d, int64_t n, int64_t a_bytes, int64_t b_bytes) {
@@ -1212,7 +1216,6 @@ int mhsw_run_kernel_forwards(mhsw_driver *d, const char *const *reads, const int
   if (rc) return rc;
   d->sig = mhsw::batch_signature(d->orientation == MHSW_ORIENT_KLIGN ? read_lens : contig_lens, n, d->max_a,
                                  d->max_b);
-  if (!d->brief_batch) drop_graph(d);
   if (d->brief_batch) {
     // one launch for both passes, from the pinned staging buffers into the pinned result views
     mhsw::OutViews dv, hv;
@@ -1715,7 +1718,8 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
     return MHSW_OK;
   };
   // A device-resident batch with all size hints is graph-eligible: the second identical
-  // call captures the enqueued work into a CUDA graph, later identical calls replay it.
+  // call captures the enqueued work into a CUDA graph, later identical calls replay it, also
+  // with other batches in between unless one of them had a buffer reallocated (buffer_moves).
   const bool hinted = !host_io && pairs->max_a_len > 0 && pairs->max_b_len > 0 && pairs->a_bytes > 0 &&
                       pairs->b_bytes > 0;
   mhsw_driver::GraphKey key{};
@@ -1737,11 +1741,16 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
     key.score2 = d->score2 ? 1 : 0;
     key.cigar = d->cigar ? 1 : 0;
   }
-  const bool same = hinted && d->use_graphs && n > 0 && d->gkey_seen && key == d->gkey;
+  const bool same =
+      hinted && d->use_graphs && n > 0 && d->gkey_seen && key == d->gkey && d->gmoves == d->buffer_moves();
   if (same && d->gexec) {
     MHSW_CK(cudaGraphLaunch(d->gexec, d->st), "graph launch");
-    d->launches = d->timing.launches;  // a replay launches what the captured call launched
     d->graph_launches++;
+    // what enqueue leaves on the handle beside the buffers
+    d->launches = d->glaunches;
+    d->fwd_order = d->gorder;
+    d->score2_n = d->score2 ? n : -1;
+    d->batch.tune.last_call_tuned = false;
   } else if (same) {
     // capture (the first identical call sized every buffer and tuned the launch shape)
     d->launches = 0;
@@ -1775,6 +1784,8 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
       } else {
         if (d->gexec) cudaGraphExecDestroy(d->gexec);
         d->gexec = ex;
+        d->glaunches = d->launches;
+        d->gorder = d->fwd_order;
         MHSW_CK(cudaGraphLaunch(d->gexec, d->st), "graph launch");
         d->graph_launches++;
       }
@@ -1784,10 +1795,12 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
       cudaGraphExecDestroy(d->gexec);
       d->gexec = nullptr;
     }
-    d->gkey = key;
-    d->gkey_seen = hinted;
+    d->gkey_seen = false;
     rc = enqueue();
     if (rc) return rc;
+    d->gkey = key;
+    d->gkey_seen = hinted;
+    d->gmoves = d->buffer_moves();
   }
   MHSW_CK(cudaEventRecord(ev[4], d->st), "event");
   if (host_io) {
@@ -2030,7 +2043,6 @@ int align_resident(mhsw_driver *d, const PairSet &in, int64_t a_bytes, int max_a
     d->timing.n_pairs = n;
     return MHSW_OK;
   }
-  drop_graph(d);
   rc = ensure_results(d, n);
   if (rc) return rc;
   MHSW_CK(d->a_code.reserve((size_t)a_bytes + 16), "cudaMalloc codes");
