@@ -1654,6 +1654,12 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
     MHSW_CK(d->h_counts.reserve(4), "cudaMallocHost");
     MHSW_CK(d->h_counts_p[slot].reserve(4), "cudaMallocHost");
     if (host_io) MHSW_CK(d->out5.reserve((size_t)n * 5), "cudaMalloc out5");
+    if (!brief) {
+      // (here, not in translate_batch alone: the CIGAR pass's host-driven rounds read the codes
+      // after a replay too; the one-launch path reads raw bytes)
+      ps.a_code = d->a_code.p;
+      ps.b_code = d->b_code.p;
+    }
   }
   rc = attach_score2(d, &ps, n, ta);
   if (rc) return rc;

@@ -138,3 +138,22 @@ def test_general_calls_in_between(built):
     assert np.array_equal(d.align_pairs(host), host_want)
     assert big.run(d) == replays[3][2]
     resident.close()
+
+
+def test_replayed_cigars_of_large_boxes(built):
+    """CIGAR mode, boxes above the register kernels' 512 rows: the generic kernel runs after the
+    replay, outside the graph, on the replayed batch's codes."""
+    torch = pytest.importorskip("torch")
+    sc = (2, 4, 4, 2, 1)
+    big = _Resident(torch, _rows(60, 700, 4), sc)
+    want, wops, wn = oracle.cigar_batch(big.p, sc, ops_cap=4096)
+    d = _driver(sc)
+    d.set_cigar(True)
+    replays = []
+    for _ in range(4):
+        replays.append(big.run(d))
+        c = d.last_cigar(big.p.n)
+        assert np.array_equal(c.nops, wn) and np.array_equal(c.mismatches, want[:, 5])
+        assert all(np.array_equal(c.of(i), wops[i, :max(int(wn[i]), 0)]) for i in range(big.p.n))
+        assert d.last_timing()["n_cigar_generic"] >= 30
+    assert replays == [0, 1, 2, 3], replays
