@@ -42,7 +42,8 @@ extern "C" {
 #define MHSW_ERR_NOMEM 4     /* host or device allocation failed */
 #define MHSW_ERR_LIMIT 5     /* a sequence exceeds the engine limits (see mhsw_limits) */
 #define MHSW_ERR_NO_GPU 6    /* no CUDA device */
-#define MHSW_ERR_INTERNAL 7  /* internal consistency check failed */
+#define MHSW_ERR_INTERNAL 7  /* internal consistency check failed: among others, pairs of a completed
+                              * batch that were not aligned (their results are not valid) */
 #define MHSW_ERR_BUSY 8      /* serving queue full (submit with MHSW_SUBMIT_NOWAIT) */
 
 /* ---- orientation ----------------------------------------------------------- */
@@ -201,6 +202,10 @@ int mhsw_driver_set_form(mhsw_driver *drv, int form);
 /* Debug knob: pairs whose score exceeds `ceiling` in the packed int16 engine are
  * re-run in int32 (default and maximum: mhsw_limits().int16_ceiling). */
 int mhsw_driver_set_int16_ceiling(mhsw_driver *drv, int ceiling);
+/* Debug knob: the blocks that share a long pair (A above 1024 bases) wait for one another at
+ * most this many polls each; a wait that gives up ends in MHSW_ERR_INTERNAL from the call (or
+ * its kernel_block).  Default and maximum 2^22 (seconds); 0: every such wait gives up at once. */
+int mhsw_driver_set_wait_limit(mhsw_driver *drv, int polls);
 /* The CUDA stream (cudaStream_t) the handle launches on. */
 int mhsw_driver_stream(mhsw_driver *drv, void **stream);
 /* Score2 mode (default off).  klign's CPU path keeps SSW's second-best score

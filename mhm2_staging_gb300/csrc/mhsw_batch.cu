@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(MODE != kModeInt && !S2 ? (G == kGKLong ? 768 
         rs.a_end[p] = -1;
         rs.b_end[p] = 0;
         rs.flag[p] = too_long ? kFlagTooLong : 0u;
+        if (too_long) atomicAdd(wl.failed, 1);
       }
       continue;
     }
@@ -421,6 +422,7 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     tr.wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
     bs.tune = tr;
     if ((e = cudaMemsetAsync(wl.ovf_count, 0, sizeof(int), st))) return fail(e, "memset");
+    if ((e = cudaMemsetAsync(wl.failed, 0, sizeof(int), st))) return fail(e, "memset");
   }
 
   // the batch: ordered with the kept configuration, then the persistent launches.  A plain

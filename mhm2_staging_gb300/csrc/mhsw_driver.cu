@@ -84,6 +84,7 @@ struct HBuf {
   }
 };
 
+constexpr int kHostCounts = 3;  // counters a batch copies back: int32 re-runs, wide searches, failed pairs
 constexpr int kInt16Ceiling = mhsw::V16::kBig - 1 - 64;  // leaves room for one match step
 
 }  // namespace
@@ -181,6 +182,7 @@ struct mhsw_driver {
   int orientation = MHSW_ORIENT_KLIGN;
   int form = MHSW_FORM_PLAIN;
   int ceiling16 = kInt16Ceiling;
+  int wait_limit = mhsw::kLongWaits;
   cudaStream_t st = nullptr;
   cudaEvent_t ev_done = nullptr;
   bool ev_live = false;
@@ -281,7 +283,7 @@ struct mhsw_driver {
     const void *ptr[7];
     int64_t n, a_bytes, b_bytes;
     int32_t max_a, max_b;
-    int form, ceiling, match, mismatch, gap_open, gap_extend, ambiguity, score2, cigar;
+    int form, ceiling, waits, match, mismatch, gap_open, gap_extend, ambiguity, score2, cigar;
     bool operator==(const GraphKey &o) const { return std::memcmp(this, &o, sizeof(GraphKey)) == 0; }
   };
   GraphKey gkey{};
@@ -299,7 +301,8 @@ struct mhsw_driver {
   HBuf<int64_t> h_aoff, h_boff;
   HBuf<int32_t> h_alen, h_blen;
   HBuf<unsigned char> h_outv;
-  HBuf<int> h_counts;
+  HBuf<int> h_counts;        // counters of the drop-in and resident batches
+  bool counts_live = false;  // h_counts is (once the batch completed) the last such batch's
 
   // drop-in protocol state
   int64_t n_batch = 0;
@@ -455,7 +458,7 @@ int ensure_results(mhsw_driver *d, int64_t n) {
   MHSW_CK(d->l_ovf.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_wide.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_bands.reserve((size_t)n + 1), "cudaMalloc lists");
-  MHSW_CK(d->l_counts.reserve(5 + 2 * mhsw::kBandClasses), "cudaMalloc lists");
+  MHSW_CK(d->l_counts.reserve(6 + 2 * mhsw::kBandClasses), "cudaMalloc lists");
   return MHSW_OK;
 }
 
@@ -631,10 +634,12 @@ mhsw::WorkLists work_lists(mhsw_driver *d, int64_t n) {
   wl.ovf_count = d->l_counts.p;
   wl.wide_count = d->l_counts.p + 1;
   wl.bands = d->l_bands.p;
-  wl.band_counts = d->l_counts.p + 2;
-  wl.long_next = d->l_counts.p + 2 + 2 * mhsw::kBandClasses;
+  wl.failed = d->l_counts.p + 2;  // (these three are read back: kHostCounts)
+  wl.band_counts = d->l_counts.p + 3;
+  wl.long_next = d->l_counts.p + 3 + 2 * mhsw::kBandClasses;
   wl.long_bnd = d->long_bnd.p;
-  wl.esc_count = d->l_counts.p + 4 + 2 * mhsw::kBandClasses;
+  wl.long_waits = d->wait_limit;
+  wl.esc_count = d->l_counts.p + 5 + 2 * mhsw::kBandClasses;
   wl.cap = n;
   return wl;
 }
@@ -774,6 +779,22 @@ int ensure_outviews(mhsw_driver *d, int64_t n, mhsw::OutViews *dv, mhsw::OutView
   carve(d->outv.p, dv);
   carve(d->h_outv.p, hv);
   return MHSW_OK;
+}
+
+// The batch's counters to the host, behind its kernels.
+int copy_counts(mhsw_driver *d, int *to) {
+  MHSW_CK(cudaMemcpyAsync(to, d->l_counts.p, kHostCounts * sizeof(int), cudaMemcpyDeviceToHost, d->st),
+          "D2H counters");
+  return MHSW_OK;
+}
+
+// The error of a completed batch with flagged pairs (c: its counters), or MHSW_OK.
+int check_failed(mhsw_driver *d, const int *c) {
+  if (c[2] <= 0) return MHSW_OK;
+  return d->fail(MHSW_ERR_INTERNAL,
+                 "%d pairs were not aligned (longer than the stated extents, a search that missed its score, or a wait "
+                 "between a long pair's blocks that gave up)",
+                 c[2]);
 }
 
 int check_scoring(mhsw_driver *d, const mhsw::Scoring &s) {
@@ -1187,6 +1208,15 @@ int mhsw_driver_set_int16_ceiling(mhsw_driver *d, int ceiling) {
   return MHSW_OK;
 }
 
+int mhsw_driver_set_wait_limit(mhsw_driver *d, int polls) {
+  if (!d) return MHSW_ERR_ARG;
+  if (polls < 0 || polls > mhsw::kLongWaits)
+    return d->fail(MHSW_ERR_ARG, "wait limit must be in [0, %d]", mhsw::kLongWaits);
+  std::lock_guard<std::mutex> lk(d->mu);
+  d->wait_limit = polls;
+  return MHSW_OK;
+}
+
 int mhsw_driver_stream(mhsw_driver *d, void **stream) {
   if (!d || !stream) return MHSW_ERR_ARG;
   if (!d->inited) return d->fail(MHSW_ERR_STATE, "driver not initialised");
@@ -1208,7 +1238,7 @@ int mhsw_run_kernel_forwards(mhsw_driver *d, const char *const *reads, const int
       return d->fail(MHSW_ERR_ARG, "pair %d longer than max_read_size/max_contig_size", i);
   if (d->ev_live) MHSW_CK(cudaEventSynchronize(d->ev_done), "wait previous batch");
   d->ev_live = false;
-  d->fwd_issued = d->rev_issued = false;
+  d->fwd_issued = d->rev_issued = d->counts_live = false;
   d->launches = 0;
   d->cigar_n = -1;
   MHSW_CK(cudaEventRecord(d->ev_t[0], d->st), "event");
@@ -1250,6 +1280,9 @@ int mhsw_run_kernel_forwards(mhsw_driver *d, const char *const *reads, const int
     rc = d->begins_done ? run_short_passes(d, ps, d->max_a, d->max_b) : forward_any(d, ps, d->max_a, d->max_b, d->form);
     if (rc) return rc;
     if ((rc = copy_score2(d, n))) return rc;
+    MHSW_CK(d->h_counts.reserve(4), "cudaMallocHost");
+    if ((rc = copy_counts(d, d->h_counts.p))) return rc;
+    d->counts_live = true;
   }
   MHSW_CK(cudaEventRecord(d->ev_t[2], d->st), "event");
   mhsw::OutViews dv, hv;
@@ -1348,9 +1381,9 @@ int mhsw_run_kernel_backwards(mhsw_driver *d, const char *const *reads, const in
     int32_t *wdst[2] = {hv.w_ref_beg, hv.w_qry_beg};
     for (int k = 0; k < 2; k++)
       MHSW_CK(cudaMemcpyAsync(wdst[k], wsrc[k], sizeof(int32_t) * n, cudaMemcpyDeviceToHost, d->st), "D2H");
-    MHSW_CK(cudaMemcpyAsync(d->h_counts.reserve(4) == cudaSuccess ? d->h_counts.p : nullptr, d->l_counts.p,
-                            2 * sizeof(int), cudaMemcpyDeviceToHost, d->st),
-            "D2H counters");
+    MHSW_CK(d->h_counts.reserve(4), "cudaMallocHost");
+    if ((rc = copy_counts(d, d->h_counts.p))) return rc;
+    d->counts_live = true;
   }
   MHSW_CK(cudaEventRecord(d->ev_t[5], d->st), "event");
   MHSW_CK(cudaEventRecord(d->ev_done, d->st), "event");
@@ -1396,7 +1429,7 @@ int mhsw_kernel_block(mhsw_driver *d) {
     d->timing.n_rev_wide = d->h_counts.p[1];
     d->timing.launches = d->launches;
   }
-  return MHSW_OK;
+  return d->counts_live ? check_failed(d, d->h_counts.p) : MHSW_OK;
 }
 
 int mhsw_get_aln_results(mhsw_driver *d, mhsw_aln_results *out) {
@@ -1484,7 +1517,7 @@ int finish_slot(mhsw_driver *d, int s) {
   r.done = elapsed(d->ev_epoch, ev[4]);
   d->history[d->history_n % mhsw_driver::kHistory] = r;
   d->history_n++;
-  return MHSW_OK;
+  return n > 0 && hc ? check_failed(d, hc) : MHSW_OK;
 }
 
 // Completes every pending batch call, oldest first.
@@ -1547,7 +1580,7 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
   if (form != MHSW_FORM_PLAIN && form != MHSW_FORM_BATCHED) return d->fail(MHSW_ERR_ARG, "unknown form %d", form);
   if (d->ev_live) MHSW_CK(cudaEventSynchronize(d->ev_done), "wait previous batch");
   d->ev_live = false;
-  d->fwd_issued = d->rev_issued = false;
+  d->fwd_issued = d->rev_issued = d->counts_live = false;
   const int64_t n = pairs->n;
   d->launches = 0;
   int ma = 0, mb = 0;
@@ -1685,7 +1718,7 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
       MHSW_CK(mark(ev[2]), "event");
       MHSW_CK(mark(ev[3]), "event");
       MHSW_CK(cudaMemcpyAsync(out5, d->out5.p, sizeof(int32_t) * 5 * n, cudaMemcpyDeviceToHost, d->st), "D2H");
-      d->h_counts_p[slot].p[0] = d->h_counts_p[slot].p[1] = 0;
+      std::fill_n(d->h_counts_p[slot].p, kHostCounts, 0);
       d->launches += 1;
       return MHSW_OK;
     }
@@ -1718,8 +1751,7 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
         MHSW_CK(mhsw::launch_pack5(result_set(d), n, out5, d->st), "pack5");
       }
       d->launches += 1;
-      MHSW_CK(cudaMemcpyAsync(d->h_counts_p[slot].p, d->l_counts.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, d->st),
-              "D2H");
+      if (int r = copy_counts(d, d->h_counts_p[slot].p)) return r;
     }
     return MHSW_OK;
   };
@@ -1739,6 +1771,7 @@ int align_pairs_begin(mhsw_driver *d, const mhsw_pairs *pairs, int32_t *out5, in
     key.max_b = mb;
     key.form = form;
     key.ceiling = d->ceiling16;
+    key.waits = d->wait_limit;
     key.match = d->sc.match;
     key.mismatch = d->sc.mismatch;
     key.gap_open = d->sc.gap_open;
@@ -2030,7 +2063,7 @@ int align_resident(mhsw_driver *d, const PairSet &in, int64_t a_bytes, int max_a
   if (form != MHSW_FORM_PLAIN && form != MHSW_FORM_BATCHED) return d->fail(MHSW_ERR_ARG, "unknown form %d", form);
   if (d->ev_live) MHSW_CK(cudaEventSynchronize(d->ev_done), "wait previous batch");
   d->ev_live = false;
-  d->fwd_issued = d->rev_issued = false;
+  d->fwd_issued = d->rev_issued = d->counts_live = false;
   d->launches = 0;
   const int64_t n = in.n;
   if (n <= 0) return MHSW_OK;
@@ -2071,9 +2104,18 @@ int align_resident(mhsw_driver *d, const PairSet &in, int64_t a_bytes, int max_a
   MHSW_CK(cudaEventRecord(d->ev_t[3], d->st), "event");
   MHSW_CK(launch_pack5(result_set(d), n, out5_dev, d->st), "pack5");
   d->launches += 1;
+  MHSW_CK(d->h_counts.reserve(4), "cudaMallocHost");
+  if ((rc = copy_counts(d, d->h_counts.p))) return rc;
+  d->counts_live = true;
   d->timing = mhsw_timing{};
   d->timing.n_pairs = n;
   return MHSW_OK;
+}
+
+int resident_check(mhsw_driver *d) {
+  if (!d) return MHSW_ERR_ARG;
+  std::lock_guard<std::mutex> lk(d->mu);
+  return d->counts_live ? check_failed(d, d->h_counts.p) : MHSW_OK;
 }
 
 void resident_timing(mhsw_driver *d) {

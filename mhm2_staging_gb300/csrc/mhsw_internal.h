@@ -31,6 +31,9 @@ void driver_gaps(mhsw_driver *d, int *gap_open, int *gap_extend);
 // Returns MHSW_ERR_STATE when the handle is not in CIGAR mode.
 int cigar_resident(mhsw_driver *d, const PairSet &ps);
 bool driver_cigar(mhsw_driver *d);
+// After the stream work of an align_resident call completed: MHSW_ERR_INTERNAL when pairs of it
+// were not aligned.
+int resident_check(mhsw_driver *d);
 // After the stream work of an align_resident call (and its CIGAR pass) completed: its
 // device times into the handle's mhsw_timing (translation to end of the begin pass).
 void resident_timing(mhsw_driver *d);

@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(256) k_fwd(PairSet ps, ResultSet rs, Scoring s
         rs.a_end[p] = -1;
         rs.b_end[p] = 0;
         rs.flag[p] = too_long ? kFlagTooLong : 0u;
+        if (too_long) atomicAdd(wl.failed, 1);
       }
       continue;
     }
@@ -456,7 +457,8 @@ __global__ void __launch_bounds__(128) k_rev_band(PairSet ps, ResultSet rs, Scor
     append_agg(wl.wide, wl.esc_count, wl.cap, p, escalate);
     if (escalate) continue;
     if (!found || fi >= M2 || fj < 0 || fj >= N2) {
-      rs.flag[p] |= kFlagTooLong;  // inconsistent; reported as an error by the driver
+      rs.flag[p] |= kFlagTooLong;  // inconsistent; the call fails
+      atomicAdd(wl.failed, 1);
       rs.a_beg[p] = -1;
       rs.b_beg[p] = 0;
       continue;
@@ -640,7 +642,8 @@ __global__ void __launch_bounds__(128) k_rev_band16(PairSet ps, ResultSet rs, Sc
     append_agg(wl.wide, wl.esc_count, wl.cap, p, escalate);
     if (escalate) continue;
     if (!found || fi < 0 || fi >= M2 || fj < 0 || fj >= N2) {
-      rs.flag[p] |= kFlagTooLong;  // inconsistent; reported as an error by the driver
+      rs.flag[p] |= kFlagTooLong;  // inconsistent; the call fails
+      atomicAdd(wl.failed, 1);
       rs.a_beg[p] = -1;
       rs.b_beg[p] = 0;
       continue;
@@ -760,6 +763,7 @@ __global__ void __launch_bounds__(256) k_rev_wave(PairSet ps, ResultSet rs, Scor
     if (too_long) {
       if (lane == 0) {
         rs.flag[p] |= kFlagTooLong;
+        atomicAdd(wl.failed, 1);
         rs.a_beg[p] = -1;
         rs.b_beg[p] = 0;
       }
@@ -772,6 +776,7 @@ __global__ void __launch_bounds__(256) k_rev_wave(PairSet ps, ResultSet rs, Scor
     if (lane == 0) {
       if (key_value(so.key) != S) {
         rs.flag[p] |= kFlagTooLong;
+        atomicAdd(wl.failed, 1);
         rs.a_beg[p] = -1;
         rs.b_beg[p] = 0;
       } else {
@@ -824,6 +829,7 @@ __global__ void k_reset_lists(WorkLists wl) {
   *wl.ovf_count = 0;
   *wl.wide_count = 0;
   *wl.esc_count = 0;
+  *wl.failed = 0;
   for (int i = 0; i < 2 * kBandClasses; i++) wl.band_counts[i] = 0;
   wl.long_next[0] = wl.long_next[1] = 0;
 }

@@ -450,7 +450,10 @@ int mhsw_klign_align(mhsw_driver *d, const mhsw_contigs *cg, const mhsw_candidat
     down(out->perfect, o_pf, (size_t)n);
     if (out->cigar_slot && mhsw::driver_cigar(d)) down(out->cigar_slot, slot, sizeof(int32_t) * n);
     if (!e) e = cudaStreamSynchronize(st);
-    if (!e && h_counts[0] > 0) mhsw::resident_timing(d);
+    if (!e && h_counts[0] > 0) {
+      rc = mhsw::resident_check(d);
+      mhsw::resident_timing(d);
+    }
   }
   if (e || rc) cudaStreamSynchronize(st);  // nothing of a failed call left in flight
   if (e) return e == cudaErrorMemoryAllocation ? MHSW_ERR_NOMEM : MHSW_ERR_CUDA;

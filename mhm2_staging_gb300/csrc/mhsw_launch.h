@@ -22,8 +22,10 @@ struct WorkLists {
   int64_t *bands;     // begin-pass pairs grouped by band class (one segment per class)
   int *band_counts;   // kBandClasses pair counts, then kBandClasses scatter cursors
   int64_t cap;        // capacity of each list
+  int *failed;        // pairs flagged kFlagTooLong: the call fails
   int *long_next;     // claim counters of the long-pair kernels (forward, begin)
   uint32_t *long_bnd; // their strip boundaries (LongPlan::bytes), or null
+  int long_waits;     // polls after which one of their waits gives up (at most kLongWaits)
 };
 
 struct FwdConfig {
@@ -139,6 +141,7 @@ cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scorin
 // scorings; not in score2 mode).
 constexpr int kLongRows = 1024;
 constexpr int kLongScore = 32000;
+constexpr int kLongWaits = 1 << 22;  // polls (of L2) before a wait gives up: seconds
 constexpr size_t kLongScratch = size_t(512) << 20;  // strip boundaries, at most
 // Batches up to this size send every such begin search there; in larger ones the banded
 // kernels (a thread per pair, far fewer cells) have pairs enough to fill the GPU.

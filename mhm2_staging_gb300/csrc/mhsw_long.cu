@@ -7,8 +7,8 @@
 // row in global memory that the producer publishes 32 columns at a time through a progress
 // word.  While the pairs are few, a pair's strips go round the blocks of a cluster (4 SMs, 32
 // warps), so a scheduler has one strip rather than four.  A strip only ever waits for an earlier one and a warp takes its
-// strips in order, so the waits end; each is bounded all the same and reports the pair as
-// inconsistent if it gives up.
+// strips in order, so the waits end; each is bounded all the same: if one gives up the pair is
+// flagged, its warps go on without waiting, and the call fails.
 //
 // The step is the keyed int16 step of mhsw_engine16.cuh with one operation more per cell
 // pair: keys are formed from H above a base kept per lane half, so scores up to
@@ -35,7 +35,6 @@ namespace {
 constexpr int kLK = 8;                  // row pairs per lane
 constexpr int kLRows = 2 * kLK * 32;    // rows per strip
 constexpr int kLChunk = 32;             // columns between progress updates
-constexpr int kLongWaits = 1 << 22;     // polls (of L2) before a wait gives up (seconds)
 
 constexpr int kLongWarps = 32;          // warps on one pair, at most
 
@@ -74,6 +73,8 @@ struct LongArgs {
   LongShared *shared;      // per cluster
   uint32_t *bnd;           // per cluster: one row of `cols` words per warp
   int64_t cols;
+  int waits;               // polls before a wait gives up
+  int *flagged;            // pairs flagged so far
 };
 
 // The keyed step with keys above a base (nbase: its negative, per half).  LAZY (gap open >= gap
@@ -126,7 +127,8 @@ __device__ __forceinline__ void long_step(int t, uint32_t zH, uint32_t zE, const
 // that reached it stop.
 template <bool LAZY>
 __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, int bdir, int N, int I, int J, int goal,
-                           const Scoring &sc, uint32_t *prof, uint32_t *bnd, int64_t cols, LongShared &sh, int warp, int W) {
+                           const Scoring &sc, uint32_t *prof, uint32_t *bnd, int64_t cols, LongShared &sh, int warp, int W,
+                           int waits) {
   using ST = Step16<kLK, 32>;
   using L = Prof16<kLK>;
   constexpr unsigned full = 0xffffffffu;
@@ -176,7 +178,7 @@ __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, 
       const unsigned long long want = ((unsigned long long)(s - 1) << 32) | (unsigned)col;
       int polls = 0;
       while (seen < want) {
-        if (++polls > kLongWaits || *(volatile int *)&sh.failed) return false;
+        if (++polls > waits || *(volatile int *)&sh.failed) return false;
         seen = prog[pw];
         fenced = false;
       }
@@ -336,7 +338,8 @@ __global__ void __launch_bounds__(256, 2) k_long(LongArgs g) {
         int I, J;
         band_sides(t, N2, S, sc, I, J);
         reset();
-        long_sweep<LAZY>(a, -1, t, b, -1, (int)min((long long)N2, (long long)t + J), I, J, S, sc, prof, bnd, g.cols, sh, warp, W);
+        long_sweep<LAZY>(a, -1, t, b, -1, (int)min((long long)N2, (long long)t + J), I, J, S, sc, prof, bnd, g.cols, sh,
+                         warp, W, g.waits);
         cluster_barrier();
         best = vs.best;
         failed = vs.failed;
@@ -346,7 +349,8 @@ __global__ void __launch_bounds__(256, 2) k_long(LongArgs g) {
       }
       if (lead) {
         if (key_value(best) != S || failed) {
-          g.rs.flag[p] |= kFlagTooLong;  // inconsistent
+          g.rs.flag[p] |= kFlagTooLong;  // inconsistent, or a wait gave up
+          atomicAdd(g.flagged, 1);
           g.rs.a_beg[p] = -1;
           g.rs.b_beg[p] = 0;
         } else {
@@ -358,13 +362,14 @@ __global__ void __launch_bounds__(256, 2) k_long(LongArgs g) {
       const int M = g.ps.a_len[p], N = g.ps.b_len[p];
       reset();
       long_sweep<LAZY>(g.ps.a_code + g.ps.a_off[p], 1, M, g.ps.b_code + g.ps.b_off[p], 1, N, M, N, 0, sc, prof, bnd, g.cols, sh,
-                 warp, W);
+                       warp, W, g.waits);
       cluster_barrier();
       if (lead) {
         const bool failed = vs.failed;
         const unsigned long long best = vs.best;
         const int S = failed ? 0 : key_value(best);
         g.rs.flag[p] = failed ? kFlagTooLong : 0u;
+        if (failed) atomicAdd(g.flagged, 1);
         g.rs.score[p] = S;
         g.rs.a_end[p] = S > 0 ? key_row(best) : -1;
         g.rs.b_end[p] = S > 0 ? key_col(best) : 0;
@@ -425,6 +430,8 @@ static void carve(LongArgs &g, const LongPlan &pl, const WorkLists &wl) {
   const size_t head = ((size_t)pl.clusters * sizeof(LongShared) + 255) / 256 * 256;
   g.bnd = wl.long_bnd + head / sizeof(uint32_t);
   g.cols = pl.cols;
+  g.waits = wl.long_waits;
+  g.flagged = wl.failed;
 }
 
 cudaError_t launch_long_forward(const LongPlan &pl, const PairSet &ps, const ResultSet &rs, const Scoring &sc,

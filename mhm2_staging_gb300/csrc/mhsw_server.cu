@@ -236,6 +236,8 @@ int mhsw_server::run_micro_batch(Slot *s, std::vector<Piece> &pieces, int64_t ro
   SRV_CK(cudaMemcpyAsync(s->h_out5.p, s->out5.p, sizeof(int32_t) * 5 * rows, cudaMemcpyDeviceToHost, st), "D2H");
   SRV_CK(cudaStreamSynchronize(st), "slot synchronise");
 #undef SRV_CK
+  rc = mhsw::resident_check(s->drv);
+  if (rc) return fail(rc, "slot alignment: %s", mhsw_driver_last_error(s->drv));
   for (auto &pc : pieces) {
     Request &r = *pc.r;
     std::memcpy(r.out5 + 5 * (int64_t)pc.first, s->h_out5.p + 5 * pc.row, sizeof(int32_t) * 5 * (size_t)pc.count);

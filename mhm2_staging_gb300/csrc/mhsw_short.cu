@@ -425,7 +425,8 @@ __global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scori
     }
     if (lane == 0) {
       if (key_value(q) != S) {
-        rs.flag[p] |= kFlagTooLong;  // inconsistent
+        rs.flag[p] |= kFlagTooLong;  // inconsistent; the call fails
+        atomicAdd(wl.failed, 1);
         rs.a_beg[p] = -1;
         rs.b_beg[p] = 0;
       } else {

@@ -17,7 +17,7 @@ struct Scoring {
 enum : uint32_t {
   kFlagOverflow16 = 1u,   // int16 ceiling crossed: forward pass re-run in int32
   kFlagRevWide = 2u,      // reverse band wider than the banded kernel's limit
-  kFlagTooLong = 4u,      // sequence beyond the engine limits (error)
+  kFlagTooLong = 4u,      // beyond the engine limits, or a search that failed: the call fails
 };
 
 struct PairSet {  // device pointers; A = SSW ref (rows), B = SSW query (columns)

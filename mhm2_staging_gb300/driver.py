@@ -191,6 +191,7 @@ SIGNATURES: dict[str, tuple] = {
     "mhsw_driver_set_orientation": (C.c_int, [_P, C.c_int]),
     "mhsw_driver_set_form": (C.c_int, [_P, C.c_int]),
     "mhsw_driver_set_int16_ceiling": (C.c_int, [_P, C.c_int]),
+    "mhsw_driver_set_wait_limit": (C.c_int, [_P, C.c_int]),
     "mhsw_driver_stream": (C.c_int, [_P, C.POINTER(_P)]),
     "mhsw_driver_set_score2": (C.c_int, [_P, C.c_int]),
     "mhsw_last_score2": (C.c_int, [_P, _P, _P, C.c_int]),
@@ -411,6 +412,10 @@ class GPUDriver:
 
     def set_int16_ceiling(self, ceiling: int) -> None:
         self._ck(self._lib.mhsw_driver_set_int16_ceiling(self._h, ceiling), "set_int16_ceiling")
+
+    def set_wait_limit(self, polls: int = 1 << 22) -> None:
+        """Polls after which a wait between the blocks of a long pair gives up (the call then fails)."""
+        self._ck(self._lib.mhsw_driver_set_wait_limit(self._h, polls), "set_wait_limit")
 
     def set_score2(self, on: bool) -> None:
         """Score2 mode: also compute SSW's second-best score (klign's aln.score2)."""
