@@ -429,7 +429,8 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   // batch that does not give every 16-lane group a pair takes those for short reads too:
   // their shorter chain is what it waits for.
   BatchShape shape = tune ? bs.shape : BatchShape{};
-  if (!tune && n <= (int64_t)sms * 64) shape.lane_rows = 0;  // any_long holds: max_a > 0
+  // (A batch of empty A only has no longer kernel to go to: any_long is max_a > lane_rows.)
+  if (!tune && max_a > 0 && n <= (int64_t)sms * 64) shape.lane_rows = 0;
   if (order_items(shape, n, 1, bs.order)) return 1;
   if (longs) {
     if ((e = launch_long_forward(plan_long(n, max_b, sms), ps, rs, sc, bs.order, queue + 8 + kBucketLong, wl, st)))
