@@ -332,9 +332,9 @@ __global__ void __launch_bounds__(256, 2) k_long(LongArgs g) {
       if (!long_begin(band_first_cap(S, sc.match, M2), S)) continue;  // the wavefront kernels take it
       const uint8_t *a = g.ps.a_code + g.ps.a_off[p] + ie, *b = g.ps.b_code + g.ps.b_off[p] + je;
       int t = band_first_cap(S, sc.match, M2);
-      unsigned long long best;
-      bool failed;
-      for (;;) {
+      unsigned long long best = 0ull;
+      bool failed = N2 > g.cols;  // (the boundary rows hold the stated longest B)
+      while (!failed) {
         int I, J;
         band_sides(t, N2, S, sc, I, J);
         reset();
@@ -360,12 +360,14 @@ __global__ void __launch_bounds__(256, 2) k_long(LongArgs g) {
       }
     } else {
       const int M = g.ps.a_len[p], N = g.ps.b_len[p];
+      const bool fits = N <= g.cols;
       reset();
-      long_sweep<LAZY>(g.ps.a_code + g.ps.a_off[p], 1, M, g.ps.b_code + g.ps.b_off[p], 1, N, M, N, 0, sc, prof, bnd, g.cols, sh,
-                       warp, W, g.waits);
+      if (fits)
+        long_sweep<LAZY>(g.ps.a_code + g.ps.a_off[p], 1, M, g.ps.b_code + g.ps.b_off[p], 1, N, M, N, 0, sc, prof, bnd,
+                         g.cols, sh, warp, W, g.waits);
       cluster_barrier();
       if (lead) {
-        const bool failed = vs.failed;
+        const bool failed = vs.failed || !fits;
         const unsigned long long best = vs.best;
         const int S = failed ? 0 : key_value(best);
         g.rs.flag[p] = failed ? kFlagTooLong : 0u;

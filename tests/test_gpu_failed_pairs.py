@@ -115,6 +115,27 @@ def test_klign_call(built):
     resident.close()
 
 
+def test_pair_beyond_the_stated_extents(built):
+    """A long pair whose B is longer than the batch's stated longest B: the kernels' scratch ends
+    there."""
+    torch = pytest.importorskip("torch")
+    from mhm2_staging_gb300.driver import DevicePairs
+
+    rng = np.random.default_rng(5)
+    w = BASES[rng.integers(0, 4, 4000)]
+    p = Pairs.from_lists([w[100:1700].tobytes(), w[500:3500].tobytes()], [w[:2000].tobytes(), w.tobytes()])
+    keep = [torch.from_numpy(x).cuda() for x in (p.a_seq, p.a_off, p.a_len, p.b_seq, p.b_off, p.b_len)]
+    ma, mb, cells, ab, bb = p.extents()
+    out = torch.zeros((p.n, 5), dtype=torch.int32, device="cuda")
+    d = _driver()
+    with pytest.raises(RuntimeError, match="status 7.*1 pairs were not aligned"):
+        d.align_pairs_device(DevicePairs(*(t.data_ptr() for t in keep), p.n, ma, 2000, cells, ab, bb), out.data_ptr())
+    want = oracle.align_batch(p, SC)
+    assert np.array_equal(out.cpu().numpy()[0], want[0])
+    d.align_pairs_device(DevicePairs(*(t.data_ptr() for t in keep), p.n, ma, mb, cells, ab, bb), out.data_ptr())
+    assert np.array_equal(out.cpu().numpy(), want)
+
+
 def test_limits_of_the_knob(built):
     d = _driver()
     for bad in (-1, (1 << 22) + 1):
