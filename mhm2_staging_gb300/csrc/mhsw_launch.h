@@ -122,6 +122,8 @@ cudaError_t launch_short(const PairSet &ps, const Scoring &sc, int max_a, int ma
                          const ResultSet *rs, bool a_is_query, cudaStream_t st);
 // The forward pass alone: out3 (n x 3) = score, a_end, b_end; -1 three times for a pair outside
 // max_a or max_b.
+// (prepare_short_forward loads its kernels, which a first launch otherwise does.)
+cudaError_t prepare_short_forward();
 cudaError_t launch_short_forward(const PairSet &ps, const Scoring &sc, int max_a, int max_b, int32_t *out3,
                                  cudaStream_t st);
 // True when some pair of a batch with these longest sequences can need the int32 pass.

@@ -21,7 +21,7 @@
 // Nothing here calls cudaMalloc, cudaFree or any library routine that allocates.
 // The first call on a device does a one-time set-up with that device current: it looks
 // up the scratch array's device address (cudaGetSymbolAddress, which also loads this
-// module onto the device) and sets the kernel's shared-memory attribute.  Make that
+// module onto the device) and loads and configures the kernels of every route.  Make that
 // first call before any stream capture begins.
 #include <cuda_runtime.h>
 
@@ -292,6 +292,8 @@ int na_setup(int dev, NaDevice **out, char *errbuf, size_t errlen) {
           (e = raise_smem_limit(reinterpret_cast<const void *>(na16_short(m)), na16_smem_short(m))) ||
           (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ_short[m], na16_short(m), 128, na16_smem_short(m))))
         return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "keyed kernel set-up: %s", cudaGetErrorString(e));
+    if ((e = prepare_short_forward()))
+      return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "short batch set-up: %s", cudaGetErrorString(e));
     if ((e = order_smem_limits()))
       return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "keyed kernel set-up: %s", cudaGetErrorString(e));
     d.scratch = static_cast<unsigned char *>(p);

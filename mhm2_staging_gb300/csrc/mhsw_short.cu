@@ -483,6 +483,14 @@ cudaError_t launch_short(const PairSet &ps, const Scoring &sc, int max_a, int ma
   return launch(g, st);
 }
 
+cudaError_t prepare_short_forward() {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, k_short<4, false, false>);
+  if (!e) e = cudaFuncGetAttributes(&a, k_short<8, false, false>);
+  if (!e) e = cudaFuncGetAttributes(&a, k_short<4, false, true>);
+  return e ? e : cudaFuncGetAttributes(&a, k_short<8, false, true>);
+}
+
 cudaError_t launch_short_forward(const PairSet &ps, const Scoring &sc, int max_a, int max_b, int32_t *out3,
                                  cudaStream_t st) {
   ShortArgs g{};
