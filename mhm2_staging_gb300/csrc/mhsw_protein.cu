@@ -96,12 +96,14 @@ struct PArgs {
 constexpr int kPadCol = kAA;                 // code of columns outside B: scores -gap open
 constexpr int kPCodes = kAA + 1;
 constexpr int kPWords = (kPCodes + 3) / 4;   // words of one row code's biased scores
+constexpr int kPCols = 65000;                // longest B (steps are 16-bit)
 
 struct P16Args {
   PArgs p;
   const uint32_t *order;
   int *ctl;                        // the order's control block
-  uint32_t *bound;                 // per group: strip boundary (max_n words; lo H, hi E^)
+  uint32_t *bound;                 // per group: strip boundary (bound_n words; lo H, hi E^)
+  int64_t bound_n;                 // longest B these kernels take, at most kPCols
   uint32_t *over;                  // pairs whose score left the keys
   int *over_n;
   int wide_from;                   // min(M, N) from which a pair goes straight to int32
@@ -306,7 +308,7 @@ __global__ void __launch_bounds__(128, 5) k_protein16(P16Args g) {
   const int grp = threadIdx.x / G, lane = threadIdx.x % G;
   const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (((threadIdx.x & 31) / G) * G);
   uint4 *tab = reinterpret_cast<uint4 *>(smem) + (size_t)grp * kPCodes * G;
-  uint32_t *bnd = g.bound ? g.bound + ((int64_t)blockIdx.x * (128 / G) + grp) * p.max_n : nullptr;
+  uint32_t *bnd = g.bound ? g.bound + ((int64_t)blockIdx.x * (128 / G) + grp) * g.bound_n : nullptr;
   const uint32_t NGE = V16::splat(-p.gE), NGO = V16::splat(-p.gO);
   const uint32_t one = (uint32_t)(p.gO >> 30) + 1u;  // a 1 the compiler cannot fold
   const int lo = G == 16 ? 0 : g.ctl[2], hi = G == 16 ? g.ctl[2] : (int)p.n;
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(128, 5) k_protein16(P16Args g) {
     const uint8_t *a = p.a_code + p.a_off[i], *b = p.b_code + p.b_off[i];
     int S = 0, ie = -1, je = 0, ib = -1, jb = 0, over = 0;
     if (M > 0 && N > 0) {
-      if (min(M, N) >= g.wide_from || N > 65000) {
+      if (min(M, N) >= g.wide_from || N > kPCols) {
         over = 1;
       } else {
         // Both passes through one call: three copies of the sweeps miss the instruction cache
@@ -581,7 +583,7 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
   }
   const bool keyed = low >= -gO && top <= 63 && top + gO <= 127 && n <= 0x7fffffff;
   const int wide_from = top > 0 ? 30000 / top : INT_MAX;  // H itself leaves int16 from there on
-  const bool over_possible = !keyed || std::min(max_m, max_n) * top > KeyBits<8>::kCap || max_n > 65000;
+  const bool over_possible = !keyed || std::min(max_m, max_n) * top > KeyBits<8>::kCap || max_n > kPCols;
   char *as = nullptr, *bs = nullptr;
   int64_t *ao = nullptr, *bo = nullptr;
   int32_t *al = nullptr, *bl = nullptr;
@@ -608,6 +610,7 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
   }
   const int64_t blocks16 = std::min<int64_t>((n + 7) / 8, (int64_t)sms * occ16);
   const int64_t blocks32 = std::min<int64_t>((n + 3) / 4, (int64_t)sms * occ32);
+  const int64_t bound_n = std::min<int64_t>(max_n, kPCols);
   // the call's arrays, laid out in the handle's call arena (sized by a first pass)
   auto lay = [&](mhsw::Carve &c) {
     if (host_io) {
@@ -633,7 +636,7 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
       c.take(&ctl, kOrderCtl + 1);
       c.take(&order, (size_t)n);
       c.take(&over, (size_t)n);
-      if (max_m > 512) c.take(&bound, (size_t)(blocks32 * 4 * max_n));
+      if (max_m > 512) c.take(&bound, (size_t)(blocks32 * 4 * bound_n));
     }
     if (over_possible) c.take(&rows, (size_t)(warps * max_n));
   };
@@ -682,7 +685,7 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
     e = cudaMemsetAsync(over_n, 0, sizeof(int), st);
     if (!e) e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, INT_MAX, true);
     if (!e) {
-      const P16Args q{g, order, ctl, bound, over, over_n, wide_from};
+      const P16Args q{g, order, ctl, bound, bound_n, over, over_n, wide_from};
       if (max_m > 256) k_protein16<32><<<(unsigned)blocks32, 128, smem32, st>>>(q);
       k_protein16<16><<<(unsigned)blocks16, 128, smem16, st>>>(q);
       e = cudaGetLastError();
