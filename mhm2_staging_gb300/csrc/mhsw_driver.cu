@@ -2131,6 +2131,7 @@ void resident_timing(mhsw_driver *d) {
 }
 
 void *driver_stream(mhsw_driver *d) { return d ? static_cast<void *>(d->st) : nullptr; }
+const Forks *driver_forks(mhsw_driver *d) { return d ? &d->forks : nullptr; }
 int driver_device(mhsw_driver *d) { return d ? d->device : -1; }
 int driver_form(mhsw_driver *d) { return d ? d->form : MHSW_FORM_PLAIN; }
 bool driver_cigar(mhsw_driver *d) { return d && d->cigar; }

@@ -24,6 +24,9 @@ int driver_device(mhsw_driver *d);
 // The handle's form for batch calls (MHSW_FORM_*) and match score.
 int driver_form(mhsw_driver *d);
 int driver_match(mhsw_driver *d);
+// The handle's side streams, for launches that may overlap on the device.
+struct Forks;
+const Forks *driver_forks(mhsw_driver *d);
 // The handle's gap penalties as positive magnitudes.
 void driver_gaps(mhsw_driver *d, int *gap_open, int *gap_extend);
 // CIGAR mode: runs the CIGAR pass over the batch of the last align_resident call (after

@@ -42,8 +42,11 @@ __device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int la
 }
 
 // Buckets of the protein kernels: A up to 128/192/256 rows (16-lane groups, K = 4/6/8), up to
-// 384/512 (32-lane groups, K = 6/8), longer (strips of 512).
-__host__ __device__ constexpr int protein_bucket(int M) {
+// 384/512 (32-lane groups, K = 6/8), longer (strips of 512)
+// -- or, for min(M, N) >= wide_from or B above kPCols, the int32 kernels (kBucketWide).
+constexpr int kPCols = 65000;
+__host__ __device__ constexpr int protein_bucket(int M, int N, int wide_from) {
+  if ((M < N ? M : N) >= wide_from || N > kPCols) return kBucketWide;
   return M <= 128 ? 0 : M <= 192 ? 1 : M <= 256 ? 2 : M <= 384 ? 4 : M <= 512 ? 5 : kBucketStrip;
 }
 
@@ -78,13 +81,13 @@ struct OrderArgs {
   uint32_t *order;
   int max_a, max_b;   // pairs longer than these go with the empty ones
   int long_rows;      // longest A of the persistent kernels
-  bool protein;       // buckets by protein_bucket (sc unused)
+  int protein_wide;   // above 0: buckets by protein_bucket with this wide_from (sc unused)
 };
 
 __device__ __forceinline__ int order_bin(const OrderArgs &g, int64_t p) {
   const int M = g.ps.a_len[p], N = g.ps.b_len[p];
   const int b = (M <= 0 || N <= 0 || M > g.max_a || N > g.max_b) ? (g.lane_rows > 0 ? 0 : kBucketFirstLong)
-                : g.protein ? protein_bucket(M) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.long_rows);
+                : g.protein_wide > 0 ? protein_bucket(M, N, g.protein_wide) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.long_rows);
   return b * kLenBins + len_class(N);
 }
 
@@ -206,9 +209,9 @@ inline cudaError_t order_smem_limits() {
 // Orders m items (pair i * stride) into `order`; clears the claim counters.
 inline cudaError_t order_pairs(const PairSet &ps, const Scoring &sc, int lane_rows, bool wide_try16, int64_t m,
                                int64_t stride, int *ctl, uint32_t *order, int sms, cudaStream_t st, int64_t *launches,
-                               int max_a = INT_MAX, int max_b = INT_MAX, int long_rows = INT_MAX, bool protein = false) {
+                               int max_a = INT_MAX, int max_b = INT_MAX, int long_rows = INT_MAX, int protein_wide = 0) {
   OrderArgs g{ps, sc, lane_rows, wide_try16, m, stride, ctl, ctl + 8, ctl + kOrderHead, ctl + kOrderHead + kOrderBins,
-              order, max_a, max_b, long_rows, protein};
+              order, max_a, max_b, long_rows, protein_wide};
   cudaError_t e = order_smem_limits();
   if (e) return e;
   if (m <= kOrderOneBlock) {

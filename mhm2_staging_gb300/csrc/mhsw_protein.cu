@@ -13,9 +13,10 @@
 // length order.  The substitution scores of a lane's rows are bytes: one 128-bit shared load per
 // step gives the column's scores for all of them, and one byte permute per cell pair spreads two
 // of them into the halves of a word (a 24-code table of words, as the DNA engine's, would leave
-// room for 4 warps an SM).  Pairs whose score leaves the keys (4032), and matrices whose
+// room for 4 warps an SM).  Pairs whose score could leave int16 (min(M, N) * largest score from
+// 30,000 on), B above 65,000 residues, and matrices whose
 // scores do not fit the bytes (below -gap open, or above 127 - gap open), take the int32
-// kernels: one warp per pair, lanes along A (K rows a lane, 32K rows a strip), B's
+// kernels, beside the others on a side stream: one warp per pair, lanes along A (K rows a lane, 32K rows a strip), B's
 // columns swept as a skewed wavefront -- lane l works on column t - l at step t and hands
 // its bottom row's H and E to lane l + 1 by shuffle; strips hand their last row to the next
 // through a per-warp global row.  int32 cells with DPX add-max / 3-way relu-max; the
@@ -87,8 +88,8 @@ struct PArgs {
   int32_t *a_beg, *b_beg;          // begins written
   int2 *rows;                      // per warp slot: H, E of a strip's last row (max_n each)
   int64_t max_n;
-  const uint32_t *list;            // int32 kernels: the pairs to take (null: all n)
-  const int *list_n;
+  const uint32_t *list;            // int32 kernels: the pair order, from item *list_first on (null: all pairs)
+  const int *list_first;
 };
 
 // ---- keyed int16 kernels ------------------------------------------------------------------
@@ -96,7 +97,6 @@ struct PArgs {
 constexpr int kPadCol = kAA;                 // code of columns outside B: scores -gap open
 constexpr int kPCodes = kAA + 1;
 constexpr int kPWords = (kPCodes + 3) / 4;   // words of one row code's biased scores
-constexpr int kPCols = 65000;                // longest B (steps are 16-bit)
 
 struct P16Args {
   PArgs p;
@@ -104,19 +104,19 @@ struct P16Args {
   int *ctl;                        // the order's control block
   uint32_t *bound;                 // per group: strip boundary (bound_n words; lo H, hi E^)
   int64_t bound_n;                 // longest B these kernels take, at most kPCols
-  uint32_t *over;                  // pairs whose score left the keys
-  int *over_n;
-  int wide_from;                   // min(M, N) from which a pair goes straight to int32
 };
 
 // One step (Step16 of mhsw_engine16.cuh) with byte scores: lo words of this step's column, hi
 // words of the previous one.  Bytes are below 128, so the permute's sign bytes are zeros.
-template <int K>
+// BASE: keys are formed from H above a base kept per lane half (nbase: its negative), as in
+// mhsw_long.cu, so they hold scores up to int16's own limit.
+template <int K, bool BASE>
 struct StepP {
   static constexpr uint32_t kKeyMask = KeyBits<K>::kMask;
   __device__ static __forceinline__ void run(int t, uint32_t zH, uint32_t zE, uint32_t sel, uint32_t l0, uint32_t l1,
                                              uint32_t p0, uint32_t p1, uint32_t (&D)[K], uint32_t (&F)[K],
-                                             uint32_t &Hlast, uint32_t &Ecout, uint32_t &Kl, uint32_t &Jp, uint32_t NGE, uint32_t NGO, uint32_t one, uint32_t eight) {
+                                             uint32_t &Hlast, uint32_t &Ecout, uint32_t &Kl, uint32_t &Jp, uint32_t NGE,
+                                             uint32_t NGO, uint32_t one, uint32_t eight, uint32_t nbase) {
     uint32_t Ev = prmt_sel(zE, Ecout, sel);
     const uint32_t Htop = prmt_sel(zH, Hlast, sel);
     auto word = [&](int k) {
@@ -140,7 +140,8 @@ struct StepP {
       }
       Ev = __viaddmax_s16x2(Ev, NGE, Hn);
       F[k] = __viaddmax_s16x2(F[k], NGE, Hn);
-      key[k] = mad_u32(Hn, eight, (uint32_t)(kKeyMask - k) * 0x00010001u);
+      const uint32_t hk = BASE ? __viaddmax_s16x2_relu(Hn, nbase, 0u) : Hn;
+      key[k] = mad_u32(hk, eight, (uint32_t)(kKeyMask - k) * 0x00010001u);
     }
     uint32_t Kn = Kl;
 #pragma unroll
@@ -155,13 +156,17 @@ struct StepP {
 
 // Sweep of A (a[adir * i], i < M) over B (b[bdir * j], j < N): the best key, and whether the
 // score left the keys.  MULTI: A in strips of 2*K*G rows, the boundary row in bnd.
-template <int K, int G, bool MULTI>
+// BASE: the base starts at 0 and moves below a half's maximum once that is 2048 above it, looked at
+// every four steps at most.  A row's H rises by at most top + gap open <= 127 a column (opening a gap
+// bounds the left neighbour from below), so keys stay below 2048 + 4 * 127 < 4096; cells at or below
+// the base, which is under a score already seen in the half, cannot be the best.
+template <int K, int G, bool MULTI, bool BASE = false>
 __device__ unsigned long long protein_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, int bdir, int N,
                                             const uint32_t *rowtab, uint4 *tab, int lane, unsigned gmask, uint32_t *bnd,
                                             uint32_t NGE, uint32_t NGO, uint32_t one, int &overflow) {
   constexpr int KB = KeyBits<K>::kBits;
   constexpr uint32_t KMASK = KeyBits<K>::kMask;
-  using ST = StepP<K>;
+  using ST = StepP<K, BASE>;
   const uint32_t scale = one << KB;
   const int nstrips = MULTI ? (M + 2 * K * G - 1) / (2 * K * G) : 1;
   const int T_end = N + 2 * G - 1;
@@ -200,6 +205,21 @@ __device__ unsigned long long protein_sweep(const uint8_t *a, int adir, int M, c
     for (int k = 0; k < K; k++) D[k] = F[k] = 0u;
     uint32_t p0 = 0u, p1 = 0u;  // the previous column's hi scores (before column 0: -gap open)
     uint32_t Hlast = 0u, Ecout = 0u, Kl = 0u, Jp = 0u;
+    int base_lo = 0, base_hi = 0;
+    uint32_t nbase = 0u;
+    auto move_base = [&]() {
+      if constexpr (BASE) {
+        static_assert(KB == 3, "keys of 12 score bits");
+        if (Kl & 0x40004000u) {
+          const int klo = (int)(Kl & 0xffffu), khi = (int)(Kl >> 16);
+          const int dlo = klo & 0x4000 ? (klo >> 3) - 1 : 0, dhi = khi & 0x4000 ? (khi >> 3) - 1 : 0;
+          base_lo += dlo;
+          base_hi += dhi;
+          Kl = (uint32_t)(klo - 8 * dlo) | ((uint32_t)(khi - 8 * dhi) << 16);
+          nbase = V16::pack(-base_lo, -base_hi);
+        }
+      }
+    };
     const uint32_t sel = lane == 0 && first ? 0x54BBu : 0x5432u;
     const int j0 = -2 * lane;
     auto code_at = [&](int j) -> int {  // (a load in bounds for every j: no branch around it)
@@ -217,7 +237,8 @@ __device__ unsigned long long protein_sweep(const uint8_t *a, int adir, int M, c
         zH = __byte_perm(w, 0u, 0x1000);
         zE = w;
       }
-      ST::run(tt, zH, zE, sel, v.x, v.y, p0, p1, D, F, Hlast, Ecout, Kl, Jp, NGE, NGO, one, scale);
+      ST::run(tt, zH, zE, sel, v.x, v.y, p0, p1, D, F, Hlast, Ecout, Kl, Jp, NGE, NGO, one, scale,
+              nbase);
       p0 = v.z;
       p1 = v.w;
       if (MULTI && !last && lane == G - 1) {
@@ -237,7 +258,10 @@ __device__ unsigned long long protein_sweep(const uint8_t *a, int adir, int M, c
       step(t + 1, c);
     };
     // (the phases of sweep16_impl; an odd step count runs one step more over pad columns)
-    for (; t < T_end && t < 2 * G - 4; t += 2) two(std::true_type{});
+    for (; t < T_end && t < 2 * G - 4; t += 2) {
+      two(std::true_type{});
+      move_base();
+    }
     ahead = b + (ptrdiff_t)bdir * (t + 2 + j0);
     // (four steps an iteration: with eight the kernel misses the instruction cache, 1.38 ms for
     // 20,000 pairs against 1.31)
@@ -247,15 +271,21 @@ __device__ unsigned long long protein_sweep(const uint8_t *a, int adir, int M, c
         two(std::false_type{});
         t += 2;
       }
+      move_base();
     }
-    for (; t < T_end; t += 2) two(std::true_type{});
+    for (; t < T_end; t += 2) {
+      two(std::true_type{});
+      move_base();
+    }
 
     unsigned long long kbest = 0ull;
     int vmax = 0;
 #pragma unroll
     for (int half = 0; half < 2; half++) {
       const uint32_t key = half ? (Kl >> 16) : (Kl & 0xffffu);
-      const int v = (int)(key >> KB), r = row0 + (half ? K : 0) + (int)KMASK - (int)(key & KMASK);
+      if (BASE && (key >> KB) == 0) continue;  // nothing above the base
+      const int v = (int)(key >> KB) + (half ? base_hi : base_lo);
+      const int r = row0 + (half ? K : 0) + (int)KMASK - (int)(key & KMASK);
       const int col = (int)(half ? (Jp >> 16) : (Jp & 0xffffu)) - 2 * lane - half;
       vmax = v > vmax ? v : vmax;
       if (v > 0 && r < M) {
@@ -263,15 +293,16 @@ __device__ unsigned long long protein_sweep(const uint8_t *a, int adir, int M, c
         kbest = kk > kbest ? kk : kbest;
       }
     }
-    if (vmax > KeyBits<K>::kCap) overflow = 1;
+    if (!BASE && vmax > KeyBits<K>::kCap) overflow = 1;
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
       const unsigned long long other = __shfl_xor_sync(gmask, kbest, o, G);
       kbest = other > kbest ? other : kbest;
-      overflow |= __shfl_xor_sync(gmask, overflow, o, G);
+      if (!BASE) overflow |= __shfl_xor_sync(gmask, overflow, o, G);
     }
     if (kbest > best) best = kbest;
     __syncwarp(gmask);
+    if (overflow) break;  // the pair is swept again: no strip after this one matters
   }
   return best;
 }
@@ -289,8 +320,24 @@ __device__ __forceinline__ unsigned long long protein_rows(const uint8_t *a, int
   return protein_sweep<8, G, true>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
 }
 
+// The sweep with keys above a base, for pairs whose score left the plain keys.  (Not inlined: beside
+// the plain sweeps' code it costs 20,000 ordinary pairs 2-3%.)
+template <int G>
+__device__ __noinline__ unsigned long long protein_based(const uint8_t *a, int adir, int M, const uint8_t *b, int bdir,
+                                                            int N, const uint32_t *rowtab, uint4 *tab, int lane,
+                                                            unsigned gmask, uint32_t *bnd, uint32_t NGE, uint32_t NGO,
+                                                            uint32_t one) {
+  int none;
+  if (G == 16 || M <= 16 * G)
+    return protein_sweep<8, G, false, true>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, none);
+  return protein_sweep<8, G, true, true>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, none);
+}
+
 // Persistent: G-lane groups claim pairs of their range of the order (16 lanes: A up to 256
-// rows) and run both passes.  The begin sweep first covers score + 32 reversed rows (an
+// rows) and run both passes.  A pair whose score leaves the keys (4032) is swept again with keys above
+// a base, which costs an operation a cell pair more, not by the int32 kernels: 2,000 near-identical
+// pairs of 1,400-1,600 residues 8.9 ms in int32 alone, 10.3 in int16 and then int32, 5.4 so; 4,000 of
+// 600-700 2.95, 3.59 and 2.59.  The begin sweep first covers score + 32 reversed rows (an
 // alignment scores at least about one a row), then the whole prefix if the score is not there.
 template <int G>
 __global__ void __launch_bounds__(128, 5) k_protein16(P16Args g) {
@@ -311,7 +358,7 @@ __global__ void __launch_bounds__(128, 5) k_protein16(P16Args g) {
   uint32_t *bnd = g.bound ? g.bound + ((int64_t)blockIdx.x * (128 / G) + grp) * g.bound_n : nullptr;
   const uint32_t NGE = V16::splat(-p.gE), NGO = V16::splat(-p.gO);
   const uint32_t one = (uint32_t)(p.gO >> 30) + 1u;  // a 1 the compiler cannot fold
-  const int lo = G == 16 ? 0 : g.ctl[2], hi = G == 16 ? g.ctl[2] : (int)p.n;
+  const int lo = G == 16 ? 0 : g.ctl[2], hi = G == 16 ? g.ctl[2] : g.ctl[8 + kBucketWide];
   for (;;) {
     int claim = 0;
     if (lane == 0) claim = atomicAdd(g.ctl + (G == 16 ? 0 : 1), 1);
@@ -320,48 +367,47 @@ __global__ void __launch_bounds__(128, 5) k_protein16(P16Args g) {
     const uint32_t i = g.order[lo + claim];
     const int M = p.a_len[i], N = p.b_len[i];
     const uint8_t *a = p.a_code + p.a_off[i], *b = p.b_code + p.b_off[i];
-    int S = 0, ie = -1, je = 0, ib = -1, jb = 0, over = 0;
+    int S = 0, ie = -1, je = 0, ib = -1, jb = 0;
     if (M > 0 && N > 0) {
-      if (min(M, N) >= g.wide_from || N > kPCols) {
-        over = 1;
-      } else {
-        // Both passes through one call: three copies of the sweeps miss the instruction cache
-        // at every change of a warp's pass (20,000 pairs 1.45 -> 1.35 ms).
-        const uint8_t *qa = a, *qb = b;
-        int dir = 1, m = M, n = N, ignored = 0;
-        for (bool forward = true;; forward = false) {
-          const unsigned long long k = protein_rows<G>(qa, dir, m, qb, dir, n, rowtab, tab, lane, gmask, bnd, NGE, NGO, one,
-                                                       forward ? over : ignored);
-          if (forward) {
-            S = key_value(k);
-            if (S <= 0 || over) break;
-            ie = key_row(k);
-            je = key_col(k);
-            qa = a + ie;
-            qb = b + je;
-            dir = -1;
-            m = min(ie + 1, S + 32);
-            n = je + 1;
-          } else if (key_value(k) != S && m < ie + 1) {
-            m = ie + 1;
-          } else {
-            ib = ie - key_row(k);
-            jb = je - key_col(k);
-            break;
+      // Both passes through one call: three copies of the sweeps miss the instruction cache
+      // at every change of a warp's pass (20,000 pairs 1.45 -> 1.35 ms).
+      const uint8_t *qa = a, *qb = b;
+      int dir = 1, m = M, n = N, left_keys = 0;
+      bool forward = true, based = false;
+      for (;;) {
+        const unsigned long long k =
+            based ? protein_based<G>(qa, dir, m, qb, dir, n, rowtab, tab, lane, gmask, bnd, NGE, NGO, one)
+                  : protein_rows<G>(qa, dir, m, qb, dir, n, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, left_keys);
+        if (forward) {
+          if (!based && left_keys) {
+            based = true;
+            continue;
           }
+          S = key_value(k);
+          if (S <= 0) break;
+          forward = false;
+          ie = key_row(k);
+          je = key_col(k);
+          qa = a + ie;
+          qb = b + je;
+          dir = -1;
+          m = min(ie + 1, S + 32);
+          n = je + 1;
+        } else if (key_value(k) != S && m < ie + 1) {
+          m = ie + 1;
+        } else {
+          ib = ie - key_row(k);
+          jb = je - key_col(k);
+          break;
         }
       }
     }
     if (lane == 0) {
-      if (over) {
-        g.over[atomicAdd(g.over_n, 1)] = i;
-      } else {
-        p.score[i] = S;
-        p.a_end[i] = ie;
-        p.b_end[i] = je;
-        p.a_beg[i] = ib;
-        p.b_beg[i] = jb;
-      }
+      p.score[i] = S;
+      p.a_end[i] = ie;
+      p.b_end[i] = je;
+      p.a_beg[i] = ib;
+      p.b_beg[i] = jb;
     }
   }
 }
@@ -380,8 +426,7 @@ __global__ void __launch_bounds__(128) k_protein(PArgs g) {
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   int2 *bound = g.rows + warp * g.max_n;
   const int gO = g.gO, gE = g.gE;
-  const int64_t total = g.list ? (int64_t)*g.list_n : g.n;
-  for (int64_t it = warp; it < total; it += nwarps) {
+  for (int64_t it = (g.list ? *g.list_first : 0) + warp; it < g.n; it += nwarps) {
     const int64_t p = g.list ? (int64_t)g.list[it] : it;
     int M, N;
     const uint8_t *A = g.a_code + g.a_off[p], *B = g.b_code + g.b_off[p];
@@ -583,7 +628,7 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
   }
   const bool keyed = low >= -gO && top <= 63 && top + gO <= 127 && n <= 0x7fffffff;
   const int wide_from = top > 0 ? 30000 / top : INT_MAX;  // H itself leaves int16 from there on
-  const bool over_possible = !keyed || std::min(max_m, max_n) * top > KeyBits<8>::kCap || max_n > kPCols;
+  const bool wide_possible = !keyed || std::min(max_m, max_n) >= wide_from || max_n > kPCols;
   char *as = nullptr, *bs = nullptr;
   int64_t *ao = nullptr, *bo = nullptr;
   int32_t *al = nullptr, *bl = nullptr;
@@ -593,7 +638,7 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
   int *bad = nullptr;
   int2 *rows = nullptr;
   int *ctl = nullptr;
-  uint32_t *order = nullptr, *over = nullptr, *bound = nullptr;
+  uint32_t *order = nullptr, *bound = nullptr;
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // one warp per pair at a time; 24 resident warps per SM (76 registers x 128 threads
@@ -633,12 +678,11 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
     c.take(&bb, (size_t)n);
     c.take(&bad, 1);
     if (keyed) {
-      c.take(&ctl, kOrderCtl + 1);
+      c.take(&ctl, kOrderCtl);
       c.take(&order, (size_t)n);
-      c.take(&over, (size_t)n);
       if (max_m > 512) c.take(&bound, (size_t)(blocks32 * 4 * bound_n));
     }
-    if (over_possible) c.take(&rows, (size_t)(warps * max_n));
+    if (wide_possible) c.take(&rows, (size_t)(warps * max_n));
   };
   mhsw::Carve sizing;
   lay(sizing);
@@ -681,24 +725,32 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
     ps.a_len = al;
     ps.b_len = bl;
     ps.n = n;
-    int *over_n = ctl + kOrderCtl;
-    e = cudaMemsetAsync(over_n, 0, sizeof(int), st);
-    if (!e) e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, INT_MAX, true);
-    if (!e) {
-      const P16Args q{g, order, ctl, bound, bound_n, over, over_n, wide_from};
-      if (max_m > 256) k_protein16<32><<<(unsigned)blocks32, 128, smem32, st>>>(q);
-      k_protein16<16><<<(unsigned)blocks16, 128, smem16, st>>>(q);
-      e = cudaGetLastError();
-    }
-    g.list = over;
-    g.list_n = over_n;
+    e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, INT_MAX, wide_from);
+    g.list = order;
+    g.list_first = ctl + 8 + kBucketWide;
+  }
+  // the int32 kernels' pairs are others than the int16 kernels': side by side
+  const Forks *fk = driver_forks(d);
+  const bool fan = keyed && wide_possible && fk && fk->fork;
+  if (!e && fan) e = fork_to(*fk, st, 1);
+  if (!e && wide_possible) {
+    const unsigned blocks = (unsigned)((warps * 32 + 127) / 128);
+    cudaStream_t ws = fan ? fk->side[0] : st;
+    k_protein<false><<<blocks, 128, 0, ws>>>(g);
+    k_protein<true><<<blocks, 128, 0, ws>>>(g);
+    e = cudaGetLastError();
+  }
+  if (!e && keyed) {
+    const P16Args q{g, order, ctl, bound, bound_n};
+    if (max_m > 256) k_protein16<32><<<(unsigned)blocks32, 128, smem32, st>>>(q);
+    k_protein16<16><<<(unsigned)blocks16, 128, smem16, st>>>(q);
+    e = cudaGetLastError();
+  }
+  if (fan) {
+    const cudaError_t j = join_from(*fk, st, 1);  // (after a failed launch too: the arena is one call's)
+    if (!e) e = j;
   }
   if (!e) {
-    if (over_possible) {
-      const unsigned blocks = (unsigned)((warps * 32 + 127) / 128);
-      k_protein<false><<<blocks, 128, 0, st>>>(g);
-      k_protein<true><<<blocks, 128, 0, st>>>(g);
-    }
     k_protein_pack<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(sc, ab, ae, bb, be, n, o5);
     e = cudaGetLastError();
   }
