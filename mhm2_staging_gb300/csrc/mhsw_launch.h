@@ -140,7 +140,7 @@ cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scorin
 // ---- long pairs (mhsw_long.cu) -------------------------------------------------------
 // A pair with more rows than this (and, in the begin pass, a search whose first row cap is
 // above it) takes a block of its own when its score bound is at most kLongScore (keyed
-// scorings; not in score2 mode).
+// scorings; not in score2 mode; many pairs of little more rows: strips_take_long).
 constexpr int kLongRows = 1024;
 constexpr int kLongScore = 32000;
 constexpr int kLongWaits = 1 << 22;  // polls (of L2) before a wait gives up: seconds

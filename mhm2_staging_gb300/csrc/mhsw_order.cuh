@@ -15,14 +15,17 @@ namespace {
 
 // Buckets: 0..3 = A up to 64/96/128/160 rows (8-lane groups, K = 4/6/8/10),
 // 4/5 = up to 192/256 rows (16-lane groups, K = 6/8), 6 = longer A (K = 8 strips),
-// 7 = could exceed the int16 keys: straight to the int32 list; 8 = A above long_rows rows: a
-// block of its own (mhsw_long.cu).  The tuned row threshold
-// (lane_rows, 160 or 128) moves A of 129..160 rows between bucket 3 and bucket 4.
+// 7 = could exceed the int16 keys: straight to the int32 list; 8, 9 = A above long_rows rows: a
+// block of its own (mhsw_long.cu), or, for bucket 8 (up to kStripRows rows, scores that fit the keys),
+// strips of one lane group where the batch has many of them (strips_take_long).  The tuned row
+// threshold (lane_rows, 160 or 128) moves A of 129..160 rows between bucket 3 and bucket 4.
 constexpr int kBucketFirstLong = 4;
 constexpr int kBucketStrip = 6;
 constexpr int kBucketWide = 7;
-constexpr int kBucketLong = 8;
-constexpr int kBuckets = 9;
+constexpr int kBucketLongStrip = 8;
+constexpr int kBucketLong = 9;
+constexpr int kBuckets = 10;
+constexpr int kStripRows = 1280;
 __host__ __device__ constexpr int bucket_k(int b) {
   return b == 0 ? 4 : b == 1 ? 6 : b == 2 ? 8 : b == 3 ? 10 : b == 4 ? 6 : 8;
 }
@@ -36,7 +39,7 @@ __device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int la
   // fits a 16-bit key: the capacity leaves 64 values of margin and H grows by at most match
   // per step, so it holds for match <= 63; larger matches keep the bound routing.
   const long long bound = (long long)(M < N ? M : N) * sc.match;
-  if (M > long_rows && bound <= kLongScore) return kBucketLong;
+  if (M > long_rows && bound <= kLongScore) return M <= kStripRows && bound <= keyed_cap(8) ? kBucketLongStrip : kBucketLong;
   if ((!wide_try16 || sc.match > 63) && bound > keyed_cap(bucket_k(b))) return kBucketWide;
   return b;
 }
@@ -69,13 +72,17 @@ __device__ __forceinline__ int len_class(int n) {  // 0 = longest
   return kLenBins - 1 - c;
 }
 
+constexpr int kOrderLongFirst = 7;
+
 struct OrderArgs {
   PairSet ps;
   Scoring sc;
   int lane_rows;
   bool wide_try16;
   int64_t m, stride;  // item i < m is pair i * stride (stride 1: the whole batch; larger: the tuner's sample)
-  int *queue;         // [0], [1]: claim counters of the short and long ranges; [2]: first item of the long range
+  int *queue;         // [0], [1]: claim counters of the short and long ranges; [2]: first item of the long range;
+                      // [4..6]: LongCells of bucket 8; [kOrderLongFirst]: first item
+                      // of the long-pair kernel
   int *first;         // first item of each bucket, then m
   int *hist, *cursor; // kOrderBins each (zeroed before the two-launch form)
   uint32_t *order;
@@ -89,6 +96,39 @@ __device__ __forceinline__ int order_bin(const OrderArgs &g, int64_t p) {
   const int b = (M <= 0 || N <= 0 || M > g.max_a || N > g.max_b) ? (g.lane_rows > 0 ? 0 : kBucketFirstLong)
                 : g.protein_wide > 0 ? protein_bucket(M, N, g.protein_wide) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.long_rows);
   return b * kLenBins + len_class(N);
+}
+
+// What strips_take_long weighs for the pairs of bucket 8, in units of 1024 cells: gathered per block,
+// then once per block in queue[4], [5] (64 bits) and [6].
+constexpr int kLongFill = 400;  // columns' worth of the long-pair kernel's time that filling its strips takes
+struct LongCells {
+  unsigned long long sum;  // rows * (columns + kLongFill)
+  unsigned int most;       // the longest pair's cells
+};
+__device__ __forceinline__ void add_long_cells(LongCells *s, const OrderArgs &g, int64_t p, int bin) {
+  if (bin < kBucketLongStrip * kLenBins || bin >= (kBucketLongStrip + 1) * kLenBins) return;
+  const long long M = g.ps.a_len[p], N = g.ps.b_len[p];
+  atomicAdd(&s->sum, (unsigned long long)(M * (N + kLongFill) >> 10));
+  atomicMax(&s->most, (unsigned int)((M * N + 1023) >> 10));
+}
+__device__ __forceinline__ void flush_long_cells(const LongCells &s, int *queue) {
+  if (threadIdx.x != 0 || s.sum == 0) return;
+  atomicAdd(reinterpret_cast<unsigned long long *>(queue + 4), s.sum);
+  atomicMax(reinterpret_cast<unsigned int *>(queue + 6), s.most);
+}
+
+// Whether bucket 8 goes to the persistent kernel's lane groups, a pair a group in strips of 256
+// rows, rather than to the long-pair kernel.  That kernel's strips of 512 rows are a third padding
+// there, but a lane group alone sweeps only about 1 G cells/s: the groups win once what the batch costs
+// the long-pair kernel is kStripShare times its longest pair's cells.  Forward pass, long-pair kernel / lane groups, 1,030-1,100
+// rows: 20,000 pairs against 300-400 columns 4.54 / 2.31 ms, against 1,030-1,100 9.67 / 6.68; 3,000
+// pairs 0.79 / 0.66 and 1.60 / 1.60, 2,000 0.57 / 0.56 and 1.14 / 1.34; against 4,000-6,000 columns
+// 12,000 pairs 22.7 / 17.9, 4,000 7.8 / 9.5.  From 1,500 rows on the long-pair kernel is level or
+// ahead up to 20,000 pairs (1,500-2,000 squared 18.5 / 19.4).
+constexpr unsigned long long kStripShare = 3700;
+__device__ __forceinline__ bool strips_take_long(const int *queue) {
+  const unsigned long long sum = *reinterpret_cast<const volatile unsigned long long *>(queue + 4);
+  return sum > 0 && sum >= kStripShare * *reinterpret_cast<const volatile unsigned int *>(queue + 6);
 }
 
 // Exclusive prefix sum of the kOrderBins counts in h, in place, by the whole block.
@@ -131,22 +171,29 @@ __device__ __forceinline__ void write_firsts(const OrderArgs &g, const int *base
   if (threadIdx.x == 0) {
     g.first[kBuckets] = (int)g.m;
     g.queue[2] = base[kBucketFirstLong * kLenBins];
+    g.queue[kOrderLongFirst] = base[(strips_take_long(g.queue) ? kBucketLong : kBucketLongStrip) * kLenBins];
   }
 }
 
 __global__ void __launch_bounds__(1024) k_order_one(OrderArgs g) {
   extern __shared__ int h[];
   for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) h[b] = 0;
-  if (threadIdx.x < 2) g.queue[threadIdx.x] = 0;
+  __shared__ LongCells cells;
+  if (threadIdx.x < 7 && threadIdx.x != 2) g.queue[threadIdx.x] = 0;
+  if (threadIdx.x == 0) cells = LongCells{0ull, 0u};
   __syncthreads();
   int bin[kOrderOneBlock / 1024];
 #pragma unroll
   for (int k = 0; k < kOrderOneBlock / 1024; k++) {
     const int64_t i = threadIdx.x + k * 1024;
     bin[k] = i < g.m ? order_bin(g, i * g.stride) : -1;
-    if (bin[k] >= 0) atomicAdd(&h[bin[k]], 1);
+    if (bin[k] >= 0) {
+      atomicAdd(&h[bin[k]], 1);
+      add_long_cells(&cells, g, i * g.stride, bin[k]);
+    }
   }
   __syncthreads();
+  flush_long_cells(cells, g.queue);
   scan_bins(h);
   write_firsts(g, h);
   __syncthreads();
@@ -157,11 +204,17 @@ __global__ void __launch_bounds__(1024) k_order_one(OrderArgs g) {
 
 __global__ void __launch_bounds__(1024) k_order_hist(OrderArgs g) {
   extern __shared__ int h[];
+  __shared__ LongCells cells;
   for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x) h[b] = 0;
+  if (threadIdx.x == 0) cells = LongCells{0ull, 0u};
   __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.m; i += (int64_t)gridDim.x * blockDim.x)
-    atomicAdd(&h[order_bin(g, i * g.stride)], 1);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.m; i += (int64_t)gridDim.x * blockDim.x) {
+    const int bin = order_bin(g, i * g.stride);
+    atomicAdd(&h[bin], 1);
+    add_long_cells(&cells, g, i * g.stride, bin);
+  }
   __syncthreads();
+  flush_long_cells(cells, g.queue);
   for (int b = threadIdx.x; b < kOrderBins; b += blockDim.x)
     if (h[b]) atomicAdd(&g.hist[b], h[b]);
 }
@@ -194,7 +247,7 @@ __global__ void __launch_bounds__(1024) k_order_place(OrderArgs g) {
   }
 }
 
-// The order's control block: [0..7] claim counters and first long item, [8..23] first item of
+// The order's control block: [0..7] as OrderArgs::queue, [8..23] first item of
 // each bucket and the item count, then the bin counts and cursors.
 constexpr size_t kOrderHead = 24;
 constexpr size_t kOrderCtl = kOrderHead + 2 * kOrderBins;
