@@ -458,7 +458,7 @@ int ensure_results(mhsw_driver *d, int64_t n) {
   MHSW_CK(d->l_ovf.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_wide.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_bands.reserve((size_t)n + 1), "cudaMalloc lists");
-  MHSW_CK(d->l_counts.reserve(6 + 2 * mhsw::kBandClasses), "cudaMalloc lists");
+  MHSW_CK(d->l_counts.reserve(7 + 2 * mhsw::kBandClasses + mhsw::kWarpClasses), "cudaMalloc lists");
   return MHSW_OK;
 }
 
@@ -640,6 +640,7 @@ mhsw::WorkLists work_lists(mhsw_driver *d, int64_t n) {
   wl.long_bnd = d->long_bnd.p;
   wl.long_waits = d->wait_limit;
   wl.esc_count = d->l_counts.p + 5 + 2 * mhsw::kBandClasses;
+  wl.warp_cost = reinterpret_cast<unsigned int *>(d->l_counts.p + 6 + 2 * mhsw::kBandClasses);
   wl.cap = n;
   return wl;
 }

@@ -153,6 +153,28 @@ __device__ __forceinline__ bool band_outgrown(int t, int N2, int S, const Scorin
   return I > L || J > 2 * G - L;
 }
 
+// Searches of the widest classes may go to the warp kernel instead: it costs about ten times a banded
+// search's instructions but not a thread's latency (0.5 us a row pair, however few the searches).
+// From the widest class down they go there while what a warp would sweep for all of them stays
+// below kWarpShare * 1024 cells per row of the longest search: about what the warps get through in
+// the time a thread takes for that search.  Whole calls with a share of 0 / 500 / 1000 / 2000 / 4000:
+// 8,500 pairs of 150 bp in 300, 15% apart, 393 / 395 / 356 / 341 / 342 us (50,000: 950 to 952); 8,500 of
+// 400-900 in 600-1,500, 2%, 3.58 / 3.93 / 4.29 / 4.24 / 4.26 ms; 100,000 uneven with CIGARs 2.83 / 2.77 /
+// 2.77 / 2.85 / 3.02.  By the batch's size alone (classes 5 and 6 up to 250,000 pairs) 50,000 pairs of
+// 150 bp, 15% apart, took 1,242 us.
+constexpr unsigned long long kWarpShare = 1000;
+// The narrowest class that goes there (kBandClasses: none).
+__device__ __forceinline__ int warp_top_class(const WorkLists &wl, bool warps) {
+  int top = kBandClasses;
+  unsigned long long sum = 0;
+#pragma unroll
+  for (int k = kWarpClasses - 1; k >= 0; k--) {
+    sum += wl.warp_cost[k];
+    if (warps && top == kBandClasses - kWarpClasses + k + 1 && sum <= kWarpShare * wl.warp_cost[kWarpClasses]) top--;
+  }
+  return top;
+}
+
 // The class a search goes to: band_fit's, or the wide list when that is at least top_class and
 // the warp kernel takes it.
 __device__ __forceinline__ int band_route(int S, int M2, int N2, const Scoring &sc, int top_class) {
@@ -166,7 +188,7 @@ __device__ __forceinline__ int band_route(int S, int M2, int N2, const Scoring &
 // s_cap: the largest score the band kernels take (the packed int16 kernels hold scores up
 // to kBand16Score); pairs above it go to the wavefront list too.
 // longs: searches over many rows go to the wide list, where the long-pair kernel takes them.
-__device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc, int64_t p, int s_cap, bool longs, int top_class) {
+__device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc, int64_t p, int s_cap, bool longs) {
   const int S = rs.score[p];
   if ((rs.flag[p] & kFlagTooLong) || S <= 0) {
     rs.a_beg[p] = -1;
@@ -174,7 +196,7 @@ __device__ __forceinline__ int band_class(const ResultSet &rs, const Scoring &sc
     return -1;
   }
   if (S > s_cap || (longs && long_begin(band_first_cap(S, sc.match, rs.a_end[p] + 1), S))) return kBandClasses;
-  return band_route(S, rs.a_end[p] + 1, rs.b_end[p] + 1, sc, top_class);
+  return band_fit(S, rs.a_end[p] + 1, rs.b_end[p] + 1, sc);
 }
 
 // Warp-aggregated append of p to the end of the list, downwards (one atomic per warp).
@@ -193,27 +215,41 @@ __device__ __forceinline__ void append_agg(int64_t *list, int *count, int64_t ca
   }
 }
 
-// Pass 1: count the pairs of each band class.
+// Pass 1: count the pairs of each band class, and what the widest classes would cost the warp kernel.
 __global__ void __launch_bounds__(256) k_rev_count(ResultSet rs, Scoring sc, const uint32_t *__restrict__ order,
-                                                   int64_t n, int *band_counts, int s_cap, bool longs,
-                                                   int top_class) {
+                                                   int64_t n, WorkLists wl, int s_cap, bool longs, bool warps) {
   __shared__ int cnt[kBandClasses];
+  __shared__ unsigned int cost[kWarpClasses + 1];
   if (threadIdx.x < kBandClasses) cnt[threadIdx.x] = 0;
+  if (threadIdx.x <= kWarpClasses) cost[threadIdx.x] = 0u;
   __syncthreads();
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = order ? (int64_t)order[idx] : idx;
-    const int c = band_class(rs, sc, p, s_cap, longs, top_class);
+    const int c = band_class(rs, sc, p, s_cap, longs);
     if (c >= 0 && c < kBandClasses) atomicAdd(&cnt[c], 1);
+    if (warps && c >= kBandClasses - kWarpClasses && c < kBandClasses) {
+      const int S = rs.score[p], M2 = rs.a_end[p] + 1, N2 = rs.b_end[p] + 1;
+      if (warp_begin(M2, N2, S, sc)) {
+        const int t = band_first_cap(S, sc.match, M2);
+        int I, J;
+        band_sides(t, N2, S, sc, I, J);
+        const int n2 = t + J < N2 ? t + J : N2;
+        atomicAdd(&cost[c - (kBandClasses - kWarpClasses)], (unsigned int)(t * n2 + 1023) >> 10);
+        atomicMax(&cost[kWarpClasses], (unsigned int)t);
+      }
+    }
   }
   __syncthreads();
-  if (threadIdx.x < kBandClasses && cnt[threadIdx.x]) atomicAdd(&band_counts[threadIdx.x], cnt[threadIdx.x]);
+  if (threadIdx.x < kBandClasses && cnt[threadIdx.x]) atomicAdd(&wl.band_counts[threadIdx.x], cnt[threadIdx.x]);
+  if (threadIdx.x < kWarpClasses && cost[threadIdx.x]) atomicAdd(&wl.warp_cost[threadIdx.x], cost[threadIdx.x]);
+  if (threadIdx.x == kWarpClasses && cost[threadIdx.x]) atomicMax(&wl.warp_cost[threadIdx.x], cost[threadIdx.x]);
 }
 
 // Pass 2: place each pair in its class segment (segments in class order, each filled in
 // the batch's order); wider pairs go to the wavefront list.
 __global__ void __launch_bounds__(256) k_rev_scatter(ResultSet rs, Scoring sc, const uint32_t *__restrict__ order,
-                                                     int64_t n, WorkLists wl, int s_cap, bool longs,
-                                                     int top_class) {
+                                                     int64_t n, WorkLists wl, int s_cap, bool longs, bool warps) {
+  const int top_class = warp_top_class(wl, warps);
   int off[kBandClasses];
   int acc = 0;
 #pragma unroll
@@ -364,7 +400,7 @@ __global__ void __launch_bounds__(128) k_rev_band(PairSet ps, ResultSet rs, Scor
   int64_t off = 0;
 #pragma unroll
   for (int c = 0; c < C; c++) off += wl.band_counts[c];
-  int64_t total = wl.band_counts[C];
+  int64_t total = wl.band_counts[kBandClasses + C];  // (those scattered: some of its count may be the warp kernel's)
   if (off + total > wl.cap) total = wl.cap - off;
   // A pair's fields are loaded one grid-stride iteration ahead of its search (their
   // chain of dependent loads then overlaps the previous pair's rows), and the A codes of
@@ -546,7 +582,7 @@ __global__ void __launch_bounds__(128) k_rev_band16(PairSet ps, ResultSet rs, Sc
   int64_t off = 0;
 #pragma unroll
   for (int c = 0; c < C; c++) off += wl.band_counts[c];
-  int64_t total = wl.band_counts[C];
+  int64_t total = wl.band_counts[kBandClasses + C];  // (those scattered: some of its count may be the warp kernel's)
   if (off + total > wl.cap) total = wl.cap - off;
   struct Meta {
     int64_t p = -1;
@@ -831,6 +867,7 @@ __global__ void k_reset_lists(WorkLists wl) {
   *wl.esc_count = 0;
   *wl.failed = 0;
   for (int i = 0; i < 2 * kBandClasses; i++) wl.band_counts[i] = 0;
+  for (int i = 0; i <= kWarpClasses; i++) wl.warp_cost[i] = 0u;
   wl.long_next[0] = wl.long_next[1] = 0;
 }
 
@@ -1043,13 +1080,8 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
                     sc.match + sc.gap_open <= 255;
     const int s_cap = bi ? kBand16Score : 0x7fffffff;
     const bool force = longs && ps.n <= kLongBeginPairs;
-    // The narrowest class that goes to the warp kernel: it costs about ten times a banded
-    // search's instructions but not a thread's latency.  Begin pass, classes 7 / 5 / 4 / 3 from:
-    // 9000 mixed pairs 184 / 135 / 127 / 123 us, 20,000 220 / 180 / 214 / 239, 100,000 uneven
-    // 362 / 324 / 463 / 733, 800,000 1390 / 1707 / 2680 / 4952.
-    const int top_class = !warps || ps.n > 250000 ? kBandClasses : ps.n > 12000 ? 5 : 4;
-    k_rev_count<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl.band_counts, s_cap, force, top_class);
-    k_rev_scatter<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap, force, top_class);
+    k_rev_count<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap, force, warps);
+    k_rev_scatter<<<grid, 256, 0, st>>>(rs, sc, order, ps.n, wl, s_cap, force, warps);
     // The classes are independent: with side streams they run concurrently, so the
     // latency-bound narrow classes share the SMs with the wide ones.
     cudaStream_t cs[kBandClasses];

@@ -10,6 +10,7 @@ struct PairSet;
 struct ResultSet;
 
 constexpr int kBandClasses = 7;  // banded begin-pass instantiations (half-widths 3 .. 31)
+constexpr int kWarpClasses = 3;  // of these, the widest, which the warp kernel may take
 
 // Work lists built on the device (no host round trip between passes).
 struct WorkLists {
@@ -21,6 +22,8 @@ struct WorkLists {
   int *esc_count;
   int64_t *bands;     // begin-pass pairs grouped by band class (one segment per class)
   int *band_counts;   // kBandClasses pair counts, then kBandClasses scatter cursors
+  unsigned int *warp_cost;  // kWarpClasses: cells a warp would sweep for the class's searches, in 1024s; then
+                            // the most rows among them
   int64_t cap;        // capacity of each list
   int *failed;        // pairs flagged kFlagTooLong: the call fails
   int *long_next;     // claim counters of the long-pair kernels (forward, begin)

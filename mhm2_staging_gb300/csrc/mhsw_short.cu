@@ -393,8 +393,9 @@ __global__ void __launch_bounds__(32) k_short(ShortArgs g) {
 }
 
 // Begin searches of the wide list, a warp each: bands wider than the banded kernels hold, those
-// that outgrew theirs, and in all but the largest batches the widest of their classes, whose threads walk a row pair in
-// 0.5 us -- 250 rows took 130-160 us however few the pairs.  Same search as k_short's.
+// that outgrew theirs, and the widest of their classes while they hold few searches (warp_top_class):
+// their threads walk a row pair in 0.5 us, so 250 rows took 130-160 us however few the pairs.  Same
+// search as k_short's.
 template <bool STEP>
 __global__ void __launch_bounds__(32) k_rev_warp(PairSet ps, ResultSet rs, Scoring sc, WorkLists wl, bool longs,
                                                  bool escaped) {
