@@ -81,13 +81,15 @@ typedef struct {
  * from their translation to the end of the begin pass; fwd_cells and the counters of
  * re-runs left 0). */
 typedef struct {
-  double fwd_ms;      /* forward kernels (incl. int32 re-runs) */
-  double rev_ms;      /* begin (reverse) kernels */
+  double fwd_ms;      /* forward kernels (incl. int32 re-runs); both passes on the one-launch path */
+  double rev_ms;      /* begin (reverse) kernels; 0 on the one-launch path (see MHSW_FORM_PLAIN for
+                       * which batches take it) */
   double total_ms;    /* all device work of the call incl. copies */
   double fwd_cells;   /* sum over pairs of len(A) * len(B) */
   int64_t n_pairs;
   int64_t n_overflow16;  /* pairs re-run in int32 */
-  int64_t n_rev_wide;    /* begin searches wider than the banded kernels */
+  int64_t n_rev_wide;    /* begin searches wider than the banded kernels hold, from the start or on
+                          * the way (whichever kernel took them; 0 on the one-launch path) */
   int64_t launches;      /* kernels launched by the call (a graph replay counts its kernels) */
   int64_t graph_replays; /* CUDA graph launches by this handle so far: a device-resident batch
                           * aligned again with the same pointers, sizes and settings is

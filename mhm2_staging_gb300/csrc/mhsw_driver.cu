@@ -84,7 +84,7 @@ struct HBuf {
   }
 };
 
-constexpr int kHostCounts = 3;  // counters a batch copies back: int32 re-runs, wide searches, failed pairs
+constexpr int kHostCounts = 4;  // counters a batch copies back: int32 re-runs, wide searches, escapes, failed pairs
 constexpr int kInt16Ceiling = mhsw::V16::kBig - 1 - 64;  // leaves room for one match step
 
 }  // namespace
@@ -458,7 +458,7 @@ int ensure_results(mhsw_driver *d, int64_t n) {
   MHSW_CK(d->l_ovf.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_wide.reserve((size_t)n + 1), "cudaMalloc lists");
   MHSW_CK(d->l_bands.reserve((size_t)n + 1), "cudaMalloc lists");
-  MHSW_CK(d->l_counts.reserve(7 + 2 * mhsw::kBandClasses + mhsw::kWarpClasses), "cudaMalloc lists");
+  MHSW_CK(d->l_counts.reserve(8 + 2 * mhsw::kBandClasses + mhsw::kWarpClasses), "cudaMalloc lists");
   return MHSW_OK;
 }
 
@@ -632,15 +632,16 @@ mhsw::WorkLists work_lists(mhsw_driver *d, int64_t n) {
   wl.ovf = d->l_ovf.p;
   wl.wide = d->l_wide.p;
   wl.ovf_count = d->l_counts.p;
-  wl.wide_count = d->l_counts.p + 1;
+  wl.wider = d->l_counts.p + 1;
+  wl.esc_count = d->l_counts.p + 2;
   wl.bands = d->l_bands.p;
-  wl.failed = d->l_counts.p + 2;  // (these three are read back: kHostCounts)
-  wl.band_counts = d->l_counts.p + 3;
-  wl.long_next = d->l_counts.p + 3 + 2 * mhsw::kBandClasses;
+  wl.failed = d->l_counts.p + 3;  // (these four are read back: kHostCounts)
+  wl.wide_count = d->l_counts.p + 4;
+  wl.band_counts = d->l_counts.p + 5;
+  wl.long_next = d->l_counts.p + 5 + 2 * mhsw::kBandClasses;
   wl.long_bnd = d->long_bnd.p;
   wl.long_waits = d->wait_limit;
-  wl.esc_count = d->l_counts.p + 5 + 2 * mhsw::kBandClasses;
-  wl.warp_cost = reinterpret_cast<unsigned int *>(d->l_counts.p + 6 + 2 * mhsw::kBandClasses);
+  wl.warp_cost = reinterpret_cast<unsigned int *>(d->l_counts.p + 7 + 2 * mhsw::kBandClasses);
   wl.cap = n;
   return wl;
 }
@@ -791,11 +792,11 @@ int copy_counts(mhsw_driver *d, int *to) {
 
 // The error of a completed batch with flagged pairs (c: its counters), or MHSW_OK.
 int check_failed(mhsw_driver *d, const int *c) {
-  if (c[2] <= 0) return MHSW_OK;
+  if (c[3] <= 0) return MHSW_OK;
   return d->fail(MHSW_ERR_INTERNAL,
                  "%d pairs were not aligned (longer than the stated extents, a search that missed its score, or a wait "
                  "between a long pair's blocks that gave up)",
-                 c[2]);
+                 c[3]);
 }
 
 int check_scoring(mhsw_driver *d, const mhsw::Scoring &s) {
@@ -1328,7 +1329,7 @@ int mhsw_run_kernel_backwards(mhsw_driver *d, const char *const *reads, const in
   if (d->brief_batch && !d->cigar) {
     // the begins came with the forward launch
     MHSW_CK(d->h_counts.reserve(4), "cudaMallocHost");
-    d->h_counts.p[0] = d->h_counts.p[1] = 0;
+    std::fill_n(d->h_counts.p, kHostCounts, 0);
     MHSW_CK(cudaEventRecord(d->ev_t[4], d->st), "event");
     MHSW_CK(cudaEventRecord(d->ev_t[5], d->st), "event");
     MHSW_CK(cudaEventRecord(d->ev_done, d->st), "event");
@@ -1427,7 +1428,7 @@ int mhsw_kernel_block(mhsw_driver *d) {
     d->timing.fwd_cells = d->fwd_cells;
     d->timing.n_pairs = d->n_batch;
     d->timing.n_overflow16 = d->h_counts.p[0];
-    d->timing.n_rev_wide = d->h_counts.p[1];
+    d->timing.n_rev_wide = d->h_counts.p[1] + d->h_counts.p[2];
     d->timing.launches = d->launches;
   }
   return d->counts_live ? check_failed(d, d->h_counts.p) : MHSW_OK;
@@ -1496,7 +1497,7 @@ int finish_slot(mhsw_driver *d, int s) {
   d->timing.fwd_cells = pd.cells;
   d->timing.n_pairs = n;
   d->timing.n_overflow16 = n > 0 && hc ? hc[0] : 0;
-  d->timing.n_rev_wide = n > 0 && hc ? hc[1] : 0;
+  d->timing.n_rev_wide = n > 0 && hc ? hc[1] + hc[2] : 0;
   d->timing.launches = d->launches;
   d->timing.graph_replays = d->graph_launches;
   d->timing.cigar_ms = d->cigar_ms;

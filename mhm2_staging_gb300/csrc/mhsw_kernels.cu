@@ -218,15 +218,19 @@ __device__ __forceinline__ void append_agg(int64_t *list, int *count, int64_t ca
 // Pass 1: count the pairs of each band class, and what the widest classes would cost the warp kernel.
 __global__ void __launch_bounds__(256) k_rev_count(ResultSet rs, Scoring sc, const uint32_t *__restrict__ order,
                                                    int64_t n, WorkLists wl, int s_cap, bool longs, bool warps) {
-  __shared__ int cnt[kBandClasses];
+  __shared__ int cnt[kBandClasses + 1];  // (the last: wider than all of them, whoever takes it)
   __shared__ unsigned int cost[kWarpClasses + 1];
-  if (threadIdx.x < kBandClasses) cnt[threadIdx.x] = 0;
+  if (threadIdx.x <= kBandClasses) cnt[threadIdx.x] = 0;
   if (threadIdx.x <= kWarpClasses) cost[threadIdx.x] = 0u;
   __syncthreads();
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = order ? (int64_t)order[idx] : idx;
     const int c = band_class(rs, sc, p, s_cap, longs);
     if (c >= 0 && c < kBandClasses) atomicAdd(&cnt[c], 1);
+    if (c == kBandClasses) {
+      const int S = rs.score[p];
+      if (!longs || S > s_cap || band_fit(S, rs.a_end[p] + 1, rs.b_end[p] + 1, sc) == c) atomicAdd(&cnt[c], 1);
+    }
     if (warps && c >= kBandClasses - kWarpClasses && c < kBandClasses) {
       const int S = rs.score[p], M2 = rs.a_end[p] + 1, N2 = rs.b_end[p] + 1;
       if (warp_begin(M2, N2, S, sc)) {
@@ -241,6 +245,7 @@ __global__ void __launch_bounds__(256) k_rev_count(ResultSet rs, Scoring sc, con
   }
   __syncthreads();
   if (threadIdx.x < kBandClasses && cnt[threadIdx.x]) atomicAdd(&wl.band_counts[threadIdx.x], cnt[threadIdx.x]);
+  if (threadIdx.x == kBandClasses && cnt[threadIdx.x]) atomicAdd(wl.wider, cnt[threadIdx.x]);
   if (threadIdx.x < kWarpClasses && cost[threadIdx.x]) atomicAdd(&wl.warp_cost[threadIdx.x], cost[threadIdx.x]);
   if (threadIdx.x == kWarpClasses && cost[threadIdx.x]) atomicMax(&wl.warp_cost[threadIdx.x], cost[threadIdx.x]);
 }
@@ -866,6 +871,7 @@ __global__ void k_reset_lists(WorkLists wl) {
   *wl.wide_count = 0;
   *wl.esc_count = 0;
   *wl.failed = 0;
+  *wl.wider = 0;
   for (int i = 0; i < 2 * kBandClasses; i++) wl.band_counts[i] = 0;
   for (int i = 0; i <= kWarpClasses; i++) wl.warp_cost[i] = 0u;
   wl.long_next[0] = wl.long_next[1] = 0;

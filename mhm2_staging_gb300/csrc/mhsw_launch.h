@@ -26,6 +26,7 @@ struct WorkLists {
                             // the most rows among them
   int64_t cap;        // capacity of each list
   int *failed;        // pairs flagged kFlagTooLong: the call fails
+  int *wider;         // searches wider than the banded kernels hold (of the wide list, which others go to as well)
   int *long_next;     // claim counters of the long-pair kernels (forward, begin)
   uint32_t *long_bnd; // their strip boundaries (LongPlan::bytes), or null
   int long_waits;     // polls after which one of their waits gives up (at most kLongWaits)

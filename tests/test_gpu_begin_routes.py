@@ -59,3 +59,29 @@ def test_rows_past_the_warp_kernel(built):
     d.init(0, 1, 1, -3, -5, -2, 0)
     d.set_ambiguity(-2)
     assert np.array_equal(d.align_pairs(p, FORM_PLAIN), oracle.align_batch(p, (1, 3, 5, 2, 2)))
+
+
+@pytest.mark.parametrize("n", [8500, 30000])
+def test_count_of_wide_searches(built, n):
+    """n_rev_wide counts the searches wider than the banded kernels hold (63 cells), not those that a
+    rule on the batch gives to other kernels."""
+    from test_band_bounds import band_sides
+
+    sc = (1, 3, 5, 2, 2)
+    rng = np.random.default_rng(n)
+    a, b = _pairs(rng, n, (140, 300), 0.12, 0)
+    p = Pairs.from_lists(a, b)
+    out = oracle.align_batch(p, sc)
+    # searches whose first rows are all their rows: nothing outgrows its band on the way
+    keep = [i for i in range(n) if 2 * out[i, 0] + 16 >= out[i, 2] + 1]
+    p, out = p.subset(keep), out[keep]
+    sides = [band_sides(int(ie) + 1, int(je) + 1, int(s), sc) for s, _, ie, _, je in out]
+    want = sum(i + j > 2 * 31 for i, j, _ in sides)
+    assert p.n > 8192 * 0.9 and 0 < want < p.n // 2
+    d = GPUDriver()
+    d.init(0, 1, 1, -3, -5, -2, 0)
+    d.set_ambiguity(-2)
+    d.fix_batch_config(128, 0, 160, False)  # (not the one-launch path)
+    got = d.align_pairs(p, FORM_BATCHED)
+    assert np.array_equal(got, out)
+    assert d.last_timing()["n_rev_wide"] == want
