@@ -816,7 +816,7 @@ constexpr int64_t kInPlaceBytes = 512 << 10;
 // general path's kernels).
 bool short_passes(mhsw_driver *d, int64_t n, int max_a, int max_b, int form) {
   return n > 0 && !(form == MHSW_FORM_BATCHED && !d->batch.autotune) &&
-         mhsw::short_batch(d->sc, ceiling_for(d), n, max_a, max_b);
+         mhsw::short_batch(d->sc, ceiling_for(d), n, max_a, max_b, d->score2);
 }
 
 // ... and is all there is to do (CIGAR mode goes on from the code arenas and result arrays).

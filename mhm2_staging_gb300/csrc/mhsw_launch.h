@@ -112,12 +112,16 @@ cudaError_t launch_finalize(const ResultSet &rs, int64_t n, bool a_is_query, int
                             cudaStream_t st);
 
 // ---- short batches (mhsw_short.cu) -------------------------------------------------
-// Largest batch (pairs, and pairs times the longest B), A and B the one-launch path takes.
+// Largest batch (pairs, and pairs times the longest B), A and B the one-launch path takes; and the
+// lower lines (short_batch) for A up to kShortNarrow rows and up to 256.
 constexpr int64_t kShortPairs = 8192;
 constexpr int64_t kShortColumns = 14000000;
 constexpr int kShortRowsMax = 512;
 constexpr int kShortColsMax = 8192;
-bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b);
+constexpr int kShortNarrow = 64;
+constexpr int64_t kNarrowPairs = 2000, kNarrowPairsS2 = 1500, kNarrowColumns = 3000000;
+constexpr int64_t kMidPairs = 6500, kMidColumns = 11000000;
+bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b, bool score2);
 // Forward and begin pass of a short batch: ps.a_seq raw bytes, B from ps.b_code or, when
 // that is null, ps.b_seq raw bytes; any of them may be pinned host memory.  Results go to out5
 // (n x 5), the drop-in views ov and the general path's arrays rs (each may be null; score2

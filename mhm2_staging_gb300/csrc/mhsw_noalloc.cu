@@ -361,7 +361,7 @@ extern "C" int mhsw_forward_noalloc(const mhsw_pairs *pairs, short match_score, 
     return na_fail(errbuf, errlen, MHSW_ERR_CUDA, "launch: %s", cudaGetErrorString(err));
   };
   const int ceiling = kCeiling16;
-  if (short_batch(sc, ceiling, n, max_a, max_b)) {
+  if (short_batch(sc, ceiling, n, max_a, max_b, false)) {
     if ((e = launch_short_forward(ps, sc, max_a, max_b, out3, st))) return launch_fail(e);
     return MHSW_OK;
   }

@@ -14,10 +14,9 @@
 // smallest row, then column, which is SSW's rule for ends and (reversed) for begins
 // (ssw_core.cpp:474-506, :1166-1178); no cell of the reversed box exceeds the score.
 //
-// Measured against the general path (whole call, resident batch): 400 mixed reads 308 -> 95 us,
-// 2,000 462 -> 186, 8,100 664 -> 474, 1,600 250 bp reads against 2-8 kb 1217 -> 969; a host
-// call of 32 pairs 222 -> 73.  At 3,000 such long references it loses (1482 against 1245):
-// kShortPairs and kShortColumns draw the line.
+// Measured against what it replaced (whole call, resident batch): 400 mixed reads 308 -> 95 us,
+// 2,000 462 -> 186, 8,100 664 -> 412; a host call of 32 pairs 207 -> 60.  short_batch draws the line to
+// the general path.
 //
 // 32 lanes per pair give the shortest serial chain (a lane step costs its rows' chain of
 // dependent maxima plus the hand-off) and no idle lanes beside a longer neighbour, at the
@@ -449,9 +448,19 @@ cudaError_t launch_rev_warp(const PairSet &ps, const ResultSet &rs, const Scorin
   return cudaGetLastError();
 }
 
-bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b) {
-  return n <= kShortPairs && n * (int64_t)max_b <= kShortColumns && sc.gap_open >= sc.gap_extend && max_a <= kShortRowsMax && max_b <= kShortColsMax && keyed_scoring(sc) &&
-         !may_need_int32(sc, ceiling, max_a, max_b);
+// What the one-launch path loses on is its 32 lanes of at least four rows each (128 rows) and a sweep
+// of every column by one warp.  Whole calls, resident, one launch / general path:
+//   A 50-64:  2,000 pairs x 1,700 columns 189 / 208 us, 3,000 x 1,000 154 / 176, 2,500 316 / 291,
+//             4,000 x 1,000 196 / 179, 1,700 295 / 230, 8,000 x 300 163 / 153, 1,000 348 / 239
+//             (score2: 2,000 x 1,700 218 / 202, 8,000 x 1,000 417 / 255);
+//   A 130-160: 6,500 x 1,000 382 / 362, 8,000 x 1,700 708 / 598 (score2 832 / 663);
+//   A 400-512: 8,000 x 1,700 2,007 / 2,110, 3,000 x 4,600 1,696 / 2,636.
+bool short_batch(const Scoring &sc, int ceiling, int64_t n, int max_a, int max_b, bool score2) {
+  const int64_t columns = n * (int64_t)max_b;
+  if (n > kShortPairs || columns > kShortColumns || max_a > kShortRowsMax || max_b > kShortColsMax) return false;
+  if (max_a <= kShortNarrow && n > (score2 ? kNarrowPairsS2 : kNarrowPairs) && columns > kNarrowColumns) return false;
+  if (max_a <= 256 && n > kMidPairs && columns > kMidColumns) return false;
+  return sc.gap_open >= sc.gap_extend && keyed_scoring(sc) && !may_need_int32(sc, ceiling, max_a, max_b);
 }
 
 static cudaError_t launch(ShortArgs g, cudaStream_t st) {
