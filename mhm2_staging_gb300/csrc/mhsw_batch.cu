@@ -41,7 +41,7 @@ __device__ __forceinline__ unsigned group_mask_b(int G) {
 template <int G, bool S2, int MODE>
 __global__ void __launch_bounds__(MODE != kModeInt && !S2 ? (G == kGKLong ? 768 : 640): 256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
                                                      const uint32_t *__restrict__ order, int *queue, int lane_rows,
-                                                     bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap,
+                                                     int min_rows, bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap,
                                                      V16::Pay *scratch, int scratch_stride) {
   constexpr bool kShort = (G == kGKShort);
   extern __shared__ __align__(16) unsigned char smem[];
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(MODE != kModeInt && !S2 ? (G == kGKLong ? 768 
     if (item >= hi) break;
     const int64_t p = order[item];
     const int M = ps.a_len[p], N = ps.b_len[p];
-    const int bucket = (M <= 0 || N <= 0) ? 0 : bucket_of(M, N, sc, lane_rows, wide_try16);
+    const int bucket = (M <= 0 || N <= 0) ? 0 : bucket_of(M, N, sc, lane_rows, wide_try16, min_rows);
     if (bucket == kBucketWide) {
       if (lane == 0) {
         rs.flag[p] = kFlagOverflow16;
@@ -264,7 +264,7 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   // order of m items (pair i * stride); clears the claim counters
   auto order_items = [&](const BatchShape &sh, int64_t m, int64_t stride, uint32_t *order) -> int {
     if ((e = order_pairs(ps, sc, sh.lane_rows, sh.wide_try16, m, stride, bs.ctl, order, sms, st, launches, INT_MAX,
-                         INT_MAX, long_rows)))
+                         INT_MAX, long_rows, sh.min_rows)))
       return fail(e, "order launch");
     return 0;
   };
@@ -318,11 +318,11 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     const bool fan = any_long && any_short && fk && fk->fork;
     if (fan && (e2 = fork_to(*fk, st, 1))) return fail(e2, "fork");
     if (any_long)
-      klong<<<grid_l, threads, smem_l, fan ? fk->side[0] : st>>>(ps, rs, sc, order, queue, sh.lane_rows, sh.wide_try16,
-                                                                 ceiling, wl, pad, bcap, scr, stride);
+      klong<<<grid_l, threads, smem_l, fan ? fk->side[0] : st>>>(ps, rs, sc, order, queue, sh.lane_rows, sh.min_rows,
+                                                                 sh.wide_try16, ceiling, wl, pad, bcap, scr, stride);
     if (any_short)
-      kshort<<<grid_s, threads, smem_s, st>>>(ps, rs, sc, order, queue, sh.lane_rows, sh.wide_try16, ceiling, wl, pad,
-                                               bcap, nullptr, stride);
+      kshort<<<grid_s, threads, smem_s, st>>>(ps, rs, sc, order, queue, sh.lane_rows, sh.min_rows, sh.wide_try16, ceiling,
+                                               wl, pad, bcap, nullptr, stride);
     e2 = cudaGetLastError();
     if (e2) return fail(e2, "persistent forward launch");
     if (fan && (e2 = join_from(*fk, st, 1))) return fail(e2, "join");
@@ -425,12 +425,22 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     if ((e = cudaMemsetAsync(wl.failed, 0, sizeof(int), st))) return fail(e, "memset");
   }
 
-  // the batch: ordered with the kept configuration, then the persistent launches.  A plain
-  // batch that does not give every 16-lane group a pair takes those for short reads too:
-  // their shorter chain is what it waits for.
+  // the batch: ordered with the kept configuration, then the persistent launches.
   BatchShape shape = tune ? bs.shape : BatchShape{};
+  // A plain batch that leaves lane groups without a pair waits for the slowest warp's chain.  Its pairs
+  // all take the longest one's bucket (up to 256 rows): a warp whose groups are of two buckets runs
+  // their sweeps one after the other (2,000 pairs of 100-250 rows x 8,200-9,000 columns 1.79 -> 1.25 ms).
+  // 16-lane groups have the shorter chain, 8-lane ones halve the warps: the lines are where the warps
+  // come to two, and six, a scheduler.  Same columns, 8 / 16 lanes: 50-64 rows, 30 pairs 622 / 742 us,
+  // 9,000 1,266 / 3,000; 100-128, 1,000 954 / 805, 1,500 958 / 996; 150-160, 3,600 1,469 / 1,312, 4,500
+  // 1,488 / 1,703.  Beyond the outer lines the buckets' own sizes pay (7,500 of 100-250 3.29 ms).
   // (A batch of empty A only has no longer kernel to go to: any_long is max_a > lane_rows.)
-  if (!tune && max_a > 0 && n <= (int64_t)sms * 64) shape.lane_rows = 0;
+  if (!tune && max_a > 0 && n <= (int64_t)sms * (max_a <= 192 ? 64 : 40)) {
+    shape.min_rows = std::min(max_a, 256);
+    const bool eight =
+        max_a <= 64 || (max_a <= 128 && n > (int64_t)sms * 8) || (max_a <= 160 && n > (int64_t)sms * 24);
+    if (!eight) shape.lane_rows = 0;
+  }
   if (order_items(shape, n, 1, bs.order)) return 1;
   // The long pairs' kernel runs beside the others: 3,000 pairs of 900-1,280 rows, a third of them
   // below 1,024, take 1.58 ms, one kernel after the other 2.46.  It is launched after them: in front

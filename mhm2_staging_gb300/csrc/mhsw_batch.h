@@ -16,6 +16,7 @@ struct BatchShape {
   int groups_per_block = 16;  // block size in units of 8 threads
   int blocks_per_sm = 0;      // 0 = occupancy maximum
   int lane_rows = 160;        // longest A (rows) given to 8-lane groups; longer A runs in 16-lane groups
+  int min_rows = 0;           // shorter A share the bucket of this many rows
   bool wide_try16 = false;    // pairs whose score bound exceeds the int16 keys: int16 first (re-run on
                               // overflow) instead of straight to int32
 };

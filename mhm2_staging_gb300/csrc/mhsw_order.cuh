@@ -30,10 +30,12 @@ __host__ __device__ constexpr int bucket_k(int b) {
   return b == 0 ? 4 : b == 1 ? 6 : b == 2 ? 8 : b == 3 ? 10 : b == 4 ? 6 : 8;
 }
 
+// min_rows: A of fewer rows go to the bucket of that many (BatchShape).
 __device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int lane_rows, bool wide_try16,
-                                         int long_rows = INT_MAX) {
-  const int b = M <= lane_rows ? (M <= 64 ? 0 : M <= 96 ? 1 : M <= 128 ? 2 : 3)
-                               : (M <= 192 ? 4 : M <= 256 ? 5 : kBucketStrip);
+                                         int min_rows = 0, int long_rows = INT_MAX) {
+  const int R = M > min_rows ? M : min_rows;
+  const int b = R <= lane_rows ? (R <= 64 ? 0 : R <= 96 ? 1 : R <= 128 ? 2 : 3)
+                               : (R <= 192 ? 4 : R <= 256 ? 5 : kBucketStrip);
   // wide_try16: the int16 engine's ceiling test sends the pairs that do overflow to int32.
   // That test sees a score cross the keys' capacity only if the first cell above it still
   // fits a 16-bit key: the capacity leaves 64 values of margin and H grows by at most match
@@ -88,13 +90,14 @@ struct OrderArgs {
   uint32_t *order;
   int max_a, max_b;   // pairs longer than these go with the empty ones
   int long_rows;      // longest A of the persistent kernels
+  int min_rows;       // bucket_of's
   int protein_wide;   // above 0: buckets by protein_bucket with this wide_from (sc unused)
 };
 
 __device__ __forceinline__ int order_bin(const OrderArgs &g, int64_t p) {
   const int M = g.ps.a_len[p], N = g.ps.b_len[p];
   const int b = (M <= 0 || N <= 0 || M > g.max_a || N > g.max_b) ? (g.lane_rows > 0 ? 0 : kBucketFirstLong)
-                : g.protein_wide > 0 ? protein_bucket(M, N, g.protein_wide) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.long_rows);
+                : g.protein_wide > 0 ? protein_bucket(M, N, g.protein_wide) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.min_rows, g.long_rows);
   return b * kLenBins + len_class(N);
 }
 
@@ -262,9 +265,10 @@ inline cudaError_t order_smem_limits() {
 // Orders m items (pair i * stride) into `order`; clears the claim counters.
 inline cudaError_t order_pairs(const PairSet &ps, const Scoring &sc, int lane_rows, bool wide_try16, int64_t m,
                                int64_t stride, int *ctl, uint32_t *order, int sms, cudaStream_t st, int64_t *launches,
-                               int max_a = INT_MAX, int max_b = INT_MAX, int long_rows = INT_MAX, int protein_wide = 0) {
+                               int max_a = INT_MAX, int max_b = INT_MAX, int long_rows = INT_MAX, int min_rows = 0,
+                               int protein_wide = 0) {
   OrderArgs g{ps, sc, lane_rows, wide_try16, m, stride, ctl, ctl + 8, ctl + kOrderHead, ctl + kOrderHead + kOrderBins,
-              order, max_a, max_b, long_rows, protein_wide};
+              order, max_a, max_b, long_rows, min_rows, protein_wide};
   cudaError_t e = order_smem_limits();
   if (e) return e;
   if (m <= kOrderOneBlock) {

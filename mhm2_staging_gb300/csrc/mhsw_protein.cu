@@ -725,7 +725,8 @@ int mhsw_align_protein(mhsw_driver *d, const mhsw_pairs *pairs, const int16_t *s
     ps.a_len = al;
     ps.b_len = bl;
     ps.n = n;
-    e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, INT_MAX, wide_from);
+    e = order_pairs(ps, Scoring{}, 1, false, n, 1, ctl, order, sms, st, nullptr, INT_MAX, INT_MAX, INT_MAX, 0,
+                    wide_from);
     g.list = order;
     g.list_first = ctl + 8 + kBucketWide;
   }
