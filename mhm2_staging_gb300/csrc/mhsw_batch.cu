@@ -230,10 +230,31 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     return 1;
   }
   const bool s2 = ps.rowmax16 != nullptr;
+  BatchShape plain;  // the plain form's configuration
+  // A plain batch that leaves lane groups without a pair waits for the slowest warp's chain.  Its pairs
+  // all take the longest one's bucket (up to 256 rows): a warp whose groups are of two buckets runs
+  // their sweeps one after the other (2,000 pairs of 100-250 rows x 8,200-9,000 columns 1.79 -> 1.25 ms).
+  // 16-lane groups have the shorter chain, 8-lane ones halve the warps: the lines are where the warps
+  // come to two, and six, a scheduler.  Same columns, 8 / 16 lanes: 50-64 rows, 30 pairs 622 / 742 us,
+  // 9,000 1,266 / 3,000; 100-128, 1,000 954 / 805, 1,500 958 / 996; 150-160, 3,600 1,469 / 1,312, 4,500
+  // 1,488 / 1,703.  Beyond the outer lines the buckets' own sizes pay (7,500 of 100-250 3.29 ms).
+  // (A batch of empty A only has no longer kernel to go to: any_long is max_a > lane_rows.)
+  if (!tune && max_a > 0 && n <= (int64_t)sms * (max_a <= 192 ? 64 : 40)) {
+    plain.min_rows = std::min(max_a, 256);
+    const bool eight =
+        max_a <= 64 || (max_a <= 128 && n > (int64_t)sms * 8) || (max_a <= 160 && n > (int64_t)sms * 24);
+    if (!eight) plain.lane_rows = 0;
+  }
   // The engine's mode by the largest score of each kernel's pairs (8-lane groups take at most
   // 160 rows).
-  const int mode_s = mode_for((long long)std::min({max_a, max_b, 160}) * sc.match, 10);
-  const int mode_l = mode_for((long long)std::min(max_a, max_b) * sc.match, 8);
+  // One bucket on up to about a warp a scheduler: integers have the shorter chain.  Calls, half or
+  // step keys / integers: 30 pairs of 600-1,000 rows squared 2.11 / 2.00 ms, 1,000 of 200-256 x
+  // 8,200-9,000 1.01 / 0.98; 2,000 of the latter 1.25 / 1.29.  On 8 lanes only six row pairs a lane gain
+  // (2,000 of 50-96 832 / 805 us; 50-64 650 / 659, 100-128 960 / 959).
+  const bool few_l = plain.min_rows > 0 && plain.lane_rows == 0 && n <= (int64_t)sms * (max_a > 256 ? 13 : 8);
+  const bool few_s = plain.min_rows > 64 && plain.min_rows <= 96 && n <= (int64_t)sms * 16;
+  const int mode_s = few_s ? kModeInt : mode_for((long long)std::min({max_a, max_b, 160}) * sc.match, 10);
+  const int mode_l = few_l ? kModeInt : mode_for((long long)std::min(max_a, max_b) * sc.match, 8);
   using Kern = decltype(&k_fwd_persist<kGKShort, false, kModeInt>);
   auto pick = [&](int mode, Kern i, Kern h, Kern t, Kern i2, Kern h2, Kern t2) -> Kern {
     return mode == kModeStep ? (s2 ? t2 : t) : mode == kModeHalf ? (s2 ? h2 : h) : (s2 ? i2 : i);
@@ -426,21 +447,7 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
   }
 
   // the batch: ordered with the kept configuration, then the persistent launches.
-  BatchShape shape = tune ? bs.shape : BatchShape{};
-  // A plain batch that leaves lane groups without a pair waits for the slowest warp's chain.  Its pairs
-  // all take the longest one's bucket (up to 256 rows): a warp whose groups are of two buckets runs
-  // their sweeps one after the other (2,000 pairs of 100-250 rows x 8,200-9,000 columns 1.79 -> 1.25 ms).
-  // 16-lane groups have the shorter chain, 8-lane ones halve the warps: the lines are where the warps
-  // come to two, and six, a scheduler.  Same columns, 8 / 16 lanes: 50-64 rows, 30 pairs 622 / 742 us,
-  // 9,000 1,266 / 3,000; 100-128, 1,000 954 / 805, 1,500 958 / 996; 150-160, 3,600 1,469 / 1,312, 4,500
-  // 1,488 / 1,703.  Beyond the outer lines the buckets' own sizes pay (7,500 of 100-250 3.29 ms).
-  // (A batch of empty A only has no longer kernel to go to: any_long is max_a > lane_rows.)
-  if (!tune && max_a > 0 && n <= (int64_t)sms * (max_a <= 192 ? 64 : 40)) {
-    shape.min_rows = std::min(max_a, 256);
-    const bool eight =
-        max_a <= 64 || (max_a <= 128 && n > (int64_t)sms * 8) || (max_a <= 160 && n > (int64_t)sms * 24);
-    if (!eight) shape.lane_rows = 0;
-  }
+  const BatchShape shape = tune ? bs.shape : plain;
   if (order_items(shape, n, 1, bs.order)) return 1;
   // The long pairs' kernel runs beside the others: 3,000 pairs of 900-1,280 rows, a third of them
   // below 1,024, take 1.58 ms, one kernel after the other 2.46.  It is launched after them: in front
