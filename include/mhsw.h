@@ -57,8 +57,8 @@ extern "C" {
 /* ---- forms ----------------------------------------------------------------- */
 /* Both forms give the same results.  They order the pairs by length on the device and run
  * persistent kernels whose lane groups claim pairs from a queue; the batched form also tunes
- * their configuration to the batch (mhsw_tuning).  Batches of a few thousand pairs take one
- * launch for both passes in either form. */
+ * their configuration to the batch (mhsw_tuning).  Batches of a few thousand pairs (at most
+ * 8,192; fewer for A up to 256 rows) take one launch for both passes in either form. */
 #define MHSW_FORM_PLAIN 0    /* default configuration */
 #define MHSW_FORM_BATCHED 1  /* configuration picked by timed trials */
 
@@ -93,7 +93,8 @@ typedef struct {
   int64_t launches;      /* kernels launched by the call (a graph replay counts its kernels) */
   int64_t graph_replays; /* CUDA graph launches by this handle so far: a device-resident batch
                           * aligned again with the same pointers, sizes and settings is
-                          * captured on its second call and replayed from then on */
+                          * captured on its second call and replayed from then on (captured
+                          * again after a call that made the handle's device buffers grow) */
   double cigar_ms;          /* CIGAR mode: the CIGAR pass (device kernels plus the host-driven
                              * rounds for wide bands), 0 otherwise */
   int64_t n_cigar_generic;  /* CIGAR mode: pairs whose band or box exceeded the register

@@ -39,10 +39,10 @@ __device__ __forceinline__ unsigned group_mask_b(int G) {
 // 12.51 -> 12.23 ms and 30,011 pairs against 2-8 kb 6.55 -> 6.47 against 96 and 128; the score2
 // kernels, which keep a row maximum per row pair, lose or spill there.
 template <int G, bool S2, int MODE>
-__global__ void __launch_bounds__(MODE != kModeInt && !S2 ? (G == kGKLong ? 768 : 640): 256) k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc,
-                                                     const uint32_t *__restrict__ order, int *queue, int lane_rows,
-                                                     int min_rows, bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap,
-                                                     V16::Pay *scratch, int scratch_stride) {
+__global__ void __launch_bounds__(MODE != kModeInt && !S2 ? (G == kGKLong ? 768 : 640) : 256)
+    k_fwd_persist(PairSet ps, ResultSet rs, Scoring sc, const uint32_t *__restrict__ order, int *queue, int lane_rows,
+                  int min_rows, bool wide_try16, int ceiling, WorkLists wl, int pad, int bcap, V16::Pay *scratch,
+                  int scratch_stride) {
   constexpr bool kShort = (G == kGKShort);
   extern __shared__ __align__(16) unsigned char smem[];
   const int gpb = blockDim.x / G;
@@ -246,8 +246,7 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     if (!eight) plain.lane_rows = 0;
   }
   // The engine's mode by the largest score of each kernel's pairs (8-lane groups take at most
-  // 160 rows).
-  // One bucket on up to about a warp a scheduler: integers have the shorter chain.  Calls, half or
+  // 160 rows).  One bucket on up to about a warp a scheduler: integers have the shorter chain.  Calls, half or
   // step keys / integers: 30 pairs of 600-1,000 rows squared 2.11 / 2.00 ms, 1,000 of 200-256 x
   // 8,200-9,000 1.01 / 0.98; 2,000 of the latter 1.25 / 1.29.  On 8 lanes only six row pairs a lane gain
   // (2,000 of 50-96 832 / 805 us; 50-64 650 / 659, 100-128 960 / 959).
@@ -270,10 +269,12 @@ int batched_forward(BatchState &bs, int device, const PairSet &ps, const ResultS
     return h ? (s2 ? half_s2 : half_w) : (s2 ? full_s2 : full);
   };
   constexpr int kZ = kCode16Zero + 1, kN = kCodeN + 1;
-  const size_t prof_short = prof_of(mode_s != kModeInt, group_prof16_bytes<10, kGKShort, kN>(), group_prof16_bytes<10, kGKShort, kZ>(),
-                                    group_prof16_bytes<10, kGKShort, kN, true>(), group_prof16_bytes<10, kGKShort, kZ, true>());
-  const size_t prof_long = prof_of(mode_l != kModeInt, group_prof16_bytes<8, kGKLong, kN>(), group_prof16_bytes<8, kGKLong, kZ>(),
-                                   group_prof16_bytes<8, kGKLong, kN, true>(), group_prof16_bytes<8, kGKLong, kZ, true>());
+  const size_t prof_short =
+      prof_of(mode_s != kModeInt, group_prof16_bytes<10, kGKShort, kN>(), group_prof16_bytes<10, kGKShort, kZ>(),
+              group_prof16_bytes<10, kGKShort, kN, true>(), group_prof16_bytes<10, kGKShort, kZ, true>());
+  const size_t prof_long =
+      prof_of(mode_l != kModeInt, group_prof16_bytes<8, kGKLong, kN>(), group_prof16_bytes<8, kGKLong, kZ>(),
+              group_prof16_bytes<8, kGKLong, kN, true>(), group_prof16_bytes<8, kGKLong, kZ, true>());
   // long pairs take blocks of their own (not in score2 mode, which needs their row maxima, nor
   // under a lowered int16 ceiling, which asks for the int32 pass)
   const bool longs = max_a > kLongRows && !s2 && wl.long_bnd && ceiling >= kCeiling16;

@@ -1275,8 +1275,8 @@ cudaError_t launch_lanes(const CigarArgs &g, int sms, int64_t most, int max_a, i
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(k_cigar_lanes<LG>), smem);
   if (e) return e;
   const int64_t need = (most + kLaneWarps * (32 / LG) - 1) / (kLaneWarps * (32 / LG));
-  k_cigar_lanes<LG><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * 8)), kLaneWarps * 32, smem, st>>>(
-      g, c_lo, c_hi, from_list, row_cap);
+  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * 8));
+  k_cigar_lanes<LG><<<(unsigned)grid, kLaneWarps * 32, smem, st>>>(g, c_lo, c_hi, from_list, row_cap);
   return cudaGetLastError();
 }
 

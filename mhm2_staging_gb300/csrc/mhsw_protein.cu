@@ -313,11 +313,14 @@ __device__ __forceinline__ unsigned long long protein_rows(const uint8_t *a, int
                                                            int N, const uint32_t *rowtab, uint4 *tab, int lane,
                                                            unsigned gmask, uint32_t *bnd, uint32_t NGE, uint32_t NGO,
                                                            uint32_t one, int &over) {
-  if (M <= 8 * G) return protein_sweep<4, G, false>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
-  if (M <= 12 * G) return protein_sweep<6, G, false>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
-  if (G == 16 || M <= 16 * G)
-    return protein_sweep<8, G, false>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
-  return protein_sweep<8, G, true>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask, bnd, NGE, NGO, one, over);
+  auto sweep = [&](auto k, auto multi) {
+    return protein_sweep<decltype(k)::value, G, decltype(multi)::value>(a, adir, M, b, bdir, N, rowtab, tab, lane, gmask,
+                                                                        bnd, NGE, NGO, one, over);
+  };
+  if (M <= 8 * G) return sweep(std::integral_constant<int, 4>{}, std::false_type{});
+  if (M <= 12 * G) return sweep(std::integral_constant<int, 6>{}, std::false_type{});
+  if (G == 16 || M <= 16 * G) return sweep(std::integral_constant<int, 8>{}, std::false_type{});
+  return sweep(std::integral_constant<int, 8>{}, std::true_type{});
 }
 
 // The sweep with keys above a base, for pairs whose score left the plain keys.  (Not inlined: beside

@@ -75,7 +75,8 @@ struct ShortStep {
   using Eng = Step16<kLay, 32, S2, STEP ? kModeStep : kModeInt>;
   static constexpr uint32_t kKeyMask = KeyBits<R>::kMask;
   static constexpr int kStepBits = STEP ? 3 : 0;
-  __device__ static __forceinline__ void load(const uint32_t *tab, int c, int lane, uint32_t (&lo)[kLay], uint32_t (&hi)[kLay]) {
+  __device__ static __forceinline__ void load(const uint32_t *tab, int c, int lane, uint32_t (&lo)[kLay],
+                                              uint32_t (&hi)[kLay]) {
     if constexpr (STEP) Eng::load_half(tab, c, lane, lo);
     else Eng::load(reinterpret_cast<const uint4 *>(tab), c, lane, lo, hi);
   }
@@ -113,7 +114,8 @@ struct ShortStep {
       } else {
         Hlast = Hn;
       }
-      key[k] = mad_u32(Hn, scale, ((uint32_t)(kKeyMask - k) * (STEP ? 8u : 1u) + (STEP ? 7u - (uint32_t)u : 0u)) * 0x00010001u);
+      const uint32_t tag = (uint32_t)(kKeyMask - k) * (STEP ? 8u : 1u) + (STEP ? 7u - (uint32_t)u : 0u);
+      key[k] = mad_u32(Hn, scale, tag * 0x00010001u);
       if constexpr (S2) Rm[k] = __viaddmax_s16x2(Hn, vmask, Rm[k]);
     }
 #pragma unroll
@@ -163,7 +165,8 @@ __device__ __forceinline__ unsigned long long sweep_warp(int M, int N, RowCode r
       base[w] = (alo[w] == kCodePad ? 0u : alo[w] == kCodeN ? vn : miss) |
                 (ahi[w] == kCodePad ? 0u : ahi[w] == kCodeN ? vn : miss) << 16;
       ST::put(prof, kCodeN, w, lane, both(w, vn));
-      if constexpr (S2) ST::put(prof, kCode16Zero, w, lane, both(w, (uint32_t)sc.gap_open));  // scores 0 against real rows
+      // (scores 0 against real rows)
+      if constexpr (S2) ST::put(prof, kCode16Zero, w, lane, both(w, (uint32_t)sc.gap_open));
     }
 #pragma unroll
     for (int c = 0; c < kCodeN; c++)
@@ -196,8 +199,8 @@ __device__ __forceinline__ unsigned long long sweep_warp(int M, int N, RowCode r
         const int jl = t + u - 2 * lane;
         vmask = ((unsigned)jl < (unsigned)N ? 0u : 0x0000C000u) | ((unsigned)(jl - 1) < (unsigned)N ? 0u : 0xC0000000u);
       }
-      ST::run(t + u, u, zH, zE, sel, lo, STEP ? lo : hi, P, F, Hlast, Ecout, STEP ? Kb : Kl, Jp, NGE, NGO, NGOh, one, scale,
-              Rm, vmask);
+      ST::run(t + u, u, zH, zE, sel, lo, STEP ? lo : hi, P, F, Hlast, Ecout, STEP ? Kb : Kl, Jp, NGE, NGO, NGOh, one,
+              scale, Rm, vmask);
 #pragma unroll
       for (int k = 0; k < K; k++) {
         lo[k] = nlo[k];
@@ -471,8 +474,11 @@ static cudaError_t launch(ShortArgs g, cudaStream_t st) {
                     : (small ? warp_prof<4, false>(step) : warp_prof<8, false>(step));
   const size_t smem =
       ((size_t)g.prof_bytes + (s2 ? (small ? 512 : 1024) + 16 : 0) + 2 * kShortPad + (size_t)g.max_b + 15) / 16 * 16;
-  auto kern = s2 ? (small ? k_short<4, true, false> : k_short<8, true, false>) : (small ? k_short<4, false, false> : k_short<8, false, false>);
-  if (step) kern = s2 ? (small ? k_short<4, true, true> : k_short<8, true, true>) : (small ? k_short<4, false, true> : k_short<8, false, true>);
+  auto kern = s2 ? (small ? k_short<4, true, false> : k_short<8, true, false>)
+                 : (small ? k_short<4, false, false> : k_short<8, false, false>);
+  if (step)
+    kern = s2 ? (small ? k_short<4, true, true> : k_short<8, true, true>)
+              : (small ? k_short<4, false, true> : k_short<8, false, true>);
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
   if (e != cudaSuccess) return e;
   kern<<<(unsigned)g.ps.n, 32, smem, st>>>(g);
